@@ -14,11 +14,11 @@
 //   - singleton SCCs only: z_v = b_v / q_v;
 //   - otherwise BiCGStab on the odd-parity Schur complement.  Every edge flips one bit, so
 //     the graph is bipartite by popcount parity and the even rows are eliminated exactly.
-//     The right preconditioner is the Schur diagonal, and inner iterations run in FP64
-//     (ESL_METHOD_DIRECT) or FP32 (ESL_METHOD_MIXED) inside FP64 iterative refinement on
-//     the true residual.  Groups whose SCCs all have at most kSwLocalMax states run the
-//     whole refinement inside one CTA per (SCC, 32 systems) (k_sw_local: block
-//     reductions, no grid-wide step); larger groups run one grid-wide kernel per step.
+//     The right preconditioner is the Schur diagonal.  Groups whose SCCs have at most
+//     kSccMaxRows rows of either parity run in one launch, a CTA per (SCC, few systems)
+//     with its vectors on chip and in FP64 throughout (k_sw_scc); larger groups run one
+//     grid-wide kernel per step, their inner iterations in FP64 (ESL_METHOD_DIRECT) or
+//     FP32 (ESL_METHOD_MIXED) inside FP64 iterative refinement on the true residual.
 //
 // Layout: every vector is [row][system], the Kp (K rounded up to 32) systems of a row
 // contiguous.  A warp handles 32 systems of one state, so every neighbour gather reads a
@@ -47,8 +47,7 @@ namespace esl {
 namespace {
 
 constexpr int kSwT = 256;            // threads per row kernel
-constexpr int kSwLocalMax = 512;     // largest SCC of a group solved CTA-locally
-constexpr int kSwLocalWarps = 16;    // most warps of a CTA-local solve
+constexpr int kSwLocalMax = 512;     // largest SCC of a kind-1 group
 constexpr int kSwPoll = 4;           // Krylov iterations launched between convergence polls
 // Poll windows in flight: the host reads the running count of window c - (depth - 1)
 // after queueing window c, so a late host leaves the GPU idle only after it has fallen
@@ -81,11 +80,14 @@ enum IScal { I_FLAGS, I_ITERS, I_NOIMP, I_TOTAL, I_STALL, I_NISCAL };
 
 struct SwGroup {
     uint32_t beg, ne, no;  // first slot, even rows, odd rows
-    int kind;              // 0 singletons, 1 CTA-local Krylov, 2 grid-wide Krylov
+    int kind;              // 0 singletons, 1 SCCs of at most kSwLocalMax states, 2 larger ones
     int max_scc;
     uint32_t scc0, nscc;   // local groups: range in the local SCC list (SCCs of >= 2 states)
     int max_odd;           // local groups: most odd rows of one SCC
     uint64_t nin;          // in-group predecessor entries of the group's rows
+    uint32_t s0, ns;       // the group's SCCs of >= 2 states: range in SweepPlan::scc
+    bool resident;         // every one of them fits k_sw_scc
+    uint32_t singles;      // rows that are SCCs of their own
     int term;              // terminal plan: the terminal SCC of the group (-1 otherwise)
     uint32_t pos0;         // terminal plan: position of the SCC's first state in the order
 };
@@ -100,9 +102,10 @@ struct SweepPlan {
     DevBuf<uint32_t> og_ptr, og_ent;     // predecessors in earlier groups
     DevBuf<uint32_t> tp_ptr, tp_ent;     // transient predecessors of terminal position p
     DevBuf<uint32_t> lsc_off;            // local SCCs: offsets into lsc_slots
-    // local SCCs: per CTA-local group, its SCCs' group-relative indices by decreasing
-    // size (the launch order of k_sw_local), or empty
-    DevBuf<uint32_t> lsc_rank;
+    // SCCs of >= 2 states, group by group, largest first: (first even slot, even rows,
+    // first odd slot, odd rows); an SCC's even and odd slots are one run each
+    DevBuf<uint4> scc;
+    std::vector<uint4> h_scc;
     DevBuf<uint32_t> lsc_ne;             // local SCCs: number of even-parity slots (listed first)
     DevBuf<uint32_t> lsc_slots;          // local SCCs: slots, SCC by SCC
     // terminal plan: per slot, the state's position in the reordering
@@ -1246,327 +1249,499 @@ __global__ void __launch_bounds__(kSwT) k_sw_warm_scale(SwArgs a, const double* 
         X64[(size_t)r * a.Kp + t.k] *= alpha;
 }
 
-// ---- CTA-local refinement for groups of small SCCs ----------------------------------------
-// One CTA per (SCC of >= 2 states, 32 systems): lane = system, warp w takes rows w, w + nw, ...
-// Every warp holds all 32 lanes, so the block-wide sums below give every warp the same
-// per-lane scalars and every decision (convergence, stagnation) is uniform across warps
-// without another barrier.  Vectors are the group's [row][Kp] buffers; a CTA touches only
-// the rows of its SCC, because SCCs of one level share no edge.
-struct SwLocal {
-    const uint32_t* off;     // SCC j: slots[off[j] .. off[j+1]), even-parity slots first
-    const uint32_t* ne;      // SCC j: number of even-parity slots
-    const uint32_t* slots;
-    const double* bS;        // reduced rhs (odd rows of the group)
-    const double* dS64;      // Schur diagonal (odd rows)
-    const float* dS32;       // its FP32 copy (mixed method)
-    double* X64;             // odd-row solution, refined in place
-    double* R64;             // odd rows: FP64 true residual
-    double* W64;             // even rows: FP64 elimination, also the FP64 inner solve's even buffer
-    double *R, *R0, *PH, *V, *SH, *TT, *D;  // odd rows, FP64 inner solve
-    // FP32 inner solve: buffers of its own, because CTAs of one launch may be in FP32 and
-    // FP64 steps at the same time
-    float *fR, *fR0, *fPH, *fV, *fSH, *fTT, *fD;  // odd rows
-    float* fW;                                    // even rows
+// ---- SCC-resident refinement --------------------------------------------------------------
+// One CTA solves one SCC for KS systems (a power of two chosen per SCC) from right-hand
+// side to result: the two vectors the operator gathers (the search direction and its
+// even-row elimination) stay in shared memory, a thread's own rows in registers, and the
+// CTA stops with its own systems.  A Krylov iteration is bounded by its chain of barriers
+// and shared-memory gathers instead of L2 latency and launches.  Against the launch per
+// step (SCCs above 512 states) and the CTA-local solve on global vectors that it replaces:
+// n=12 x 64 rate sets 14.7 -> 2.8 ms, n=17 x 185 systems 64.6 -> 24.0 ms, one n=22 solve
+// 277 -> 71 ms.
+//
+// A work item is (SCC, tile of KS systems); the SCCs of a launch are listed largest first
+// and cut into buckets of equal KS.  CTAs past the last item serve the group's singleton
+// SCCs (rows without in-group predecessors): z = b / q.
+constexpr int kSccMaxRows = 4096;  // most odd (or even) rows of an SCC solved by one CTA
+// threads of a CTA with one row per thread, and with several (whose registers hold more)
+constexpr int kSccThreads1 = 1024, kSccThreads = 512;
+__host__ __device__ constexpr int scc_threads(int NR) { return NR > 1 ? kSccThreads : kSccThreads1; }
+constexpr int kSccBuckets = 6;     // KS = 1, 2, 4, ..., 32
+constexpr size_t kSccMaxSmem = 227 * 1024;
+
+struct SccBucket {
+    uint32_t item0, scc0;  // first work item, first SCC (relative to SccArgs::scc)
+    int lks;               // log2 KS
+};
+
+struct SccArgs {
+    SwArgs a;
+    const uint4* scc;  // the launch's SCCs: (first even slot, even rows, first odd slot, odd rows)
+    SccBucket b[kSccBuckets];
+    int nb;
+    uint32_t items;    // CTAs before those of the singleton rows
+    const uint32_t *og_ptr, *og_ent;
+    const double* x0;
+    size_t x0_ld;
+    const double* warm;  // K x N warm start by state, or null
+    size_t warm_ld;
+    double* Z;           // [slot][Kp]
+    double* BS;          // reduced right-hand sides, [odd row of the group][Kp]
     double tol2, accept2;
-    int max_iters, max_refine, mixed;
+    int max_iters, max_outer, stall;
     unsigned long long* ratio;  // per system: max over SCCs of final |r|^2 / |b|^2 (bits of a double >= 0)
     int* fail;                  // per system: 1 once an SCC stays above the acceptance residual
-    int* iters;                 // per system: inner iterations, max over SCCs
-    // the SCC at place p of the launch order is the group's SCC rank[p] (largest first),
-    // or SCC p when null
-    const uint32_t* rank;
+    int* iters;                 // the group's most inner iterations
+    // deflated (terminal) groups: kernels into Rb[k][pos[slot]], normalised to sum 1
+    const uint32_t* pos;
+    double* Rb;
+    int TS;
 };
 
-struct LocalRows {
-    const uint32_t* ev;  // even slots of the SCC
-    const uint32_t* od;  // odd slots
-    int se, so, warp, nw;
-    uint32_t obase;      // first odd slot of the group
+__device__ __forceinline__ void scc_sync(int nact) { asm volatile("bar.sync 1, %0;" ::"r"(nact) : "memory"); }
+
+// sum over a row's entries of rate(entry) * X[entry row][system s], X and the rates in
+// shared memory as [row << lks | s]
+__device__ __forceinline__ double scc_gather(const uint32_t* __restrict__ ent, int cnt, const double* X,
+                                             const double* rate, int lks, int s, uint32_t base) {
+    double acc = 0.0;
+    int j = 0;
+    for (; j + 4 <= cnt; j += 4) {
+        uint32_t e[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) e[u] = __ldg(ent + j + u);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            acc += rate[(ent_rate(e[u]) << lks) | s] * X[((ent_slot(e[u]) - base) << lks) | s];
+    }
+    for (; j < cnt; j++) {
+        const uint32_t e = __ldg(ent + j);
+        acc += rate[(ent_rate(e) << lks) | s] * X[((ent_slot(e) - base) << lks) | s];
+    }
+    return acc;
+}
+
+// Sums of NV values over the CTA's threads of one system; every thread of a system gets
+// the same bits.  `red` holds NV x warps x KS doubles; calls without a barrier in between
+// must use different buffers.
+template <int NV>
+__device__ __forceinline__ void scc_sum(double* red, int lks, int s, int nact, double (&v)[NV]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nact >> 5, KS = 1 << lks;
+#pragma unroll
+    for (int j = 0; j < NV; j++)
+        for (int o = 16; o >= KS; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+    if (lane < KS)
+#pragma unroll
+        for (int j = 0; j < NV; j++) red[((j * nw + warp) << lks) | lane] = v[j];
+    scc_sync(nact);
+#pragma unroll
+    for (int j = 0; j < NV; j++) {
+        double acc = 0.0;
+        for (int w = 0; w < nw; w++) acc += red[((j * nw + w) << lks) | s];
+        v[j] = acc;
+    }
+}
+
+// out-rate sum of state v (out-mask f) for system s
+__device__ __forceinline__ double scc_q(const double* rate, uint32_t v, uint32_t f, int lks, int s) {
+    double q = 0.0;
+    while (f) {
+        const int i = __ffs(f) - 1;
+        f &= f - 1;
+        q += rate[((2 * i + (int)((v >> i) & 1u)) << lks) | s];
+    }
+    return q;
+}
+
+// Singleton rows of a group, z = (x0 + inflow from earlier groups) / q.  KW = min(32, K
+// rounded up to a power of two) adjacent lanes serve the systems of one row, so that
+// small batches fill the warp with rows.
+__device__ __forceinline__ void scc_singles(const SccArgs& g, uint32_t cta, uint32_t ctas) {
+    const SwArgs& a = g.a;
+    int lw = 0;
+    while (lw < 5 && (1 << lw) < a.K) lw++;
+    const int KW = 1 << lw;
+    const uint32_t rows = a.ne + a.no, tiles = (uint32_t)((a.K + KW - 1) >> lw), rpb = blockDim.x >> lw;
+    for (uint64_t u = (uint64_t)cta * rpb + (threadIdx.x >> lw); u < (uint64_t)rows * tiles; u += (uint64_t)ctas * rpb) {
+        const uint32_t t = (uint32_t)(u / rows), r = (uint32_t)(u - (uint64_t)t * rows);
+        const int k = (int)(t << lw) + (int)(threadIdx.x & (KW - 1));
+        if (k >= a.K) continue;
+        const uint32_t slot = a.beg + r;
+        const uint4 d = a.desc[slot];
+        if (d.w) continue;  // in an SCC of two or more states
+        double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + d.x];
+        const uint32_t p1 = g.og_ptr[slot + 1];
+        for (uint32_t p = g.og_ptr[slot]; p < p1; p++) {
+            const uint32_t e = __ldg(g.og_ent + p);
+            acc += __ldg(a.rateT + (size_t)ent_rate(e) * a.Kp + k) * g.Z[(size_t)ent_slot(e) * a.Kp + k];
+        }
+        double q = 0.0;
+        for (uint32_t f = d.y; f; f &= f - 1) {
+            const int i = __ffs(f) - 1;
+            q += __ldg(a.rateT + (size_t)(2 * i + (int)((d.x >> i) & 1u)) * a.Kp + k);
+        }
+        g.Z[(size_t)slot * a.Kp + k] = acc / q;
+    }
+}
+
+// A thread's own values of one vector (rows rs, rs + RS, ...): registers when a thread has
+// one row, else its own entries of a shared-memory array.
+template <int NR>
+struct SccVec {
+    double reg;
+    double* sm;
+    __device__ __forceinline__ double get(int idx) const { return NR > 1 ? sm[idx] : reg; }
+    __device__ __forceinline__ void set(int idx, double x) {
+        if (NR > 1) sm[idx] = x;
+        else reg = x;
+    }
 };
 
-// Sums of two per-lane values over the CTA's warps, double-buffered so that the next
-// call may write while slow warps still read the previous result.
-__device__ __forceinline__ void local_sum2(double* red, int& site, const LocalRows& L, int lane, double v0, double v1,
-                                           double& o0, double& o1) {
-    double* rb = red + (site & 1) * (2 * kSwLocalWarps * 32);
-    site++;
-    rb[L.warp * 32 + lane] = v0;
-    rb[kSwLocalWarps * 32 + L.warp * 32 + lane] = v1;
-    __syncthreads();
-    double s0 = 0.0, s1 = 0.0;
-    for (int w = 0; w < L.nw; w++) {
-        s0 += rb[w * 32 + lane];
-        s1 += rb[kSwLocalWarps * 32 + w * 32 + lane];
-    }
-    o0 = s0;
-    o1 = s1;
+// shared-memory doubles of an SCC's work item (see the carving in k_sw_scc)
+__host__ __device__ inline size_t scc_smem_doubles(int NR, int n, int se, int so, int lks, int nact) {
+    const size_t m = (size_t)(se > so ? se : so), KS = (size_t)1 << lks;
+    return (m + se + 2 * n + 6 * (size_t)(nact >> 5) + (NR > 1 ? 4 * (size_t)so + se : 0)) * KS;
 }
 
-// even rows: W_e = (sum over odd in-SCC predecessors o of rate(o -> e) X_o) / q_e
-template <class TC, class TX, class TW>
-__device__ __forceinline__ void local_elim(const SwArgs& a, const Tile& t, const TC* s, const LocalRows& L,
-                                           const TX* X, TW* W, bool act) {
-    for (int i = L.warp; i < L.se; i += L.nw) {
-        const uint32_t slot = L.ev[i];
-        const uint2 row = a.rows[slot];
-        const uint32_t p0 = a.ig_ptr[slot];
-        const TC acc = sw_gather<TC, TX>(s, t, a.Kp, a.ig_ent, p0, (int)(a.ig_ptr[slot + 1] - p0), X, L.obase,
-                                         act, (TC)0);
-        if (act) W[(size_t)(slot - a.beg) * a.Kp + t.k] = (TW)(acc / sw_q(s, row.x, row.y, t));
+// NR: most odd (or even) rows of a thread.  DEFL: the deflated operator of a terminal SCC
+// (see k_sw_defl_fin): S x + u gamma(x), u_o = q_o / s, whose gamma is summed at the
+// barrier that the elimination ends with anyway.
+template <int NR, bool DEFL>
+__global__ void __launch_bounds__(scc_threads(NR)) k_sw_scc(const __grid_constant__ SccArgs g) {
+    extern __shared__ double s_scc[];
+    const SwArgs& a = g.a;
+    if (blockIdx.x >= g.items) {
+        if (!DEFL) scc_singles(g, blockIdx.x - g.items, gridDim.x - g.items);
+        return;
     }
-}
-
-// BiCGStab on the SCC's odd-row Schur complement (right preconditioner: its diagonal) for
-// the residual R64 scaled by `scale` (1/|R64|, so that FP32 neither underflows nor
-// overflows); the scaled correction is left in D.  `target` is in scaled units.  Lanes
-// with run == false do not write.
-template <class T>
-__device__ int local_inner(const SwArgs& a, const SwLocal& l, const Tile& t, const T* s, const LocalRows& L,
-                           double* red, int& site, bool run, double scale, double target) {
-    constexpr bool f64 = sizeof(T) == 8;
-    T* R = f64 ? (T*)l.R : (T*)l.fR;
-    T* R0 = f64 ? (T*)l.R0 : (T*)l.fR0;
-    T* PH = f64 ? (T*)l.PH : (T*)l.fPH;
-    T* V = f64 ? (T*)l.V : (T*)l.fV;
-    T* SH = f64 ? (T*)l.SH : (T*)l.fSH;
-    T* TT = f64 ? (T*)l.TT : (T*)l.fTT;
-    T* D = f64 ? (T*)l.D : (T*)l.fD;
-    T* WW = f64 ? (T*)l.W64 : (T*)l.fW;
-    const T* dS = sizeof(T) == 8 ? (const T*)l.dS64 : (const T*)l.dS32;
+    int bk = 0;
+    while (bk + 1 < g.nb && blockIdx.x >= g.b[bk + 1].item0) bk++;
+    const int lks = g.b[bk].lks, KS = 1 << lks;
+    const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), item = blockIdx.x - g.b[bk].item0;
+    const uint4 sc = g.scc[g.b[bk].scc0 + item / tiles];
+    const uint32_t ev0 = sc.x, od0 = sc.z;
+    const int se = (int)sc.y, so = (int)sc.w, sm = max(se, so);
+    // threads past one per (row, system) pair leave; barriers count the others
+    const int nact = min((int)blockDim.x, (sm * KS + 31) & ~31);
+    if ((int)threadIdx.x >= nact) return;
+    const int s = threadIdx.x & (KS - 1), rs = threadIdx.x >> lks, RS = nact >> lks;
+    const int k = (int)(item % tiles) * KS + s;
     const size_t Kp = a.Kp;
-    if (run) {
-        for (int i = L.warp; i < L.so; i += L.nw) {
-            const size_t idx = (size_t)(L.od[i] - L.obase) * Kp + t.k;
-            const T x = (T)(l.R64[idx] * scale);
-            R[idx] = x;
-            R0[idx] = x;
-            D[idx] = 0;
-            PH[idx] = 0;
-            V[idx] = 0;
+    const bool act = k < a.K;
+    double* A = s_scc;                       // odd rows: the vector whose product is formed
+    double* W = A + ((size_t)sm << lks);     // even rows: its elimination
+    double* rate = W + ((size_t)se << lks);
+    double* red0 = rate + ((size_t)(2 * a.n) << lks);
+    double* red1 = red0 + ((size_t)(2 * (nact >> 5)) << lks);
+    double* red2 = red1 + ((size_t)(3 * (nact >> 5)) << lks);
+    SccVec<NR> R, V, P, T, IQ;
+    if constexpr (NR > 1) {
+        R.sm = red2 + ((size_t)(nact >> 5) << lks);
+        V.sm = R.sm + ((size_t)so << lks);
+        P.sm = V.sm + ((size_t)so << lks);
+        T.sm = P.sm + ((size_t)so << lks);
+        IQ.sm = T.sm + ((size_t)so << lks);
+    }
+    double R0[NR], D[NR], dS[NR], q[NR];
+    uint32_t po[NR], pe[NR];  // own rows' entries: offset from the SCC's first, << 5 | count
+    for (int idx = threadIdx.x; idx < (2 * a.n) << lks; idx += nact)
+        rate[idx] = a.rateT[(size_t)(idx >> lks) * Kp + (size_t)(item % tiles) * KS + (idx & (KS - 1))];
+    const uint32_t pe0 = a.desc[ev0].z, po0 = a.desc[od0].z;
+    const uint32_t *ent_e = a.ig_ent + pe0, *ent_o = a.ig_ent + po0;
+    const double inv_s = 1.0 / (double)(se + so);
+    auto rhs = [&](uint32_t slot, uint32_t v) {
+        double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + v];
+        const uint32_t p1 = g.og_ptr[slot + 1];
+        for (uint32_t p = g.og_ptr[slot]; p < p1; p++) {
+            const uint32_t e = __ldg(g.og_ent + p);
+            acc += rate[(ent_rate(e) << lks) | s] * g.Z[(size_t)ent_slot(e) * Kp + k];
+        }
+        return acc;
+    };
+    scc_sync(nact);
+    // even rows: 1 / q (in A too, for the Schur diagonal), and b / q, kept in Z until the end
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        const int r = rs + i * RS, idx = (r << lks) | s;
+        pe[i] = 0;
+        if (r < se) {
+            const uint32_t slot = ev0 + r;
+            const uint4 d = a.desc[slot];
+            pe[i] = (d.z - pe0) << 5 | d.w;
+            const double iq = 1.0 / scc_q(rate, d.x, d.y, lks, s);
+            IQ.set(idx, iq);
+            A[idx] = iq;
+            double w = 0.0;
+            if (!DEFL && act) {
+                w = rhs(slot, d.x) * iq;
+                g.Z[(size_t)slot * Kp + k] = w;
+            }
+            W[idx] = w;
         }
     }
-    __syncthreads();
-    double rho = 1.0, alpha = 0.0, omega = 1.0, beta = 0.0, best = 1.0, dmy;
-    int its = 0, stall = 0;
-    while (__any_sync(0xffffffffu, run)) {
-        if (run) {
-            const T b = (T)beta, w = (T)omega;
-            for (int i = L.warp; i < L.so; i += L.nw) {
-                const size_t idx = (size_t)(L.od[i] - L.obase) * Kp + t.k;
-                const T d = dS[idx];
-                PH[idx] = (R[idx] + b * (d * PH[idx] - w * V[idx])) / d;
+    scc_sync(nact);
+    // odd rows: q, Schur diagonal, reduced right-hand side, starting iterate
+    double sum1[1] = {0.0};
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        const int r = rs + i * RS, idx = (r << lks) | s;
+        po[i] = 0;
+        if (r < so) {
+            const uint32_t slot = od0 + r;
+            const uint4 d = a.desc[slot];
+            po[i] = (d.z - po0) << 5 | d.w;
+            const double qv = scc_q(rate, d.x, d.y, lks, s);
+            double dv = qv;
+            for (uint32_t j = 0; j < d.w; j++) {
+                const uint32_t e = __ldg(a.ig_ent + d.z + j);
+                const int ri = ent_rate(e);
+                // rate(e -> o) is the entry's; rate(o -> e) flips the same bit the other way
+                if ((d.y >> (ri >> 1)) & 1u)
+                    dv -= rate[(ri << lks) | s] * rate[((ri ^ 1) << lks) | s] * A[((ent_slot(e) - ev0) << lks) | s];
             }
-        }
-        __syncthreads();
-        local_elim<T, T, T>(a, t, s, L, PH, WW, run);
-        __syncthreads();
-        double r0v = 0.0;
-        for (int i = L.warp; i < L.so; i += L.nw) {
-            const uint32_t slot = L.od[i];
-            const uint2 row = a.rows[slot];
-            const uint32_t p0 = a.ig_ptr[slot];
-            const T flow = sw_gather<T, T>(s, t, a.Kp, a.ig_ent, p0, (int)(a.ig_ptr[slot + 1] - p0), WW, a.beg,
-                                           run, (T)0);
-            if (run) {
-                const size_t idx = (size_t)(slot - L.obase) * Kp + t.k;
-                const T y = sw_q(s, row.x, row.y, t) * PH[idx] - flow;
-                V[idx] = y;
-                r0v += (double)R0[idx] * (double)y;
-            }
-        }
-        local_sum2(red, site, L, t.lane, r0v, 0.0, r0v, dmy);
-        alpha = r0v != 0.0 ? rho / r0v : 0.0;
-        if (run) {
-            const T al = (T)alpha;
-            for (int i = L.warp; i < L.so; i += L.nw) {
-                const size_t idx = (size_t)(L.od[i] - L.obase) * Kp + t.k;
-                SH[idx] = (R[idx] - al * V[idx]) / dS[idx];
-            }
-        }
-        __syncthreads();
-        local_elim<T, T, T>(a, t, s, L, SH, WW, run);
-        __syncthreads();
-        double ts = 0.0, tt = 0.0;
-        for (int i = L.warp; i < L.so; i += L.nw) {
-            const uint32_t slot = L.od[i];
-            const uint2 row = a.rows[slot];
-            const uint32_t p0 = a.ig_ptr[slot];
-            const T flow = sw_gather<T, T>(s, t, a.Kp, a.ig_ent, p0, (int)(a.ig_ptr[slot + 1] - p0), WW, a.beg,
-                                           run, (T)0);
-            if (run) {
-                const size_t idx = (size_t)(slot - L.obase) * Kp + t.k;
-                const T sh = SH[idx];
-                const T y = sw_q(s, row.x, row.y, t) * sh - flow;
-                TT[idx] = y;
-                ts += (double)y * ((double)dS[idx] * (double)sh);
-                tt += (double)y * (double)y;
-            }
-        }
-        local_sum2(red, site, L, t.lane, ts, tt, ts, tt);
-        omega = tt > 0.0 ? ts / tt : 0.0;
-        double rr = 0.0, rn = 0.0;
-        if (run) {
-            const T al = (T)alpha, w = (T)omega;
-            for (int i = L.warp; i < L.so; i += L.nw) {
-                const size_t idx = (size_t)(L.od[i] - L.obase) * Kp + t.k;
-                const T sh = SH[idx];
-                D[idx] += al * PH[idx] + w * sh;
-                const T rv = dS[idx] * sh - w * TT[idx];
-                R[idx] = rv;
-                rr += (double)rv * (double)rv;
-                rn += (double)R0[idx] * (double)rv;
-            }
-        }
-        local_sum2(red, site, L, t.lane, rr, rn, rr, rn);
-        if (run) {
-            its++;
-            if (rr < 0.5 * best) {
-                best = rr;
-                stall = 0;
+            q[i] = qv;
+            dS[i] = dv;
+            double b;
+            if (DEFL) {
+                b = qv * inv_s;
             } else {
-                stall++;
+                b = act ? rhs(slot, d.x) : 0.0;
+                b += scc_gather(a.ig_ent + d.z, (int)d.w, W, rate, lks, s, ev0);
             }
-            const bool stop = !(rr > target) || its >= l.max_iters || r0v == 0.0 || omega == 0.0 || rn == 0.0 ||
-                              !isfinite(rr) || !isfinite(alpha) || stall >= kSwStall;
-            if (stop) {
-                run = false;
-            } else {
-                beta = (rn / rho) * (alpha / omega);
-                rho = rn;
-            }
-        }
-    }
-    return its;
-}
-
-__global__ void __launch_bounds__(kSwLocalWarps * 32) k_sw_local(SwArgs a, SwLocal l) {
-    extern __shared__ unsigned char s_raw[];
-    double* s64 = reinterpret_cast<double*>(s_raw);
-    float* s32 = reinterpret_cast<float*>(s64 + 2 * a.n * 32);
-    __shared__ double red[2 * 2 * kSwLocalWarps * 32];
-    Tile t;
-    t.KT = 32;
-    t.TR = 32;
-    t.lane = threadIdx.x & 31;
-    t.rsub = threadIdx.x >> 5;
-    t.RB = blockDim.x >> 5;
-    // CTA b solves 32-system tile b % tiles of the SCC at place b / tiles in the launch
-    // order: every tile of the largest SCCs is dispatched first, so that the CTAs with
-    // the longest refinements do not start in a late wave
-    const uint32_t tiles = (uint32_t)a.Kp / 32, tile = blockIdx.x % tiles, place = blockIdx.x / tiles;
-    const uint32_t j = l.rank ? l.rank[place] : place;
-    t.k = tile * 32 + t.lane;
-    for (int idx = threadIdx.x; idx < 2 * a.n * 32; idx += blockDim.x) {
-        const double r = a.rateT[(size_t)(idx >> 5) * a.Kp + tile * 32 + (idx & 31)];
-        s64[idx] = r;
-        s32[idx] = (float)r;
-    }
-    __syncthreads();
-    const uint32_t off = l.off[j];
-    LocalRows L;
-    L.se = (int)l.ne[j];
-    L.so = (int)(l.off[j + 1] - off) - L.se;
-    L.ev = l.slots + off;
-    L.od = L.ev + L.se;
-    L.warp = t.rsub;
-    L.nw = t.RB;
-    L.obase = a.beg + a.ne;
-    const bool act = t.k < a.K;
-    const size_t Kp = a.Kp;
-    int site = 0;
-    double b2 = 0.0, dmy;
-    if (act) {
-        for (int i = L.warp; i < L.so; i += L.nw) {
-            const double b = l.bS[(size_t)(L.od[i] - L.obase) * Kp + t.k];
-            b2 += b * b;
-        }
-    }
-    local_sum2(red, site, L, t.lane, b2, 0.0, b2, dmy);
-    // Refinement.  The mixed method takes FP32 inner steps first; a system whose FP32 step
-    // raised the true residual has that step undone, and a system whose FP32 steps stop
-    // cutting the residual by 4x (or after three of them) continues with FP64 steps.
-    // Inner solves of one kind run together: the other systems wait for that step.
-    bool done = !act || !(b2 > 0.0), failed = false, use64 = !l.mixed, stepped = false, last32 = false;
-    double prev = 0.0, rr = 0.0, last_nrm = 0.0;
-    int noimp = 0, its = 0, n32 = 0;
-    for (int outer = 0;; outer++) {
-        // true residual R64 = bS - S X64, in FP64
-        local_elim<double, double, double>(a, t, s64, L, l.X64, l.W64, act);
-        __syncthreads();
-        double r2 = 0.0;
-        for (int i = L.warp; i < L.so; i += L.nw) {
-            const uint32_t slot = L.od[i];
-            const uint2 row = a.rows[slot];
-            const uint32_t p0 = a.ig_ptr[slot];
-            const double flow = sw_gather<double, double>(s64, t, a.Kp, a.ig_ent, p0,
-                                                          (int)(a.ig_ptr[slot + 1] - p0), l.W64, a.beg, act, 0.0);
+            sum1[0] += b * b;
+            R.set(idx, b);
             if (act) {
-                const size_t idx = (size_t)(slot - L.obase) * Kp + t.k;
-                const double res = l.bS[idx] - (sw_q(s64, row.x, row.y, t) * l.X64[idx] - flow);
-                l.R64[idx] = res;
-                r2 += res * res;
+                g.BS[(size_t)(slot - a.beg - a.ne) * Kp + k] = b;
+                g.Z[(size_t)slot * Kp + k] = !DEFL && g.warm ? g.warm[(size_t)k * g.warm_ld + d.x] : 0.0;
             }
         }
-        local_sum2(red, site, L, t.lane, r2, 0.0, rr, dmy);
-        bool revert = false;
+    }
+    scc_sum<1>(red1, lks, s, nact, sum1);
+    const double b2 = sum1[0];
+    double gamma = 0.0;
+    // W = elimination of A (and gamma(A)), with the barrier after it
+    auto elim = [&]() {
+        double gm[1] = {0.0};
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS, idx = (r << lks) | s;
+            if (r < se) {
+                const double w =
+                    scc_gather(ent_e + (pe[i] >> 5), (int)(pe[i] & 31u), A, rate, lks, s, od0) * IQ.get(idx);
+                W[idx] = w;
+                if (DEFL) gm[0] += w;
+            }
+            if (DEFL && r < so) gm[0] += A[idx];
+        }
+        if (DEFL) {
+            scc_sum<1>(red2, lks, s, nact, gm);
+            gamma = gm[0];
+        } else {
+            scc_sync(nact);
+        }
+    };
+    // own odd row's value of the operator applied to A
+    auto apply = [&](int i, int idx) {
+        double y = q[i] * A[idx] - scc_gather(ent_o + (po[i] >> 5), (int)(po[i] & 31u), W, rate, lks, s, ev0);
+        if (DEFL) y += gamma * (q[i] * inv_s);
+        return y;
+    };
+    auto load_x = [&]() {
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS;
+            if (r < so) A[(r << lks) | s] = act ? g.Z[(size_t)(od0 + r) * Kp + k] : 0.0;
+        }
+        scc_sync(nact);
+    };
+    bool done = !act || !(b2 > 0.0), failed = false;
+    const bool warm = !DEFL && g.warm != nullptr;
+    if (warm) {
+        // least-squares multiple (S x . b) / (S x . S x) of the warm start: its residual is
+        // never larger than that of a zero start
+        load_x();
+        elim();
+        double v[2] = {0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS, idx = (r << lks) | s;
+            if (r < so) {
+                const double y = apply(i, idx);
+                v[0] += y * R.get(idx);
+                v[1] += y * y;
+            }
+        }
+        scc_sum<2>(red0, lks, s, nact, v);
+        const double al = v[1] > 0.0 ? v[0] / v[1] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS;
+            if (r < so && act) g.Z[(size_t)(od0 + r) * Kp + k] *= al;
+        }
+    }
+    double prev = 0.0, rr = b2;
+    int noimp = 0, its = 0;
+    for (int outer = 0;; outer++) {
+        if (outer > 0 || warm) {
+            // true residual r = b - S x
+            load_x();
+            elim();
+            double v[1] = {0.0};
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const int r = rs + i * RS, idx = (r << lks) | s;
+                if (r < so) {
+                    const double b = act ? g.BS[(size_t)(od0 + r - a.beg - a.ne) * Kp + k] : 0.0;
+                    const double res = b - apply(i, idx);
+                    R.set(idx, res);
+                    v[0] += res * res;
+                }
+            }
+            scc_sum<1>(red1, lks, s, nact, v);
+            rr = v[0];
+        }
         if (!done) {
-            if (rr <= l.tol2 * b2) {
+            if (rr <= g.tol2 * b2) {
                 done = true;
-            } else if (stepped && last32 && !(rr < prev)) {
-                revert = true;
             } else {
-                if (stepped && last32 && !(rr < 0.25 * prev)) use64 = true;
-                if (stepped && !last32 && !(rr < 0.25 * prev)) noimp++;
+                if (outer > 0 && !(rr < 0.25 * prev)) noimp++;
                 if (noimp >= 2 || !isfinite(rr)) {
                     // stagnation: accepted within the acceptance residual
                     done = true;
-                    failed = !(rr <= l.accept2 * b2);
-                } else if (outer >= l.max_refine + 3) {
+                    failed = !(rr <= g.accept2 * b2);
+                } else if (outer >= g.max_outer) {
                     // out of refinement steps while still improving: the fallback redoes it
                     done = true;
                     failed = true;
                 }
             }
         }
-        if (__any_sync(0xffffffffu, revert)) {
-            if (revert) {
-                for (int i = L.warp; i < L.so; i += L.nw) {
-                    const size_t idx = (size_t)(L.od[i] - L.obase) * Kp + t.k;
-                    l.X64[idx] -= last_nrm * (double)l.fD[idx];
-                }
-                use64 = true;
-            }
-            stepped = false;
-            __syncthreads();
-            continue;  // the residual of the restored iterate
-        }
         if (!__any_sync(0xffffffffu, !done)) break;
         prev = rr;
-        const bool want32 = !done && !use64;
-        const bool phase32 = __any_sync(0xffffffffu, want32);
-        const bool run = phase32 ? want32 : !done;
+        const bool started = !done;
+        bool run = started;
         const double nrm = sqrt(rr), scale = nrm > 0.0 ? 1.0 / nrm : 0.0;
-        const double target = fmax(phase32 ? 1e-10 : 1e-26, 0.01 * l.tol2 * b2 * scale * scale);
-        if (phase32)
-            its += local_inner<float>(a, l, t, s32, L, red, site, run, scale, target);
-        else
-            its += local_inner<double>(a, l, t, s64, L, red, site, run, scale, target);
-        if (run) {
-            for (int i = L.warp; i < L.so; i += L.nw) {
-                const size_t idx = (size_t)(L.od[i] - L.obase) * Kp + t.k;
-                l.X64[idx] += nrm * (phase32 ? (double)l.fD[idx] : l.D[idx]);
+        const double target = fmax(1e-26, 0.01 * g.tol2 * b2 * scale * scale);
+        // BiCGStab on the residual scaled to unit norm, right preconditioner dS; the next
+        // search direction needs no barrier of its own: beta = -(r0 . t) / (r0 . v)
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS, idx = (r << lks) | s;
+            if (r < so) {
+                const double x = R.get(idx) * scale;
+                R.set(idx, x);
+                R0[i] = x;
+                D[i] = 0.0;
+                A[idx] = x / dS[i];
             }
         }
-        stepped = run;
-        last32 = phase32;
-        last_nrm = nrm;
-        if (run && phase32 && ++n32 >= 3) use64 = true;
-        __syncthreads();
+        scc_sync(nact);
+        double rho = 1.0, best = 1.0;
+        int it = 0, stall = 0;
+        while (__any_sync(0xffffffffu, run)) {
+            elim();
+            double v1[1] = {0.0};
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const int r = rs + i * RS, idx = (r << lks) | s;
+                if (r < so) {
+                    const double y = apply(i, idx);
+                    V.set(idx, y);
+                    v1[0] += R0[i] * y;
+                }
+            }
+            scc_sum<1>(red0, lks, s, nact, v1);
+            const double r0v = v1[0], alpha = r0v != 0.0 ? rho / r0v : 0.0;
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const int r = rs + i * RS, idx = (r << lks) | s;
+                if (r < so) {
+                    P.set(idx, A[idx]);
+                    A[idx] = (R.get(idx) - alpha * V.get(idx)) / dS[i];
+                }
+            }
+            scc_sync(nact);
+            elim();
+            double v3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const int r = rs + i * RS, idx = (r << lks) | s;
+                if (r < so) {
+                    const double y = apply(i, idx);
+                    T.set(idx, y);
+                    v3[0] += y * (dS[i] * A[idx]);
+                    v3[1] += y * y;
+                    v3[2] += R0[i] * y;
+                }
+            }
+            scc_sum<3>(red1, lks, s, nact, v3);
+            const double omega = v3[1] > 0.0 ? v3[0] / v3[1] : 0.0, beta = r0v != 0.0 ? -v3[2] / r0v : 0.0;
+            double v2[2] = {0.0, 0.0};
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const int r = rs + i * RS, idx = (r << lks) | s;
+                if (r < so) {
+                    const double sh = A[idx], ph = P.get(idx), d = dS[i];
+                    if (run) D[i] += alpha * ph + omega * sh;
+                    const double rv = d * sh - omega * T.get(idx);
+                    R.set(idx, rv);
+                    v2[0] += rv * rv;
+                    v2[1] += R0[i] * rv;
+                    A[idx] = (rv + beta * (d * ph - omega * V.get(idx))) / d;
+                }
+            }
+            scc_sum<2>(red0, lks, s, nact, v2);
+            if (run) {
+                it++;
+                if (v2[0] < 0.5 * best) {
+                    best = v2[0];
+                    stall = 0;
+                } else {
+                    stall++;
+                }
+                run = !(!(v2[0] > target) || it >= g.max_iters || r0v == 0.0 || omega == 0.0 || v2[1] == 0.0 ||
+                        !isfinite(v2[0]) || !isfinite(alpha) || stall >= g.stall);
+                rho = v2[1];
+            }
+        }
+        its += it;
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS;
+            if (r < so && started) g.Z[(size_t)(od0 + r) * Kp + k] += nrm * D[i];
+        }
     }
-    if (act && L.warp == 0) {
-        atomicMax(l.ratio + t.k, (unsigned long long)__double_as_longlong(b2 > 0.0 ? rr / b2 : 0.0));
-        if (failed) l.fail[t.k] = 1;
-        atomicMax(l.iters + t.k, its);
+    // even rows from the odd solution
+    load_x();
+    double total[1] = {0.0};
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        const int r = rs + i * RS, idx = (r << lks) | s;
+        if (r < se) {
+            const double w = scc_gather(ent_e + (pe[i] >> 5), (int)(pe[i] & 31u), A, rate, lks, s, od0) * IQ.get(idx);
+            if (DEFL) {
+                W[idx] = w;
+                total[0] += w;
+            } else if (act) {
+                g.Z[(size_t)(ev0 + r) * Kp + k] += w;
+            }
+        }
+        if (DEFL && r < so) total[0] += A[idx];
+    }
+    if (DEFL) {
+        scc_sum<1>(red1, lks, s, nact, total);
+        const double inv = total[0] != 0.0 ? 1.0 / total[0] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const int r = rs + i * RS, idx = (r << lks) | s;
+            if (act && r < se) g.Rb[(size_t)k * g.TS + g.pos[ev0 + r]] = W[idx] * inv;
+            if (act && r < so) g.Rb[(size_t)k * g.TS + g.pos[od0 + r]] = A[idx] * inv;
+        }
+    }
+    if (act && rs == 0) {
+        atomicMax(g.ratio + k, (unsigned long long)__double_as_longlong(b2 > 0.0 ? rr / b2 : 0.0));
+        if (failed) g.fail[k] = 1;
+        atomicMax(g.iters, its);
     }
 }
 
@@ -1621,7 +1796,7 @@ __global__ void k_sw_rate_table(int n, int K, int Kp, int nrhs, const double* __
 
 // ---- host side ------------------------------------------------------------------------------
 enum SwSlot { W_Z, W_RATET, W_BV, W_BS, W_R64, W_DS64, W_DS32, W_W64, W_WT, W_R, W_R0, W_PH, W_V, W_SH, W_TT,
-              W_D, W_SCAL, W_ISCAL, W_CNT, W_LOC, W_QO, W_IQE, W_PERM, W_F0, W_COUNT = W_F0 + 8 };
+              W_D, W_SCAL, W_ISCAL, W_CNT, W_LOC, W_QO, W_IQE, W_PERM, W_COUNT };
 
 bool debug_on();
 
@@ -1658,6 +1833,9 @@ int build_terminal_plan(const std::vector<int32_t>& order, const std::vector<int
             }
             (par ? g.no : g.ne) = (uint32_t)rows.size() - g.beg - (par ? g.ne : 0);
         }
+        g.s0 = (uint32_t)TP->h_scc.size();
+        g.ns = 1;
+        TP->h_scc.push_back(make_uint4(g.beg, g.ne, g.beg + g.ne, g.no));
         TP->max_rows = std::max(TP->max_rows, g.ne + g.no);
         TP->max_even = std::max(TP->max_even, g.ne);
         TP->max_odd = std::max(TP->max_odd, g.no);
@@ -1974,6 +2152,24 @@ __global__ void k_pl_groups(int T, int TS, const int32_t* __restrict__ offsets, 
     }
 }
 
+// SCCs of >= 2 states in list order (idx: exclusive scan of their flags)
+__global__ void k_pl_scc2(int NT, const uint32_t* __restrict__ ssize, uint32_t* __restrict__ flag) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c > NT) return;
+    flag[c] = (c < NT && ssize[c] >= 2) ? 1u : 0u;
+}
+__global__ void k_pl_scc_list(int NT, int T, int TS, const int32_t* __restrict__ offsets,
+                              const uint32_t* __restrict__ gid_incl, const uint32_t* __restrict__ ssize,
+                              const uint32_t* __restrict__ E, const uint32_t* __restrict__ info,
+                              const uint32_t* __restrict__ idx, uint4* __restrict__ out) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= NT || ssize[c] < 2) return;
+    const uint32_t* in = info + (size_t)(gid_incl[c] - 1) * 8;
+    const uint32_t p0 = in[0], ne = in[1], cs = (uint32_t)(offsets[T + c] - TS), ce = cs + ssize[c];
+    const uint32_t er = E[cs] - E[p0], se = E[ce] - E[cs];
+    out[idx[c]] = make_uint4(p0 + er, se, p0 + ne + (cs - p0) - er, ssize[c] - se);
+}
+
 // slot of every transient position: rows, slot_of (by state), group of each slot
 __global__ void k_pl_slots(uint32_t M, int TS, const int32_t* __restrict__ order, const uint32_t* __restrict__ F,
                            const uint32_t* __restrict__ E, const uint32_t* __restrict__ sccpos,
@@ -2208,6 +2404,24 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         ESL_CUDA(cudaMemcpyAsync(&tot[2], qidx.get() + NT, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaMemcpyAsync(&tot[3], qoff.get() + NT, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
+        // the list of SCCs of >= 2 states (qsize and qoff are free again)
+        uint32_t n2 = 0;
+        for (uint32_t g = 0; g < G; g++) n2 += h_info[(size_t)g * 8 + 6];
+        if (n2 > 0) {
+            ESL_TRY(P->scc.alloc(n2));
+            ESL_COUNT_LAUNCH();
+            k_pl_scc2<<<nblk((uint64_t)NT + 1), 256, 0, s>>>(NT, ssize.get(), qsize.get());
+            DevBuf<uint32_t> sidx;
+            ESL_TRY(sidx.alloc((size_t)NT + 1));
+            ESL_TRY(scan_excl(tmp, qsize.get(), sidx.get(), (uint32_t)NT + 1, s));
+            ESL_COUNT_LAUNCH();
+            k_pl_scc_list<<<nblk(NT), 256, 0, s>>>(NT, T, TS, offsets, gid.get(), ssize.get(), E.get(), info.get(),
+                                                   sidx.get(), P->scc.get());
+            ESL_CUDA(cudaGetLastError());
+            P->h_scc.resize(n2);
+            ESL_CUDA(cudaMemcpyAsync(P->h_scc.data(), P->scc.get(), (size_t)n2 * sizeof(uint4), cudaMemcpyDeviceToHost,
+                                     s));
+        }
         ESL_TRY(P->ig_ent.alloc(std::max<uint32_t>(tot[0], 1)));
         ESL_TRY(P->og_ent.alloc(std::max<uint32_t>(tot[1], 1)));
         ESL_TRY(P->desc.alloc(M));
@@ -2263,6 +2477,7 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         ESL_CUDA(cudaGetLastError());
     }
     // the group table on the host
+    uint32_t s0 = 0;
     for (uint32_t g = 0; g < G; g++) {
         const uint32_t* in = &h_info[(size_t)g * 8];
         SwGroup gr{};
@@ -2278,6 +2493,9 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
             gr.max_odd = (int)in[7];
         }
         gr.nin = h_tail[2 * g + 1];
+        gr.s0 = s0;
+        gr.ns = in[6];
+        s0 += gr.ns;
         P->max_rows = std::max(P->max_rows, gr.ne + gr.no);
         P->max_even = std::max(P->max_even, gr.ne);
         P->max_odd = std::max(P->max_odd, gr.no);
@@ -2306,31 +2524,33 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     return ESL_OK;
 }
 
-// Launch order of the CTA-local groups: per group, its SCCs' group-relative indices by
-// decreasing size (ties by index), read by k_sw_local through SwLocal::rank.  A group
-// lasts as long as its slowest CTA, the one of its largest SCC; started first, that CTA
-// no longer waits for a free slot behind the small ones.
-int build_local_rank(esl_ctx* ctx, SweepPlan* P) {
-    uint32_t nl = 0;
-    for (const SwGroup& g : P->groups)
-        if (g.kind == 1) nl = std::max(nl, g.scc0 + g.nscc);
-    if (nl == 0) return ESL_OK;
-    cudaStream_t s = ctx->stream;
-    std::vector<uint32_t> off((size_t)nl + 1), rank(nl);
-    ESL_CUDA(cudaMemcpyAsync(off.data(), P->lsc_off.get(), ((size_t)nl + 1) * 4, cudaMemcpyDeviceToHost, s));
-    ESL_CUDA(cudaStreamSynchronize(s));
-    for (const SwGroup& g : P->groups) {
-        if (g.kind != 1) continue;
-        std::vector<uint32_t> idx(g.nscc);
-        for (uint32_t j = 0; j < g.nscc; j++) idx[j] = j;
-        std::stable_sort(idx.begin(), idx.end(), [&](uint32_t x, uint32_t y) {
-            return off[g.scc0 + x + 1] - off[g.scc0 + x] > off[g.scc0 + y + 1] - off[g.scc0 + y];
-        });
-        std::copy(idx.begin(), idx.end(), rank.begin() + g.scc0);
+// Most rows of one parity of an SCC
+inline uint32_t scc_rows(const uint4& c) { return std::max(c.y, c.w); }
+
+// Sorts each group's SCC list by decreasing size (the launch order of k_sw_scc: a group
+// lasts as long as the CTA of its largest SCC, which must not start behind the small ones)
+// and marks the groups whose SCCs all fit a CTA.
+int finish_scc_list(esl_ctx* ctx, int n, SweepPlan* P) {
+    for (SwGroup& g : P->groups) {
+        const auto b = P->h_scc.begin() + g.s0, e = b + g.ns;
+        std::stable_sort(b, e, [](const uint4& x, const uint4& y) { return scc_rows(x) > scc_rows(y); });
+        g.resident = true;
+        g.singles = g.ne + g.no;
+        for (auto c = b; c != e; ++c) {
+            g.singles -= c->y + c->w;
+            const uint32_t m = scc_rows(*c);
+            g.resident = g.resident && m <= (uint32_t)kSccMaxRows &&
+                         scc_smem_doubles(m > kSccThreads1 ? 2 : 1, n, (int)c->y, (int)c->w, 0,
+                                          (int)std::min<uint32_t>(kSccThreads1, (m + 31) & ~31u)) *
+                                 8 <=
+                             kSccMaxSmem;
+        }
     }
-    ESL_TRY(P->lsc_rank.alloc(nl));
-    ESL_CUDA(cudaMemcpyAsync(P->lsc_rank.get(), rank.data(), (size_t)nl * 4, cudaMemcpyHostToDevice, s));
-    ESL_CUDA(cudaStreamSynchronize(s));
+    if (P->h_scc.empty()) return ESL_OK;
+    if (!P->scc.get()) ESL_TRY(P->scc.alloc(P->h_scc.size()));
+    ESL_CUDA(cudaMemcpyAsync(P->scc.get(), P->h_scc.data(), P->h_scc.size() * sizeof(uint4), cudaMemcpyHostToDevice,
+                             ctx->stream));
+    ESL_CUDA(cudaStreamSynchronize(ctx->stream));
     return ESL_OK;
 }
 
@@ -2344,7 +2564,9 @@ int build_plan(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     }
     SweepPlan* P = nullptr;
     ESL_TRY(build_plan_device(ctx, net, P));
-    if (int rc = build_local_rank(ctx, P); rc != ESL_OK) {
+    int rc = finish_scc_list(ctx, net->n, P);
+    if (rc == ESL_OK && P->term) rc = finish_scc_list(ctx, net->n, P->term);
+    if (rc != ESL_OK) {
         delete P;
         return rc;
     }
@@ -2401,6 +2623,58 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
     if (want > cap) want = cap;
     if (want == 0) want = 1;
     return dim3((unsigned)want, ty);
+}
+
+// Launches k_sw_scc over SCCs [j0, j1) of group g (sorted by decreasing size) and, with
+// `singles`, its singleton rows.  KS, the systems of one CTA, is the largest power of two
+// that keeps one thread per (row, system) pair within kSccPairs threads (1 above).
+constexpr int kSccPairs = 256;
+int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t j0, uint32_t j1, bool singles, bool defl,
+               SccArgs ga) {
+    const int K = ga.a.K, n = ga.a.n;
+    int lmax = 0;
+    while (lmax < 5 && (1 << lmax) < K) lmax++;
+    ga.scc = P->scc.get() + g.s0;
+    ga.nb = 0;
+    uint64_t items = 0;
+    int nr = 1, threads = 32;
+    size_t smem = 0;
+    for (uint32_t j = j0; j < j1; j++) {
+        const int m = (int)scc_rows(P->h_scc[g.s0 + j]);
+        if (m > kSccThreads1) nr = std::max(nr, m > 4 * kSccThreads ? 8 : 4);
+    }
+    for (uint32_t j = j0; j < j1; j++) {
+        const uint4& c = P->h_scc[g.s0 + j];
+        const int m = (int)scc_rows(c);
+        int lks = 0;
+        while (lks < lmax && (m << (lks + 1)) <= kSccPairs) lks++;
+        if (ga.nb == 0 || ga.b[ga.nb - 1].lks != lks) ga.b[ga.nb++] = SccBucket{(uint32_t)items, j, lks};
+        items += (uint64_t)((K + (1 << lks) - 1) >> lks);
+        const int nact = std::min(scc_threads(nr), ((m << lks) + 31) & ~31);
+        threads = std::max(threads, nact);
+        smem = std::max(smem, scc_smem_doubles(nr, n, (int)c.y, (int)c.w, lks, nact) * 8);
+    }
+    ga.items = (uint32_t)items;
+    uint64_t ctas = 0;
+    if (singles) {
+        threads = std::max(threads, 128);
+        const uint64_t pairs = (uint64_t)(g.ne + g.no) * (uint64_t)K;
+        ctas = std::max<uint64_t>(1, std::min<uint64_t>((pairs + threads - 1) / threads, (uint64_t)ctx->sm_count * 8));
+    }
+    if (items + ctas == 0) return ESL_OK;
+    if (items + ctas > 0x7FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
+    const unsigned grid = (unsigned)(items + ctas);
+    cudaStream_t s = ctx->stream;
+    auto go = [&](auto kern) -> int {
+        if (smem > 48 * 1024)
+            ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
+        ESL_COUNT_LAUNCH();
+        kern<<<grid, threads, smem, s>>>(ga);
+        ESL_CUDA(cudaGetLastError());
+        return ESL_OK;
+    };
+    if (defl) return nr == 1 ? go(k_sw_scc<1, true>) : nr == 4 ? go(k_sw_scc<4, true>) : go(k_sw_scc<8, true>);
+    return nr == 1 ? go(k_sw_scc<1, false>) : nr == 4 ? go(k_sw_scc<4, false>) : go(k_sw_scc<8, false>);
 }
 
 // the graphs (one per poll slot) of a Krylov solve, released on scope exit
@@ -2572,12 +2846,14 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     double* scal = (double*)ws.get(W_SCAL, (size_t)C_NSCAL * Kp * 8, &st_);
     int* iscal = (int*)ws.get(W_ISCAL, (size_t)I_NISCAL * Kp * 4, &st_);
     int* d_cnt = (int*)ws.get(W_CNT, 64, &st_);
-    // per-system results of the CTA-local groups: max |r|^2/|b|^2, failure flag, iterations
-    unsigned long long* loc_ratio = (unsigned long long*)ws.get(W_LOC, (size_t)Kp * 16, &st_);
+    // results of the SCC-resident groups: per system max |r|^2/|b|^2 and failure flag, per
+    // group the most iterations
+    const size_t loc_bytes = (size_t)Kp * 12 + P->groups.size() * 4;
+    unsigned long long* loc_ratio = (unsigned long long*)ws.get(W_LOC, loc_bytes, &st_);
     if (st_ != ESL_OK) return st_;
     int* loc_fail = reinterpret_cast<int*>(loc_ratio + Kp);
     int* loc_iters = loc_fail + Kp;
-    ESL_CUDA(cudaMemsetAsync(loc_ratio, 0, (size_t)Kp * 16, s));
+    ESL_CUDA(cudaMemsetAsync(loc_ratio, 0, loc_bytes, s));
     SwScalPtr sc;
     for (int j = 0; j < C_NSCAL; j++) sc.c[j] = scal + (size_t)j * Kp;
     for (int j = 0; j < I_NISCAL; j++) sc.i[j] = iscal + (size_t)j * Kp;
@@ -2625,11 +2901,47 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         const uint32_t rows = g.ne + g.no;
         a.gam = nullptr;
         a.inv_s = 1.0 / (double)std::max<uint32_t>(rows, 1);
-        if (g.kind == 0) {
+        // singleton SCCs only: a row kernel, or the singleton CTAs of k_sw_scc, whose lanes
+        // hold rows when there are fewer than 32 systems
+        if (g.kind == 0 && K >= 32) {
             ESL_COUNT_LAUNCH();
             k_sw_rhs<true><<<row_grid(rows, Kp, KT64, ctx->sm_count), kSwT, sm64, s>>>(
                 a, P->og_ptr.get(), P->og_ent.get(), x0, x0_ld, Z, nullptr);
             ESL_CUDA(cudaGetLastError());
+            continue;
+        }
+        if (g.resident) {
+            SccArgs ga{};
+            ga.a = a;
+            ga.og_ptr = P->og_ptr.get();
+            ga.og_ent = P->og_ent.get();
+            ga.x0 = x0;
+            ga.x0_ld = x0_ld;
+            ga.warm = term ? nullptr : o.d_warm;
+            ga.warm_ld = (size_t)net->N;
+            ga.Z = Z;
+            ga.BS = (double*)ws.get(W_BS, (size_t)std::max<uint32_t>(P->max_odd, 1) * Kp * 8, &st_);
+            if (st_ != ESL_OK) return st_;
+            ga.tol2 = tol * tol;
+            ga.accept2 = kSwAcceptRel * kSwAcceptRel;
+            ga.max_iters = max_iters;
+            ga.max_outer = g.kind == 2 ? max_refine : max_refine + 3;
+            ga.stall = g.kind == 2 ? kSwStall64 : kSwStall;
+            ga.ratio = loc_ratio;
+            ga.fail = loc_fail;
+            ga.iters = loc_iters + (&g - P->groups.data());
+            if (term) {
+                ga.pos = P->pos.get();
+                ga.Rb = y;
+                ga.TS = net->term_states;
+            }
+            st.local_groups++;
+            ESL_TRY(launch_scc(ctx, P, g, 0, g.ns, !term && g.singles > 0, term, ga));
+            if (debug_on()) {
+                ESL_CUDA(cudaStreamSynchronize(s));
+                fprintf(stderr, "[esl-sweep] local group beg %u even %u odd %u max_scc %d sccs %u singles %u, %.3f ms\n",
+                        g.beg, g.ne, g.no, g.max_scc, g.ns, g.singles, g_ms());
+            }
             continue;
         }
         double* Bv = (double*)ws.get(W_BV, (size_t)P->max_rows * Kp * 8, &st_);
@@ -2641,11 +2953,8 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             k_sw_rhs<false><<<row_grid(rows, Kp, KT64, ctx->sm_count), kSwT, sm64, s>>>(
                 a, P->og_ptr.get(), P->og_ent.get(), x0, x0_ld, Z, Bv);
         ESL_CUDA(cudaGetLastError());
-        // ---- Krylov group (CTA-local or grid-wide) ----
-        if (g.kind == 1)
-            st.local_groups++;
-        else
-            st.krylov_groups++;
+        // ---- grid-wide Krylov group ----
+        st.krylov_groups++;
         const size_t vo = (size_t)std::max<uint32_t>(P->max_odd, 1) * Kp, ve = (size_t)std::max<uint32_t>(P->max_even, 1) * Kp;
         double* bS = (double*)ws.get(W_BS, vo * 8, &st_);
         double* R64 = (double*)ws.get(W_R64, vo * 8, &st_);
@@ -2683,16 +2992,14 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         ESL_CUDA(cudaMemsetAsync(iscal, 0, (size_t)I_NISCAL * Kp * 4, s));
         ESL_COUNT_LAUNCH();
         k_sw_diag<<<go, kSwT, gsm64, s>>>(a, dS64, dS32);
-        if (g.kind == 2) {
-            // out-rate sums of the rows, read by the FP64 operator kernels of this group
-            double* Qo = (double*)ws.get(W_QO, vo * 8, &st_);
-            double* IQe = (double*)ws.get(W_IQE, ve * 8, &st_);
-            if (st_ != ESL_OK) return st_;
-            ESL_COUNT_LAUNCH();
-            k_sw_qrows<<<row_grid(g.ne + g.no, Kp, gKT64, ctx->sm_count), kSwT, gsm64, s>>>(a, Qo, IQe);
-            a.Qo = Qo;
-            a.IQe = IQe;
-        }
+        // out-rate sums of the rows, read by the FP64 operator kernels of this group
+        double* Qo = (double*)ws.get(W_QO, vo * 8, &st_);
+        double* IQe = (double*)ws.get(W_IQE, ve * 8, &st_);
+        if (st_ != ESL_OK) return st_;
+        ESL_COUNT_LAUNCH();
+        k_sw_qrows<<<row_grid(g.ne + g.no, Kp, gKT64, ctx->sm_count), kSwT, gsm64, s>>>(a, Qo, IQe);
+        a.Qo = Qo;
+        a.IQe = IQe;
         // reduced rhs bS = b_odd + A_oe (b_even / q_e)
         ESL_COUNT_LAUNCH();
         k_sw_elim<1, double, double, double><<<ge, kSwT, gsm64, s>>>(a, Bv, (const double*)nullptr, W64);
@@ -2703,73 +3010,6 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         const double* warm = term ? nullptr : o.d_warm;
         k_sw_init<<<go, kSwT, 0, s>>>(a, warm, (size_t)net->N, bS, dS64, X64);
         ESL_CUDA(cudaGetLastError());
-        if (g.kind == 1) {
-            SwLocal l{};
-            l.off = P->lsc_off.get() + g.scc0;
-            l.rank = P->lsc_rank.get() ? P->lsc_rank.get() + g.scc0 : nullptr;
-            l.ne = P->lsc_ne.get() + g.scc0;
-            l.slots = P->lsc_slots.get();
-            l.bS = bS;
-            l.dS64 = dS64;
-            l.dS32 = dS32;
-            l.X64 = X64;
-            l.R64 = R64;
-            l.W64 = W64;
-            l.R = (double*)vR;
-            l.R0 = (double*)vR0;
-            l.PH = (double*)vPH;
-            l.V = (double*)vV;
-            l.SH = (double*)vSH;
-            l.TT = (double*)vTT;
-            l.D = (double*)vD;
-            if (mixed) {
-                const size_t lo = (size_t)std::max<uint32_t>(P->max_odd_local, 1) * Kp;
-                const size_t le = (size_t)std::max<uint32_t>(P->max_even_local, 1) * Kp;
-                float** fv[7] = {&l.fR, &l.fR0, &l.fPH, &l.fV, &l.fSH, &l.fTT, &l.fD};
-                for (int j = 0; j < 7; j++) *fv[j] = (float*)ws.get(W_F0 + j, lo * 4, &st_);
-                l.fW = (float*)ws.get(W_F0 + 7, le * 4, &st_);
-                if (st_ != ESL_OK) return st_;
-            }
-            l.tol2 = tol * tol;
-            l.accept2 = kSwAcceptRel * kSwAcceptRel;
-            l.max_iters = max_iters;
-            l.max_refine = max_refine;
-            l.mixed = mixed ? 1 : 0;
-            l.ratio = loc_ratio;
-            l.fail = loc_fail;
-            l.iters = loc_iters;
-            const int nw = std::max(1, std::min(kSwLocalWarps, (g.max_odd + 3) / 4));
-            const size_t smem = (size_t)2 * n * 32 * (8 + 4);
-            if (g.nscc > 0) {
-                ESL_COUNT_LAUNCH();
-                k_sw_local<<<(unsigned)g.nscc * (unsigned)(Kp / 32), nw * 32, smem, s>>>(a, l);
-            }
-            // even rows of the group from the odd solution, straight into Z
-            a.flags = nullptr;
-            a.KT = gKT64;
-            ESL_COUNT_LAUNCH();
-            k_sw_elim<1, double, double, double><<<ge, kSwT, gsm64, s>>>(a, Bv, X64, Z + (size_t)g.beg * Kp);
-            ESL_CUDA(cudaGetLastError());
-            if (debug_on()) {
-                std::vector<unsigned long long> h_loc((size_t)Kp * 2);
-                ESL_CUDA(cudaMemcpyAsync(h_loc.data(), loc_ratio, (size_t)Kp * 16, cudaMemcpyDeviceToHost, s));
-                ESL_CUDA(cudaStreamSynchronize(s));
-                const int* h_fail = reinterpret_cast<const int*>(h_loc.data() + Kp);
-                int nf = 0;
-                double worst = 0.0;
-                for (int k = 0; k < K; k++) {
-                    double ratio;
-                    memcpy(&ratio, &h_loc[k], 8);
-                    worst = std::max(worst, ratio);
-                    nf += h_fail[k] != 0;
-                }
-                fprintf(stderr,
-                        "[esl-sweep] local group beg %u even %u odd %u max_scc %d sccs %u warps %d: failed %d "
-                        "worst relres so far %.3e, %.3f ms\n",
-                        g.beg, g.ne, g.no, g.max_scc, g.nscc, nw, nf, std::sqrt(worst), g_ms());
-            }
-            continue;
-        }
         // An NVTX range names the grid solve of the largest level group, so that a
         // profiler can select that group's launches (`ncu --nvtx --nvtx-include
         // "esl_largest_level_group/"`); without a profiler attached it costs nothing.
@@ -3195,22 +3435,30 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
                                                                         o.d_occupation);
         ESL_CUDA(cudaGetLastError());
     }
-    // results of the CTA-local groups
+    // results of the SCC-resident groups
     if (st.local_groups > 0) {
-        std::vector<unsigned long long> h_loc((size_t)Kp * 2);
-        ESL_CUDA(cudaMemcpyAsync(h_loc.data(), loc_ratio, (size_t)Kp * 16, cudaMemcpyDeviceToHost, s));
+        std::vector<unsigned char> h_loc(loc_bytes);
+        ESL_CUDA(cudaMemcpyAsync(h_loc.data(), loc_ratio, loc_bytes, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
-        const int* h_fail = reinterpret_cast<const int*>(h_loc.data() + Kp);
-        const int* h_its = h_fail + Kp;
-        int loc_its = 0;
+        std::vector<int> h_its(P->groups.size());
+        std::memcpy(h_its.data(), h_loc.data() + (size_t)Kp * 12, h_its.size() * 4);
         for (int k = 0; k < K; k++) {
             double ratio;
-            memcpy(&ratio, &h_loc[k], 8);
+            int bad;
+            std::memcpy(&ratio, h_loc.data() + (size_t)k * 8, 8);
+            std::memcpy(&bad, h_loc.data() + (size_t)Kp * 8 + (size_t)k * 4, 4);
             st.relres = std::max(st.relres, std::sqrt(ratio));
-            if (h_fail[k]) failed[k] = 1;
-            loc_its = std::max(loc_its, h_its[k]);
+            if (bad) failed[k] = 1;
         }
-        total_iters += loc_its;
+        // groups of larger SCCs add their iterations, groups of small ones run beside them
+        int small = 0;
+        for (size_t j = 0; j < h_its.size(); j++) {
+            if (P->groups[j].kind == 2)
+                total_iters += h_its[j];
+            else
+                small = std::max(small, h_its[j]);
+        }
+        total_iters += small;
     }
     st.iters = total_iters;
     st.failed.clear();
