@@ -1746,7 +1746,9 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
             int smax = 0;
             for (int t : dense_list) smax = std::max(smax, net->h_offsets[t + 1] - net->h_offsets[t]);
             size_t smem = (size_t)smax * (smax + 1) * 8 + (size_t)smax * 4 + 16;
-            ESL_CUDA(cudaFuncSetAttribute(k_dense_terminal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            // the same limit from every thread: contexts of esl_solve_many set it concurrently
+            constexpr int kDenseTermSmem = kDenseTerm * (kDenseTerm + 1) * 8 + kDenseTerm * 4 + 16;
+            ESL_CUDA(cudaFuncSetAttribute(k_dense_terminal, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseTermSmem));
             ESL_COUNT_LAUNCH();
             k_dense_terminal<<<dim3((unsigned)dense_list.size(), B), 256, smem, s>>>(
                 n, d_list, net->offsets.get(), net->order.get(), net->F.get(), d_rates, TS, Rb);
