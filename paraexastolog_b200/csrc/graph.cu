@@ -7,11 +7,11 @@
 //
 // Graph: edge s -> s ^ (1<<i) iff bit i of F[s]; edge s ^ (1<<i) -> s iff bit i of G[s].
 // SCCs: iterated trim (a state with no live successor or no live predecessor is a
-// singleton SCC), then rounds of forward max-colour propagation followed by a
-// backward reach within each colour from its root (the state whose colour is its
-// own id, i.e. the largest id of its SCC); every round removes at least one SCC
-// per colour.  Labels are made canonical afterwards: the label of an SCC is its
-// smallest state, the same label the reference gives singletons.
+// singleton SCC), then rounds of forward max-priority propagation followed by a backward
+// reach within each colour from its root (the state whose colour is its own priority,
+// i.e. the largest of its SCC); every round removes at least one SCC per colour.  Labels
+// are made canonical afterwards: the label of an SCC is its smallest state, the same
+// label the reference gives singletons.
 // Levels: level 1 = SCC without out-edges to other SCCs (terminal); otherwise
 // 1 + max level of its successor SCCs (the reference's labelling fixpoint).
 // Order: terminal SCCs by label ascending, then the others by decreasing level and,
@@ -36,142 +36,305 @@ constexpr int kThreads = 256;
 
 inline unsigned blocks_for(uint64_t N) { return (unsigned)((N + kThreads - 1) / kThreads); }
 
-// flag slot 0: "changed" for the running fixpoint
-__global__ void k_trim(int n, uint64_t N, const uint32_t* __restrict__ F, const uint32_t* __restrict__ G,
-                       int32_t* __restrict__ lab, unsigned long long* __restrict__ flags) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N || lab[v] >= 0) return;
-    uint32_t f = F[v], g = G[v];
-    bool out_live = false, in_live = false;
-    while (f && !out_live) {
-        int i = __ffs(f) - 1;
-        f &= f - 1;
-        out_live = lab[v ^ (1ull << i)] < 0;
+// ---- SCCs, canonical labels and levels in one cooperative launch ---------------------------
+// Every fixpoint of the decomposition is monotone, so its states may be relaxed in any
+// order and read any mixture of old and new neighbour values: threads run several passes
+// over their states between two grid barriers, and the barriers only decide termination
+// (a phase in which no state changed).  With a launch per pass and a host read of the flag
+// per few passes, launches and reads took most of the time: the n=20 network 27.4 ms (1,587
+// launches, 474 reads) against 8.4 ms here, the n=13 one 4.1 against 1.0 ms.  A pass over
+// 2^20 states (17 us) is bound by the L2 traffic of the neighbour reads (whole-warp walks of
+// the union of flips and four states in flight measured the same), a pass over few states
+// by round trips to L2, a level per pass at worst (114 passes, 2.1 ms, at n=20).
+//
+// A CTA owns the 32-state chunks c with c % grid == its index, which spreads live states
+// evenly, and keeps the list of its live states.  Colours are pseudo-random priorities
+// (a bijection of the state index): with the index itself as colour the same network took
+// 28 rounds whose live sets shrink 2.5 times slower.
+constexpr int kSccT = 1024;
+constexpr uint32_t kReached = 0x80000000u;
+constexpr unsigned kBarrierPolls = 1u << 24;  // bound of a barrier wait (seconds)
+
+struct GraphState {        // device, zeroed before the launch
+    unsigned arrived;      // grid barrier: arrivals so far
+    int status;            // 0, or 1: a budget ran out, 2: a barrier wait ran out
+    unsigned changed[3];   // by phase % 3
+    unsigned live[3];      // by round % 3
+    unsigned rounds, phases;
+};
+
+struct GraphArgs {
+    int n;
+    uint32_t N;
+    const uint32_t *F, *G;
+    int32_t* lab;
+    uint32_t* color;   // 0: dead; priority + 1, kReached once it reaches its colour's root
+    int32_t* canon;
+    int32_t* level;
+    uint32_t* list;    // grid x cap
+    uint32_t cap;      // states per CTA
+    uint64_t* keys;
+    int32_t* vals;
+    int64_t budget;    // passes per fixpoint
+    GraphState* st;
+};
+
+// Bijection of [0, 2^n): odd multiplications and xor-shifts
+__device__ __forceinline__ uint32_t priority_of(uint32_t v, int n) {
+    const uint32_t m = (1u << n) - 1u;
+    const int h = max(n >> 1, 1);
+    v = (v * 0x9E3779B1u) & m;
+    v ^= v >> h;
+    v = (v * 0x85EBCA6Bu) & m;
+    v ^= v >> (h + 1);
+    return (v * 0xC2B2AE35u) & m;
+}
+
+// Grid barrier with a bounded wait; false once the launch has failed anywhere.
+__device__ bool grid_barrier(GraphState* st, unsigned& target) {
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&st->arrived, 1u);
+        unsigned polls = 0;
+        while (*(volatile unsigned*)&st->arrived < target && *(volatile int*)&st->status != 2)
+            if (++polls > kBarrierPolls) atomicExch(&st->status, 2);
+        __threadfence();
     }
-    while (g && !in_live) {
-        int i = __ffs(g) - 1;
-        g &= g - 1;
-        in_live = lab[v ^ (1ull << i)] < 0;
-    }
-    if (!(out_live && in_live)) {
-        lab[v] = (int32_t)v;
-        flags[0] = 1;
-        atomicAdd(&flags[1], 1ull);
+    __syncthreads();
+    return *(volatile int*)&st->status == 0;
+}
+
+// Calls fn on the values of arr at the neighbours of v in mask, eight at a time (0 past the
+// last), until it returns true.  A pass over few states is a chain of L2 round trips:
+// eight loads in flight make it one or two of them.
+template <class Fn>
+__device__ __forceinline__ void for_neighbours(uint32_t v, uint32_t mask, const uint32_t* arr, Fn fn) {
+    while (mask) {
+        uint32_t x[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const uint32_t bit = mask & (0u - mask);
+            x[j] = bit ? __ldcg(arr + (v ^ bit)) : 0u;
+            mask ^= bit;
+        }
+        if (fn(x)) return;
     }
 }
 
-__global__ void k_color_init(uint64_t N, const int32_t* __restrict__ lab, int32_t* __restrict__ color,
-                             uint8_t* __restrict__ reached) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    color[v] = lab[v] < 0 ? (int32_t)v : -1;
-    reached[v] = 0;
-}
-
-// colour(v) = max colour over live predecessors (chaotic, monotone)
-__global__ void k_color_fw(uint64_t N, const uint32_t* __restrict__ G, const int32_t* __restrict__ lab,
-                           int32_t* __restrict__ color, unsigned long long* __restrict__ flags) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N || lab[v] >= 0) return;
-    int32_t c = color[v], m = c;
-    uint32_t g = G[v];
-    while (g) {
-        int i = __ffs(g) - 1;
-        g &= g - 1;
-        uint64_t u = v ^ (1ull << i);
-        if (lab[u] < 0) m = max(m, color[u]);
+__global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
+    const uint32_t tid = threadIdx.x, cta = blockIdx.x, ctas = gridDim.x;
+    GraphState* st = g.st;
+    uint32_t* list = g.list + (size_t)cta * g.cap;
+    __shared__ unsigned s_warp[kSccT / 32 + 1];
+    unsigned target = 0, phase = 0;
+    // state i of this CTA
+    auto state_at = [&](uint32_t i) { return ((i >> 5) * ctas + cta) * 32u + (i & 31u); };
+    const uint32_t chunks = (g.N + 31) / 32;
+    const uint32_t own = (chunks / ctas + (cta < chunks % ctas ? 1u : 0u)) * 32u;
+    // keeps the states of the list with a nonzero colour; returns their count
+    auto compact = [&](uint32_t count, bool init) {
+        uint32_t kept = 0;
+        for (uint32_t i0 = 0; i0 < count; i0 += kSccT) {
+            const uint32_t i = i0 + tid;
+            uint32_t v = 0;
+            bool keep = false;
+            if (i < count) {
+                v = init ? state_at(i) : list[i];
+                keep = v < g.N && (init || __ldcg(g.color + v) != 0u);
+            }
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
+            if ((tid & 31) == 0) s_warp[tid >> 5] = __popc(m);
+            __syncthreads();
+            if (tid < 32) {
+                unsigned x = s_warp[tid], y = x;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned z = __shfl_up_sync(0xFFFFFFFFu, y, o);
+                    if ((int)tid >= o) y += z;
+                }
+                s_warp[tid] = y - x;
+                if (tid == 31) s_warp[32] = y;
+            }
+            __syncthreads();
+            if (keep) list[kept + s_warp[tid >> 5] + __popc(m & ((1u << (tid & 31)) - 1u))] = v;
+            kept += s_warp[32];
+            __syncthreads();
+        }
+        return kept;
+    };
+    // Runs pass(place) over the CTA's first `count` list places until a whole phase changes
+    // nothing: `passes` sweeps per phase while the states are few (a sweep is then shorter
+    // than a barrier).  `seeded`: this thread changed states that the passes read since the
+    // last barrier, which the first phase may not see everywhere.  False: failed.
+    auto fixpoint = [&](uint32_t count, unsigned passes, bool seeded, auto pass) -> bool {
+        bool ch = seeded;
+        for (int64_t used = 0;; ch = false) {
+            const unsigned p = (unsigned)min((int64_t)passes, max(g.budget - used, (int64_t)1));
+            for (unsigned k = 0; k < p; k++)
+                for (uint32_t i = tid; i < count; i += kSccT) ch |= pass(i);
+            used += p;
+            if (cta == 0 && tid == 0) st->changed[(phase + 1) % 3] = 0;
+            if (__syncthreads_or(ch) && tid == 0) st->changed[phase % 3] = 1;
+            if (!grid_barrier(st, target)) return false;
+            const unsigned any = *(volatile unsigned*)&st->changed[phase % 3];
+            phase++;
+            if (!any) return true;
+            if (used >= g.budget) {
+                if (tid == 0) atomicCAS(&st->status, 0, 1);
+                // every CTA sees the same flag and budget: all leave here
+                return false;
+            }
+        }
+    };
+    uint32_t count = compact(own, true);
+    for (uint32_t i = tid; i < count; i += kSccT) {
+        const uint32_t v = list[i];
+        g.color[v] = 1u;  // live
+        g.canon[v] = 0x7FFFFFFF;
+        g.level[v] = 1;
     }
-    if (m > c) {
-        color[v] = m;
-        flags[0] = 1;
-    }
-}
-
-__global__ void k_root_init(uint64_t N, const int32_t* __restrict__ lab, const int32_t* __restrict__ color,
-                            uint8_t* __restrict__ reached) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    reached[v] = (lab[v] < 0 && color[v] == (int32_t)v) ? 1 : 0;
-}
-
-// v reaches its colour's root through live successors of the same colour
-__global__ void k_reach_bw(uint64_t N, const uint32_t* __restrict__ F, const int32_t* __restrict__ lab,
-                           const int32_t* __restrict__ color, uint8_t* __restrict__ reached,
-                           unsigned long long* __restrict__ flags) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N || lab[v] >= 0 || reached[v]) return;
-    int32_t c = color[v];
-    uint32_t f = F[v];
-    while (f) {
-        int i = __ffs(f) - 1;
-        f &= f - 1;
-        uint64_t w = v ^ (1ull << i);
-        if (lab[w] < 0 && color[w] == c && reached[w]) {
-            reached[v] = 1;
-            flags[0] = 1;
+    if (!grid_barrier(st, target)) return;
+    uint32_t live = g.N;
+    unsigned round = 0;
+    bool seeded = false;
+    // a state without a live successor or without a live predecessor is its own SCC
+    auto trim = [&](uint32_t i) {
+        const uint32_t v = list[i];
+        if (__ldcg(g.color + v) == 0u) return false;
+        bool out = false, in = false;
+        auto alive = [](bool& hit) {
+            return [&hit](const uint32_t (&x)[8]) {
+                hit = (x[0] | x[1] | x[2] | x[3] | x[4] | x[5] | x[6] | x[7]) != 0u;
+                return hit;
+            };
+        };
+        for_neighbours(v, g.F[v], g.color, alive(out));
+        if (out) for_neighbours(v, g.G[v], g.color, alive(in));
+        if (in) return false;
+        g.lab[v] = (int32_t)priority_of(v, g.n);
+        __stcg(g.color + v, 0u);
+        return true;
+    };
+    for (;; round++) {
+        const unsigned passes = live > 2u * kSccT * ctas ? 1u : 4u;
+        if (!fixpoint(count, passes, seeded, trim)) return;
+        count = compact(count, false);
+        if (cta == 0 && tid == 0) st->live[(round + 1) % 3] = 0;
+        if (tid == 0 && count) atomicAdd(&st->live[round % 3], count);
+        for (uint32_t i = tid; i < count; i += kSccT) __stcg(g.color + list[i], priority_of(list[i], g.n) + 1u);
+        if (!grid_barrier(st, target)) return;
+        live = *(volatile unsigned*)&st->live[round % 3];
+        if (live == 0) break;
+        // largest priority among the live ancestors
+        if (!fixpoint(count, passes, false, [&](uint32_t i) {
+                const uint32_t v = list[i], c = __ldcg(g.color + v);
+                uint32_t m = c;
+                for_neighbours(v, g.G[v], g.color, [&](const uint32_t (&x)[8]) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) m = max(m, x[j]);
+                    return false;
+                });
+                if (m > c) __stcg(g.color + v, m);
+                return m > c;
+            }))
             return;
+        // backward from each colour's root (the state of that priority) within the colour
+        seeded = false;
+        for (uint32_t i = tid; i < count; i += kSccT) {
+            const uint32_t v = list[i], c = priority_of(v, g.n) + 1u;
+            if (__ldcg(g.color + v) == c) {
+                __stcg(g.color + v, c | kReached);
+                seeded = true;
+            }
+        }
+        if (!fixpoint(count, passes, seeded, [&](uint32_t i) {
+                const uint32_t v = list[i], c = __ldcg(g.color + v);
+                if (c & kReached) return false;
+                bool hit = false;
+                for_neighbours(v, g.F[v], g.color, [&](const uint32_t (&x)[8]) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) hit |= x[j] == (c | kReached);
+                    return hit;
+                });
+                if (hit) __stcg(g.color + v, c | kReached);
+                return hit;
+            }))
+            return;
+        seeded = false;
+        for (uint32_t i = tid; i < count; i += kSccT) {
+            const uint32_t v = list[i], c = __ldcg(g.color + v);
+            if (c & kReached) {
+                g.lab[v] = (int32_t)((c & ~kReached) - 1u);
+                __stcg(g.color + v, 0u);
+                seeded = true;
+            }
         }
     }
-}
-
-__global__ void k_assign(uint64_t N, int32_t* __restrict__ lab, const int32_t* __restrict__ color,
-                         const uint8_t* __restrict__ reached, unsigned long long* __restrict__ flags) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N || lab[v] >= 0 || !reached[v]) return;
-    lab[v] = color[v];
-    atomicAdd(&flags[1], 1ull);
-}
-
-__global__ void k_fill(uint64_t N, int32_t* __restrict__ a, int32_t val) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < N) a[v] = val;
-}
-
-__global__ void k_canon_min(uint64_t N, const int32_t* __restrict__ lab, int32_t* __restrict__ canon) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < N) atomicMin(&canon[lab[v]], (int32_t)v);
-}
-
-__global__ void k_canon_apply(uint64_t N, int32_t* __restrict__ lab, const int32_t* __restrict__ canon) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < N) lab[v] = canon[lab[v]];
-}
-
-// level per SCC stored at its label; 1 + max successor level
-__global__ void k_level(uint64_t N, const uint32_t* __restrict__ F, const int32_t* __restrict__ lab,
-                        int32_t* __restrict__ level, unsigned long long* __restrict__ flags) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    int32_t c = lab[v];
-    int32_t best = 0;
-    uint32_t f = F[v];
-    while (f) {
-        int i = __ffs(f) - 1;
-        f &= f - 1;
-        int32_t d = lab[v ^ (1ull << i)];
-        if (d != c) best = max(best, level[d]);
+    if (cta == 0 && tid == 0) {
+        st->rounds = round;
+        st->phases = phase;
     }
-    best += 1;
-    if (best > level[c]) {
-        atomicMax(&level[c], best);
-        flags[0] = 1;
+    // canonical labels: smallest state of each SCC
+    for (uint32_t i = tid; i < own; i += kSccT) {
+        const uint32_t v = state_at(i);
+        if (v < g.N) atomicMin(&g.canon[g.lab[v]], (int32_t)v);
     }
-}
-
-// sort key: terminal -> label; other -> (1, MAXLVL - level, MAXLBL - label)
-__global__ void k_keys(uint64_t N, const int32_t* __restrict__ lab, const int32_t* __restrict__ level,
-                       uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    int32_t c = lab[v];
-    int32_t l = level[c];
-    uint64_t k;
-    if (l == 1)
-        k = (uint64_t)c;
-    else
-        k = (1ull << 62) | ((uint64_t)(0x3FFFFFFF - l) << 31) | (uint64_t)(0x7FFFFFFF - c);
-    keys[v] = k;
-    vals[v] = (int32_t)v;
+    if (!grid_barrier(st, target)) return;
+    for (uint32_t i = tid; i < own; i += kSccT) {
+        const uint32_t v = state_at(i);
+        if (v < g.N) g.lab[v] = __ldcg(g.canon + g.lab[v]);
+    }
+    if (!grid_barrier(st, target)) return;
+    // levels, stored at the SCC's label: 1 + the largest level among successor SCCs.  The
+    // list takes each state's flips that leave its SCC, the colours a copy of its SCC's
+    // level, which neighbours read without going through the label.
+    for (uint32_t i = tid; i < own; i += kSccT) {
+        const uint32_t v = state_at(i);
+        uint32_t x = 0;
+        if (v < g.N) {
+            const int32_t c = g.lab[v];
+            for (uint32_t f = g.F[v]; f; f &= f - 1) {
+                const uint32_t bit = f & (0u - f);
+                if (__ldcg(g.lab + (v ^ bit)) != c) x |= bit;
+            }
+            __stcg(g.color + v, 1u);
+        }
+        list[i] = x;
+    }
+    if (!grid_barrier(st, target)) return;
+    if (!fixpoint(own, g.N > 2u * kSccT * ctas ? 1u : 4u, false, [&](uint32_t i) {
+            const uint32_t v = state_at(i);
+            if (v >= g.N) return false;
+            const int32_t c = g.lab[v];
+            const uint32_t l = (uint32_t)__ldcg(g.level + c);
+            bool ch = false;
+            if (l > __ldcg(g.color + v)) {
+                __stcg(g.color + v, l);
+                ch = true;
+            }
+            uint32_t best = 0;
+            for_neighbours(v, list[i], g.color, [&](const uint32_t (&x)[8]) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) best = max(best, x[j]);
+                return false;
+            });
+            if (best >= l && best > 0) {
+                atomicMax(&g.level[c], (int32_t)best + 1);
+                ch = true;
+            }
+            return ch;
+        }))
+        return;
+    // sort key: terminal -> label; other -> (1, MAXLVL - level, MAXLBL - label)
+    for (uint32_t i = tid; i < own; i += kSccT) {
+        const uint32_t v = state_at(i);
+        if (v >= g.N) continue;
+        const int32_t c = g.lab[v], l = __ldcg(g.level + c);
+        g.keys[v] = l == 1 ? (uint64_t)c
+                           : (1ull << 62) | ((uint64_t)(0x3FFFFFFF - l) << 31) | (uint64_t)(0x7FFFFFFF - c);
+        g.vals[v] = (int32_t)v;
+    }
 }
 
 __global__ void k_heads(uint64_t N, const uint64_t* __restrict__ keys, int32_t* __restrict__ pos_out,
@@ -227,40 +390,6 @@ __global__ void k_domain_masks(int n, uint64_t N, const uint32_t* __restrict__ F
     Gd[v] = gd;
 }
 
-struct Flags {
-    esl_ctx* ctx;
-    int64_t reads = 0;
-    int reset() {
-        ESL_CUDA(cudaMemsetAsync(ctx->d_flag.get(), 0, 8 * sizeof(unsigned long long), ctx->stream));
-        return ESL_OK;
-    }
-    int reset_changed() {
-        ESL_CUDA(cudaMemsetAsync(ctx->d_flag.get(), 0, sizeof(unsigned long long), ctx->stream));
-        return ESL_OK;
-    }
-    int read(unsigned long long* out, int count) {
-        reads++;
-        ESL_CUDA(cudaMemcpyAsync(ctx->h_flag, ctx->d_flag.get(), count * sizeof(unsigned long long),
-                                 cudaMemcpyDeviceToHost, ctx->stream));
-        ESL_CUDA(cudaStreamSynchronize(ctx->stream));
-        std::memcpy(out, ctx->h_flag, count * sizeof(unsigned long long));
-        return ESL_OK;
-    }
-};
-
-// Runs `sweep` until it reports no change; `per_check` sweeps per host check.
-template <class Sweep>
-int fixpoint(Flags& fl, Sweep sweep, int per_check, int64_t budget, const char* what) {
-    for (int64_t it = 0; it < budget; it += per_check) {
-        ESL_TRY(fl.reset_changed());
-        for (int k = 0; k < per_check; k++) ESL_TRY(sweep());
-        unsigned long long ch = 0;
-        ESL_TRY(fl.read(&ch, 1));
-        if (!ch) return ESL_OK;
-    }
-    return fail(ESL_ERR_TIMEOUT, std::string("fixpoint budget exceeded in ") + what);
-}
-
 }  // namespace
 
 int build_graph(esl_ctx* ctx, esl_net* net) {
@@ -270,108 +399,70 @@ int build_graph(esl_ctx* ctx, esl_net* net) {
     const unsigned nb = blocks_for(N);
     const uint32_t* F = net->F.get();
     const uint32_t* G = net->G.get();
-    Flags fl{ctx};
     const bool dbg = getenv("ESL_DEBUG") != nullptr;
     const auto t0 = std::chrono::steady_clock::now();
     auto ms_since = [&]() {
         return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     };
-    // budgets: a sweep can only fail to progress once per state (or the context's budget)
-    const int64_t budget = ctx->graph_sweeps > 0 ? ctx->graph_sweeps : (int64_t)N + 64;
-    // nominal algorithmic bytes of one fixpoint sweep (measurement hook): one pass over
-    // every state's mask, label and colour / level word, 4 B each.  States already
-    // assigned read only their label, so later sweeps move less than this.
-    const double sweep_bytes = 12.0 * (double)N;
-
     ESL_TRY(net->labels.alloc(N));
     int32_t* lab = net->labels.get();
-    DevBuf<int32_t> color, canon, level;
-    DevBuf<uint8_t> reached;
-    ESL_TRY(color.alloc(N));
-    ESL_TRY(reached.alloc(N));
-    ESL_COUNT_LAUNCH();
-    k_fill<<<nb, kThreads, 0, s>>>(N, lab, -1);
-    ESL_CUDA(cudaGetLastError());
-    ESL_TRY(fl.reset());
-
-    auto trim = [&]() -> int {
-        return fixpoint(fl, [&]() -> int {
-            ProfScope ps(ctx, "graph_sweep", sweep_bytes);
-            ESL_COUNT_LAUNCH();
-            k_trim<<<nb, kThreads, 0, s>>>(n, N, F, G, lab, ctx->d_flag.get());
-            ESL_CUDA(cudaGetLastError());
-            return ESL_OK;
-        }, 2, budget, "trim");
-    };
-    ESL_TRY(trim());
-    unsigned long long st[2];
-    ESL_TRY(fl.read(st, 2));
-    int64_t rounds = 0;
-    while (st[1] < N) {
-        if (++rounds > (int64_t)N) return fail(ESL_ERR_TIMEOUT, "SCC colouring rounds exceeded");
-        ESL_COUNT_LAUNCH();
-        k_color_init<<<nb, kThreads, 0, s>>>(N, lab, color.get(), reached.get());
-        ESL_CUDA(cudaGetLastError());
-        ESL_TRY(fixpoint(fl, [&]() -> int {
-            ProfScope ps(ctx, "graph_sweep", sweep_bytes);
-            ESL_COUNT_LAUNCH();
-            k_color_fw<<<nb, kThreads, 0, s>>>(N, G, lab, color.get(), ctx->d_flag.get());
-            ESL_CUDA(cudaGetLastError());
-            return ESL_OK;
-        }, 4, budget, "forward colouring"));
-        ESL_COUNT_LAUNCH();
-        k_root_init<<<nb, kThreads, 0, s>>>(N, lab, color.get(), reached.get());
-        ESL_CUDA(cudaGetLastError());
-        ESL_TRY(fixpoint(fl, [&]() -> int {
-            ProfScope ps(ctx, "graph_sweep", sweep_bytes);
-            ESL_COUNT_LAUNCH();
-            k_reach_bw<<<nb, kThreads, 0, s>>>(N, F, lab, color.get(), reached.get(), ctx->d_flag.get());
-            ESL_CUDA(cudaGetLastError());
-            return ESL_OK;
-        }, 4, budget, "backward reach"));
-        ESL_COUNT_LAUNCH();
-        k_assign<<<nb, kThreads, 0, s>>>(N, lab, color.get(), reached.get(), ctx->d_flag.get());
-        ESL_CUDA(cudaGetLastError());
-        ESL_TRY(trim());
-        ESL_TRY(fl.read(st, 2));
-    }
-    if (dbg) fprintf(stderr, "[esl-graph] SCC: %lld rounds, %lld flag reads, %.1f ms\n", (long long)rounds,
-                     (long long)fl.reads, ms_since());
-    // canonical labels: smallest state of each SCC
-    ESL_TRY(canon.alloc(N));
-    ESL_COUNT_LAUNCH();
-    k_fill<<<nb, kThreads, 0, s>>>(N, canon.get(), 0x7FFFFFFF);
-    ESL_COUNT_LAUNCH();
-    k_canon_min<<<nb, kThreads, 0, s>>>(N, lab, canon.get());
-    ESL_COUNT_LAUNCH();
-    k_canon_apply<<<nb, kThreads, 0, s>>>(N, lab, canon.get());
-    ESL_CUDA(cudaGetLastError());
-
-    // levels (indexed by label)
+    DevBuf<int32_t> level;
+    DevBuf<uint64_t> keys;
+    DevBuf<int32_t> vals;
     ESL_TRY(level.alloc(N));
-    ESL_COUNT_LAUNCH();
-    k_fill<<<nb, kThreads, 0, s>>>(N, level.get(), 0);
-    ESL_CUDA(cudaGetLastError());
-    ESL_TRY(fixpoint(fl, [&]() -> int {
-        ProfScope ps(ctx, "graph_sweep", sweep_bytes);
-        ESL_COUNT_LAUNCH();
-        k_level<<<nb, kThreads, 0, s>>>(N, F, lab, level.get(), ctx->d_flag.get());
-        ESL_CUDA(cudaGetLastError());
-        return ESL_OK;
-    }, 4, budget, "levels"));
+    ESL_TRY(keys.alloc(N));
+    ESL_TRY(vals.alloc(N));
+    {
+        DevBuf<uint32_t> color, list;
+        DevBuf<int32_t> canon;
+        DevBuf<GraphState> state;
+        ESL_TRY(color.alloc(N));
+        ESL_TRY(canon.alloc(N));
+        ESL_TRY(state.alloc(1));
+        GraphArgs ga{};
+        // one state per thread while that leaves SMs free: fewer CTAs, shorter barriers
+        const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)ctx->sm_count, (N + kSccT - 1) / kSccT);
+        ga.n = n;
+        ga.N = (uint32_t)N;
+        ga.F = F;
+        ga.G = G;
+        ga.lab = lab;
+        ga.color = color.get();
+        ga.canon = canon.get();
+        ga.level = level.get();
+        ga.cap = (uint32_t)(((N + 31) / 32 + grid - 1) / grid * 32);
+        ESL_TRY(list.alloc((size_t)ga.cap * grid));
+        ga.list = list.get();
+        ga.keys = keys.get();
+        ga.vals = vals.get();
+        // a pass can only fail to progress once per state (or the context's budget)
+        ga.budget = ctx->graph_sweeps > 0 ? ctx->graph_sweeps : (int64_t)N + 64;
+        ga.st = state.get();
+        ESL_CUDA(cudaMemsetAsync(state.get(), 0, sizeof(GraphState), s));
+        GraphState h{};
+        {
+            // nominal algorithmic bytes (measurement hook): masks, label, colour and level
+            // of every state once
+            ProfScope ps(ctx, "graph_sweep", 24.0 * (double)N);
+            void* args[] = {&ga};
+            ESL_COUNT_LAUNCH();
+            ESL_CUDA(cudaLaunchCooperativeKernel((const void*)k_scc, dim3(grid), dim3(kSccT), args, 0, s));
+        }
+        ESL_CUDA(cudaMemcpyAsync(&h, state.get(), sizeof h, cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaStreamSynchronize(s));
+        if (h.status == 1) return fail(ESL_ERR_TIMEOUT, "fixpoint budget exceeded in the SCC decomposition or the levels");
+        if (h.status) return fail(ESL_ERR_TIMEOUT, "a grid barrier of the SCC decomposition did not complete in time");
+        if (dbg)
+            fprintf(stderr, "[esl-graph] SCCs and levels: %u rounds, %u phases, %.1f ms\n", h.rounds, h.phases, ms_since());
+    }
 
     // ordering by a stable radix sort of (class, level, label) keys
     {
-        DevBuf<uint64_t> keys, keys_out;
-        DevBuf<int32_t> vals, pos;
+        DevBuf<uint64_t> keys_out;
+        DevBuf<int32_t> pos;
         DevBuf<uint8_t> head;
-        ESL_TRY(keys.alloc(N));
         ESL_TRY(keys_out.alloc(N));
-        ESL_TRY(vals.alloc(N));
         ESL_TRY(net->order.alloc(N));
-        ESL_COUNT_LAUNCH();
-        k_keys<<<nb, kThreads, 0, s>>>(N, lab, level.get(), keys.get(), vals.get());
-        ESL_CUDA(cudaGetLastError());
         size_t tmp_bytes = 0;
         ESL_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.get(), keys_out.get(), vals.get(),
                                                  net->order.get(), (int64_t)N, 0, 64, s));
@@ -436,7 +527,7 @@ int build_graph(esl_ctx* ctx, esl_net* net) {
     k_domain_masks<<<nb, kThreads, 0, s>>>(n, N, F, G, net->term_of.get(), net->Fdom.get(), net->Gdom.get());
     ESL_CUDA(cudaGetLastError());
     ESL_CUDA(cudaStreamSynchronize(s));
-    if (dbg) fprintf(stderr, "[esl-graph] done: %lld flag reads, %.1f ms\n", (long long)fl.reads, ms_since());
+    if (dbg) fprintf(stderr, "[esl-graph] done: %.1f ms\n", ms_since());
     return ESL_OK;
 }
 
