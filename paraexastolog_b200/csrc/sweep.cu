@@ -36,6 +36,7 @@
 #include <memory>
 #include <mutex>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include <cub/device/device_scan.cuh>
@@ -106,6 +107,14 @@ struct SweepPlan {
     // first odd slot, odd rows); an SCC's even and odd slots are one run each
     DevBuf<uint4> scc;
     std::vector<uint4> h_scc;
+    // Predecessors of the rows of SCCs solved by one CTA (k_sw_scc), by slices of 32 rows of
+    // one parity: scc_sl = an SCC's first even and first odd slice, sl = a slice's (lines,
+    // first line of ell).  Line j holds entries 4j .. 4j + 3 of each row, 16 bytes a row:
+    // local row of the other parity << 9 | rate index << 3, so that masked and shifted they
+    // are byte offsets (row * 8 after >> 6); past a row's last entry the local row is the
+    // other parity's row count.
+    DevBuf<uint2> scc_sl, sl;
+    DevBuf<uint4> ell;
     DevBuf<uint32_t> lsc_ne;             // local SCCs: number of even-parity slots (listed first)
     DevBuf<uint32_t> lsc_slots;          // local SCCs: slots, SCC by SCC
     // terminal plan: per slot, the state's position in the reordering
@@ -1253,40 +1262,47 @@ __global__ void __launch_bounds__(kSwT) k_sw_warm_scale(SwArgs a, const double* 
 // One CTA solves one SCC for KS systems (a power of two chosen per SCC) from right-hand
 // side to result: the two vectors the operator gathers (the search direction and its
 // even-row elimination) stay in shared memory, a thread's own rows in registers, and the
-// CTA stops with its own systems.  A Krylov iteration is bounded by its chain of barriers
-// and shared-memory gathers instead of L2 latency and launches.  Against the launch per
-// step (SCCs above 512 states) and the CTA-local solve on global vectors that it replaces:
-// n=12 x 64 rate sets 14.7 -> 2.8 ms, n=17 x 185 systems 64.6 -> 24.0 ms, one n=22 solve
-// 277 -> 71 ms.
+// CTA stops with its own systems.  A Krylov iteration is bounded by its chain of FP64
+// reductions, barriers and shared-memory gathers (3.9 us at 256 rows, 27 us at 4,096)
+// instead of L2 latency and launches.  Against the launch per step (SCCs above 512 states)
+// and the CTA-local solve on global vectors that it replaces: n=12 x 64 rate sets 14.7 ->
+// 1.5 ms, n=17 x 185 systems 64.6 -> 14.9 ms, one n=22 solve 277 -> 61 ms.
 //
-// A work item is (SCC, tile of KS systems); the SCCs of a launch are listed largest first
-// and cut into buckets of equal KS.  CTAs past the last item serve the group's singleton
-// SCCs (rows without in-group predecessors): z = b / q.
+// A work item is (SCC, tile of KS systems) and has a team of warps; a CTA holds several
+// teams of small SCCs, each with a barrier and a part of shared memory of its own, because
+// a group may have thousands of them beside one of 512 rows, whose CTAs fill an SM each.
+// The SCCs of a launch are listed largest first and cut into buckets of equal KS and team
+// size.  CTAs past the last item serve the group's singleton SCCs (rows without in-group
+// predecessors): z = b / q.
 constexpr int kSccMaxRows = 4096;  // most odd (or even) rows of an SCC solved by one CTA
-// threads of a CTA with one row per thread, and with several (whose registers hold more)
-constexpr int kSccThreads1 = 1024, kSccThreads = 512;
-__host__ __device__ constexpr int scc_threads(int NR) { return NR > 1 ? kSccThreads : kSccThreads1; }
-constexpr int kSccBuckets = 6;     // KS = 1, 2, 4, ..., 32
+// threads of a CTA with one row per thread (128 registers each), and with several
+constexpr int kSccThreads = 512, kSccThreadsBig = 1024;
+constexpr int kSccBuckets = 16;    // most (KS, team size) pairs of a launch
 constexpr size_t kSccMaxSmem = 227 * 1024;
 
 struct SccBucket {
-    uint32_t item0, scc0;  // first work item, first SCC (relative to SccArgs::scc)
-    int lks;               // log2 KS
+    uint32_t cta0, items;  // first CTA, work items
+    uint32_t scc0;         // first SCC (relative to SccArgs::scc)
+    uint32_t stride;       // doubles of shared memory per team
+    uint8_t lks, lteam;    // log2 KS, log2 threads of a team
+    uint8_t teams;         // teams per CTA
 };
 
 struct SccArgs {
     SwArgs a;
     const uint4* scc;  // the launch's SCCs: (first even slot, even rows, first odd slot, odd rows)
+    const uint2 *scc_sl, *sl;  // see SweepPlan
+    const uint4* ell;
     SccBucket b[kSccBuckets];
     int nb;
-    uint32_t items;    // CTAs before those of the singleton rows
+    uint32_t ctas;     // CTAs before those of the singleton rows
     const uint32_t *og_ptr, *og_ent;
     const double* x0;
     size_t x0_ld;
     const double* warm;  // K x N warm start by state, or null
     size_t warm_ld;
     double* Z;           // [slot][Kp]
-    double* BS;          // reduced right-hand sides, [odd row of the group][Kp]
+    double* own[5];      // BIG: group-sized scratch, odd rows x Kp each
     double tol2, accept2;
     int max_iters, max_outer, stall;
     unsigned long long* ratio;  // per system: max over SCCs of final |r|^2 / |b|^2 (bits of a double >= 0)
@@ -1298,48 +1314,64 @@ struct SccArgs {
     int TS;
 };
 
-__device__ __forceinline__ void scc_sync(int nact) { asm volatile("bar.sync 1, %0;" ::"r"(nact) : "memory"); }
-
-// sum over a row's entries of rate(entry) * X[entry row][system s], X and the rates in
-// shared memory as [row << lks | s]
-__device__ __forceinline__ double scc_gather(const uint32_t* __restrict__ ent, int cnt, const double* X,
-                                             const double* rate, int lks, int s, uint32_t base) {
-    double acc = 0.0;
-    int j = 0;
-    for (; j + 4 <= cnt; j += 4) {
-        uint32_t e[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) e[u] = __ldg(ent + j + u);
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-            acc += rate[(ent_rate(e[u]) << lks) | s] * X[((ent_slot(e[u]) - base) << lks) | s];
-    }
-    for (; j < cnt; j++) {
-        const uint32_t e = __ldg(ent + j);
-        acc += rate[(ent_rate(e) << lks) | s] * X[((ent_slot(e) - base) << lks) | s];
-    }
-    return acc;
+// a team's barrier: `threads` of the CTA, named by the team
+struct SccTeam {
+    int id, threads, tid;
+};
+__device__ __forceinline__ void scc_sync(const SccTeam& m) {
+    if (m.threads == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(m.id), "r"(m.threads) : "memory");
 }
 
-// Sums of NV values over the CTA's threads of one system; every thread of a system gets
+// The row gathers are bound by the instructions they issue (77% of issue slots at 18
+// instructions per entry when entries were loaded, tested and decoded one by one): four
+// entries come in one load, untested, already scaled to byte offsets, and shared memory is
+// addressed in 32 bits.
+__device__ __forceinline__ double lds_f64(uint32_t addr) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t shared_addr(const double* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// byte offsets of an entry's rate and gathered row in arrays of 1 << lks systems
+__device__ __forceinline__ uint32_t ell_rate(uint32_t e, int lks) { return (e & 0x1F8u) << lks; }
+__device__ __forceinline__ uint32_t ell_row(uint32_t e, int lks) { return (e >> 6 & ~7u) << lks; }
+// acc += sum over four entries of rate * X (shared addresses, this thread's system included)
+__device__ __forceinline__ void ell_add(double& acc, const uint4& e, uint32_t X, uint32_t rate, int lks) {
+    const double r0 = lds_f64(rate + ell_rate(e.x, lks)), x0 = lds_f64(X + ell_row(e.x, lks));
+    const double r1 = lds_f64(rate + ell_rate(e.y, lks)), x1 = lds_f64(X + ell_row(e.y, lks));
+    const double r2 = lds_f64(rate + ell_rate(e.z, lks)), x2 = lds_f64(X + ell_row(e.z, lks));
+    const double r3 = lds_f64(rate + ell_rate(e.w, lks)), x3 = lds_f64(X + ell_row(e.w, lks));
+    acc += r0 * x0;
+    acc += r1 * x1;
+    acc += r2 * x2;
+    acc += r3 * x3;
+}
+
+// Sums of NV values over a team's threads of one system; every thread of a system gets
 // the same bits.  `red` holds NV x warps x KS doubles; calls without a barrier in between
-// must use different buffers.
+// must use different buffers.  Both levels are butterflies, the values interleaved: each
+// thread adding up the warps' partial sums itself took 3,000 cycles a value at 32 warps,
+// two thirds of an iteration.
 template <int NV>
-__device__ __forceinline__ void scc_sum(double* red, int lks, int s, int nact, double (&v)[NV]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nact >> 5, KS = 1 << lks;
+__device__ __forceinline__ void scc_sum(double* red, int lks, const SccTeam& m, double (&v)[NV]) {
+    const int lane = m.tid & 31, warp = m.tid >> 5, KS = 1 << lks, total = (m.threads >> 5) << lks;
+    for (int o = 16; o >= KS; o >>= 1)
 #pragma unroll
-    for (int j = 0; j < NV; j++)
-        for (int o = 16; o >= KS; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+        for (int j = 0; j < NV; j++) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
     if (lane < KS)
 #pragma unroll
-        for (int j = 0; j < NV; j++) red[((j * nw + warp) << lks) | lane] = v[j];
-    scc_sync(nact);
+        for (int j = 0; j < NV; j++) red[j * total + (warp << lks) + lane] = v[j];
+    scc_sync(m);
+    // lane l takes the partial sums l, l + 32, ... of its system l % KS
 #pragma unroll
-    for (int j = 0; j < NV; j++) {
-        double acc = 0.0;
-        for (int w = 0; w < nw; w++) acc += red[((j * nw + w) << lks) | s];
-        v[j] = acc;
-    }
+    for (int j = 0; j < NV; j++) v[j] = lane < total ? red[j * total + lane] : 0.0;
+    for (int w = lane + 32; w < total; w += 32)
+#pragma unroll
+        for (int j = 0; j < NV; j++) v[j] += red[j * total + w];
+    for (int o = 16; o >= KS; o >>= 1)
+#pragma unroll
+        for (int j = 0; j < NV; j++) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
 }
 
 // out-rate sum of state v (out-mask f) for system s
@@ -1384,70 +1416,163 @@ __device__ __forceinline__ void scc_singles(const SccArgs& g, uint32_t cta, uint
     }
 }
 
-// A thread's own values of one vector (rows rs, rs + RS, ...): registers when a thread has
-// one row, else its own entries of a shared-memory array.
-template <int NR>
+// Own-row vectors of a thread.  One row per thread (BIG false): registers.  Else values of
+// an array, indexed [row << lks | s], that only this thread touches.
+template <bool BIG>
 struct SccVec {
     double reg;
-    double* sm;
-    __device__ __forceinline__ double get(int idx) const { return NR > 1 ? sm[idx] : reg; }
+    double* mem;
+    __device__ __forceinline__ double get(int idx) const { return BIG ? mem[idx] : reg; }
     __device__ __forceinline__ void set(int idx, double x) {
-        if (NR > 1) sm[idx] = x;
+        if (BIG) mem[idx] = x;
         else reg = x;
     }
 };
 
-// shared-memory doubles of an SCC's work item (see the carving in k_sw_scc)
-__host__ __device__ inline size_t scc_smem_doubles(int NR, int n, int se, int so, int lks, int nact) {
+// SCCs of at most kSccDense odd rows are solved by elimination: a Krylov iteration is a
+// chain of FP64 reductions, about 4 us however small the SCC, an elimination step one
+// barrier and a division (n=12 x 64 rate sets 1.93 -> 1.5 ms; at 32 rows the steps cost as
+// much as the iterations, n=22 67 -> 61 ms).  A budget of fewer iterations than rows is too
+// small for it.
+constexpr int kSccDense = 16;
+__host__ __device__ inline bool scc_dense(int so, int max_iters) { return so <= kSccDense && so <= max_iters; }
+__host__ __device__ inline int scc_dense_ld(int so) { return (so + 1) | 1; }
+
+// shared-memory doubles of a work item (see the carving in k_sw_scc)
+__host__ __device__ inline size_t scc_smem_doubles(bool big, bool dense, int n, int se, int so, int lks, int nact) {
     const size_t m = (size_t)(se > so ? se : so), KS = (size_t)1 << lks;
-    return (m + se + 2 * n + 6 * (size_t)(nact >> 5) + (NR > 1 ? 4 * (size_t)so + se : 0)) * KS;
+    return (m + 1 + se + 1 + 2 * n + 6 * (size_t)(nact >> 5) + (big ? 4 * (size_t)so + se : 0) +
+            (dense ? (size_t)so * scc_dense_ld(so) + 2 : 0)) *
+           KS;
 }
 
-// NR: most odd (or even) rows of a thread.  DEFL: the deflated operator of a terminal SCC
-// (see k_sw_defl_fin): S x + u gamma(x), u_o = q_o / s, whose gamma is summed at the
-// barrier that the elimination ends with anyway.
-template <int NR, bool DEFL>
-__global__ void __launch_bounds__(scc_threads(NR)) k_sw_scc(const __grid_constant__ SccArgs g) {
-    extern __shared__ double s_scc[];
+// BIG false: SCCs of at most kSccThreads rows of either parity, a thread per row and system,
+// everything but the gathered vectors in registers, the row's first entries included.
+// BIG true: several rows per thread; r, v, p, t and 1 / q in shared memory, r0, d, the
+// Schur diagonal, q and the right-hand side in memory (streamed, an item's own run).
+// DEFL: the deflated operator of a terminal SCC (see k_sw_defl_fin): S x + u gamma(x),
+// u_o = q_o / s, whose gamma is summed at the barrier that the elimination ends with anyway.
+template <bool BIG, bool DEFL>
+__global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_scc(const __grid_constant__ SccArgs g) {
+    extern __shared__ double s_all[];
     const SwArgs& a = g.a;
-    if (blockIdx.x >= g.items) {
-        if (!DEFL) scc_singles(g, blockIdx.x - g.items, gridDim.x - g.items);
+    if (blockIdx.x >= g.ctas) {
+        if (!DEFL) scc_singles(g, blockIdx.x - g.ctas, gridDim.x - g.ctas);
         return;
     }
     int bk = 0;
-    while (bk + 1 < g.nb && blockIdx.x >= g.b[bk + 1].item0) bk++;
-    const int lks = g.b[bk].lks, KS = 1 << lks;
-    const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), item = blockIdx.x - g.b[bk].item0;
-    const uint4 sc = g.scc[g.b[bk].scc0 + item / tiles];
+    while (bk + 1 < g.nb && blockIdx.x >= g.b[bk + 1].cta0) bk++;
+    const SccBucket& bu = g.b[bk];
+    const int lteam = BIG ? 10 : bu.lteam;
+    const SccTeam team = {BIG ? 0 : (int)(threadIdx.x >> lteam), 1 << lteam, (int)(threadIdx.x & ((1u << lteam) - 1u))};
+    const uint32_t item = BIG ? blockIdx.x - bu.cta0 : (blockIdx.x - bu.cta0) * bu.teams + team.id;
+    if (!BIG && (team.id >= bu.teams || item >= bu.items)) return;
+    double* s_scc = BIG ? s_all : s_all + (size_t)team.id * bu.stride;
+    const int lks = bu.lks, KS = 1 << lks;
+    const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), tile = item % tiles;
+    const uint4 sc = g.scc[bu.scc0 + item / tiles];
+    const uint2 first = g.scc_sl[bu.scc0 + item / tiles];
     const uint32_t ev0 = sc.x, od0 = sc.z;
     const int se = (int)sc.y, so = (int)sc.w, sm = max(se, so);
-    // threads past one per (row, system) pair leave; barriers count the others
-    const int nact = min((int)blockDim.x, (sm * KS + 31) & ~31);
-    if ((int)threadIdx.x >= nact) return;
-    const int s = threadIdx.x & (KS - 1), rs = threadIdx.x >> lks, RS = nact >> lks;
-    const int k = (int)(item % tiles) * KS + s;
+    const int nact = team.threads;
+    const int s = team.tid & (KS - 1), rs = team.tid >> lks, RS = nact >> lks;
+    const int k = (int)tile * KS + s;
     const size_t Kp = a.Kp;
     const bool act = k < a.K;
-    double* A = s_scc;                       // odd rows: the vector whose product is formed
-    double* W = A + ((size_t)sm << lks);     // even rows: its elimination
-    double* rate = W + ((size_t)se << lks);
+    // both with a zero row past the last, for the entries that a row of a slice lacks
+    double* A = s_scc;                           // odd rows: the vector whose product is formed
+    double* W = A + ((size_t)(sm + 1) << lks);   // even rows: its elimination
+    double* rate = W + ((size_t)(se + 1) << lks);
     double* red0 = rate + ((size_t)(2 * a.n) << lks);
     double* red1 = red0 + ((size_t)(2 * (nact >> 5)) << lks);
     double* red2 = red1 + ((size_t)(3 * (nact >> 5)) << lks);
-    SccVec<NR> R, V, P, T, IQ;
-    if constexpr (NR > 1) {
-        R.sm = red2 + ((size_t)(nact >> 5) << lks);
-        V.sm = R.sm + ((size_t)so << lks);
-        P.sm = V.sm + ((size_t)so << lks);
-        T.sm = P.sm + ((size_t)so << lks);
-        IQ.sm = T.sm + ((size_t)so << lks);
+    SccVec<BIG> R, V, P, T, IQ, R0, D, dS, q, BS;
+    if constexpr (BIG) {
+        R.mem = red2 + ((size_t)(nact >> 5) << lks);
+        V.mem = R.mem + ((size_t)so << lks);
+        P.mem = V.mem + ((size_t)so << lks);
+        T.mem = P.mem + ((size_t)so << lks);
+        IQ.mem = T.mem + ((size_t)so << lks);
+        // the SCC's so x Kp block of a group vector, tile by tile
+        const size_t o = (size_t)(od0 - a.beg - a.ne) * Kp + (size_t)tile * KS * so;
+        R0.mem = g.own[0] + o;
+        D.mem = g.own[1] + o;
+        dS.mem = g.own[2] + o;
+        q.mem = g.own[3] + o;
+        BS.mem = g.own[4] + o;
     }
-    double R0[NR], D[NR], dS[NR], q[NR];
-    uint32_t po[NR], pe[NR];  // own rows' entries: offset from the SCC's first, << 5 | count
-    for (int idx = threadIdx.x; idx < (2 * a.n) << lks; idx += nact)
-        rate[idx] = a.rateT[(size_t)(idx >> lks) * Kp + (size_t)(item % tiles) * KS + (idx & (KS - 1))];
-    const uint32_t pe0 = a.desc[ev0].z, po0 = a.desc[od0].z;
-    const uint32_t *ent_e = a.ig_ent + pe0, *ent_o = a.ig_ent + po0;
+    // one row per thread: its first two lines stay in registers
+    uint4 ee[2], eo[2];
+    uint2 le = make_uint2(0u, 0u), lo = make_uint2(0u, 0u);
+    if (!BIG) {
+        if (rs < se) le = __ldg(g.sl + first.x + (rs >> 5));
+        if (rs < so) lo = __ldg(g.sl + first.y + (rs >> 5));
+        for (int j = 0; j < 2; j++) {
+            if (j < (int)le.x) ee[j] = __ldg(g.ell + (size_t)(le.y + j) * 32 + (rs & 31));
+            if (j < (int)lo.x) eo[j] = __ldg(g.ell + (size_t)(lo.y + j) * 32 + (rs & 31));
+        }
+    }
+    const uint32_t rate_at = shared_addr(rate + s);
+    // fn(row, index) of the own rows below count
+    auto each = [&](int count, auto fn) {
+        if constexpr (BIG) {
+            for (int r = rs; r < count; r += RS) fn(r, (r << lks) | s);
+        } else if (rs < count) {
+            fn(rs, (rs << lks) | s);
+        }
+    };
+    // fn(row, index, sum over its entries of X) of the own even or odd rows; with several,
+    // the next line, of the same row or the next one, is in flight while one is summed
+    auto gather = [&](auto even, const double* X, auto fn) {
+        constexpr bool EVEN = decltype(even)::value;
+        const int count = EVEN ? se : so;
+        const uint32_t xs = shared_addr(X + s);
+        if constexpr (BIG) {
+            if (rs >= count) return;
+            const uint2* sl = g.sl + (EVEN ? first.x : first.y);
+            const uint2 none = make_uint2(0u, 0u);
+            uint2 cur = __ldg(sl + (rs >> 5)), nxt = rs + RS < count ? __ldg(sl + ((rs + RS) >> 5)) : none;
+            const uint4* line = g.ell + (size_t)cur.y * 32 + (rs & 31);
+            uint4 e = cur.x ? __ldg(line) : make_uint4(0u, 0u, 0u, 0u);
+            for (int r = rs; r < count; r += RS) {
+                const uint4* line2 = g.ell + (size_t)nxt.y * 32 + ((r + RS) & 31);
+                const uint32_t next_lines = nxt.x;
+                uint32_t left = cur.x;
+                double acc = 0.0;
+                uint4 f = e;
+                while (left > 1) {
+                    line += 32;
+                    f = __ldg(line);
+                    ell_add(acc, e, xs, rate_at, lks);
+                    e = f;
+                    left--;
+                }
+                if (next_lines) f = __ldg(line2);
+                cur = nxt;
+                nxt = r + 2 * RS < count ? __ldg(sl + ((r + 2 * RS) >> 5)) : none;
+                if (left) ell_add(acc, e, xs, rate_at, lks);
+                e = f;
+                line = line2;
+                fn(r, (r << lks) | s, acc);
+            }
+        } else if (rs < count) {
+            const uint2 l = EVEN ? le : lo;
+            double acc = 0.0;
+            if (l.x > 0) ell_add(acc, EVEN ? ee[0] : eo[0], xs, rate_at, lks);
+            if (l.x > 1) ell_add(acc, EVEN ? ee[1] : eo[1], xs, rate_at, lks);
+            for (uint32_t j = 2; j < l.x; j++)
+                ell_add(acc, __ldg(g.ell + (size_t)(l.y + j) * 32 + (rs & 31)), xs, rate_at, lks);
+            fn(rs, (rs << lks) | s, acc);
+        }
+    };
+    constexpr auto even_rows = std::true_type{};
+    constexpr auto odd_rows = std::false_type{};
+    for (int idx = team.tid; idx < (2 * a.n) << lks; idx += nact)
+        rate[idx] = a.rateT[(size_t)(idx >> lks) * Kp + (size_t)tile * KS + (idx & (KS - 1))];
+    if (rs == 0) {
+        A[(se << lks) | s] = 0.0;
+        W[(se << lks) | s] = 0.0;
+    }
     const double inv_s = 1.0 / (double)(se + so);
     auto rhs = [&](uint32_t slot, uint32_t v) {
         double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + v];
@@ -1458,147 +1583,162 @@ __global__ void __launch_bounds__(scc_threads(NR)) k_sw_scc(const __grid_constan
         }
         return acc;
     };
-    scc_sync(nact);
+    scc_sync(team);
     // even rows: 1 / q (in A too, for the Schur diagonal), and b / q, kept in Z until the end
-#pragma unroll
-    for (int i = 0; i < NR; i++) {
-        const int r = rs + i * RS, idx = (r << lks) | s;
-        pe[i] = 0;
-        if (r < se) {
-            const uint32_t slot = ev0 + r;
-            const uint4 d = a.desc[slot];
-            pe[i] = (d.z - pe0) << 5 | d.w;
-            const double iq = 1.0 / scc_q(rate, d.x, d.y, lks, s);
-            IQ.set(idx, iq);
-            A[idx] = iq;
-            double w = 0.0;
-            if (!DEFL && act) {
-                w = rhs(slot, d.x) * iq;
-                g.Z[(size_t)slot * Kp + k] = w;
-            }
-            W[idx] = w;
+    each(se, [&](int r, int idx) {
+        const uint32_t slot = ev0 + r;
+        const uint2 d = a.rows[slot];
+        const double iq = 1.0 / scc_q(rate, d.x, d.y, lks, s);
+        IQ.set(idx, iq);
+        A[idx] = iq;
+        double w = 0.0;
+        if (!DEFL && act) {
+            w = rhs(slot, d.x) * iq;
+            g.Z[(size_t)slot * Kp + k] = w;
         }
-    }
-    scc_sync(nact);
+        W[idx] = w;
+    });
+    scc_sync(team);
     // odd rows: q, Schur diagonal, reduced right-hand side, starting iterate
     double sum1[1] = {0.0};
+    gather(odd_rows, W, [&](int r, int idx, double inflow) {
+        const uint32_t slot = od0 + r;
+        const uint2 d = a.rows[slot];
+        const double qv = scc_q(rate, d.x, d.y, lks, s);
+        double dv = qv;
+        const uint2 sl = __ldg(g.sl + first.y + (r >> 5));
+        for (uint32_t j = 0; j < 4 * sl.x; j++) {
+            const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(g.ell + (size_t)(sl.y + j / 4) * 32 + (r & 31)) + j % 4);
+            const uint32_t ri = e >> 3 & 63u;
+            // rate(e -> o) is the entry's; rate(o -> e) flips the same bit the other way
+            if ((d.y >> (ri >> 1)) & 1u)
+                dv -= rate[(ri << lks) | s] * rate[((ri ^ 1u) << lks) | s] * A[((e >> 9) << lks) | s];
+        }
+        q.set(idx, qv);
+        dS.set(idx, dv);
+        const double b = DEFL ? qv * inv_s : (act ? rhs(slot, d.x) : 0.0) + inflow;
+        sum1[0] += b * b;
+        R.set(idx, b);
+        BS.set(idx, b);
+        if (act) g.Z[(size_t)slot * Kp + k] = !DEFL && g.warm ? g.warm[(size_t)k * g.warm_ld + d.x] : 0.0;
+    });
+    const bool dense = !BIG && !DEFL && scc_dense(so, g.max_iters);
+    const int ld = scc_dense_ld(so);
+    double* M = red2 + ((size_t)(nact >> 5) << lks);  // [row][column], the right-hand side last
+    double* pivot = M + ((size_t)(so * ld) << lks);   // 1 / pivot of this and the next step
+    auto at = [&](int r, int c) -> double& { return M[((r * ld + c) << lks) | s]; };
+    if (!BIG && dense && rs < so) {
+        // own row of the Schur complement: q_o - sum over e of rate(e -> o) / q_e rate(o' -> e)
+        for (int c = 0; c < so; c++) at(rs, c) = 0.0;
+        at(rs, rs) = q.get(0);
+        at(rs, so) = R.get(0);
+        for (uint32_t j = 0; j < lo.x; j++) {
+            const uint4 e4 = __ldg(g.ell + (size_t)(lo.y + j) * 32 + (rs & 31));
+            const uint32_t es[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
-    for (int i = 0; i < NR; i++) {
-        const int r = rs + i * RS, idx = (r << lks) | s;
-        po[i] = 0;
-        if (r < so) {
-            const uint32_t slot = od0 + r;
-            const uint4 d = a.desc[slot];
-            po[i] = (d.z - po0) << 5 | d.w;
-            const double qv = scc_q(rate, d.x, d.y, lks, s);
-            double dv = qv;
-            for (uint32_t j = 0; j < d.w; j++) {
-                const uint32_t e = __ldg(a.ig_ent + d.z + j);
-                const int ri = ent_rate(e);
-                // rate(e -> o) is the entry's; rate(o -> e) flips the same bit the other way
-                if ((d.y >> (ri >> 1)) & 1u)
-                    dv -= rate[(ri << lks) | s] * rate[((ri ^ 1) << lks) | s] * A[((ent_slot(e) - ev0) << lks) | s];
-            }
-            q[i] = qv;
-            dS[i] = dv;
-            double b;
-            if (DEFL) {
-                b = qv * inv_s;
-            } else {
-                b = act ? rhs(slot, d.x) : 0.0;
-                b += scc_gather(a.ig_ent + d.z, (int)d.w, W, rate, lks, s, ev0);
-            }
-            sum1[0] += b * b;
-            R.set(idx, b);
-            if (act) {
-                g.BS[(size_t)(slot - a.beg - a.ne) * Kp + k] = b;
-                g.Z[(size_t)slot * Kp + k] = !DEFL && g.warm ? g.warm[(size_t)k * g.warm_ld + d.x] : 0.0;
+            for (int u = 0; u < 4; u++) {
+                const uint32_t er = es[u] >> 9;
+                if ((int)er == se) break;
+                const double w = rate[((es[u] >> 3 & 63u) << lks) | s] * A[(er << lks) | s];
+                const uint2 sl = __ldg(g.sl + first.x + (er >> 5));
+                for (uint32_t i = 0; i < sl.x; i++) {
+                    const uint4 f4 = __ldg(g.ell + (size_t)(sl.y + i) * 32 + (er & 31));
+                    const uint32_t fs[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                    for (int x = 0; x < 4; x++)
+                        if ((int)(fs[x] >> 9) != so)
+                            at(rs, (int)(fs[x] >> 9)) -= w * rate[((fs[x] >> 3 & 63u) << lks) | s];
+                }
             }
         }
+        if (rs == 0) pivot[s] = 1.0 / at(0, 0);
     }
-    scc_sum<1>(red1, lks, s, nact, sum1);
+    scc_sum<1>(red1, lks, team, sum1);
     const double b2 = sum1[0];
+    if (rs == 0) A[(so << lks) | s] = 0.0;  // 1 / q of an even row until here
+    if (!BIG && dense) {
+        // Gauss-Jordan without pivoting (the rows of an M-matrix, diagonally dominant by
+        // columns); the true residual below decides whether it is good enough
+        for (int j = 0; j < so; j++) {
+            if (rs < so && rs != j) {
+                const double f = at(rs, j) * pivot[((j & 1) << lks) | s];
+#pragma unroll 4
+                for (int c = j + 1; c <= so; c++) at(rs, c) -= f * at(j, c);
+                if (rs == j + 1) pivot[(((j + 1) & 1) << lks) | s] = 1.0 / at(rs, rs);
+            }
+            scc_sync(team);
+        }
+        if (rs < so && act) g.Z[(size_t)(od0 + rs) * Kp + k] = at(rs, so) / at(rs, rs);
+    }
     double gamma = 0.0;
     // W = elimination of A (and gamma(A)), with the barrier after it
     auto elim = [&]() {
         double gm[1] = {0.0};
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS, idx = (r << lks) | s;
-            if (r < se) {
-                const double w =
-                    scc_gather(ent_e + (pe[i] >> 5), (int)(pe[i] & 31u), A, rate, lks, s, od0) * IQ.get(idx);
-                W[idx] = w;
-                if (DEFL) gm[0] += w;
-            }
-            if (DEFL && r < so) gm[0] += A[idx];
-        }
+        gather(even_rows, A, [&](int, int idx, double sum) {
+            const double w = sum * IQ.get(idx);
+            W[idx] = w;
+            if (DEFL) gm[0] += w;
+        });
         if (DEFL) {
-            scc_sum<1>(red2, lks, s, nact, gm);
+            each(so, [&](int, int idx) { gm[0] += A[idx]; });
+            scc_sum<1>(red2, lks, team, gm);
             gamma = gm[0];
         } else {
-            scc_sync(nact);
+            scc_sync(team);
         }
     };
-    // own odd row's value of the operator applied to A
-    auto apply = [&](int i, int idx) {
-        double y = q[i] * A[idx] - scc_gather(ent_o + (po[i] >> 5), (int)(po[i] & 31u), W, rate, lks, s, ev0);
-        if (DEFL) y += gamma * (q[i] * inv_s);
-        return y;
+    // fn(index, own odd row's value of the operator applied to A)
+    auto apply = [&](auto fn) {
+        gather(odd_rows, W, [&](int, int idx, double sum) {
+            const double qv = q.get(idx);
+            double y = qv * A[idx] - sum;
+            if (DEFL) y += gamma * (qv * inv_s);
+            fn(idx, y);
+        });
     };
     auto load_x = [&]() {
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS;
-            if (r < so) A[(r << lks) | s] = act ? g.Z[(size_t)(od0 + r) * Kp + k] : 0.0;
-        }
-        scc_sync(nact);
+        each(so, [&](int r, int idx) { A[idx] = act ? g.Z[(size_t)(od0 + r) * Kp + k] : 0.0; });
+        scc_sync(team);
     };
     bool done = !act || !(b2 > 0.0), failed = false;
-    const bool warm = !DEFL && g.warm != nullptr;
+    const bool warm = !DEFL && !dense && g.warm != nullptr;
     if (warm) {
         // least-squares multiple (S x . b) / (S x . S x) of the warm start: its residual is
         // never larger than that of a zero start
         load_x();
         elim();
         double v[2] = {0.0, 0.0};
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS, idx = (r << lks) | s;
-            if (r < so) {
-                const double y = apply(i, idx);
-                v[0] += y * R.get(idx);
-                v[1] += y * y;
-            }
-        }
-        scc_sum<2>(red0, lks, s, nact, v);
+        apply([&](int idx, double y) {
+            v[0] += y * BS.get(idx);
+            v[1] += y * y;
+        });
+        scc_sum<2>(red0, lks, team, v);
         const double al = v[1] > 0.0 ? v[0] / v[1] : 0.0;
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS;
-            if (r < so && act) g.Z[(size_t)(od0 + r) * Kp + k] *= al;
-        }
+        if (act) each(so, [&](int r, int) { g.Z[(size_t)(od0 + r) * Kp + k] *= al; });
     }
     double prev = 0.0, rr = b2;
     int noimp = 0, its = 0;
     for (int outer = 0;; outer++) {
-        if (outer > 0 || warm) {
+        if (outer > 0 || warm || dense) {
             // true residual r = b - S x
             load_x();
             elim();
             double v[1] = {0.0};
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-                const int r = rs + i * RS, idx = (r << lks) | s;
-                if (r < so) {
-                    const double b = act ? g.BS[(size_t)(od0 + r - a.beg - a.ne) * Kp + k] : 0.0;
-                    const double res = b - apply(i, idx);
-                    R.set(idx, res);
-                    v[0] += res * res;
-                }
-            }
-            scc_sum<1>(red1, lks, s, nact, v);
+            apply([&](int idx, double y) {
+                const double res = BS.get(idx) - y;
+                R.set(idx, res);
+                v[0] += res * res;
+            });
+            scc_sum<1>(red1, lks, team, v);
             rr = v[0];
+            if (dense && outer == 0 && !done && !(rr < b2)) {
+                // a zero start is better (a singular block, overflow)
+                each(so, [&](int r, int idx) {
+                    g.Z[(size_t)(od0 + r) * Kp + k] = 0.0;
+                    R.set(idx, BS.get(idx));
+                });
+                rr = b2;
+            }
         }
         if (!done) {
             if (rr <= g.tol2 * b2) {
@@ -1616,6 +1756,7 @@ __global__ void __launch_bounds__(scc_threads(NR)) k_sw_scc(const __grid_constan
                 }
             }
         }
+        // every warp holds every system of the CTA, and its sums are the same everywhere
         if (!__any_sync(0xffffffffu, !done)) break;
         prev = rr;
         const bool started = !done;
@@ -1624,73 +1765,51 @@ __global__ void __launch_bounds__(scc_threads(NR)) k_sw_scc(const __grid_constan
         const double target = fmax(1e-26, 0.01 * g.tol2 * b2 * scale * scale);
         // BiCGStab on the residual scaled to unit norm, right preconditioner dS; the next
         // search direction needs no barrier of its own: beta = -(r0 . t) / (r0 . v)
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS, idx = (r << lks) | s;
-            if (r < so) {
-                const double x = R.get(idx) * scale;
-                R.set(idx, x);
-                R0[i] = x;
-                D[i] = 0.0;
-                A[idx] = x / dS[i];
-            }
-        }
-        scc_sync(nact);
+        each(so, [&](int, int idx) {
+            const double x = R.get(idx) * scale;
+            R.set(idx, x);
+            R0.set(idx, x);
+            D.set(idx, 0.0);
+            A[idx] = x / dS.get(idx);
+        });
+        scc_sync(team);
         double rho = 1.0, best = 1.0;
         int it = 0, stall = 0;
         while (__any_sync(0xffffffffu, run)) {
             elim();
             double v1[1] = {0.0};
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-                const int r = rs + i * RS, idx = (r << lks) | s;
-                if (r < so) {
-                    const double y = apply(i, idx);
-                    V.set(idx, y);
-                    v1[0] += R0[i] * y;
-                }
-            }
-            scc_sum<1>(red0, lks, s, nact, v1);
+            apply([&](int idx, double y) {
+                V.set(idx, y);
+                v1[0] += R0.get(idx) * y;
+            });
+            scc_sum<1>(red0, lks, team, v1);
             const double r0v = v1[0], alpha = r0v != 0.0 ? rho / r0v : 0.0;
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-                const int r = rs + i * RS, idx = (r << lks) | s;
-                if (r < so) {
-                    P.set(idx, A[idx]);
-                    A[idx] = (R.get(idx) - alpha * V.get(idx)) / dS[i];
-                }
-            }
-            scc_sync(nact);
+            each(so, [&](int, int idx) {
+                P.set(idx, A[idx]);
+                A[idx] = (R.get(idx) - alpha * V.get(idx)) / dS.get(idx);
+            });
+            scc_sync(team);
             elim();
             double v3[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-                const int r = rs + i * RS, idx = (r << lks) | s;
-                if (r < so) {
-                    const double y = apply(i, idx);
-                    T.set(idx, y);
-                    v3[0] += y * (dS[i] * A[idx]);
-                    v3[1] += y * y;
-                    v3[2] += R0[i] * y;
-                }
-            }
-            scc_sum<3>(red1, lks, s, nact, v3);
+            apply([&](int idx, double y) {
+                T.set(idx, y);
+                v3[0] += y * (dS.get(idx) * A[idx]);
+                v3[1] += y * y;
+                v3[2] += R0.get(idx) * y;
+            });
+            scc_sum<3>(red1, lks, team, v3);
             const double omega = v3[1] > 0.0 ? v3[0] / v3[1] : 0.0, beta = r0v != 0.0 ? -v3[2] / r0v : 0.0;
             double v2[2] = {0.0, 0.0};
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-                const int r = rs + i * RS, idx = (r << lks) | s;
-                if (r < so) {
-                    const double sh = A[idx], ph = P.get(idx), d = dS[i];
-                    if (run) D[i] += alpha * ph + omega * sh;
-                    const double rv = d * sh - omega * T.get(idx);
-                    R.set(idx, rv);
-                    v2[0] += rv * rv;
-                    v2[1] += R0[i] * rv;
-                    A[idx] = (rv + beta * (d * ph - omega * V.get(idx))) / d;
-                }
-            }
-            scc_sum<2>(red0, lks, s, nact, v2);
+            each(so, [&](int, int idx) {
+                const double sh = A[idx], ph = P.get(idx), d = dS.get(idx);
+                if (run) D.set(idx, D.get(idx) + (alpha * ph + omega * sh));
+                const double rv = d * sh - omega * T.get(idx);
+                R.set(idx, rv);
+                v2[0] += rv * rv;
+                v2[1] += R0.get(idx) * rv;
+                A[idx] = (rv + beta * (d * ph - omega * V.get(idx))) / d;
+            });
+            scc_sum<2>(red0, lks, team, v2);
             if (run) {
                 it++;
                 if (v2[0] < 0.5 * best) {
@@ -1705,37 +1824,27 @@ __global__ void __launch_bounds__(scc_threads(NR)) k_sw_scc(const __grid_constan
             }
         }
         its += it;
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS;
-            if (r < so && started) g.Z[(size_t)(od0 + r) * Kp + k] += nrm * D[i];
-        }
+        if (started) each(so, [&](int r, int idx) { g.Z[(size_t)(od0 + r) * Kp + k] += nrm * D.get(idx); });
     }
     // even rows from the odd solution
     load_x();
     double total[1] = {0.0};
-#pragma unroll
-    for (int i = 0; i < NR; i++) {
-        const int r = rs + i * RS, idx = (r << lks) | s;
-        if (r < se) {
-            const double w = scc_gather(ent_e + (pe[i] >> 5), (int)(pe[i] & 31u), A, rate, lks, s, od0) * IQ.get(idx);
-            if (DEFL) {
-                W[idx] = w;
-                total[0] += w;
-            } else if (act) {
-                g.Z[(size_t)(ev0 + r) * Kp + k] += w;
-            }
+    gather(even_rows, A, [&](int r, int idx, double sum) {
+        const double w = sum * IQ.get(idx);
+        if (DEFL) {
+            W[idx] = w;
+            total[0] += w;
+        } else if (act) {
+            g.Z[(size_t)(ev0 + r) * Kp + k] += w;
         }
-        if (DEFL && r < so) total[0] += A[idx];
-    }
+    });
     if (DEFL) {
-        scc_sum<1>(red1, lks, s, nact, total);
+        each(so, [&](int, int idx) { total[0] += A[idx]; });
+        scc_sum<1>(red1, lks, team, total);
         const double inv = total[0] != 0.0 ? 1.0 / total[0] : 0.0;
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            const int r = rs + i * RS, idx = (r << lks) | s;
-            if (act && r < se) g.Rb[(size_t)k * g.TS + g.pos[ev0 + r]] = W[idx] * inv;
-            if (act && r < so) g.Rb[(size_t)k * g.TS + g.pos[od0 + r]] = A[idx] * inv;
+        if (act) {
+            each(se, [&](int r, int idx) { g.Rb[(size_t)k * g.TS + g.pos[ev0 + r]] = W[idx] * inv; });
+            each(so, [&](int r, int idx) { g.Rb[(size_t)k * g.TS + g.pos[od0 + r]] = A[idx] * inv; });
         }
     }
     if (act && rs == 0) {
@@ -2527,6 +2636,54 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
 // Most rows of one parity of an SCC
 inline uint32_t scc_rows(const uint4& c) { return std::max(c.y, c.w); }
 
+// Slices of SCC j (see SweepPlan::sl): source[slice] = (first slot, rows, first slot of the
+// other parity, rows of the other parity)
+__global__ void k_pl_slices(uint32_t count, const uint4* __restrict__ scc, const uint2* __restrict__ scc_sl,
+                            uint4* __restrict__ source) {
+    const uint32_t j = blockIdx.x;
+    if (j >= count) return;
+    const uint4 c = scc[j];
+    const uint2 f = scc_sl[j];
+    if (f.x == kNoSlot) return;  // not solved by one CTA
+    for (uint32_t r = threadIdx.x * 32; r < c.y; r += blockDim.x * 32)
+        source[f.x + r / 32] = make_uint4(c.x + r, min(32u, c.y - r), c.z, c.w);
+    for (uint32_t r = threadIdx.x * 32; r < c.w; r += blockDim.x * 32)
+        source[f.y + r / 32] = make_uint4(c.z + r, min(32u, c.w - r), c.x, c.y);
+}
+
+// One warp per slice.  FILL false: its line count (four entries a line, the most of a row);
+// true: the lines.
+template <bool FILL>
+__global__ void k_pl_ell(uint32_t slices, const uint4* __restrict__ source, const uint32_t* __restrict__ ig_ptr,
+                         const uint32_t* __restrict__ ig_ent, uint32_t* __restrict__ width,
+                         const uint32_t* __restrict__ off, uint2* __restrict__ sl, uint4* __restrict__ ell) {
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= slices) return;
+    const uint4 src = source[w];
+    const bool row = lane < src.y;
+    const uint32_t p = row ? ig_ptr[src.x + lane] : 0u;
+    const uint32_t cnt = row ? ig_ptr[src.x + lane + 1] - p : 0u;
+    if (!FILL) {
+        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, cnt);
+        if (lane == 0) width[w] = (most + 3) / 4;
+        return;
+    }
+    const uint32_t lines = width[w];
+    if (lane == 0) sl[w] = make_uint2(lines, off[w]);
+    for (uint32_t j = 0; j < lines; j++) {
+        uint32_t e[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            e[u] = src.w << 9;
+            if (4 * j + u < cnt) {
+                const uint32_t x = ig_ent[p + 4 * j + u];
+                e[u] = (ent_slot(x) - src.z) << 9 | (uint32_t)ent_rate(x) << 3;
+            }
+        }
+        ell[((size_t)off[w] + j) * 32 + lane] = make_uint4(e[0], e[1], e[2], e[3]);
+    }
+}
+
 // Sorts each group's SCC list by decreasing size (the launch order of k_sw_scc: a group
 // lasts as long as the CTA of its largest SCC, which must not start behind the small ones)
 // and marks the groups whose SCCs all fit a CTA.
@@ -2540,17 +2697,55 @@ int finish_scc_list(esl_ctx* ctx, int n, SweepPlan* P) {
             g.singles -= c->y + c->w;
             const uint32_t m = scc_rows(*c);
             g.resident = g.resident && m <= (uint32_t)kSccMaxRows &&
-                         scc_smem_doubles(m > kSccThreads1 ? 2 : 1, n, (int)c->y, (int)c->w, 0,
-                                          (int)std::min<uint32_t>(kSccThreads1, (m + 31) & ~31u)) *
+                         scc_smem_doubles(m > kSccThreads, false, n, (int)c->y, (int)c->w, 0,
+                                          (int)std::min<uint32_t>(kSccThreadsBig, (m + 31) & ~31u)) *
                                  8 <=
                              kSccMaxSmem;
         }
     }
     if (P->h_scc.empty()) return ESL_OK;
-    if (!P->scc.get()) ESL_TRY(P->scc.alloc(P->h_scc.size()));
-    ESL_CUDA(cudaMemcpyAsync(P->scc.get(), P->h_scc.data(), P->h_scc.size() * sizeof(uint4), cudaMemcpyHostToDevice,
-                             ctx->stream));
-    ESL_CUDA(cudaStreamSynchronize(ctx->stream));
+    cudaStream_t s = ctx->stream;
+    const uint32_t count = (uint32_t)P->h_scc.size();
+    std::vector<uint2> first(count, make_uint2(kNoSlot, kNoSlot));
+    uint32_t slices = 0;
+    for (const SwGroup& g : P->groups)
+        for (uint32_t j = g.s0; g.resident && j < g.s0 + g.ns; j++) {
+            first[j].x = slices;
+            slices += (P->h_scc[j].y + 31) / 32;
+            first[j].y = slices;
+            slices += (P->h_scc[j].w + 31) / 32;
+        }
+    if (!P->scc.get()) ESL_TRY(P->scc.alloc(count));
+    ESL_TRY(P->scc_sl.alloc(count));
+    ESL_CUDA(cudaMemcpyAsync(P->scc.get(), P->h_scc.data(), (size_t)count * sizeof(uint4), cudaMemcpyHostToDevice, s));
+    ESL_CUDA(cudaMemcpyAsync(P->scc_sl.get(), first.data(), (size_t)count * sizeof(uint2), cudaMemcpyHostToDevice, s));
+    DevBuf<uint4> source;
+    DevBuf<uint32_t> width, off;
+    DevBuf<uint8_t> tmp;
+    ESL_TRY(source.alloc(std::max(slices, 1u)));
+    ESL_TRY(width.alloc((size_t)slices + 1));
+    ESL_TRY(off.alloc((size_t)slices + 1));
+    ESL_TRY(P->sl.alloc(std::max(slices, 1u)));
+    uint32_t lines = 0;
+    if (slices > 0) {
+        ESL_COUNT_LAUNCH();
+        k_pl_slices<<<count, 32, 0, s>>>(count, P->scc.get(), P->scc_sl.get(), source.get());
+        ESL_CUDA(cudaMemsetAsync(width.get() + slices, 0, 4, s));
+        ESL_COUNT_LAUNCH();
+        k_pl_ell<false><<<nblk((uint64_t)slices * 32), 256, 0, s>>>(slices, source.get(), P->ig_ptr.get(),
+                                                                    P->ig_ent.get(), width.get(), nullptr, nullptr,
+                                                                    nullptr);
+        ESL_TRY(scan_excl(tmp, width.get(), off.get(), slices + 1, s));
+        ESL_CUDA(cudaMemcpyAsync(&lines, off.get() + slices, 4, cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaStreamSynchronize(s));
+        ESL_TRY(P->ell.alloc((size_t)lines * 32));
+        ESL_COUNT_LAUNCH();
+        k_pl_ell<true><<<nblk((uint64_t)slices * 32), 256, 0, s>>>(slices, source.get(), P->ig_ptr.get(),
+                                                                   P->ig_ent.get(), width.get(), off.get(),
+                                                                   P->sl.get(), P->ell.get());
+        ESL_CUDA(cudaGetLastError());
+    }
+    ESL_CUDA(cudaStreamSynchronize(s));
     return ESL_OK;
 }
 
@@ -2625,56 +2820,98 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
     return dim3((unsigned)want, ty);
 }
 
-// Launches k_sw_scc over SCCs [j0, j1) of group g (sorted by decreasing size) and, with
-// `singles`, its singleton rows.  KS, the systems of one CTA, is the largest power of two
-// that keeps one thread per (row, system) pair within kSccPairs threads (1 above).
+// Launches k_sw_scc over group g: its SCCs of more than kSccThreads rows, then the others
+// with its singleton rows.  KS, the systems of one CTA, is the largest power of two that
+// keeps (row, system) pairs of small SCCs within kSccPairs threads; large SCCs, one CTA per
+// SM, take more systems while shared memory holds them and the SMs stay filled.
 constexpr int kSccPairs = 256;
-int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t j0, uint32_t j1, bool singles, bool defl,
-               SccArgs ga) {
+constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
+int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, SccArgs ga) {
     const int K = ga.a.K, n = ga.a.n;
     int lmax = 0;
     while (lmax < 5 && (1 << lmax) < K) lmax++;
     ga.scc = P->scc.get() + g.s0;
-    ga.nb = 0;
-    uint64_t items = 0;
-    int nr = 1, threads = 32;
-    size_t smem = 0;
-    for (uint32_t j = j0; j < j1; j++) {
-        const int m = (int)scc_rows(P->h_scc[g.s0 + j]);
-        if (m > kSccThreads1) nr = std::max(nr, m > 4 * kSccThreads ? 8 : 4);
+    ga.scc_sl = P->scc_sl.get() + g.s0;
+    ga.sl = P->sl.get();
+    ga.ell = P->ell.get();
+    const uint4* list = P->h_scc.data() + g.s0;
+    uint32_t nbig = 0;
+    while (nbig < g.ns && scc_rows(list[nbig]) > (uint32_t)kSccThreads) nbig++;
+    for (int part = 0; part < 2; part++) {
+        const bool big = part == 0;
+        const uint32_t j0 = big ? 0 : nbig, j1 = big ? nbig : g.ns;
+        // buckets, and the items that a CTA per item would make
+        uint64_t all = 0;
+        ga.nb = 0;
+        for (uint32_t j = j0; j < j1; j++) {
+            const int se = (int)list[j].y, so = (int)list[j].w, m = std::max(se, so);
+            const bool dense = !big && !defl && scc_dense(so, ga.max_iters);
+            auto lteam = [&](int l) {
+                int t = big ? 10 : 5;
+                while (!big && (1 << t) < (m << l)) t++;
+                return t;
+            };
+            auto doubles = [&](int l) { return scc_smem_doubles(big, dense, n, se, so, l, 1 << lteam(l)); };
+            int lks = 0;
+            if (big)
+                while (lks < lmax && doubles(lks + 1) * 8 <= kSccMaxSmem &&
+                       (uint64_t)nbig * (uint64_t)((K + (2 << lks) - 1) >> (lks + 1)) >= (uint64_t)ctx->sm_count)
+                    lks++;
+            else
+                while (lks < lmax && (m << (lks + 1)) <= kSccPairs &&
+                       (!dense || doubles(lks + 1) * 8 <= kSccDenseSmem))
+                    lks++;
+            // an SCC's KS is at least that of the larger ones before it
+            if (ga.nb > 0) lks = std::max<int>(lks, ga.b[ga.nb - 1].lks);
+            const int lt = lteam(lks);
+            if (ga.nb == 0 || ga.b[ga.nb - 1].lks != lks || ga.b[ga.nb - 1].lteam != lt) {
+                if (ga.nb == kSccBuckets) return fail(ESL_ERR_INVALID, "too many buckets");
+                ga.b[ga.nb++] = SccBucket{0, 0, j, 0, (uint8_t)lks, (uint8_t)lt, 1};
+            }
+            SccBucket& b = ga.b[ga.nb - 1];
+            const uint64_t its = (uint64_t)((K + (1 << lks) - 1) >> lks);
+            if (all + its > 0x3FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
+            b.items += (uint32_t)its;
+            all += its;
+            b.stride = std::max<uint32_t>(b.stride, (uint32_t)doubles(lks));
+        }
+        // Items share CTAs once there are more of them than SMs; a CTA then has the threads
+        // of the largest team at least
+        int threads = 32;
+        size_t smem = 0;
+        uint32_t items = 0, ctas = 0;
+        for (int j = 0; j < ga.nb; j++) threads = std::max(threads, 1 << ga.b[j].lteam);
+        if (!big && all > (uint64_t)ctx->sm_count) threads = std::max(threads, kSccPairs);
+        for (int j = 0; j < ga.nb; j++) {
+            SccBucket& b = ga.b[j];
+            if (!big && all > (uint64_t)ctx->sm_count)
+                b.teams = (uint8_t)std::max<size_t>(
+                    1, std::min<size_t>({(size_t)(threads >> b.lteam), (size_t)16, kSccTeamSmem / (b.stride * 8)}));
+            b.cta0 = items;
+            items += (b.items + b.teams - 1) / b.teams;
+            smem = std::max(smem, (size_t)b.teams * b.stride * 8);
+        }
+        ga.ctas = items;
+        if (!big && !defl && g.singles > 0) {
+            threads = std::max(threads, 128);
+            const uint64_t pairs = (uint64_t)(g.ne + g.no) * (uint64_t)K;
+            ctas = (uint32_t)std::max<uint64_t>(
+                1, std::min<uint64_t>((pairs + threads - 1) / threads, (uint64_t)ctx->sm_count * 8));
+        }
+        if (items + ctas == 0) continue;
+        auto go = [&](auto kern) -> int {
+            // the same limit from every thread: contexts set it concurrently
+            if (smem > 48 * 1024)
+                ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
+            ESL_COUNT_LAUNCH();
+            kern<<<items + ctas, threads, smem, ctx->stream>>>(ga);
+            ESL_CUDA(cudaGetLastError());
+            return ESL_OK;
+        };
+        if (defl) ESL_TRY(big ? go(k_sw_scc<true, true>) : go(k_sw_scc<false, true>));
+        else ESL_TRY(big ? go(k_sw_scc<true, false>) : go(k_sw_scc<false, false>));
     }
-    for (uint32_t j = j0; j < j1; j++) {
-        const uint4& c = P->h_scc[g.s0 + j];
-        const int m = (int)scc_rows(c);
-        int lks = 0;
-        while (lks < lmax && (m << (lks + 1)) <= kSccPairs) lks++;
-        if (ga.nb == 0 || ga.b[ga.nb - 1].lks != lks) ga.b[ga.nb++] = SccBucket{(uint32_t)items, j, lks};
-        items += (uint64_t)((K + (1 << lks) - 1) >> lks);
-        const int nact = std::min(scc_threads(nr), ((m << lks) + 31) & ~31);
-        threads = std::max(threads, nact);
-        smem = std::max(smem, scc_smem_doubles(nr, n, (int)c.y, (int)c.w, lks, nact) * 8);
-    }
-    ga.items = (uint32_t)items;
-    uint64_t ctas = 0;
-    if (singles) {
-        threads = std::max(threads, 128);
-        const uint64_t pairs = (uint64_t)(g.ne + g.no) * (uint64_t)K;
-        ctas = std::max<uint64_t>(1, std::min<uint64_t>((pairs + threads - 1) / threads, (uint64_t)ctx->sm_count * 8));
-    }
-    if (items + ctas == 0) return ESL_OK;
-    if (items + ctas > 0x7FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
-    const unsigned grid = (unsigned)(items + ctas);
-    cudaStream_t s = ctx->stream;
-    auto go = [&](auto kern) -> int {
-        if (smem > 48 * 1024)
-            ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
-        ESL_COUNT_LAUNCH();
-        kern<<<grid, threads, smem, s>>>(ga);
-        ESL_CUDA(cudaGetLastError());
-        return ESL_OK;
-    };
-    if (defl) return nr == 1 ? go(k_sw_scc<1, true>) : nr == 4 ? go(k_sw_scc<4, true>) : go(k_sw_scc<8, true>);
-    return nr == 1 ? go(k_sw_scc<1, false>) : nr == 4 ? go(k_sw_scc<4, false>) : go(k_sw_scc<8, false>);
+    return ESL_OK;
 }
 
 // the graphs (one per poll slot) of a Krylov solve, released on scope exit
@@ -2920,8 +3157,12 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ga.warm = term ? nullptr : o.d_warm;
             ga.warm_ld = (size_t)net->N;
             ga.Z = Z;
-            ga.BS = (double*)ws.get(W_BS, (size_t)std::max<uint32_t>(P->max_odd, 1) * Kp * 8, &st_);
-            if (st_ != ESL_OK) return st_;
+            if (g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads) {
+                const int slots[5] = {W_R0, W_D, W_DS64, W_QO, W_BS};
+                for (int j = 0; j < 5; j++)
+                    ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(P->max_odd, 1) * Kp * 8, &st_);
+                if (st_ != ESL_OK) return st_;
+            }
             ga.tol2 = tol * tol;
             ga.accept2 = kSwAcceptRel * kSwAcceptRel;
             ga.max_iters = max_iters;
@@ -2936,7 +3177,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
                 ga.TS = net->term_states;
             }
             st.local_groups++;
-            ESL_TRY(launch_scc(ctx, P, g, 0, g.ns, !term && g.singles > 0, term, ga));
+            ESL_TRY(launch_scc(ctx, P, g, term, ga));
             if (debug_on()) {
                 ESL_CUDA(cudaStreamSynchronize(s));
                 fprintf(stderr, "[esl-sweep] local group beg %u even %u odd %u max_scc %d sccs %u singles %u, %.3f ms\n",
