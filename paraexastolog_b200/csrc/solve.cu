@@ -613,21 +613,36 @@ __global__ void k_terminal_mass(int n, int T, int term_states, int nrhs, int x0_
     if (t >= 0 && (lane == 0 || tprev != t)) atomicAdd(&y[(size_t)k * T + t], acc);
 }
 
-// x_inf[k][v] = R_b[pos] * y[k][t] on terminal states; marginals accumulated
-__global__ void k_scatter_xinf(int n, int T, int term_states, int nrhs, size_t N, const int32_t* __restrict__ order,
-                               const int32_t* __restrict__ term_of, const double* __restrict__ Rb,
-                               const double* __restrict__ y, double* __restrict__ x_inf, double* __restrict__ marg) {
-    const int k = blockIdx.y;
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= term_states) return;
-    const int b = k / nrhs;
-    uint32_t v = (uint32_t)order[p];
-    int t = term_of[v];
-    double val = Rb[(size_t)b * term_states + p] * y[(size_t)k * T + t];
-    x_inf[(size_t)k * N + v] = val;
-    if (marg && val != 0.0) {
-        for (int i = 0; i < n; i++)
-            if ((v >> i) & 1u) atomicAdd(&marg[(size_t)k * n + i], val);
+// x_inf[k][v] = R_b[pos] * y[k][t] on terminal states; marginals accumulated.  A thread sums
+// its states' contributions to each node in its own column of shared memory and the CTA adds
+// one value per node: an atomic per state and set bit, all on the n addresses of a system,
+// took 4.1 ms for 32,640 terminal states x 64 systems.
+constexpr int kScatterT = 128;
+__global__ void __launch_bounds__(kScatterT) k_scatter_xinf(int n, int T, int term_states, int nrhs, size_t N,
+                                                            const int32_t* __restrict__ order,
+                                                            const int32_t* __restrict__ term_of,
+                                                            const double* __restrict__ Rb,
+                                                            const double* __restrict__ y, double* __restrict__ x_inf,
+                                                            double* __restrict__ marg) {
+    extern __shared__ double s_marg[];  // [node][thread]
+    const int k = blockIdx.y, b = k / nrhs, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (marg)
+        for (int i = 0; i < n; i++) s_marg[i * kScatterT + threadIdx.x] = 0.0;
+    for (int p = blockIdx.x * kScatterT + threadIdx.x; p < term_states; p += gridDim.x * kScatterT) {
+        const uint32_t v = (uint32_t)order[p];
+        const double val = Rb[(size_t)b * term_states + p] * y[(size_t)k * T + term_of[v]];
+        x_inf[(size_t)k * N + v] = val;
+        if (marg)
+            for (uint32_t m = v; m; m &= m - 1) s_marg[(__ffs(m) - 1) * kScatterT + threadIdx.x] += val;
+    }
+    if (!marg) return;
+    __syncthreads();
+    for (int i = warp; i < n; i += kScatterT / 32) {
+        double sum = 0.0;
+#pragma unroll
+        for (int j = 0; j < kScatterT; j += 32) sum += s_marg[i * kScatterT + j + lane];
+        sum = warp_sum(sum);
+        if (lane == 0 && sum != 0.0) atomicAdd(&marg[(size_t)k * n + i], sum);
     }
 }
 
@@ -1996,8 +2011,10 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         ESL_CUDA(cudaMemsetAsync(d_x_inf, 0, (size_t)K * N * 8, s));
         if (d_marg) ESL_CUDA(cudaMemsetAsync(d_marg, 0, (size_t)K * n * 8, s));
         ESL_COUNT_LAUNCH();
-        k_scatter_xinf<<<dim3((TS + 127) / 128, K), 128, 0, s>>>(n, T, TS, R, N, net->order.get(),
-                                                                   net->term_of.get(), Rb, y, d_x_inf, d_marg);
+        // up to eight CTAs of several states per thread for a system
+        const int parts = std::max(1, std::min(8, (TS + 4 * kScatterT - 1) / (4 * kScatterT)));
+        k_scatter_xinf<<<dim3(parts, K), kScatterT, (size_t)n * kScatterT * 8, s>>>(
+            n, T, TS, R, N, net->order.get(), net->term_of.get(), Rb, y, d_x_inf, d_marg);
         ESL_CUDA(cudaGetLastError());
     }
     // ---- absorption matrix L (backward form, first rate set) ----
