@@ -1302,7 +1302,9 @@ struct SccArgs {
     const double* warm;  // K x N warm start by state, or null
     size_t warm_ld;
     double* Z;           // [slot][Kp]
-    double* own[5];      // BIG: group-sized scratch, odd rows x Kp each
+    double* own[12];     // group-sized scratch: 5 odd-row vectors (kSccBig), all 12 (kSccGrid)
+    unsigned* bar;       // kSccGrid: barrier arrivals (0 before the launch), and a failure flag
+    double* part;        // kSccGrid: 2 x CTAs x 3 x KS partial sums
     double tol2, accept2;
     int max_iters, max_outer, stall;
     unsigned long long* ratio;  // per system: max over SCCs of final |r|^2 / |b|^2 (bits of a double >= 0)
@@ -1312,6 +1314,34 @@ struct SccArgs {
     const uint32_t* pos;
     double* Rb;
     int TS;
+};
+
+// Barrier of a cooperative launch.  A wait is bounded: past the bound it sets the failure
+// flag and neither this CTA nor, once they see the flag, the others wait any more (their
+// iteration budgets end the launch; the host reports the flag).
+constexpr unsigned kGridPolls = 1u << 24;
+struct GridBarrier {
+    unsigned* bar;
+    unsigned target;
+    bool dead;
+    __device__ __forceinline__ void wait() {
+        __syncthreads();
+        target += gridDim.x;
+        if (threadIdx.x == 0 && !dead) {
+            __threadfence();
+            atomicAdd(bar, 1u);
+            unsigned polls = 0;
+            while ((int)(*(volatile unsigned*)bar - target) < 0) {
+                if (*(volatile unsigned*)(bar + 1)) {
+                    dead = true;
+                    break;
+                }
+                if (++polls > kGridPolls) atomicExch(bar + 1, 1u);
+            }
+            __threadfence();
+        }
+        __syncthreads();
+    }
 };
 
 // a team's barrier: `threads` of the CTA, named by the team
@@ -1446,47 +1476,62 @@ __host__ __device__ inline size_t scc_smem_doubles(bool big, bool dense, int n, 
            KS;
 }
 
-// BIG false: SCCs of at most kSccThreads rows of either parity, a thread per row and system,
-// everything but the gathered vectors in registers, the row's first entries included.
-// BIG true: several rows per thread; r, v, p, t and 1 / q in shared memory, r0, d, the
+// kSccSmall: SCCs of at most kSccThreads rows of either parity, a thread per row and
+// system, everything but the gathered vectors in registers, the row's first entries included.
+// kSccBig: several rows per thread; r, v, p, t and 1 / q in shared memory, r0, d, the
 // Schur diagonal, q and the right-hand side in memory (streamed, an item's own run).
+// kSccGrid: the whole group, all systems (at most 32), by the whole grid of a cooperative
+// launch; every vector in memory as [row][KS].  For groups beyond a CTA's shared memory when
+// there are at most 32 systems: the row kernels would move 32 / K times the bytes and launch
+// seven kernels per iteration (n=22, one system, 11 groups of 16K to 370K rows: 24 -> 4 ms;
+// split over two or more tiles it is no faster than the row kernels, 58K rows x 512 systems
+// 144 against 65 ms).
 // DEFL: the deflated operator of a terminal SCC (see k_sw_defl_fin): S x + u gamma(x),
 // u_o = q_o / s, whose gamma is summed at the barrier that the elimination ends with anyway.
-template <bool BIG, bool DEFL>
-__global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_scc(const __grid_constant__ SccArgs g) {
+enum { kSccSmall, kSccBig, kSccGrid };
+template <int MODE, bool DEFL>
+__global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsBig, 1)
+    k_sw_scc(const __grid_constant__ SccArgs g) {
+    constexpr bool BIG = MODE == kSccBig, GRID = MODE == kSccGrid, MEM = BIG || GRID;
     extern __shared__ double s_all[];
     const SwArgs& a = g.a;
-    if (blockIdx.x >= g.ctas) {
+    if (!GRID && blockIdx.x >= g.ctas) {
         if (!DEFL) scc_singles(g, blockIdx.x - g.ctas, gridDim.x - g.ctas);
         return;
     }
     int bk = 0;
     while (bk + 1 < g.nb && blockIdx.x >= g.b[bk + 1].cta0) bk++;
     const SccBucket& bu = g.b[bk];
-    const int lteam = BIG ? 10 : bu.lteam;
-    const SccTeam team = {BIG ? 0 : (int)(threadIdx.x >> lteam), 1 << lteam, (int)(threadIdx.x & ((1u << lteam) - 1u))};
-    const uint32_t item = BIG ? blockIdx.x - bu.cta0 : (blockIdx.x - bu.cta0) * bu.teams + team.id;
-    if (!BIG && (team.id >= bu.teams || item >= bu.items)) return;
-    double* s_scc = BIG ? s_all : s_all + (size_t)team.id * bu.stride;
+    const int lteam = MEM ? 10 : bu.lteam;
+    const SccTeam team = {MEM ? 0 : (int)(threadIdx.x >> lteam), 1 << lteam, (int)(threadIdx.x & ((1u << lteam) - 1u))};
+    const uint32_t item = GRID ? 0u : BIG ? blockIdx.x - bu.cta0 : (blockIdx.x - bu.cta0) * bu.teams + team.id;
+    if (!MEM && (team.id >= bu.teams || item >= bu.items)) return;
+    double* s_scc = MEM ? s_all : s_all + (size_t)team.id * bu.stride;
     const int lks = bu.lks, KS = 1 << lks;
     const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), tile = item % tiles;
-    const uint4 sc = g.scc[bu.scc0 + item / tiles];
-    const uint2 first = g.scc_sl[bu.scc0 + item / tiles];
+    const uint4 sc = GRID ? make_uint4(a.beg, a.ne, a.beg + a.ne, a.no) : g.scc[bu.scc0 + item / tiles];
+    const uint2 first = GRID ? make_uint2(0u, 0u) : g.scc_sl[bu.scc0 + item / tiles];
     const uint32_t ev0 = sc.x, od0 = sc.z;
     const int se = (int)sc.y, so = (int)sc.w, sm = max(se, so);
     const int nact = team.threads;
-    const int s = team.tid & (KS - 1), rs = team.tid >> lks, RS = nact >> lks;
+    const int s = team.tid & (KS - 1);
+    const int rs = ((GRID ? (int)blockIdx.x * nact : 0) + team.tid) >> lks, RS = ((GRID ? (int)gridDim.x : 1) * nact) >> lks;
     const int k = (int)tile * KS + s;
     const size_t Kp = a.Kp;
     const bool act = k < a.K;
     // both with a zero row past the last, for the entries that a row of a slice lacks
-    double* A = s_scc;                           // odd rows: the vector whose product is formed
-    double* W = A + ((size_t)(sm + 1) << lks);   // even rows: its elimination
-    double* rate = W + ((size_t)(se + 1) << lks);
+    double* A = GRID ? g.own[5] : s_scc;                           // odd rows: the vector whose product is formed
+    double* W = GRID ? g.own[6] : A + ((size_t)(sm + 1) << lks);   // even rows: its elimination
+    double* rate = GRID ? s_scc : W + ((size_t)(se + 1) << lks);
     double* red0 = rate + ((size_t)(2 * a.n) << lks);
     double* red1 = red0 + ((size_t)(2 * (nact >> 5)) << lks);
     double* red2 = red1 + ((size_t)(3 * (nact >> 5)) << lks);
-    SccVec<BIG> R, V, P, T, IQ, R0, D, dS, q, BS;
+    SccVec<MEM> R, V, P, T, IQ, R0, D, dS, q, BS;
+    if constexpr (GRID) {
+        SccVec<MEM>* const all[10] = {&R0, &D, &dS, &q, &BS, &R, &V, &P, &T, &IQ};
+#pragma unroll
+        for (int j = 0; j < 10; j++) all[j]->mem = g.own[j < 5 ? j : j + 2];
+    }
     if constexpr (BIG) {
         R.mem = red2 + ((size_t)(nact >> 5) << lks);
         V.mem = R.mem + ((size_t)so << lks);
@@ -1504,7 +1549,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
     // one row per thread: its first two lines stay in registers
     uint4 ee[2], eo[2];
     uint2 le = make_uint2(0u, 0u), lo = make_uint2(0u, 0u);
-    if (!BIG) {
+    if (!MEM) {
         if (rs < se) le = __ldg(g.sl + first.x + (rs >> 5));
         if (rs < so) lo = __ldg(g.sl + first.y + (rs >> 5));
         for (int j = 0; j < 2; j++) {
@@ -1515,7 +1560,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
     const uint32_t rate_at = shared_addr(rate + s);
     // fn(row, index) of the own rows below count
     auto each = [&](int count, auto fn) {
-        if constexpr (BIG) {
+        if constexpr (MEM) {
             for (int r = rs; r < count; r += RS) fn(r, (r << lks) | s);
         } else if (rs < count) {
             fn(rs, (rs << lks) | s);
@@ -1526,8 +1571,26 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
     auto gather = [&](auto even, const double* X, auto fn) {
         constexpr bool EVEN = decltype(even)::value;
         const int count = EVEN ? se : so;
-        const uint32_t xs = shared_addr(X + s);
-        if constexpr (BIG) {
+        [[maybe_unused]] const uint32_t xs = GRID ? 0u : shared_addr(X + s);
+        if constexpr (GRID) {
+            const uint32_t base = EVEN ? od0 : ev0;
+            for (int r = rs; r < count; r += RS) {
+                const uint2 zw = __ldg(reinterpret_cast<const uint2*>(a.desc + (EVEN ? ev0 : od0) + r) + 1);
+                double acc = 0.0;
+                for (uint32_t j = 0; j < zw.y; j += 8) {
+                    uint32_t e[8];
+                    double x[8];
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; u++) e[u] = j + u < zw.y ? __ldg(a.ig_ent + zw.x + j + u) : 0u;
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; u++)
+                        x[u] = j + u < zw.y ? __ldcg(X + ((size_t)(ent_slot(e[u]) - base) << lks) + s) : 0.0;
+#pragma unroll
+                    for (uint32_t u = 0; u < 8; u++) acc += rate[(ent_rate(e[u]) << lks) | s] * x[u];
+                }
+                fn(r, (r << lks) | s, acc);
+            }
+        } else if constexpr (BIG) {
             if (rs >= count) return;
             const uint2* sl = g.sl + (EVEN ? first.x : first.y);
             const uint2 none = make_uint2(0u, 0u);
@@ -1567,9 +1630,35 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
     };
     constexpr auto even_rows = std::true_type{};
     constexpr auto odd_rows = std::false_type{};
+    // barrier of all threads of the item, and sums over them (see scc_sum); a grid's CTAs
+    // add up their sums in one order, so that they take the same decisions
+    GridBarrier gb = {g.bar, 0u, false};
+    auto sync = [&]() {
+        if constexpr (GRID) gb.wait();
+        else scc_sync(team);
+    };
+    unsigned sums = 0;
+    auto sum = [&](double* red, auto& v) {
+        constexpr int NV = (int)(sizeof(v) / sizeof(double));
+        scc_sum<NV>(red, lks, team, v);
+        if constexpr (GRID) {
+            double* part = g.part + (size_t)(sums++ & 1u) * ((size_t)gridDim.x * 3 << lks);
+            if (team.tid < KS)
+#pragma unroll
+                for (int j = 0; j < NV; j++) __stcg(part + ((size_t)(blockIdx.x * 3 + j) << lks) + s, v[j]);
+            gb.wait();
+#pragma unroll
+            for (int j = 0; j < NV; j++) v[j] = 0.0;
+            for (int c = team.tid >> lks; c < (int)gridDim.x; c += nact >> lks)
+#pragma unroll
+                for (int j = 0; j < NV; j++) v[j] += __ldcg(part + ((size_t)(c * 3 + j) << lks) + s);
+            scc_sum<NV>(red, lks, team, v);
+            __syncthreads();  // red is free again
+        }
+    };
     for (int idx = team.tid; idx < (2 * a.n) << lks; idx += nact)
         rate[idx] = a.rateT[(size_t)(idx >> lks) * Kp + (size_t)tile * KS + (idx & (KS - 1))];
-    if (rs == 0) {
+    if (!GRID && rs == 0) {
         A[(se << lks) | s] = 0.0;
         W[(se << lks) | s] = 0.0;
     }
@@ -1583,7 +1672,8 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
         }
         return acc;
     };
-    scc_sync(team);
+    if (GRID) __syncthreads();
+    else scc_sync(team);
     // even rows: 1 / q (in A too, for the Schur diagonal), and b / q, kept in Z until the end
     each(se, [&](int r, int idx) {
         const uint32_t slot = ev0 + r;
@@ -1598,7 +1688,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
         }
         W[idx] = w;
     });
-    scc_sync(team);
+    sync();
     // odd rows: q, Schur diagonal, reduced right-hand side, starting iterate
     double sum1[1] = {0.0};
     gather(odd_rows, W, [&](int r, int idx, double inflow) {
@@ -1606,13 +1696,23 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
         const uint2 d = a.rows[slot];
         const double qv = scc_q(rate, d.x, d.y, lks, s);
         double dv = qv;
-        const uint2 sl = __ldg(g.sl + first.y + (r >> 5));
-        for (uint32_t j = 0; j < 4 * sl.x; j++) {
-            const uint32_t e = __ldg(reinterpret_cast<const uint32_t*>(g.ell + (size_t)(sl.y + j / 4) * 32 + (r & 31)) + j % 4);
-            const uint32_t ri = e >> 3 & 63u;
-            // rate(e -> o) is the entry's; rate(o -> e) flips the same bit the other way
-            if ((d.y >> (ri >> 1)) & 1u)
-                dv -= rate[(ri << lks) | s] * rate[((ri ^ 1u) << lks) | s] * A[((e >> 9) << lks) | s];
+        // rate(e -> o) rate(o -> e) / q_e where both edges exist: the reverse flips the same bit
+        auto diag = [&](uint32_t ri, double iq) {
+            if ((d.y >> (ri >> 1)) & 1u) dv -= rate[(ri << lks) | s] * rate[((ri ^ 1u) << lks) | s] * iq;
+        };
+        if constexpr (GRID) {
+            const uint4 full = a.desc[slot];
+            for (uint32_t j = full.z; j < full.z + full.w; j++) {
+                const uint32_t e = __ldg(a.ig_ent + j);
+                diag((uint32_t)ent_rate(e), __ldcg(A + ((size_t)(ent_slot(e) - ev0) << lks) + s));
+            }
+        } else {
+            const uint2 sl = __ldg(g.sl + first.y + (r >> 5));
+            for (uint32_t j = 0; j < 4 * sl.x; j++) {
+                const uint32_t e =
+                    __ldg(reinterpret_cast<const uint32_t*>(g.ell + (size_t)(sl.y + j / 4) * 32 + (r & 31)) + j % 4);
+                diag(e >> 3 & 63u, A[((e >> 9) << lks) | s]);
+            }
         }
         q.set(idx, qv);
         dS.set(idx, dv);
@@ -1622,12 +1722,12 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
         BS.set(idx, b);
         if (act) g.Z[(size_t)slot * Kp + k] = !DEFL && g.warm ? g.warm[(size_t)k * g.warm_ld + d.x] : 0.0;
     });
-    const bool dense = !BIG && !DEFL && scc_dense(so, g.max_iters);
+    const bool dense = !MEM && !DEFL && scc_dense(so, g.max_iters);
     const int ld = scc_dense_ld(so);
     double* M = red2 + ((size_t)(nact >> 5) << lks);  // [row][column], the right-hand side last
     double* pivot = M + ((size_t)(so * ld) << lks);   // 1 / pivot of this and the next step
     auto at = [&](int r, int c) -> double& { return M[((r * ld + c) << lks) | s]; };
-    if (!BIG && dense && rs < so) {
+    if (!MEM && dense && rs < so) {
         // own row of the Schur complement: q_o - sum over e of rate(e -> o) / q_e rate(o' -> e)
         for (int c = 0; c < so; c++) at(rs, c) = 0.0;
         at(rs, rs) = q.get(0);
@@ -1653,10 +1753,10 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
         }
         if (rs == 0) pivot[s] = 1.0 / at(0, 0);
     }
-    scc_sum<1>(red1, lks, team, sum1);
+    sum(red1, sum1);
     const double b2 = sum1[0];
-    if (rs == 0) A[(so << lks) | s] = 0.0;  // 1 / q of an even row until here
-    if (!BIG && dense) {
+    if (!GRID && rs == 0) A[(so << lks) | s] = 0.0;  // 1 / q of an even row until here
+    if (!MEM && dense) {
         // Gauss-Jordan without pivoting (the rows of an M-matrix, diagonally dominant by
         // columns); the true residual below decides whether it is good enough
         for (int j = 0; j < so; j++) {
@@ -1681,10 +1781,10 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
         });
         if (DEFL) {
             each(so, [&](int, int idx) { gm[0] += A[idx]; });
-            scc_sum<1>(red2, lks, team, gm);
+            sum(red2, gm);
             gamma = gm[0];
         } else {
-            scc_sync(team);
+            sync();
         }
     };
     // fn(index, own odd row's value of the operator applied to A)
@@ -1698,7 +1798,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
     };
     auto load_x = [&]() {
         each(so, [&](int r, int idx) { A[idx] = act ? g.Z[(size_t)(od0 + r) * Kp + k] : 0.0; });
-        scc_sync(team);
+        sync();
     };
     bool done = !act || !(b2 > 0.0), failed = false;
     const bool warm = !DEFL && !dense && g.warm != nullptr;
@@ -1712,7 +1812,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
             v[0] += y * BS.get(idx);
             v[1] += y * y;
         });
-        scc_sum<2>(red0, lks, team, v);
+        sum(red0, v);
         const double al = v[1] > 0.0 ? v[0] / v[1] : 0.0;
         if (act) each(so, [&](int r, int) { g.Z[(size_t)(od0 + r) * Kp + k] *= al; });
     }
@@ -1729,7 +1829,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
                 R.set(idx, res);
                 v[0] += res * res;
             });
-            scc_sum<1>(red1, lks, team, v);
+            sum(red1, v);
             rr = v[0];
             if (dense && outer == 0 && !done && !(rr < b2)) {
                 // a zero start is better (a singular block, overflow)
@@ -1772,7 +1872,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
             D.set(idx, 0.0);
             A[idx] = x / dS.get(idx);
         });
-        scc_sync(team);
+        sync();
         double rho = 1.0, best = 1.0;
         int it = 0, stall = 0;
         while (__any_sync(0xffffffffu, run)) {
@@ -1782,13 +1882,13 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
                 V.set(idx, y);
                 v1[0] += R0.get(idx) * y;
             });
-            scc_sum<1>(red0, lks, team, v1);
+            sum(red0, v1);
             const double r0v = v1[0], alpha = r0v != 0.0 ? rho / r0v : 0.0;
             each(so, [&](int, int idx) {
                 P.set(idx, A[idx]);
                 A[idx] = (R.get(idx) - alpha * V.get(idx)) / dS.get(idx);
             });
-            scc_sync(team);
+            sync();
             elim();
             double v3[3] = {0.0, 0.0, 0.0};
             apply([&](int idx, double y) {
@@ -1797,7 +1897,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
                 v3[1] += y * y;
                 v3[2] += R0.get(idx) * y;
             });
-            scc_sum<3>(red1, lks, team, v3);
+            sum(red1, v3);
             const double omega = v3[1] > 0.0 ? v3[0] / v3[1] : 0.0, beta = r0v != 0.0 ? -v3[2] / r0v : 0.0;
             double v2[2] = {0.0, 0.0};
             each(so, [&](int, int idx) {
@@ -1809,7 +1909,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
                 v2[1] += R0.get(idx) * rv;
                 A[idx] = (rv + beta * (d * ph - omega * V.get(idx))) / d;
             });
-            scc_sum<2>(red0, lks, team, v2);
+            sum(red0, v2);
             if (run) {
                 it++;
                 if (v2[0] < 0.5 * best) {
@@ -1840,7 +1940,7 @@ __global__ void __launch_bounds__(BIG ? kSccThreadsBig : kSccThreads, 1) k_sw_sc
     });
     if (DEFL) {
         each(so, [&](int, int idx) { total[0] += A[idx]; });
-        scc_sum<1>(red1, lks, team, total);
+        sum(red1, total);
         const double inv = total[0] != 0.0 ? 1.0 / total[0] : 0.0;
         if (act) {
             each(se, [&](int r, int idx) { g.Rb[(size_t)k * g.TS + g.pos[ev0 + r]] = W[idx] * inv; });
@@ -1905,7 +2005,7 @@ __global__ void k_sw_rate_table(int n, int K, int Kp, int nrhs, const double* __
 
 // ---- host side ------------------------------------------------------------------------------
 enum SwSlot { W_Z, W_RATET, W_BV, W_BS, W_R64, W_DS64, W_DS32, W_W64, W_WT, W_R, W_R0, W_PH, W_V, W_SH, W_TT,
-              W_D, W_SCAL, W_ISCAL, W_CNT, W_LOC, W_QO, W_IQE, W_PERM, W_COUNT };
+              W_D, W_SCAL, W_ISCAL, W_CNT, W_LOC, W_QO, W_IQE, W_PERM, W_PART, W_COUNT };
 
 bool debug_on();
 
@@ -2908,9 +3008,30 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, Sc
             ESL_CUDA(cudaGetLastError());
             return ESL_OK;
         };
-        if (defl) ESL_TRY(big ? go(k_sw_scc<true, true>) : go(k_sw_scc<false, true>));
-        else ESL_TRY(big ? go(k_sw_scc<true, false>) : go(k_sw_scc<false, false>));
+        if (defl) ESL_TRY(big ? go(k_sw_scc<kSccBig, true>) : go(k_sw_scc<kSccSmall, true>));
+        else ESL_TRY(big ? go(k_sw_scc<kSccBig, false>) : go(k_sw_scc<kSccSmall, false>));
     }
+    return ESL_OK;
+}
+
+// Launches k_sw_scc<kSccGrid> over group g: all of its rows, all systems (at most 32).
+int launch_scc_grid(esl_ctx* ctx, const SwGroup& g, bool defl, SccArgs ga) {
+    int lks = 0;
+    while ((1 << lks) < ga.a.K) lks++;
+    ga.nb = 1;
+    ga.b[0] = SccBucket{0, 1, 0, 0, (uint8_t)lks, 10, 1};
+    // one CTA per SM: its registers are all taken, and a launch that cannot be resident fails
+    const uint64_t pairs = (uint64_t)std::max(g.ne, g.no) << lks;
+    const unsigned grid = (unsigned)std::max<uint64_t>(
+        1, std::min<uint64_t>((uint64_t)ctx->sm_count, (pairs + kSccThreadsBig - 1) / kSccThreadsBig));
+    const size_t smem = ((size_t)(2 * ga.a.n + 6 * (kSccThreadsBig / 32)) << lks) * 8;
+    const void* kern = defl ? (const void*)k_sw_scc<kSccGrid, true> : (const void*)k_sw_scc<kSccGrid, false>;
+    if (smem > 48 * 1024)
+        ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
+    ESL_CUDA(cudaMemsetAsync(ga.bar, 0, sizeof(unsigned), ctx->stream));
+    void* args[] = {&ga};
+    ESL_COUNT_LAUNCH();
+    ESL_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kSccThreadsBig), args, smem, ctx->stream));
     return ESL_OK;
 }
 
@@ -3091,6 +3212,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     int* loc_fail = reinterpret_cast<int*>(loc_ratio + Kp);
     int* loc_iters = loc_fail + Kp;
     ESL_CUDA(cudaMemsetAsync(loc_ratio, 0, loc_bytes, s));
+    ESL_CUDA(cudaMemsetAsync(d_cnt + 8, 0, 8, s));
     SwScalPtr sc;
     for (int j = 0; j < C_NSCAL; j++) sc.c[j] = scal + (size_t)j * Kp;
     for (int j = 0; j < I_NISCAL; j++) sc.i[j] = iscal + (size_t)j * Kp;
@@ -3147,7 +3269,8 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ESL_CUDA(cudaGetLastError());
             continue;
         }
-        if (g.resident) {
+        // (kSccGrid: where the rule lies, see there)
+        if (g.resident || K <= 32) {
             SccArgs ga{};
             ga.a = a;
             ga.og_ptr = P->og_ptr.get();
@@ -3157,12 +3280,18 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ga.warm = term ? nullptr : o.d_warm;
             ga.warm_ld = (size_t)net->N;
             ga.Z = Z;
-            if (g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads) {
-                const int slots[5] = {W_R0, W_D, W_DS64, W_QO, W_BS};
-                for (int j = 0; j < 5; j++)
-                    ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(P->max_odd, 1) * Kp * 8, &st_);
-                if (st_ != ESL_OK) return st_;
+            const int slots[12] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
+            const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
+            for (int j = 0; j < (g.resident ? (big ? 5 : 0) : 12); j++) {
+                const bool even = slots[j] == W_W64 || slots[j] == W_IQE;
+                ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(even ? P->max_even : P->max_odd, 1) * Kp * 8,
+                                            &st_);
             }
+            if (!g.resident) {
+                ga.bar = reinterpret_cast<unsigned*>(d_cnt) + 8;
+                ga.part = (double*)ws.get(W_PART, (size_t)2 * ctx->sm_count * 3 * 32 * 8, &st_);
+            }
+            if (st_ != ESL_OK) return st_;
             ga.tol2 = tol * tol;
             ga.accept2 = kSwAcceptRel * kSwAcceptRel;
             ga.max_iters = max_iters;
@@ -3177,7 +3306,8 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
                 ga.TS = net->term_states;
             }
             st.local_groups++;
-            ESL_TRY(launch_scc(ctx, P, g, term, ga));
+            if (g.resident) ESL_TRY(launch_scc(ctx, P, g, term, ga));
+            else ESL_TRY(launch_scc_grid(ctx, g, term, ga));
             if (debug_on()) {
                 ESL_CUDA(cudaStreamSynchronize(s));
                 fprintf(stderr, "[esl-sweep] local group beg %u even %u odd %u max_scc %d sccs %u singles %u, %.3f ms\n",
@@ -3679,8 +3809,11 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     // results of the SCC-resident groups
     if (st.local_groups > 0) {
         std::vector<unsigned char> h_loc(loc_bytes);
+        int h_bar[2] = {0, 0};
         ESL_CUDA(cudaMemcpyAsync(h_loc.data(), loc_ratio, loc_bytes, cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaMemcpyAsync(h_bar, d_cnt + 8, 8, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
+        if (h_bar[1]) return fail(ESL_ERR_TIMEOUT, "a grid barrier of the level sweep did not complete in time");
         std::vector<int> h_its(P->groups.size());
         std::memcpy(h_its.data(), h_loc.data() + (size_t)Kp * 12, h_its.size() * 4);
         for (int k = 0; k < K; k++) {
