@@ -469,9 +469,11 @@ class Mlp:
             raise ValueError(f"{ks.numel()} rate-set indices but {vs.numel()} states")
         sets = rates.numel() // (2 * self.net.n)
         if ks.numel():
-            if int(ks.min()) < 0 or int(ks.max()) >= sets:
+            # one device-to-host read for the four bounds
+            k0, k1, v0, v1 = torch.stack((*torch.aminmax(ks), *torch.aminmax(vs))).tolist()
+            if k0 < 0 or k1 >= sets:
                 raise ValueError(f"rate-set index outside [0, {sets})")
-            if int(vs.min()) < 0 or int(vs.max()) >= self.net.N:
+            if v0 < 0 or v1 >= self.net.N:
                 raise ValueError(f"state outside [0, {self.net.N})")
         return rates, ks, vs
 

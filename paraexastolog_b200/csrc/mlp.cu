@@ -118,66 +118,78 @@ __global__ void k_mlp_rate_features(int B, int n, const double* __restrict__ rat
     }
 }
 
-// ---- SIMT tiled GEMM:  C[m][n] (op)= sum_k A(m, k) B(k, n) --------------------------------
-// A(m, k) = A[m * sam + k * sak], B(k, n) = B[k * sbk + n * sbn]; 64 x 64 tiles, 256 threads
-// of 4 x 4 outputs, K in chunks of 16; blockIdx.z splits K (G_ATOMIC only).
-enum { G_STORE, G_BIAS, G_BIAS_RELU, G_MASK, G_ATOMIC };
+// ---- SIMT tiled GEMM:  C[m][n] = sum_k A(m, k) B(k, n) -----------------------------------
+// A(m, k) = A[m * sam + k * sak], B(k, n) = B[k * sbk + n * sbn]; 128 x 128 tiles, 256 threads
+// of 8 x 8 outputs, K in chunks of 16, the next chunk in registers while one is used.  FP32
+// throughout (sums in order of k), bound by the FP32 pipes and shared-memory reads: 8 x 8
+// outputs per thread read 2 x 8 words for 64 products (16,384 x 128 x 128: 27 us, 35 us
+// with 4 x 4 outputs and no prefetch).
+enum { G_STORE, G_BIAS, G_BIAS_RELU, G_MASK };
+constexpr int kGt = 128, kGk = 16, kGld = kGt + 4;
+
+// 64 products of a thread's rows ty * 4 + {0..3, 64..67} and columns tx * 4 + {0..3, 64..67}
+__device__ __forceinline__ void gemm_step(const float* a_row, const float* b_row, int ty, int tx, float (&acc)[8][8]) {
+    float a[8], b[8];
+    *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(a_row + ty * 4);
+    *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(a_row + 64 + ty * 4);
+    *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(b_row + tx * 4);
+    *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(b_row + 64 + tx * 4);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[i][j] += a[i] * b[j];
+}
+__device__ __forceinline__ int gemm_place(int t, int i) { return (i < 4 ? 0 : 64) + t * 4 + (i & 3); }
 
 template <int EPI>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* __restrict__ A, long sam, long sak,
+__global__ void __launch_bounds__(256, 2) k_gemm(int M, int N, int K, const float* __restrict__ A, long sam, long sak,
                                               const float* __restrict__ Bm, long sbk, long sbn, float* __restrict__ C,
-                                              long ldc, const float* __restrict__ bias, const float* __restrict__ mask,
-                                              int kper) {
-    __shared__ float As[16][68], Bs[16][68];
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int kb = blockIdx.z * kper, ke = min(K, kb + kper);
+                                              long ldc, const float* __restrict__ bias,
+                                              const float* __restrict__ mask) {
+    __shared__ __align__(16) float As[kGk][kGld], Bs[kGk][kGld];
+    const int m0 = blockIdx.y * kGt, n0 = blockIdx.x * kGt;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-    for (int k0 = kb; k0 < ke; k0 += 16) {
-        for (int i = threadIdx.x; i < 1024; i += 256) {
-            int mm, kk;
-            if (sam == 1) {
-                mm = i & 63;
-                kk = i >> 6;
-            } else {
-                mm = i >> 4;
-                kk = i & 15;
-            }
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < ke) ? A[(long)m * sam + (long)k * sak] : 0.0f;
-            int nn, kq;
-            if (sbn == 1) {
-                nn = i & 63;
-                kq = i >> 6;
-            } else {
-                nn = i >> 4;
-                kq = i & 15;
-            }
-            const int n = n0 + nn, kk2 = k0 + kq;
-            Bs[kq][nn] = (n < N && kk2 < ke) ? Bm[(long)kk2 * sbk + (long)n * sbn] : 0.0f;
+    float acc[8][8] = {};
+    float ra[8], rb[8];
+    // element u of this thread in a chunk: (row or column, k), k fastest where it is contiguous
+    auto place = [&](int u, bool k_fast, int& x, int& kk) {
+        const int i = u * 256 + threadIdx.x;
+        x = k_fast ? i >> 4 : i & (kGt - 1);
+        kk = k_fast ? i & 15 : i >> 7;
+    };
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            int x, kk;
+            place(u, sak == 1, x, kk);
+            ra[u] = (m0 + x < M && k0 + kk < K) ? A[(long)(m0 + x) * sam + (long)(k0 + kk) * sak] : 0.0f;
+            place(u, sbk == 1, x, kk);
+            rb[u] = (n0 + x < N && k0 + kk < K) ? Bm[(long)(k0 + kk) * sbk + (long)(n0 + x) * sbn] : 0.0f;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += kGk) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            int x, kk;
+            place(u, sak == 1, x, kk);
+            As[kk][x] = ra[u];
+            place(u, sbk == 1, x, kk);
+            Bs[kk][x] = rb[u];
         }
         __syncthreads();
+        if (k0 + kGk < K) fetch(k0 + kGk);
 #pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] += a[i] * b[j];
-        }
+        for (int kk = 0; kk < kGk; kk++) gemm_step(As[kk], Bs[kk], ty, tx, acc);
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
+    for (int i = 0; i < 8; i++) {
+        const int m = m0 + gemm_place(ty, i);
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
+        for (int j = 0; j < 8; j++) {
+            const int n = n0 + gemm_place(tx, j);
             if (n >= N) continue;
             float* c = C + (long)m * ldc + n;
             const float v = acc[i][j];
@@ -185,9 +197,84 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float* 
             if (EPI == G_BIAS) *c = v + bias[n];
             if (EPI == G_BIAS_RELU) *c = fmaxf(v + bias[n], 0.0f);
             if (EPI == G_MASK) *c = mask[(long)m * ldc + n] > 0.0f ? v : 0.0f;
-            if (EPI == G_ATOMIC) atomicAdd(c, v);
         }
     }
+}
+
+// ---- weight gradients ------------------------------------------------------------------------
+// part[CTA][parameter] = sum over the CTA's samples of the parameter's gradient, all layers:
+// CTAs of blockIdx.y 0: dW2 = dZ2^T H1 and db2, dw3 = H2^T dy and db3; 1: dW1 = dZ1^T X and db1.
+// The contraction runs over the samples, so a CTA takes a slab of them and keeps a whole
+// 128 x 128 (or 77) product in registers; k_mlp_wgrad_sum adds up the slabs in order.  In
+// place of GEMMs split over 16 slabs of 64 x 64 tiles with atomics and one column-sum kernel
+// per bias (650 us for 16,384 samples): 48 us, and 9 us for the sum.
+constexpr int kWgradCtas = 74;  // per blockIdx.y: one CTA per SM together
+__global__ void __launch_bounds__(256) k_mlp_wgrad(int S, const float* __restrict__ X, const float* __restrict__ H1,
+                                                   const float* __restrict__ H2, const float* __restrict__ dZ1,
+                                                   const float* __restrict__ dZ2, const float* __restrict__ dy,
+                                                   float* __restrict__ part) {
+    __shared__ __align__(16) float As[kGk][kGld], Bs[kGk][kGld];
+    const bool first = blockIdx.y == 1;
+    const float *A = first ? dZ1 : dZ2, *B = first ? X : H1;
+    const int ldb = first ? kXld : kH, nb = first ? kIn : kH, oW = first ? oW1 : oW2, oB = first ? oB1 : oB2;
+    float* out = part + (size_t)blockIdx.x * kParams;
+    const int per = (S + gridDim.x - 1) / gridDim.x, s0 = min(S, (int)blockIdx.x * per), s1 = min(S, s0 + per);
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    // two rows of 16-byte pieces per thread: piece c of sample rows r and r + 8
+    const int c = (threadIdx.x & 31) * 4, r = threadIdx.x >> 5;
+    float acc[8][8] = {}, db[8] = {}, w3 = 0.0f, b3 = 0.0f;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 ra[2], rb[2];
+    auto fetch = [&](int s) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int row = s + r + 8 * u;
+            ra[u] = row < s1 ? *reinterpret_cast<const float4*>(A + (size_t)row * kH + c) : zero;
+            rb[u] = row < s1 && c < ldb ? *reinterpret_cast<const float4*>(B + (size_t)row * ldb + c) : zero;
+        }
+    };
+    fetch(s0);
+    for (int s = s0; s < s1; s += kGk) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            *reinterpret_cast<float4*>(&As[r + 8 * u][c]) = ra[u];
+            *reinterpret_cast<float4*>(&Bs[r + 8 * u][c]) = rb[u];
+        }
+        __syncthreads();
+        if (s + kGk < s1) fetch(s + kGk);
+#pragma unroll
+        for (int kk = 0; kk < kGk; kk++) gemm_step(As[kk], Bs[kk], ty, tx, acc);
+        if (tx == 0)
+#pragma unroll
+            for (int kk = 0; kk < kGk; kk++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) db[i] += As[kk][gemm_place(ty, i)];
+        if (!first && threadIdx.x < kH)
+            for (int kk = 0; kk < min(kGk, s1 - s); kk++) w3 += H2[(size_t)(s + kk) * kH + threadIdx.x] * dy[s + kk];
+        if (!first && threadIdx.x == kH)
+            for (int kk = 0; kk < min(kGk, s1 - s); kk++) b3 += dy[s + kk];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int m = gemm_place(ty, i);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int n = gemm_place(tx, j);
+            if (n < nb) out[oW + m * nb + n] = acc[i][j];
+        }
+        if (tx == 0) out[oB + m] = db[i];
+    }
+    if (!first && threadIdx.x < kH) out[oW3 + threadIdx.x] = w3;
+    if (!first && threadIdx.x == kH) out[oB3] = b3;
+}
+__global__ void k_mlp_wgrad_sum(int slabs, const float* __restrict__ part, float* __restrict__ G) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kParams) return;
+    float a = 0.0f;
+#pragma unroll 8
+    for (int c = 0; c < slabs; c++) a += part[(size_t)c * kParams + i];
+    G[i] = a;
 }
 
 // ---- training pieces ------------------------------------------------------------------------
@@ -237,40 +324,62 @@ __global__ void k_mlp_label_stats(int S, uint64_t seed, int B, int nt, const uin
     }
 }
 
-// output layer, one warp per sample: y = H2 . w3 + b3, loss += w (y - t)^2 / S,
-// dy = 2 w (y - t) / S, dZ2 = dy w3 [H2 > 0]
-__global__ void k_mlp_head(int S, const float* __restrict__ H2, const float* __restrict__ Wq,
-                           const float* __restrict__ ts, const float* __restrict__ ws, float* __restrict__ y,
-                           float* __restrict__ dy, float* __restrict__ dZ2, float* __restrict__ loss) {
-    const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// output layer, one warp per sample: y = H2 . w3 + b3, lpart[block] = sum of
+// w (y - t)^2 / S over the block's samples (ws null: w = 1), dy = 2 w (y - t) / S,
+// dZ2 = dy w3 [H2 > 0].  An atomic per sample on the one loss took half of the kernel's time.
+constexpr int kHeadWarps = 8;
+__global__ void __launch_bounds__(kHeadWarps * 32) k_mlp_head(int S, const float* __restrict__ H2,
+                                                              const float* __restrict__ Wq,
+                                                              const float* __restrict__ ts,
+                                                              const float* __restrict__ ws, float* __restrict__ y,
+                                                              float* __restrict__ dy, float* __restrict__ dZ2,
+                                                              float* __restrict__ lpart) {
+    __shared__ float s_loss[kHeadWarps];
+    const int s = blockIdx.x * kHeadWarps + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (s >= S) return;
-    const float* h = H2 + (size_t)s * kH;
-    const float* w3 = Wq + oW3;
-    float a = 0.0f;
-    for (int j = lane; j < kH; j += 32) a += h[j] * w3[j];
-    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    const float yy = a + Wq[oB3];
-    const float r = yy - ts[s];
-    const float g = 2.0f * ws[s] * r / (float)S;
-    if (lane == 0) {
-        if (y) y[s] = yy;
-        if (dy) dy[s] = g;
-        if (loss) atomicAdd(loss, ws[s] * r * r / (float)S);
+    if (s < S) {
+        const float4 h = *reinterpret_cast<const float4*>(H2 + (size_t)s * kH + lane * 4);
+        float w[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) w[j] = Wq[oW3 + lane * 4 + j];
+        float a = h.x * w[0] + h.y * w[1] + h.z * w[2] + h.w * w[3];
+        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        const float yy = a + Wq[oB3];
+        const float r = yy - ts[s], wt = ws ? ws[s] : 1.0f;
+        const float g = 2.0f * wt * r / (float)S;
+        if (lane == 0) {
+            if (y) y[s] = yy;
+            if (dy) dy[s] = g;
+            s_loss[threadIdx.x >> 5] = wt * r * r / (float)S;
+        }
+        if (dZ2)
+            *reinterpret_cast<float4*>(dZ2 + (size_t)s * kH + lane * 4) =
+                make_float4(h.x > 0.0f ? g * w[0] : 0.0f, h.y > 0.0f ? g * w[1] : 0.0f, h.z > 0.0f ? g * w[2] : 0.0f,
+                            h.w > 0.0f ? g * w[3] : 0.0f);
+    } else if (lane == 0) {
+        s_loss[threadIdx.x >> 5] = 0.0f;
     }
-    if (dZ2)
-        for (int j = lane; j < kH; j += 32) dZ2[(size_t)s * kH + j] = h[j] > 0.0f ? g * w3[j] : 0.0f;
+    if (!lpart) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float a = 0.0f;
+        for (int j = 0; j < kHeadWarps; j++) a += s_loss[j];
+        lpart[blockIdx.x] = a;
+    }
 }
-
-// column sums of an S x W matrix, added into out[W]
-__global__ void k_colsum(int S, int W, const float* __restrict__ X, float* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= W) return;
-    const int per = (S + gridDim.y - 1) / gridDim.y;
-    const int s0 = blockIdx.y * per, s1 = min(S, s0 + per);
-    float a = 0.0f;
-    for (int s = s0; s < s1; s++) a += X[(size_t)s * W + j];
-    atomicAdd(out + j, a);
+// *loss = sum of the parts, in FP64 (one CTA)
+__global__ void __launch_bounds__(256) k_mlp_loss(int parts, const float* __restrict__ lpart, float* __restrict__ loss) {
+    __shared__ double s_sum[8];
+    double a = 0.0;
+    for (int i = threadIdx.x; i < parts; i += 256) a += (double)lpart[i];
+    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double b = 0.0;
+        for (int j = 0; j < 8; j++) b += s_sum[j];
+        *loss = (float)b;
+    }
 }
 
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
@@ -653,7 +762,7 @@ struct esl_mlp {
     DevBuf<float> P, G, M1, M2, Wq, Xs, A1;
     DevBuf<__nv_bfloat16> W2h;
     // per-call scratch (grow-only)
-    DevBuf<float> X, H1, H2, dZ2, dZ1, y, dy, ts, ws, C1, Xr, loss;
+    DevBuf<float> X, H1, H2, dZ2, dZ1, y, dy, ts, ws, C1, Xr, loss, lpart, wpart;
     DevBuf<int32_t> ks, vs;
     DevBuf<double> stats;
     DevBuf<int> tc_err;  // timeout flag of the tcgen05 inference
@@ -673,6 +782,7 @@ int grow(esl_mlp* m, int S) {
     ESL_TRY(m->dy.alloc(S));
     ESL_TRY(m->ts.alloc(S));
     ESL_TRY(m->ws.alloc(S));
+    ESL_TRY(m->lpart.alloc((size_t)(S + kHeadWarps - 1) / kHeadWarps));
     ESL_TRY(m->ks.alloc(S));
     ESL_TRY(m->vs.alloc(S));
     m->cap = S;
@@ -681,11 +791,10 @@ int grow(esl_mlp* m, int S) {
 
 template <int EPI>
 int gemm(cudaStream_t s, int M, int N, int K, const float* A, long sam, long sak, const float* B, long sbk, long sbn,
-         float* C, long ldc, const float* bias = nullptr, const float* mask = nullptr, int split = 1) {
-    const int kper = (K + split - 1) / split;
-    dim3 g((N + 63) / 64, (M + 63) / 64, split);
+         float* C, long ldc, const float* bias = nullptr, const float* mask = nullptr) {
+    dim3 g((N + kGt - 1) / kGt, (M + kGt - 1) / kGt);
     ESL_COUNT_LAUNCH();
-    k_gemm<EPI><<<g, 256, 0, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias, mask, (kper + 15) / 16 * 16);
+    k_gemm<EPI><<<g, 256, 0, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, bias, mask);
     ESL_CUDA(cudaGetLastError());
     return ESL_OK;
 }
@@ -698,36 +807,33 @@ int quantize(esl_mlp* m) {
     return ESL_OK;
 }
 
-// forward (and with grad != 0 backward) over S samples whose features are in X;
-// gradients are added into G, loss into *dloss
-int pass(esl_mlp* m, int S, bool grad, float* dloss) {
+// forward (and with grad != 0 backward) over S samples whose features are in X, with the
+// targets ts and weights ws (null: 1); gradients into G, loss into *dloss
+int pass(esl_mlp* m, int S, bool grad, float* dloss, const float* ws) {
     cudaStream_t s = m->ctx->stream;
     const float* Wq = m->Wq.get();
-    float* G = m->G.get();
     ESL_TRY(gemm<G_BIAS_RELU>(s, S, kH, kIn, m->X.get(), kXld, 1, Wq + oW1, 1, kIn, m->H1.get(), kH, Wq + oB1));
     ESL_TRY(gemm<G_BIAS_RELU>(s, S, kH, kH, m->H1.get(), kH, 1, Wq + oW2, 1, kH, m->H2.get(), kH, Wq + oB2));
+    const int head_blocks = (S + kHeadWarps - 1) / kHeadWarps;
     ESL_COUNT_LAUNCH();
-    k_mlp_head<<<(S + 7) / 8, 256, 0, s>>>(S, m->H2.get(), Wq, m->ts.get(), m->ws.get(), m->y.get(),
-                                          grad ? m->dy.get() : nullptr, grad ? m->dZ2.get() : nullptr, dloss);
+    k_mlp_head<<<head_blocks, kHeadWarps * 32, 0, s>>>(S, m->H2.get(), Wq, m->ts.get(), ws, m->y.get(),
+                                                       grad ? m->dy.get() : nullptr, grad ? m->dZ2.get() : nullptr,
+                                                       dloss ? m->lpart.get() : nullptr);
     ESL_CUDA(cudaGetLastError());
+    if (dloss) {
+        ESL_COUNT_LAUNCH();
+        k_mlp_loss<<<1, 256, 0, s>>>(head_blocks, m->lpart.get(), dloss);
+        ESL_CUDA(cudaGetLastError());
+    }
     if (!grad) return ESL_OK;
-    const int split = std::max(1, std::min(64, S / 1024));
-    // dw3 = H2^T dy, db3 = sum dy
-    ESL_TRY(gemm<G_ATOMIC>(s, kH, 1, S, m->H2.get(), 1, kH, m->dy.get(), 1, 0, G + oW3, 1, nullptr, nullptr, split));
-    ESL_COUNT_LAUNCH();
-    k_colsum<<<dim3(1, 64), 32, 0, s>>>(S, 1, m->dy.get(), G + oB3);
-    // dW2 = dZ2^T H1, db2 = colsum dZ2
-    ESL_TRY(gemm<G_ATOMIC>(s, kH, kH, S, m->dZ2.get(), 1, kH, m->H1.get(), kH, 1, G + oW2, kH, nullptr, nullptr,
-                           split));
-    ESL_COUNT_LAUNCH();
-    k_colsum<<<dim3(1, 64), kH, 0, s>>>(S, kH, m->dZ2.get(), G + oB2);
     // dZ1 = (dZ2 W2) [H1 > 0]
     ESL_TRY(gemm<G_MASK>(s, S, kH, kH, m->dZ2.get(), kH, 1, Wq + oW2, kH, 1, m->dZ1.get(), kH, nullptr, m->H1.get()));
-    // dW1 = dZ1^T X, db1 = colsum dZ1
-    ESL_TRY(gemm<G_ATOMIC>(s, kH, kIn, S, m->dZ1.get(), 1, kH, m->X.get(), kXld, 1, G + oW1, kIn, nullptr, nullptr,
-                           split));
+    if (!m->wpart.get()) ESL_TRY(m->wpart.alloc((size_t)kWgradCtas * kParams));
     ESL_COUNT_LAUNCH();
-    k_colsum<<<dim3(1, 64), kH, 0, s>>>(S, kH, m->dZ1.get(), G + oB1);
+    k_mlp_wgrad<<<dim3(kWgradCtas, 2), 256, 0, s>>>(S, m->X.get(), m->H1.get(), m->H2.get(), m->dZ1.get(), m->dZ2.get(),
+                                                   m->dy.get(), m->wpart.get());
+    ESL_COUNT_LAUNCH();
+    k_mlp_wgrad_sum<<<(kParams + 127) / 128, 128, 0, s>>>(kWgradCtas, m->wpart.get(), m->G.get());
     ESL_CUDA(cudaGetLastError());
     return ESL_OK;
 }
@@ -903,11 +1009,7 @@ int esl_mlp_loss_grad(esl_mlp* m, int S, const double* d_rates, const int32_t* d
     ESL_TRY(grow(m, S));
     ESL_TRY(esl_mlp_features(m, S, d_rates, d_k, d_state, m->X.get()));
     ESL_CUDA(cudaMemcpyAsync(m->ts.get(), d_target, (size_t)S * 4, cudaMemcpyDeviceToDevice, s));
-    std::vector<float> ones(S, 1.0f);
-    ESL_CUDA(cudaMemcpyAsync(m->ws.get(), ones.data(), (size_t)S * 4, cudaMemcpyHostToDevice, s));
-    ESL_CUDA(cudaMemsetAsync(m->G.get(), 0, kParams * 4, s));
-    ESL_CUDA(cudaMemsetAsync(m->loss.get(), 0, 4, s));
-    ESL_TRY(pass(m, S, grad != nullptr, m->loss.get()));
+    ESL_TRY(pass(m, S, grad != nullptr, m->loss.get(), nullptr));
     ESL_CUDA(cudaMemcpyAsync(loss, m->loss.get(), 4, cudaMemcpyDeviceToHost, s));
     if (grad) ESL_CUDA(cudaMemcpyAsync(grad, m->G.get(), kParams * 4, cudaMemcpyDeviceToHost, s));
     ESL_CUDA(cudaStreamSynchronize(s));
@@ -946,10 +1048,7 @@ int esl_mlp_train(esl_mlp* m, int B, const double* d_rates, const double* d_occu
                                                          (size_t)m->N, d_occupation, m->mu, m->sigma, m->ks.get(),
                                                          m->vs.get(), m->ts.get(), m->ws.get());
         ESL_TRY(esl_mlp_features(m, batch, d_rates, m->ks.get(), m->vs.get(), m->X.get()));
-        ESL_CUDA(cudaMemsetAsync(m->G.get(), 0, kParams * 4, s));
-        const bool last = it + 1 == steps;
-        if (last) ESL_CUDA(cudaMemsetAsync(m->loss.get(), 0, 4, s));
-        ESL_TRY(pass(m, batch, true, last ? m->loss.get() : nullptr));
+        ESL_TRY(pass(m, batch, true, it + 1 == steps ? m->loss.get() : nullptr, m->ws.get()));
         const float c1 = 1.0f - std::pow(b1, (float)m->step), c2 = 1.0f - std::pow(b2, (float)m->step);
         ESL_COUNT_LAUNCH();
         k_mlp_adam<<<(kParams + 255) / 256, 256, 0, s>>>(kParams, m->P.get(), m->G.get(), m->M1.get(), m->M2.get(), lr,
@@ -1031,8 +1130,7 @@ int esl_mlp_forward(esl_mlp* m, int S, const double* d_rates, const int32_t* d_k
     ESL_TRY(grow(m, S));
     ESL_TRY(esl_mlp_features(m, S, d_rates, d_k, d_state, m->X.get()));
     ESL_CUDA(cudaMemsetAsync(m->ts.get(), 0, (size_t)S * 4, s));
-    ESL_CUDA(cudaMemsetAsync(m->ws.get(), 0, (size_t)S * 4, s));
-    ESL_TRY(pass(m, S, false, nullptr));
+    ESL_TRY(pass(m, S, false, nullptr, nullptr));
     ESL_CUDA(cudaMemcpyAsync(d_y, m->y.get(), (size_t)S * 4, cudaMemcpyDeviceToDevice, s));
     return ESL_OK;
 }
