@@ -195,6 +195,8 @@ int table_pass(esl_ctx* ctx, const Model& m, const double* rates, DevBuf<uint32_
         ProfScope ps(ctx, "k_flip_masks", (double)N * (want_G ? 8.0 : 4.0) + 4.0 * blocks);
         ESL_TRY(launch_flip_masks(dm, F.get(), want_G ? G.get() : nullptr, counts.get(), s));
     }
+    nnz = host_edges(m, rates);
+    if (nnz >= 0) return ESL_OK;
     std::vector<uint32_t> h(blocks);
     ESL_CUDA(cudaMemcpyAsync(h.data(), counts.get(), blocks * 4, cudaMemcpyDeviceToHost, s));
     ESL_CUDA(cudaStreamSynchronize(s));
@@ -535,6 +537,10 @@ int esl_initial_state(esl_ctx* ctx, const esl_model* m, int n_fixed, const char*
 int esl_table_nnz(esl_ctx* ctx, const esl_model* m, const double* rates, int64_t* nnz) {
     StreamScope stream_scope_(ctx);
     if (!ctx || !m || !nnz) return fail(ESL_ERR_INVALID, "NULL argument");
+    // from the rules where they have tables (no pass over the states), else by counting
+    ESL_TRY(check_rates(m->m, rates));
+    *nnz = host_edges(m->m, rates);
+    if (*nnz >= 0) return ESL_OK;
     DevBuf<uint32_t> F, G, counts;
     ESL_TRY(table_pass(ctx, m->m, rates, F, G, counts, *nnz, false));
     return ESL_OK;

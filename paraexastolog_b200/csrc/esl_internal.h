@@ -264,10 +264,9 @@ struct DevModel {
     uint32_t up_ok, down_ok, self_dep;
 };
 struct DevModelBufs {
-    DevBuf<int32_t> off;
-    DevBuf<uint32_t> pos, neg, tab;
-    DevBuf<uint4> info;
+    DevBuf<uint32_t> all;
 };
+int64_t host_edges(const Model& m, const double* rates);
 int upload_model(const Model& m, DevModelBufs& b, const double* rates, DevModel& dm, cudaStream_t s);
 // zero-rate masks of a rate vector: bit i of up_ok / down_ok = rate 2i / 2i+1 nonzero
 void rate_masks(int n, const double* rates, uint32_t& up_ok, uint32_t& down_ok);
