@@ -186,13 +186,16 @@ struct esl_net {
     void (*plan_free)(void*) = nullptr;
     // slot plan of the state-major level sweep, built on first use
     void* sweep = nullptr;
+    // the same for the whole transient part as one group, forward and backward (small networks)
+    void* whole[2] = {nullptr, nullptr};
     // level-sweep tiling picked by esl_net_autotune: L2 slice budget in MB (0: default)
     // and two systems per thread on wide tiles (-1: default, on)
     int tune_tile_mb = 0, tune_s2 = -1;
     void (*sweep_free)(void*) = nullptr;
     ~esl_net() {
         if (plan && plan_free) plan_free(plan);
-        if (sweep && sweep_free) sweep_free(sweep);
+        for (void* p : {sweep, whole[0], whole[1]})
+            if (p && sweep_free) sweep_free(p);
     }
 };
 
@@ -309,6 +312,14 @@ int sweep_forward(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const doubl
 int sweep_terminal(esl_ctx* ctx, const esl_net* net, int B, const double* rates, const esl_solve_opts& o, double* Rb,
                    SweepStats& st);
 void free_sweep_workspace(void* w);
+// The transient part of a small network as one block (whole_supported): forward masses as
+// sweep_forward, and the absorption matrix L (T x N, terminal states included) of the first
+// rate set.  ESL_ERR_NOT_CONVERGED: nothing usable was written, another path must solve it.
+bool whole_supported(const esl_net* net);
+int sweep_whole(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const double* rates, const double* x0, size_t x0_ld,
+                const esl_solve_opts& o, double* y, SweepStats& st);
+int sweep_absorption(esl_ctx* ctx, const esl_net* net, const double* rates, const esl_solve_opts& o, double* d_L,
+                     SweepStats& st);
 // checksums (FNV-1a 64) of the 12 parts of a freshly built level-sweep plan: rows, desc,
 // ig_ptr, ig_ent, og_ptr, og_ent, tp_ptr, tp_ent, lsc_off, lsc_ne, lsc_slots, group table;
 // host != 0 builds it with the host reference builder instead of the device one

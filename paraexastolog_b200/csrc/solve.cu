@@ -1905,6 +1905,19 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         }
         swept = true;
     }
+    if (!swept && has_transient && o.method == ESL_METHOD_FP64 && whole_supported(net)) {
+        SweepStats sw;
+        const int rc = sweep_whole(ctx, net, K, R, d_rates, d_x0, N, o, y, sw);
+        if (rc == ESL_OK) {
+            agg.iters += sw.iters;
+            agg.relres = std::max(agg.relres, sw.relres);
+            swept = true;
+        } else if (rc != ESL_ERR_NOT_CONVERGED) {
+            return rc;
+        } else {
+            ESL_CUDA(cudaMemsetAsync(y, 0, (size_t)K * T * 8, s));
+        }
+    }
     if (swept) {
         // terminal masses are in y
     } else if (has_transient) {
@@ -2019,7 +2032,21 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
     }
     // ---- absorption matrix L (backward form, first rate set) ----
     if (d_L) {
-        if (has_transient) {
+        esl_solve_opts lo = o;
+        lo.d_warm = nullptr;
+        lo.d_occupation = nullptr;
+        lo.max_iters = std::max(o.max_iters, 5000);
+        SweepStats sa;
+        int small_rc = ESL_ERR_NOT_CONVERGED;
+        if (has_transient && whole_supported(net)) {
+            esl_solve_opts wo = lo;
+            wo.method = ESL_METHOD_FP64;
+            small_rc = sweep_absorption(ctx, net, d_rates, wo, d_L, sa);
+            if (small_rc != ESL_OK && small_rc != ESL_ERR_NOT_CONVERGED) return small_rc;
+        }
+        if (small_rc == ESL_OK) {
+            // L is complete
+        } else if (has_transient) {
             Layout L;
             ESL_TRY(make_layout(ctx, ws, net, 0, nullptr, false, L, T));
             const size_t vec = (size_t)T * L.ld;
@@ -2032,10 +2059,6 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
             ESL_CUDA(cudaGetLastError());
             double *x64 = nullptr, *zE = nullptr;
             SolveOut so;
-            esl_solve_opts lo = o;
-            lo.d_warm = nullptr;
-            lo.d_occupation = nullptr;
-            lo.max_iters = std::max(o.max_iters, 5000);
             const int rc = krylov_solve<false>(ctx, ws, L, d_rates, T, bE, bO, nullptr, 0, lo, x64, zE, so);
             if (rc == ESL_OK) {
                 ESL_COUNT_LAUNCH();

@@ -119,6 +119,8 @@ struct SweepPlan {
     DevBuf<uint32_t> lsc_slots;          // local SCCs: slots, SCC by SCC
     // terminal plan: per slot, the state's position in the reordering
     DevBuf<uint32_t> pos;
+    // backward plan of the whole transient part: per slot, the in-mask among transient states
+    DevBuf<uint32_t> rev;
     // the terminal SCCs above kDenseTerminalMax states, one deflated grid group each
     // (slots of their own; in-group predecessor lists only), or null
     SweepPlan* term = nullptr;
@@ -1301,6 +1303,7 @@ struct SccArgs {
     size_t x0_ld;
     const double* warm;  // K x N warm start by state, or null
     size_t warm_ld;
+    const uint32_t* rev; // per slot, flips whose reverse of the row's entries exists (null: the out-mask)
     double* Z;           // [slot][Kp]
     double* own[12];     // group-sized scratch: 5 odd-row vectors (kSccBig), all 12 (kSccGrid)
     unsigned* bar;       // kSccGrid: barrier arrivals (0 before the launch), and a failure flag
@@ -1697,8 +1700,9 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         const double qv = scc_q(rate, d.x, d.y, lks, s);
         double dv = qv;
         // rate(e -> o) rate(o -> e) / q_e where both edges exist: the reverse flips the same bit
+        const uint32_t both = g.rev ? g.rev[slot] : d.y;
         auto diag = [&](uint32_t ri, double iq) {
-            if ((d.y >> (ri >> 1)) & 1u) dv -= rate[(ri << lks) | s] * rate[((ri ^ 1u) << lks) | s] * iq;
+            if ((both >> (ri >> 1)) & 1u) dv -= rate[(ri << lks) | s] * rate[((ri ^ 1u) << lks) | s] * iq;
         };
         if constexpr (GRID) {
             const uint4 full = a.desc[slot];
@@ -2872,6 +2876,126 @@ int build_plan(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     return ESL_OK;
 }
 
+// The transient part of a small network as one group, even-parity states first: what the
+// whole-system form (ESL_METHOD_FP64) and the absorption matrix solve.  back: the transposed
+// system, whose rows gather from their successors at the row's own rates.
+int build_whole_plan(esl_ctx* ctx, const esl_net* net, bool back, SweepPlan*& out) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    esl_net* mnet = const_cast<esl_net*>(net);
+    void*& kept = mnet->whole[back];
+    if (kept) {
+        out = static_cast<SweepPlan*>(kept);
+        return ESL_OK;
+    }
+    cudaStream_t s = ctx->stream;
+    const size_t N = (size_t)net->N;
+    const int TS = net->term_states;
+    std::vector<int32_t> order(N), term_of(N);
+    std::vector<uint32_t> F(N), G(N);
+    ESL_CUDA(cudaMemcpyAsync(order.data(), net->order.get(), N * 4, cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaMemcpyAsync(term_of.data(), net->term_of.get(), N * 4, cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaMemcpyAsync(F.data(), net->F.get(), N * 4, cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaMemcpyAsync(G.data(), net->G.get(), N * 4, cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaStreamSynchronize(s));
+    std::unique_ptr<SweepPlan> P(new SweepPlan());
+    const uint32_t M = (uint32_t)(N - (size_t)TS);
+    P->M = M;
+    P->TS = back ? 0 : TS;
+    SwGroup g{};
+    g.kind = 2;
+    g.term = -1;
+    g.max_scc = (int)M;
+    std::vector<uint2> rows;
+    std::vector<uint32_t> slot_of(N, kNoSlot), rev;
+    for (int par = 0; par < 2; par++)
+        for (uint32_t v = 0; v < N; v++)
+            if (term_of[v] < 0 && (__builtin_popcount(v) & 1) == par) {
+                slot_of[v] = (uint32_t)rows.size();
+                rows.push_back(make_uint2(v, F[v]));
+                (par ? g.no : g.ne)++;
+            }
+    g.ns = 1;
+    P->h_scc.push_back(make_uint4(0, g.ne, g.ne, g.no));
+    P->max_rows = M;
+    P->max_even = g.ne;
+    P->max_odd = g.no;
+    std::vector<uint32_t> ig_ptr(M + 1, 0), og_ptr(M + 1, 0), ig, tp_ptr{0}, tp;
+    std::vector<uint4> desc(M);
+    auto entries = [&](uint32_t v, std::vector<uint32_t>& e) {
+        uint32_t kept_flips = 0;
+        for (uint32_t m = back ? F[v] : G[v]; m; m &= m - 1) {
+            const uint32_t i = (uint32_t)__builtin_ctz(m), su = slot_of[v ^ (1u << i)];
+            if (su == kNoSlot) continue;
+            // the rate of the edge's source: the neighbour's, or (back) the row's own
+            const uint32_t b = ((v >> i) & 1u) ^ (back ? 0u : 1u);
+            e.push_back((su << kEntShift) | (2u * i + b));
+            kept_flips |= 1u << i;
+        }
+        return kept_flips;
+    };
+    for (uint32_t sl = 0; sl < M; sl++) {
+        const uint32_t v = rows[sl].x;
+        entries(v, ig);
+        ig_ptr[sl + 1] = (uint32_t)ig.size();
+        desc[sl] = make_uint4(v, F[v], ig_ptr[sl], ig_ptr[sl + 1] - ig_ptr[sl]);
+        if (back) rev.push_back(G[v]);
+    }
+    g.nin = ig.size();
+    for (int p = 0; p < P->TS; p++) {
+        entries((uint32_t)order[p], tp);
+        tp_ptr.push_back((uint32_t)tp.size());
+    }
+    P->groups.push_back(g);
+    int rc = ESL_OK;
+    auto up = [&](auto& d, const auto& h) {
+        if (rc != ESL_OK) return;
+        rc = d.alloc(std::max<size_t>(h.size(), 1));
+        if (rc == ESL_OK && !h.empty() &&
+            cudaMemcpyAsync(d.get(), h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, s) != cudaSuccess)
+            rc = fail(ESL_ERR_CUDA, "plan upload failed");
+    };
+    up(P->rows, rows);
+    up(P->desc, desc);
+    up(P->ig_ptr, ig_ptr);
+    up(P->ig_ent, ig);
+    up(P->og_ptr, og_ptr);
+    up(P->og_ent, std::vector<uint32_t>{});
+    up(P->tp_ptr, tp_ptr);
+    up(P->tp_ent, tp);
+    if (back) up(P->rev, rev);
+    if (rc == ESL_OK && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(ESL_ERR_CUDA, "plan upload failed");
+    if (rc == ESL_OK) rc = finish_scc_list(ctx, net->n, P.get());
+    if (rc != ESL_OK) return rc;
+    mnet->sweep_free = free_plan_sweep;
+    out = P.get();
+    kept = P.release();
+    return ESL_OK;
+}
+
+// L[t][v] of the backward plan's solution (rows: Z[slot][t]) and of the terminal states
+__global__ void k_sw_scatter_L(uint32_t M, int Kp, size_t N, const uint2* __restrict__ rows, const double* __restrict__ Z,
+                               const int32_t* __restrict__ term_of, double* __restrict__ L) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.y;
+    if (i < N && term_of[i] >= 0) L[(size_t)t * N + i] = term_of[i] == t ? 1.0 : 0.0;
+    if (i < M) L[(size_t)t * N + rows[i].x] = Z[i * Kp + t];
+}
+// b[t][v] = rate of v's edges into terminal SCC t, for transient v (0 elsewhere)
+__global__ void k_sw_back_rhs(int n, size_t N, const uint32_t* __restrict__ F, const int32_t* __restrict__ term_of,
+                              const double* __restrict__ rates, double* __restrict__ b) {
+    const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.y;
+    if (v >= N) return;
+    double sum = 0.0;
+    if (term_of[v] < 0)
+        for (uint32_t f = F[v]; f; f &= f - 1) {
+            const int i = __ffs(f) - 1;
+            if (term_of[v ^ ((size_t)1 << i)] == t) sum += rates[2 * i + ((v >> i) & 1u)];
+        }
+    b[(size_t)t * N + v] = sum;
+}
+
 // systems per CTA tile: a divisor of Kp, at most 128, and rates of the tile within 36 KB
 // (with the reduction arrays the kernels stay inside the default 48 KB of shared memory).
 // With `rows` > 0 the tile is also narrowed (down to 32) until one tile's slice of a
@@ -3279,6 +3403,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ga.x0_ld = x0_ld;
             ga.warm = term ? nullptr : o.d_warm;
             ga.warm_ld = (size_t)net->N;
+            ga.rev = P->rev.get();
             ga.Z = Z;
             const int slots[12] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
             const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
@@ -3855,6 +3980,48 @@ int sweep_forward(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const doubl
     SweepPlan* P = nullptr;
     ESL_TRY(build_plan(ctx, net, P));
     return sweep_run(ctx, net, P, false, K, nrhs, rates, x0, x0_ld, o, y, st);
+}
+
+// The whole-system form is solved as one resident block while CTA-sized (8,192 transient
+// states of a network of at most 13 nodes): its Krylov launches, seven per iteration over
+// vectors of one state each, took 1.2 ms where the block takes 0.3 (n=11, one system).
+bool whole_supported(const esl_net* net) {
+    return net->n <= 13 && net->N - net->term_states >= 4 && (int64_t)net->term_states < net->N;
+}
+
+int sweep_whole(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const double* rates, const double* x0, size_t x0_ld,
+                const esl_solve_opts& o, double* y, SweepStats& st) {
+    SweepPlan* P = nullptr;
+    ESL_TRY(build_whole_plan(ctx, net, false, P));
+    if (!P->groups[0].resident || !P->max_even || !P->max_odd)
+        return fail(ESL_ERR_NOT_CONVERGED, "the transient part is not one block");
+    return sweep_run(ctx, net, P, false, K, nrhs, rates, x0, x0_ld, o, y, st);
+}
+
+int sweep_absorption(esl_ctx* ctx, const esl_net* net, const double* rates, const esl_solve_opts& o, double* d_L,
+                     SweepStats& st) {
+    SweepPlan* P = nullptr;
+    ESL_TRY(build_whole_plan(ctx, net, true, P));
+    if (!P->groups[0].resident || !P->max_even || !P->max_odd)
+        return fail(ESL_ERR_NOT_CONVERGED, "the transient part is not one block");
+    const size_t N = (size_t)net->N;
+    const int T = net->T, Kp = (T + 31) & ~31;
+    if (!ctx->sweep_work) ctx->sweep_work = new Workspace();
+    Workspace& ws = *static_cast<Workspace*>(ctx->sweep_work);
+    int st_ = ESL_OK;
+    double* b = (double*)ws.get(W_BV, (size_t)T * N * 8, &st_);
+    if (st_ != ESL_OK) return st_;
+    cudaStream_t s = ctx->stream;
+    const dim3 grid((unsigned)((N + 255) / 256), T);
+    ESL_COUNT_LAUNCH();
+    k_sw_back_rhs<<<grid, 256, 0, s>>>(net->n, N, net->F.get(), net->term_of.get(), rates, b);
+    ESL_CUDA(cudaGetLastError());
+    ESL_TRY(sweep_run(ctx, net, P, false, T, T, rates, b, N, o, nullptr, st));
+    const double* Z = (const double*)ws.get(W_Z, (size_t)P->M * Kp * 8, &st_);
+    ESL_COUNT_LAUNCH();
+    k_sw_scatter_L<<<grid, 256, 0, s>>>(P->M, Kp, N, P->rows.get(), Z, net->term_of.get(), d_L);
+    ESL_CUDA(cudaGetLastError());
+    return ESL_OK;
 }
 
 int sweep_terminal(esl_ctx* ctx, const esl_net* net, int B, const double* rates, const esl_solve_opts& o, double* Rb,
