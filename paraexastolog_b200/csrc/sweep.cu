@@ -1436,9 +1436,19 @@ __device__ __forceinline__ void scc_singles(const SccArgs& g, uint32_t cta, uint
         if (d.w) continue;  // in an SCC of two or more states
         double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + d.x];
         const uint32_t p1 = g.og_ptr[slot + 1];
-        for (uint32_t p = g.og_ptr[slot]; p < p1; p++) {
-            const uint32_t e = __ldg(g.og_ent + p);
-            acc += __ldg(a.rateT + (size_t)ent_rate(e) * a.Kp + k) * g.Z[(size_t)ent_slot(e) * a.Kp + k];
+        for (uint32_t p = g.og_ptr[slot]; p < p1; p += 4) {
+            uint32_t e[4];
+            double z[4], r4[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) e[u] = p + u < p1 ? __ldg(g.og_ent + p + u) : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                z[u] = p + u < p1 ? g.Z[(size_t)ent_slot(e[u]) * a.Kp + k] : 0.0;
+                r4[u] = __ldg(a.rateT + (size_t)ent_rate(e[u]) * a.Kp + k);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++)
+                if (p + u < p1) acc += r4[u] * z[u];
         }
         double q = 0.0;
         for (uint32_t f = d.y; f; f &= f - 1) {
@@ -1471,6 +1481,14 @@ constexpr int kSccDense = 16;
 __host__ __device__ inline bool scc_dense(int so, int max_iters) { return so <= kSccDense && so <= max_iters; }
 __host__ __device__ inline int scc_dense_ld(int so) { return (so + 1) | 1; }
 
+// 1 / x to about an ulp: two Newton steps from a single-precision reciprocal (not finite
+// where x is outside its range; the elimination's residual check then rejects the result)
+__device__ __forceinline__ double scc_recip(double x) {
+    double r = (double)(1.0f / (float)x);
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+
 // shared-memory doubles of a work item (see the carving in k_sw_scc)
 __host__ __device__ inline size_t scc_smem_doubles(bool big, bool dense, int n, int se, int so, int lks, int nact) {
     const size_t m = (size_t)(se > so ? se : so), KS = (size_t)1 << lks;
@@ -1499,7 +1517,11 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     extern __shared__ double s_all[];
     const SwArgs& a = g.a;
     if (!GRID && blockIdx.x >= g.ctas) {
-        if (!DEFL) scc_singles(g, blockIdx.x - g.ctas, gridDim.x - g.ctas);
+        if (!DEFL) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            scc_singles(g, blockIdx.x - g.ctas, gridDim.x - g.ctas);
+        }
         return;
     }
     int bk = 0;
@@ -1514,19 +1536,23 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), tile = item % tiles;
     const uint4 sc = GRID ? make_uint4(a.beg, a.ne, a.beg + a.ne, a.no) : g.scc[bu.scc0 + item / tiles];
     const uint2 first = GRID ? make_uint2(0u, 0u) : g.scc_sl[bu.scc0 + item / tiles];
+    // the rates, in flight with the SCC's description
+    const int nact = team.threads;
+    double* rate = s_scc;
+#pragma unroll 4
+    for (int idx = team.tid; idx < (2 * a.n) << lks; idx += nact)
+        rate[idx] = a.rateT[(size_t)(idx >> lks) * a.Kp + (size_t)tile * KS + (idx & (KS - 1))];
     const uint32_t ev0 = sc.x, od0 = sc.z;
     const int se = (int)sc.y, so = (int)sc.w, sm = max(se, so);
-    const int nact = team.threads;
     const int s = team.tid & (KS - 1);
     const int rs = ((GRID ? (int)blockIdx.x * nact : 0) + team.tid) >> lks, RS = ((GRID ? (int)gridDim.x : 1) * nact) >> lks;
     const int k = (int)tile * KS + s;
     const size_t Kp = a.Kp;
     const bool act = k < a.K;
     // both with a zero row past the last, for the entries that a row of a slice lacks
-    double* A = GRID ? g.own[5] : s_scc;                           // odd rows: the vector whose product is formed
-    double* W = GRID ? g.own[6] : A + ((size_t)(sm + 1) << lks);   // even rows: its elimination
-    double* rate = GRID ? s_scc : W + ((size_t)(se + 1) << lks);
-    double* red0 = rate + ((size_t)(2 * a.n) << lks);
+    double* A = GRID ? g.own[5] : rate + ((size_t)(2 * a.n) << lks);  // odd rows: the vector whose product is formed
+    double* W = GRID ? g.own[6] : A + ((size_t)(sm + 1) << lks);      // even rows: its elimination
+    double* red0 = GRID ? rate + ((size_t)(2 * a.n) << lks) : W + ((size_t)(se + 1) << lks);
     double* red1 = red0 + ((size_t)(2 * (nact >> 5)) << lks);
     double* red2 = red1 + ((size_t)(3 * (nact >> 5)) << lks);
     SccVec<MEM> R, V, P, T, IQ, R0, D, dS, q, BS;
@@ -1552,9 +1578,19 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     // one row per thread: its first two lines stay in registers
     uint4 ee[2], eo[2];
     uint2 le = make_uint2(0u, 0u), lo = make_uint2(0u, 0u);
+    uint2 row_e = le, row_o = le, og_e = le, og_o = le;
     if (!MEM) {
         if (rs < se) le = __ldg(g.sl + first.x + (rs >> 5));
         if (rs < so) lo = __ldg(g.sl + first.y + (rs >> 5));
+        // and so do the rows and the first entries from earlier groups
+        if (rs < se) {
+            row_e = a.rows[ev0 + rs];
+            if (!DEFL) og_e = make_uint2(g.og_ptr[ev0 + rs], g.og_ptr[ev0 + rs + 1]);
+        }
+        if (rs < so) {
+            row_o = a.rows[od0 + rs];
+            if (!DEFL) og_o = make_uint2(g.og_ptr[od0 + rs], g.og_ptr[od0 + rs + 1]);
+        }
         for (int j = 0; j < 2; j++) {
             if (j < (int)le.x) ee[j] = __ldg(g.ell + (size_t)(le.y + j) * 32 + (rs & 31));
             if (j < (int)lo.x) eo[j] = __ldg(g.ell + (size_t)(lo.y + j) * 32 + (rs & 31));
@@ -1659,44 +1695,61 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             __syncthreads();  // red is free again
         }
     };
-    for (int idx = team.tid; idx < (2 * a.n) << lks; idx += nact)
-        rate[idx] = a.rateT[(size_t)(idx >> lks) * Kp + (size_t)tile * KS + (idx & (KS - 1))];
     if (!GRID && rs == 0) {
         A[(se << lks) | s] = 0.0;
         W[(se << lks) | s] = 0.0;
     }
     const double inv_s = 1.0 / (double)(se + so);
-    auto rhs = [&](uint32_t slot, uint32_t v) {
+    // (four entries in flight: small groups are chains of such round trips to L2)
+    auto rhs = [&](uint2 og, uint32_t v) {
         double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + v];
-        const uint32_t p1 = g.og_ptr[slot + 1];
-        for (uint32_t p = g.og_ptr[slot]; p < p1; p++) {
-            const uint32_t e = __ldg(g.og_ent + p);
-            acc += rate[(ent_rate(e) << lks) | s] * g.Z[(size_t)ent_slot(e) * Kp + k];
+        const uint32_t p1 = og.y;
+        for (uint32_t p = og.x; p < p1; p += 4) {
+            uint32_t e[4];
+            double z[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) e[u] = p + u < p1 ? __ldg(g.og_ent + p + u) : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) z[u] = p + u < p1 ? g.Z[(size_t)ent_slot(e[u]) * Kp + k] : 0.0;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++)
+                if (p + u < p1) acc += rate[(ent_rate(e[u]) << lks) | s] * z[u];
         }
         return acc;
     };
+    auto og_of = [&](uint32_t slot) { return make_uint2(g.og_ptr[slot], g.og_ptr[slot + 1]); };
+    // From here on this launch reads what earlier ones of the sweep wrote (and lets the next
+    // one start up to this point, which only reads the plan and the rates).
+    if (!GRID) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     if (GRID) __syncthreads();
     else scc_sync(team);
     // even rows: 1 / q (in A too, for the Schur diagonal), and b / q, kept in Z until the end
     each(se, [&](int r, int idx) {
         const uint32_t slot = ev0 + r;
-        const uint2 d = a.rows[slot];
+        const uint2 d = MEM ? a.rows[slot] : row_e;
         const double iq = 1.0 / scc_q(rate, d.x, d.y, lks, s);
         IQ.set(idx, iq);
         A[idx] = iq;
         double w = 0.0;
         if (!DEFL && act) {
-            w = rhs(slot, d.x) * iq;
+            w = rhs(MEM ? og_of(slot) : og_e, d.x) * iq;
             g.Z[(size_t)slot * Kp + k] = w;
         }
         W[idx] = w;
     });
+    if (!DEFL)
+        each(so, [&](int r, int idx) {
+            R.set(idx, !act ? 0.0 : MEM ? rhs(og_of(od0 + r), a.rows[od0 + r].x) : rhs(og_o, row_o.x));
+        });
     sync();
     // odd rows: q, Schur diagonal, reduced right-hand side, starting iterate
     double sum1[1] = {0.0};
     gather(odd_rows, W, [&](int r, int idx, double inflow) {
         const uint32_t slot = od0 + r;
-        const uint2 d = a.rows[slot];
+        const uint2 d = MEM ? a.rows[slot] : row_o;
         const double qv = scc_q(rate, d.x, d.y, lks, s);
         double dv = qv;
         // rate(e -> o) rate(o -> e) / q_e where both edges exist: the reverse flips the same bit
@@ -1720,7 +1773,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         }
         q.set(idx, qv);
         dS.set(idx, dv);
-        const double b = DEFL ? qv * inv_s : (act ? rhs(slot, d.x) : 0.0) + inflow;
+        const double b = DEFL ? qv * inv_s : R.get(idx) + inflow;
         sum1[0] += b * b;
         R.set(idx, b);
         BS.set(idx, b);
@@ -1755,7 +1808,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
                 }
             }
         }
-        if (rs == 0) pivot[s] = 1.0 / at(0, 0);
+        if (rs == 0) pivot[s] = scc_recip(at(0, 0));
     }
     sum(red1, sum1);
     const double b2 = sum1[0];
@@ -1766,9 +1819,11 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         for (int j = 0; j < so; j++) {
             if (rs < so && rs != j) {
                 const double f = at(rs, j) * pivot[((j & 1) << lks) | s];
+                const double x = at(rs, j + 1) - f * at(j, j + 1);
+                at(rs, j + 1) = x;
+                if (rs == j + 1) pivot[(((j + 1) & 1) << lks) | s] = scc_recip(x);
 #pragma unroll 4
-                for (int c = j + 1; c <= so; c++) at(rs, c) -= f * at(j, c);
-                if (rs == j + 1) pivot[(((j + 1) & 1) << lks) | s] = 1.0 / at(rs, rs);
+                for (int c = j + 2; c <= so; c++) at(rs, c) -= f * at(j, c);
             }
             scc_sync(team);
         }
@@ -3050,7 +3105,9 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
 // SM, take more systems while shared memory holds them and the SMs stay filled.
 constexpr int kSccPairs = 256;
 constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
-int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, SccArgs ga) {
+// overlap: the launch may start, up to its first read of the sweep's vectors, before the
+// previous one ends (not for the sweep's first: the rates are being written).
+int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, bool overlap, SccArgs ga) {
     const int K = ga.a.K, n = ga.a.n;
     int lmax = 0;
     while (lmax < 5 && (1 << lmax) < K) lmax++;
@@ -3128,8 +3185,18 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, Sc
             if (smem > 48 * 1024)
                 ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
             ESL_COUNT_LAUNCH();
-            kern<<<items + ctas, threads, smem, ctx->stream>>>(ga);
-            ESL_CUDA(cudaGetLastError());
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr.val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(items + ctas);
+            cfg.blockDim = dim3(threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = ctx->stream;
+            cfg.attrs = &attr;
+            cfg.numAttrs = overlap ? 1 : 0;
+            ESL_CUDA(cudaLaunchKernelEx(&cfg, kern, ga));
+            overlap = true;
             return ESL_OK;
         };
         if (defl) ESL_TRY(big ? go(k_sw_scc<kSccBig, true>) : go(k_sw_scc<kSccSmall, true>));
@@ -3365,6 +3432,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     std::vector<char> failed(K, 0);
     int total_iters = 0;
 
+    bool first_launch = true;
     for (const SwGroup& g : P->groups) {
         // debug timing: wall time of the group with the stream drained on both sides
         std::chrono::steady_clock::time_point g_t0;
@@ -3431,7 +3499,9 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
                 ga.TS = net->term_states;
             }
             st.local_groups++;
-            if (g.resident) ESL_TRY(launch_scc(ctx, P, g, term, ga));
+            const bool overlap = !first_launch;
+            first_launch = false;
+            if (g.resident) ESL_TRY(launch_scc(ctx, P, g, term, overlap, ga));
             else ESL_TRY(launch_scc_grid(ctx, g, term, ga));
             if (debug_on()) {
                 ESL_CUDA(cudaStreamSynchronize(s));
