@@ -87,7 +87,8 @@ struct SwGroup {
     int max_odd;           // local groups: most odd rows of one SCC
     uint64_t nin;          // in-group predecessor entries of the group's rows
     uint32_t s0, ns;       // the group's SCCs of >= 2 states: range in SweepPlan::scc
-    bool resident;         // every one of them fits k_sw_scc
+    bool resident;         // every one of them fits a CTA or a cluster of k_sw_scc
+    bool split;            // one of them needs a cluster
     uint32_t singles;      // rows that are SCCs of their own
     int term;              // terminal plan: the terminal SCC of the group (-1 otherwise)
     uint32_t pos0;         // terminal plan: position of the SCC's first state in the order
@@ -112,7 +113,8 @@ struct SweepPlan {
     // first line of ell).  Line j holds entries 4j .. 4j + 3 of each row, 16 bytes a row:
     // local row of the other parity << 9 | rate index << 3, so that masked and shifted they
     // are byte offsets (row * 8 after >> 6); past a row's last entry the local row is the
-    // other parity's row count.
+    // other parity's row count.  In an SCC split over a cluster the local row is the owner's
+    // rank << 13 | its row there, and past the last entry the own rank's row kSccMaxRows.
     DevBuf<uint2> scc_sl, sl;
     DevBuf<uint4> ell;
     DevBuf<uint32_t> lsc_ne;             // local SCCs: number of even-parity slots (listed first)
@@ -1277,6 +1279,10 @@ __global__ void __launch_bounds__(kSwT) k_sw_warm_scale(SwArgs a, const double* 
 // size.  CTAs past the last item serve the group's singleton SCCs (rows without in-group
 // predecessors): z = b / q.
 constexpr int kSccMaxRows = 4096;  // most odd (or even) rows of an SCC solved by one CTA
+// Most CTAs that share a larger one.  512 systems: SCCs of 16K states (two) 11.2 -> 6 ms and
+// of 26K to 31K (four) 31 -> 28 and 22 -> 14 ms against the row kernels; of 53K to 58K states
+// (eight) 31 -> 38 and 64 -> 78 ms.
+constexpr int kSccMaxCluster = 4;
 // threads of a CTA with one row per thread (128 registers each), and with several
 constexpr int kSccThreads = 512, kSccThreadsBig = 1024;
 constexpr int kSccBuckets = 16;    // most (KS, team size) pairs of a launch
@@ -1379,6 +1385,29 @@ __device__ __forceinline__ void ell_add(double& acc, const uint4& e, uint32_t X,
     acc += r1 * x1;
     acc += r2 * x2;
     acc += r3 * x3;
+}
+
+// The same of an SCC split over a cluster (one system): the entry's row is in the shared
+// memory of CTA e >> 22 of the cluster.
+__device__ __forceinline__ double lds_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote));
+    return v;
+}
+__device__ __forceinline__ void ell_add_cluster(double& acc, const uint4& e, uint32_t X, uint32_t rate) {
+    const double r0 = lds_f64(rate + (e.x & 0x1F8u)), x0 = lds_cluster(X + (e.x >> 6 & 0xFFF8u), e.x >> 22);
+    const double r1 = lds_f64(rate + (e.y & 0x1F8u)), x1 = lds_cluster(X + (e.y >> 6 & 0xFFF8u), e.y >> 22);
+    const double r2 = lds_f64(rate + (e.z & 0x1F8u)), x2 = lds_cluster(X + (e.z >> 6 & 0xFFF8u), e.z >> 22);
+    const double r3 = lds_f64(rate + (e.w & 0x1F8u)), x3 = lds_cluster(X + (e.w >> 6 & 0xFFF8u), e.w >> 22);
+    acc += r0 * x0;
+    acc += r1 * x1;
+    acc += r2 * x2;
+    acc += r3 * x3;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Sums of NV values over a team's threads of one system; every thread of a system gets
@@ -1501,6 +1530,10 @@ __host__ __device__ inline size_t scc_smem_doubles(bool big, bool dense, int n, 
 // system, everything but the gathered vectors in registers, the row's first entries included.
 // kSccBig: several rows per thread; r, v, p, t and 1 / q in shared memory, r0, d, the
 // Schur diagonal, q and the right-hand side in memory (streamed, an item's own run).
+// kSccCluster: kSccBig over a cluster of up to kSccMaxCluster CTAs for one system, each with
+// kSccMaxRows rows of either parity; gathers read the owner's shared memory, sums are
+// exchanged through it (a network of two SCCs of 16,384 states, 64 and 16 systems: 8.1 ->
+// 5.5 ms).
 // kSccGrid: the whole group, all systems (at most 32), by the whole grid of a cooperative
 // launch; every vector in memory as [row][KS].  For groups beyond a CTA's shared memory when
 // there are at most 32 systems: the row kernels would move 32 / K times the bytes and launch
@@ -1509,14 +1542,20 @@ __host__ __device__ inline size_t scc_smem_doubles(bool big, bool dense, int n, 
 // 144 against 65 ms).
 // DEFL: the deflated operator of a terminal SCC (see k_sw_defl_fin): S x + u gamma(x),
 // u_o = q_o / s, whose gamma is summed at the barrier that the elimination ends with anyway.
-enum { kSccSmall, kSccBig, kSccGrid };
+enum { kSccSmall, kSccBig, kSccGrid, kSccCluster };
 template <int MODE, bool DEFL>
 __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsBig, 1)
     k_sw_scc(const __grid_constant__ SccArgs g) {
-    constexpr bool BIG = MODE == kSccBig, GRID = MODE == kSccGrid, MEM = BIG || GRID;
+    constexpr bool CLUSTER = MODE == kSccCluster, BIG = MODE == kSccBig || CLUSTER, GRID = MODE == kSccGrid,
+                   MEM = BIG || GRID;
+    uint32_t rank = 0, ranks = 1;
+    if (CLUSTER) {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    }
     extern __shared__ double s_all[];
     const SwArgs& a = g.a;
-    if (!GRID && blockIdx.x >= g.ctas) {
+    if (!GRID && !CLUSTER && blockIdx.x >= g.ctas) {
         if (!DEFL) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1525,25 +1564,38 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         return;
     }
     int bk = 0;
-    while (bk + 1 < g.nb && blockIdx.x >= g.b[bk + 1].cta0) bk++;
+    while (!CLUSTER && bk + 1 < g.nb && blockIdx.x >= g.b[bk + 1].cta0) bk++;
     const SccBucket& bu = g.b[bk];
     const int lteam = MEM ? 10 : bu.lteam;
     const SccTeam team = {MEM ? 0 : (int)(threadIdx.x >> lteam), 1 << lteam, (int)(threadIdx.x & ((1u << lteam) - 1u))};
-    const uint32_t item = GRID ? 0u : BIG ? blockIdx.x - bu.cta0 : (blockIdx.x - bu.cta0) * bu.teams + team.id;
+    const uint32_t item = GRID ? 0u : CLUSTER ? blockIdx.x / ranks : BIG ? blockIdx.x - bu.cta0 : (blockIdx.x - bu.cta0) * bu.teams + team.id;
     if (!MEM && (team.id >= bu.teams || item >= bu.items)) return;
     double* s_scc = MEM ? s_all : s_all + (size_t)team.id * bu.stride;
     const int lks = bu.lks, KS = 1 << lks;
     const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), tile = item % tiles;
     const uint4 sc = GRID ? make_uint4(a.beg, a.ne, a.beg + a.ne, a.no) : g.scc[bu.scc0 + item / tiles];
-    const uint2 first = GRID ? make_uint2(0u, 0u) : g.scc_sl[bu.scc0 + item / tiles];
+    uint2 first = GRID ? make_uint2(0u, 0u) : g.scc_sl[bu.scc0 + item / tiles];
     // the rates, in flight with the SCC's description
     const int nact = team.threads;
     double* rate = s_scc;
 #pragma unroll 4
     for (int idx = team.tid; idx < (2 * a.n) << lks; idx += nact)
         rate[idx] = a.rateT[(size_t)(idx >> lks) * a.Kp + (size_t)tile * KS + (idx & (KS - 1))];
-    const uint32_t ev0 = sc.x, od0 = sc.z;
-    const int se = (int)sc.y, so = (int)sc.w, sm = max(se, so);
+    uint32_t ev0 = sc.x, od0 = sc.z;
+    int se = (int)sc.y, so = (int)sc.w;
+    const double inv_s = 1.0 / (double)(se + so);
+    if (CLUSTER) {
+        // this CTA's rows
+        const int r0 = (int)rank * kSccMaxRows;
+        ev0 += r0;
+        od0 += r0;
+        first.x += r0 / 32;
+        first.y += r0 / 32;
+        se = min(max(se - r0, 0), kSccMaxRows);
+        so = min(max(so - r0, 0), kSccMaxRows);
+    }
+    // rows that the arrays are laid out for: the same in every CTA of a cluster
+    const int le_rows = CLUSTER ? kSccMaxRows : se, lo_rows = CLUSTER ? kSccMaxRows : so, sm = max(le_rows, lo_rows);
     const int s = team.tid & (KS - 1);
     const int rs = ((GRID ? (int)blockIdx.x * nact : 0) + team.tid) >> lks, RS = ((GRID ? (int)gridDim.x : 1) * nact) >> lks;
     const int k = (int)tile * KS + s;
@@ -1552,7 +1604,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     // both with a zero row past the last, for the entries that a row of a slice lacks
     double* A = GRID ? g.own[5] : rate + ((size_t)(2 * a.n) << lks);  // odd rows: the vector whose product is formed
     double* W = GRID ? g.own[6] : A + ((size_t)(sm + 1) << lks);      // even rows: its elimination
-    double* red0 = GRID ? rate + ((size_t)(2 * a.n) << lks) : W + ((size_t)(se + 1) << lks);
+    double* red0 = GRID ? rate + ((size_t)(2 * a.n) << lks) : W + ((size_t)(le_rows + 1) << lks);
     double* red1 = red0 + ((size_t)(2 * (nact >> 5)) << lks);
     double* red2 = red1 + ((size_t)(3 * (nact >> 5)) << lks);
     SccVec<MEM> R, V, P, T, IQ, R0, D, dS, q, BS;
@@ -1563,12 +1615,12 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     }
     if constexpr (BIG) {
         R.mem = red2 + ((size_t)(nact >> 5) << lks);
-        V.mem = R.mem + ((size_t)so << lks);
-        P.mem = V.mem + ((size_t)so << lks);
-        T.mem = P.mem + ((size_t)so << lks);
-        IQ.mem = T.mem + ((size_t)so << lks);
-        // the SCC's so x Kp block of a group vector, tile by tile
-        const size_t o = (size_t)(od0 - a.beg - a.ne) * Kp + (size_t)tile * KS * so;
+        V.mem = R.mem + ((size_t)lo_rows << lks);
+        P.mem = V.mem + ((size_t)lo_rows << lks);
+        T.mem = P.mem + ((size_t)lo_rows << lks);
+        IQ.mem = T.mem + ((size_t)lo_rows << lks);
+        // the SCC's block of odd rows x Kp of a group vector, tile by tile (row by row there)
+        const size_t o = (size_t)(sc.z - a.beg - a.ne) * Kp + (size_t)tile * KS * sc.w + (CLUSTER ? rank * kSccMaxRows : 0);
         R0.mem = g.own[0] + o;
         D.mem = g.own[1] + o;
         dS.mem = g.own[2] + o;
@@ -1630,6 +1682,10 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
                 fn(r, (r << lks) | s, acc);
             }
         } else if constexpr (BIG) {
+            auto add = [&](double& acc, const uint4& e) {
+                if constexpr (CLUSTER) ell_add_cluster(acc, e, xs, rate_at);
+                else ell_add(acc, e, xs, rate_at, lks);
+            };
             if (rs >= count) return;
             const uint2* sl = g.sl + (EVEN ? first.x : first.y);
             const uint2 none = make_uint2(0u, 0u);
@@ -1645,14 +1701,14 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
                 while (left > 1) {
                     line += 32;
                     f = __ldg(line);
-                    ell_add(acc, e, xs, rate_at, lks);
+                    add(acc, e);
                     e = f;
                     left--;
                 }
                 if (next_lines) f = __ldg(line2);
                 cur = nxt;
                 nxt = r + 2 * RS < count ? __ldg(sl + ((r + 2 * RS) >> 5)) : none;
-                if (left) ell_add(acc, e, xs, rate_at, lks);
+                if (left) add(acc, e);
                 e = f;
                 line = line2;
                 fn(r, (r << lks) | s, acc);
@@ -1674,12 +1730,28 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     GridBarrier gb = {g.bar, 0u, false};
     auto sync = [&]() {
         if constexpr (GRID) gb.wait();
+        else if constexpr (CLUSTER) cluster_sync();
         else scc_sync(team);
     };
     unsigned sums = 0;
     auto sum = [&](double* red, auto& v) {
         constexpr int NV = (int)(sizeof(v) / sizeof(double));
         scc_sum<NV>(red, lks, team, v);
+        if constexpr (CLUSTER) {
+            // the CTAs' sums, added in rank order by every thread
+            __shared__ double s_xch[2][3];
+            double* x = s_xch[sums++ & 1u];
+            if (team.tid == 0)
+#pragma unroll
+                for (int j = 0; j < NV; j++) x[j] = v[j];
+            cluster_sync();
+            const uint32_t at = shared_addr(x);
+#pragma unroll
+            for (int j = 0; j < NV; j++) {
+                v[j] = 0.0;
+                for (uint32_t c = 0; c < ranks; c++) v[j] += lds_cluster(at + 8 * j, c);
+            }
+        }
         if constexpr (GRID) {
             double* part = g.part + (size_t)(sums++ & 1u) * ((size_t)gridDim.x * 3 << lks);
             if (team.tid < KS)
@@ -1696,10 +1768,9 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         }
     };
     if (!GRID && rs == 0) {
-        A[(se << lks) | s] = 0.0;
-        W[(se << lks) | s] = 0.0;
+        A[(le_rows << lks) | s] = 0.0;
+        W[(le_rows << lks) | s] = 0.0;
     }
-    const double inv_s = 1.0 / (double)(se + so);
     // (four entries in flight: small groups are chains of such round trips to L2)
     auto rhs = [&](uint2 og, uint32_t v) {
         double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + v];
@@ -1725,7 +1796,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     if (GRID) __syncthreads();
-    else scc_sync(team);
+    else sync();
     // even rows: 1 / q (in A too, for the Schur diagonal), and b / q, kept in Z until the end
     each(se, [&](int r, int idx) {
         const uint32_t slot = ev0 + r;
@@ -1768,7 +1839,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             for (uint32_t j = 0; j < 4 * sl.x; j++) {
                 const uint32_t e =
                     __ldg(reinterpret_cast<const uint32_t*>(g.ell + (size_t)(sl.y + j / 4) * 32 + (r & 31)) + j % 4);
-                diag(e >> 3 & 63u, A[((e >> 9) << lks) | s]);
+                diag(e >> 3 & 63u, CLUSTER ? lds_cluster(shared_addr(A) + (e >> 6 & 0xFFF8u), e >> 22) : A[((e >> 9) << lks) | s]);
             }
         }
         q.set(idx, qv);
@@ -1812,7 +1883,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     }
     sum(red1, sum1);
     const double b2 = sum1[0];
-    if (!GRID && rs == 0) A[(so << lks) | s] = 0.0;  // 1 / q of an even row until here
+    if (!GRID && rs == 0) A[(lo_rows << lks) | s] = 0.0;  // 1 / q of an even row until here
     if (!MEM && dense) {
         // Gauss-Jordan without pivoting (the rows of an M-matrix, diagonally dominant by
         // columns); the true residual below decides whether it is good enough
@@ -2006,7 +2077,8 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             each(so, [&](int r, int idx) { g.Rb[(size_t)k * g.TS + g.pos[od0 + r]] = A[idx] * inv; });
         }
     }
-    if (act && rs == 0) {
+    if (CLUSTER) cluster_sync();  // no CTA leaves while others may read its shared memory
+    if (act && rs == 0 && rank == 0) {
         atomicMax(g.ratio + k, (unsigned long long)__double_as_longlong(b2 > 0.0 ? rr / b2 : 0.0));
         if (failed) g.fail[k] = 1;
         atomicMax(g.iters, its);
@@ -2795,19 +2867,20 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
 // Most rows of one parity of an SCC
 inline uint32_t scc_rows(const uint4& c) { return std::max(c.y, c.w); }
 
-// Slices of SCC j (see SweepPlan::sl): source[slice] = (first slot, rows, first slot of the
-// other parity, rows of the other parity)
+// Slices of SCC j (see SweepPlan::sl): source[slice] = (first slot, rows | 64 and the cluster
+// rank << 7 for an SCC split over a cluster, first slot of the other parity, its rows)
 __global__ void k_pl_slices(uint32_t count, const uint4* __restrict__ scc, const uint2* __restrict__ scc_sl,
                             uint4* __restrict__ source) {
     const uint32_t j = blockIdx.x;
     if (j >= count) return;
     const uint4 c = scc[j];
     const uint2 f = scc_sl[j];
-    if (f.x == kNoSlot) return;  // not solved by one CTA
+    if (f.x == kNoSlot) return;  // not solved by a CTA or a cluster
+    const bool split = max(c.y, c.w) > (uint32_t)kSccMaxRows;
     for (uint32_t r = threadIdx.x * 32; r < c.y; r += blockDim.x * 32)
-        source[f.x + r / 32] = make_uint4(c.x + r, min(32u, c.y - r), c.z, c.w);
+        source[f.x + r / 32] = make_uint4(c.x + r, min(32u, c.y - r) | (split ? 64u | r / kSccMaxRows << 7 : 0u), c.z, c.w);
     for (uint32_t r = threadIdx.x * 32; r < c.w; r += blockDim.x * 32)
-        source[f.y + r / 32] = make_uint4(c.z + r, min(32u, c.w - r), c.x, c.y);
+        source[f.y + r / 32] = make_uint4(c.z + r, min(32u, c.w - r) | (split ? 64u | r / kSccMaxRows << 7 : 0u), c.x, c.y);
 }
 
 // One warp per slice.  FILL false: its line count (four entries a line, the most of a row);
@@ -2819,7 +2892,7 @@ __global__ void k_pl_ell(uint32_t slices, const uint4* __restrict__ source, cons
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= slices) return;
     const uint4 src = source[w];
-    const bool row = lane < src.y;
+    const bool row = lane < (src.y & 63u);
     const uint32_t p = row ? ig_ptr[src.x + lane] : 0u;
     const uint32_t cnt = row ? ig_ptr[src.x + lane + 1] - p : 0u;
     if (!FILL) {
@@ -2828,15 +2901,17 @@ __global__ void k_pl_ell(uint32_t slices, const uint4* __restrict__ source, cons
         return;
     }
     const uint32_t lines = width[w];
+    const bool split = src.y & 64u;  // (see kSccCluster)
+    const uint32_t none = split ? (src.y >> 7) << 13 | (uint32_t)kSccMaxRows : src.w;
     if (lane == 0) sl[w] = make_uint2(lines, off[w]);
     for (uint32_t j = 0; j < lines; j++) {
         uint32_t e[4];
 #pragma unroll
         for (uint32_t u = 0; u < 4; u++) {
-            e[u] = src.w << 9;
+            e[u] = none << 9;
             if (4 * j + u < cnt) {
-                const uint32_t x = ig_ent[p + 4 * j + u];
-                e[u] = (ent_slot(x) - src.z) << 9 | (uint32_t)ent_rate(x) << 3;
+                const uint32_t x = ig_ent[p + 4 * j + u], r = ent_slot(x) - src.z;
+                e[u] = (split ? (r / kSccMaxRows) << 13 | r % kSccMaxRows : r) << 9 | (uint32_t)ent_rate(x) << 3;
             }
         }
         ell[((size_t)off[w] + j) * 32 + lane] = make_uint4(e[0], e[1], e[2], e[3]);
@@ -2855,7 +2930,13 @@ int finish_scc_list(esl_ctx* ctx, int n, SweepPlan* P) {
         for (auto c = b; c != e; ++c) {
             g.singles -= c->y + c->w;
             const uint32_t m = scc_rows(*c);
-            g.resident = g.resident && m <= (uint32_t)kSccMaxRows &&
+            const bool split = m > (uint32_t)kSccMaxRows;
+            g.split |= split;
+            if (split)
+                g.resident = g.resident && m <= (uint32_t)(kSccMaxRows * kSccMaxCluster) &&
+                             scc_smem_doubles(true, false, n, kSccMaxRows, kSccMaxRows, 0, kSccThreadsBig) * 8 <= kSccMaxSmem - 256;
+            else
+                g.resident = g.resident &&
                          scc_smem_doubles(m > kSccThreads, false, n, (int)c->y, (int)c->w, 0,
                                           (int)std::min<uint32_t>(kSccThreadsBig, (m + 31) & ~31u)) *
                                  8 <=
@@ -3104,6 +3185,8 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
 // keeps (row, system) pairs of small SCCs within kSccPairs threads; large SCCs, one CTA per
 // SM, take more systems while shared memory holds them and the SMs stay filled.
 constexpr int kSccPairs = 256;
+constexpr int kSccClusterMin = 8;  // fewer systems: kSccGrid uses more of the chip
+constexpr size_t kSccClusterSmem = kSccMaxSmem - 256;  // (static exchange buffers)
 constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
 // overlap: the launch may start, up to its first read of the sweep's vectors, before the
 // previous one ends (not for the sweep's first: the rates are being written).
@@ -3116,11 +3199,41 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, bo
     ga.sl = P->sl.get();
     ga.ell = P->ell.get();
     const uint4* list = P->h_scc.data() + g.s0;
-    uint32_t nbig = 0;
+    uint32_t nsplit = 0;
+    while (nsplit < g.ns && scc_rows(list[nsplit]) > (uint32_t)kSccMaxRows) nsplit++;
+    // SCCs split over clusters: one launch per cluster size
+    for (uint32_t j = 0; j < nsplit;) {
+        auto size = [&](uint32_t i) { return (scc_rows(list[i]) + kSccMaxRows - 1) / kSccMaxRows; };
+        uint32_t j1 = j + 1;
+        while (j1 < nsplit && size(j1) == size(j)) j1++;
+        if ((uint64_t)(j1 - j) * K * size(j) > 0x7FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
+        ga.nb = 1;
+        ga.b[0] = SccBucket{0, (j1 - j) * (uint32_t)K, j, 0, 0, 10, 1};
+        cudaLaunchAttribute attr[2]{};
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size(j);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((j1 - j) * (uint32_t)K * size(j));
+        cfg.blockDim = dim3(kSccThreadsBig);
+        cfg.dynamicSmemBytes = scc_smem_doubles(true, false, n, kSccMaxRows, kSccMaxRows, 0, kSccThreadsBig) * 8;
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = overlap ? 2 : 1;
+        auto kern = defl ? k_sw_scc<kSccCluster, true> : k_sw_scc<kSccCluster, false>;
+        ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccClusterSmem));
+        ESL_COUNT_LAUNCH();
+        ESL_CUDA(cudaLaunchKernelEx(&cfg, kern, ga));
+        overlap = true;
+        j = j1;
+    }
+    uint32_t nbig = nsplit;
     while (nbig < g.ns && scc_rows(list[nbig]) > (uint32_t)kSccThreads) nbig++;
     for (int part = 0; part < 2; part++) {
         const bool big = part == 0;
-        const uint32_t j0 = big ? 0 : nbig, j1 = big ? nbig : g.ns;
+        const uint32_t j0 = big ? nsplit : nbig, j1 = big ? nbig : g.ns;
         // buckets, and the items that a CTA per item would make
         uint64_t all = 0;
         ga.nb = 0;
@@ -3136,7 +3249,7 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, bo
             int lks = 0;
             if (big)
                 while (lks < lmax && doubles(lks + 1) * 8 <= kSccMaxSmem &&
-                       (uint64_t)nbig * (uint64_t)((K + (2 << lks) - 1) >> (lks + 1)) >= (uint64_t)ctx->sm_count)
+                       (uint64_t)(nbig - nsplit) * (uint64_t)((K + (2 << lks) - 1) >> (lks + 1)) >= (uint64_t)ctx->sm_count)
                     lks++;
             else
                 while (lks < lmax && (m << (lks + 1)) <= kSccPairs &&
@@ -3462,7 +3575,8 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             continue;
         }
         // (kSccGrid: where the rule lies, see there)
-        if (g.resident || K <= 32) {
+        const bool resident = g.resident && (!g.split || K >= kSccClusterMin);
+        if (resident || K <= 32) {
             SccArgs ga{};
             ga.a = a;
             ga.og_ptr = P->og_ptr.get();
@@ -3475,12 +3589,12 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ga.Z = Z;
             const int slots[12] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
             const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
-            for (int j = 0; j < (g.resident ? (big ? 5 : 0) : 12); j++) {
+            for (int j = 0; j < (resident ? (big ? 5 : 0) : 12); j++) {
                 const bool even = slots[j] == W_W64 || slots[j] == W_IQE;
                 ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(even ? P->max_even : P->max_odd, 1) * Kp * 8,
                                             &st_);
             }
-            if (!g.resident) {
+            if (!resident) {
                 ga.bar = reinterpret_cast<unsigned*>(d_cnt) + 8;
                 ga.part = (double*)ws.get(W_PART, (size_t)2 * ctx->sm_count * 3 * 32 * 8, &st_);
             }
@@ -3501,7 +3615,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             st.local_groups++;
             const bool overlap = !first_launch;
             first_launch = false;
-            if (g.resident) ESL_TRY(launch_scc(ctx, P, g, term, overlap, ga));
+            if (resident) ESL_TRY(launch_scc(ctx, P, g, term, overlap, ga));
             else ESL_TRY(launch_scc_grid(ctx, g, term, ga));
             if (debug_on()) {
                 ESL_CUDA(cudaStreamSynchronize(s));
