@@ -81,6 +81,7 @@ enum IScal { I_FLAGS, I_ITERS, I_NOIMP, I_TOTAL, I_STALL, I_NISCAL };
 
 struct SwGroup {
     uint32_t beg, ne, no;  // first slot, even rows, odd rows
+    uint32_t ob;           // first odd slot (beg + ne, except in a piece of a group)
     int kind;              // 0 singletons, 1 SCCs of at most kSwLocalMax states, 2 larger ones
     int max_scc;
     uint32_t scc0, nscc;   // local groups: range in the local SCC list (SCCs of >= 2 states)
@@ -141,7 +142,8 @@ struct SwArgs {
     const uint4* desc;       // per slot: (state, out-mask, first in-group entry, in-group count)
     const uint32_t* ig_ptr;
     const uint32_t* ig_ent;
-    uint32_t beg, ne, no;
+    // rows: ne even ones from slot beg, no odd ones from slot ob
+    uint32_t beg, ob, ne, no;
     const int* flags;        // per-system flags or null
     // FP64 out-rate sums of the group's rows, [row][Kp], or null (then recomputed from
     // the out-masks): q of the odd rows and 1 / q of the even rows
@@ -152,6 +154,9 @@ struct SwArgs {
     double* gam;
     double inv_s;
 };
+
+// slot of row r of a group (even rows first)
+__device__ __forceinline__ uint32_t sw_slot(const SwArgs& a, uint32_t r) { return r < a.ne ? a.beg + r : a.ob + (r - a.ne); }
 
 // A tile is KT systems of one row handled by TR = KT / S threads, S systems per thread:
 // thread `lane` of the row owns the adjacent systems k = lane * S, ..., k + S - 1 of the
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_rhs(SwArgs a, const uint32_t* __res
     if (__all_sync(0xffffffffu, !act)) return;
     const uint32_t cnt = a.ne + a.no;
     for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < cnt; r += gridDim.x * t.RB) {
-        const uint32_t slot = a.beg + r;
+        const uint32_t slot = sw_slot(a, r);
         const uint2 row = a.rows[slot];
         const uint32_t v = row.x;
         const uint32_t p0 = og_ptr[slot];
@@ -375,7 +380,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_diag(SwArgs a, double* __restrict__
     sw_rates(s_rate, a, t);
     if (t.k >= a.K) return;
     for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < a.no; r += gridDim.x * t.RB) {
-        const uint32_t slot = a.beg + a.ne + r;
+        const uint32_t slot = a.ob + r;
         const uint2 row = a.rows[slot];
         const uint32_t o = row.x;
         double d = sw_q(s_rate, o, row.y, t);
@@ -401,7 +406,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_qrows(SwArgs a, double* __restrict_
     sw_rates(s_rate, a, t);
     if (t.k >= a.K) return;
     for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < a.ne + a.no; r += gridDim.x * t.RB) {
-        const uint2 row = a.rows[a.beg + r];
+        const uint2 row = a.rows[sw_slot(a, r)];
         const double q = sw_q(s_rate, row.x, row.y, t);
         if (r < a.ne)
             IQe[(size_t)r * a.Kp + t.k] = 1.0 / q;
@@ -434,7 +439,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_elim(SwArgs a, const double* __rest
     // the gathers shuffle across the warp: a warp runs the row loop if any lane is active
     const bool wany = __any_sync(0xffffffffu, any);
     if (!DEFL && !wany) return;
-    const uint32_t obase = a.beg + a.ne;
+    const uint32_t obase = a.ob;
     for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < (wany ? a.ne : 0u); r += gridDim.x * t.RB) {
         // (state, out-mask, first entry, count) in one load
         const uint4 d = a.desc[a.beg + r];
@@ -506,7 +511,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_apply(SwArgs a, const T* __restrict
     }
     if (__any_sync(0xffffffffu, any)) {
         for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < a.no; r += gridDim.x * t.RB) {
-            const uint4 d = a.desc[a.beg + a.ne + r];  // (state, out-mask, first entry, count)
+            const uint4 d = a.desc[a.ob + r];  // (state, out-mask, first entry, count)
             const size_t idx = (size_t)r * a.Kp + t.k;
             T flow[S];
 #pragma unroll
@@ -689,7 +694,7 @@ __global__ void __launch_bounds__(kSwT, 8) k_sw_elim_pr(SwArgs a, const double* 
     act[1] = !sw_skip(a, t.k + 1);
     const bool any = act[0] || act[1];
     if (!__any_sync(0xffffffffu, any)) return;
-    const uint32_t count = a.ne, rs = gridDim.x * t.RB, obase = a.beg + a.ne;
+    const uint32_t count = a.ne, rs = gridDim.x * t.RB, obase = a.ob;
     // the warp's two rows are rw and rw + 1; the loop condition is warp-uniform
     for (uint32_t rw = blockIdx.x * t.RB + (t.rsub & ~1); rw < count; rw += rs) {
         const uint32_t r = rw + (t.rsub & 1);
@@ -723,7 +728,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_apply_pr(SwArgs a, const double* __
     act[1] = !sw_skip(a, t.k + 1);
     const bool any = act[0] || act[1];
     if (__any_sync(0xffffffffu, any)) {
-        const uint32_t count = a.no, rs = gridDim.x * t.RB, rowbase = a.beg + a.ne;
+        const uint32_t count = a.no, rs = gridDim.x * t.RB, rowbase = a.ob;
         for (uint32_t rw = blockIdx.x * t.RB + (t.rsub & ~1); rw < count; rw += rs) {
             const uint32_t r = rw + (t.rsub & 1);
             const PrRow p = pr_row(a, rowbase, r, count, (a.beg << kEntShift) | (uint32_t)(2 * a.n));
@@ -831,7 +836,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_defl_rhs(SwArgs a, double* __restri
     sw_rates(s_rate, a, t);
     if (t.k >= a.K) return;
     for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < a.ne + a.no; r += gridDim.x * t.RB) {
-        const uint2 row = a.rows[a.beg + r];
+        const uint2 row = a.rows[sw_slot(a, r)];
         Bv[(size_t)r * a.Kp + t.k] = r < a.ne ? 0.0 : sw_q(s_rate, row.x, row.y, t) * a.inv_s;
     }
 }
@@ -845,7 +850,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_term_out(SwArgs a, const uint32_t* 
     double d = 0.0;
     if (t.k < a.K) {
         for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < a.ne + a.no; r += gridDim.x * t.RB) {
-            const uint32_t slot = a.beg + r;
+            const uint32_t slot = sw_slot(a, r);
             const double v = Z[(size_t)slot * a.Kp + t.k];
             Rb[(size_t)t.k * TS + pos[slot]] = v;
             d += v;
@@ -1240,7 +1245,7 @@ __global__ void __launch_bounds__(kSwT) k_sw_init(SwArgs a, const double* __rest
     const Tile t = tile_of(a.KT);
     if (t.k >= a.K) return;
     for (uint32_t r = blockIdx.x * t.RB + t.rsub; r < a.no; r += gridDim.x * t.RB) {
-        const uint32_t slot = a.beg + a.ne + r;
+        const uint32_t slot = a.ob + r;
         const size_t idx = (size_t)r * a.Kp + t.k;
         double x;
         if (a.ig_ptr[slot] == a.ig_ptr[slot + 1])
@@ -1283,6 +1288,7 @@ constexpr int kSccMaxRows = 4096;  // most odd (or even) rows of an SCC solved b
 // of 26K to 31K (four) 31 -> 28 and 22 -> 14 ms against the row kernels; of 53K to 58K states
 // (eight) 31 -> 38 and 64 -> 78 ms.
 constexpr int kSccMaxCluster = 4;
+constexpr uint32_t kSccClusterRows = kSccMaxRows * kSccMaxCluster;
 // threads of a CTA with one row per thread (128 registers each), and with several
 constexpr int kSccThreads = 512, kSccThreadsBig = 1024;
 constexpr int kSccBuckets = 16;    // most (KS, team size) pairs of a launch
@@ -1460,7 +1466,7 @@ __device__ __forceinline__ void scc_singles(const SccArgs& g, uint32_t cta, uint
         const uint32_t t = (uint32_t)(u / rows), r = (uint32_t)(u - (uint64_t)t * rows);
         const int k = (int)(t << lw) + (int)(threadIdx.x & (KW - 1));
         if (k >= a.K) continue;
-        const uint32_t slot = a.beg + r;
+        const uint32_t slot = sw_slot(a, r);
         const uint4 d = a.desc[slot];
         if (d.w) continue;  // in an SCC of two or more states
         double acc = g.x0[(size_t)(k % a.nrhs) * g.x0_ld + d.x];
@@ -1573,7 +1579,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     double* s_scc = MEM ? s_all : s_all + (size_t)team.id * bu.stride;
     const int lks = bu.lks, KS = 1 << lks;
     const uint32_t tiles = (uint32_t)((a.K + KS - 1) >> lks), tile = item % tiles;
-    const uint4 sc = GRID ? make_uint4(a.beg, a.ne, a.beg + a.ne, a.no) : g.scc[bu.scc0 + item / tiles];
+    const uint4 sc = GRID ? make_uint4(a.beg, a.ne, a.ob, a.no) : g.scc[bu.scc0 + item / tiles];
     uint2 first = GRID ? make_uint2(0u, 0u) : g.scc_sl[bu.scc0 + item / tiles];
     // the rates, in flight with the SCC's description
     const int nact = team.threads;
@@ -2920,28 +2926,18 @@ __global__ void k_pl_ell(uint32_t slices, const uint4* __restrict__ source, cons
 
 // Sorts each group's SCC list by decreasing size (the launch order of k_sw_scc: a group
 // lasts as long as the CTA of its largest SCC, which must not start behind the small ones)
-// and marks the groups whose SCCs all fit a CTA.
-int finish_scc_list(esl_ctx* ctx, int n, SweepPlan* P) {
+// and lays out the predecessor lines of the SCCs that a CTA or a cluster solves.  Any SCC of
+// at most kSccMaxRows rows of either parity fits a CTA's shared memory at one system.
+static_assert((2 * (kSccMaxRows + 1) + 2 * 26 + 6 * (kSccThreadsBig / 32) + 5 * kSccMaxRows) * 8 <= (int)kSccMaxSmem - 256,
+              "k_sw_scc's arrays");
+int finish_scc_list(esl_ctx* ctx, SweepPlan* P) {
     for (SwGroup& g : P->groups) {
         const auto b = P->h_scc.begin() + g.s0, e = b + g.ns;
         std::stable_sort(b, e, [](const uint4& x, const uint4& y) { return scc_rows(x) > scc_rows(y); });
-        g.resident = true;
         g.singles = g.ne + g.no;
-        for (auto c = b; c != e; ++c) {
-            g.singles -= c->y + c->w;
-            const uint32_t m = scc_rows(*c);
-            const bool split = m > (uint32_t)kSccMaxRows;
-            g.split |= split;
-            if (split)
-                g.resident = g.resident && m <= (uint32_t)(kSccMaxRows * kSccMaxCluster) &&
-                             scc_smem_doubles(true, false, n, kSccMaxRows, kSccMaxRows, 0, kSccThreadsBig) * 8 <= kSccMaxSmem - 256;
-            else
-                g.resident = g.resident &&
-                         scc_smem_doubles(m > kSccThreads, false, n, (int)c->y, (int)c->w, 0,
-                                          (int)std::min<uint32_t>(kSccThreadsBig, (m + 31) & ~31u)) *
-                                 8 <=
-                             kSccMaxSmem;
-        }
+        for (auto c = b; c != e; ++c) g.singles -= c->y + c->w;
+        g.resident = g.ns == 0 || scc_rows(*b) <= kSccClusterRows;
+        g.split = g.ns > 0 && scc_rows(*b) > (uint32_t)kSccMaxRows;
     }
     if (P->h_scc.empty()) return ESL_OK;
     cudaStream_t s = ctx->stream;
@@ -2949,7 +2945,8 @@ int finish_scc_list(esl_ctx* ctx, int n, SweepPlan* P) {
     std::vector<uint2> first(count, make_uint2(kNoSlot, kNoSlot));
     uint32_t slices = 0;
     for (const SwGroup& g : P->groups)
-        for (uint32_t j = g.s0; g.resident && j < g.s0 + g.ns; j++) {
+        for (uint32_t j = g.s0; j < g.s0 + g.ns; j++) {
+            if (scc_rows(P->h_scc[j]) > kSccClusterRows) continue;
             first[j].x = slices;
             slices += (P->h_scc[j].y + 31) / 32;
             first[j].y = slices;
@@ -2999,8 +2996,8 @@ int build_plan(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     }
     SweepPlan* P = nullptr;
     ESL_TRY(build_plan_device(ctx, net, P));
-    int rc = finish_scc_list(ctx, net->n, P);
-    if (rc == ESL_OK && P->term) rc = finish_scc_list(ctx, net->n, P->term);
+    int rc = finish_scc_list(ctx, P);
+    if (rc == ESL_OK && P->term) rc = finish_scc_list(ctx, P->term);
     if (rc != ESL_OK) {
         delete P;
         return rc;
@@ -3101,7 +3098,7 @@ int build_whole_plan(esl_ctx* ctx, const esl_net* net, bool back, SweepPlan*& ou
     up(P->tp_ent, tp);
     if (back) up(P->rev, rev);
     if (rc == ESL_OK && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(ESL_ERR_CUDA, "plan upload failed");
-    if (rc == ESL_OK) rc = finish_scc_list(ctx, net->n, P.get());
+    if (rc == ESL_OK) rc = finish_scc_list(ctx, P.get());
     if (rc != ESL_OK) return rc;
     mnet->sweep_free = free_plan_sweep;
     out = P.get();
@@ -3180,7 +3177,7 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
     return dim3((unsigned)want, ty);
 }
 
-// Launches k_sw_scc over group g: its SCCs of more than kSccThreads rows, then the others
+// Launches k_sw_scc over group g without its first `skip` SCCs: its SCCs of more than kSccThreads rows, then the others
 // with its singleton rows.  KS, the systems of one CTA, is the largest power of two that
 // keeps (row, system) pairs of small SCCs within kSccPairs threads; large SCCs, one CTA per
 // SM, take more systems while shared memory holds them and the SMs stay filled.
@@ -3190,7 +3187,7 @@ constexpr size_t kSccClusterSmem = kSccMaxSmem - 256;  // (static exchange buffe
 constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
 // overlap: the launch may start, up to its first read of the sweep's vectors, before the
 // previous one ends (not for the sweep's first: the rates are being written).
-int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, bool overlap, SccArgs ga) {
+int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t skip, bool defl, bool overlap, SccArgs ga) {
     const int K = ga.a.K, n = ga.a.n;
     int lmax = 0;
     while (lmax < 5 && (1 << lmax) < K) lmax++;
@@ -3199,10 +3196,10 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, bool defl, bo
     ga.sl = P->sl.get();
     ga.ell = P->ell.get();
     const uint4* list = P->h_scc.data() + g.s0;
-    uint32_t nsplit = 0;
+    uint32_t nsplit = skip;
     while (nsplit < g.ns && scc_rows(list[nsplit]) > (uint32_t)kSccMaxRows) nsplit++;
     // SCCs split over clusters: one launch per cluster size
-    for (uint32_t j = 0; j < nsplit;) {
+    for (uint32_t j = skip; j < nsplit;) {
         auto size = [&](uint32_t i) { return (scc_rows(list[i]) + kSccMaxRows - 1) / kSccMaxRows; };
         uint32_t j1 = j + 1;
         while (j1 < nsplit && size(j1) == size(j)) j1++;
@@ -3545,6 +3542,46 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     std::vector<char> failed(K, 0);
     int total_iters = 0;
 
+    // arguments of k_sw_scc for group g (the row range is a's); resident: not kSccGrid
+    auto scc_args = [&](const SwGroup& g, bool resident, SccArgs& ga) -> int {
+        ga.a = a;
+        ga.og_ptr = P->og_ptr.get();
+        ga.og_ent = P->og_ent.get();
+        ga.x0 = x0;
+        ga.x0_ld = x0_ld;
+        ga.warm = term ? nullptr : o.d_warm;
+        ga.warm_ld = (size_t)net->N;
+        ga.rev = P->rev.get();
+        ga.Z = Z;
+        const int slots[12] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
+        const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
+        for (int j = 0; j < (resident ? (big ? 5 : 0) : 12); j++) {
+            const bool even = slots[j] == W_W64 || slots[j] == W_IQE;
+            ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(even ? P->max_even : P->max_odd, 1) * Kp * 8,
+                                        &st_);
+        }
+        if (!resident) {
+            ga.bar = reinterpret_cast<unsigned*>(d_cnt) + 8;
+            ga.part = (double*)ws.get(W_PART, (size_t)2 * ctx->sm_count * 3 * 32 * 8, &st_);
+        }
+        if (st_ != ESL_OK) return st_;
+        ga.tol2 = tol * tol;
+        ga.accept2 = kSwAcceptRel * kSwAcceptRel;
+        ga.max_iters = max_iters;
+        ga.max_outer = g.kind == 2 ? max_refine : max_refine + 3;
+        ga.stall = g.kind == 2 ? kSwStall64 : kSwStall;
+        ga.ratio = loc_ratio;
+        ga.fail = loc_fail;
+        ga.iters = loc_iters + (&g - P->groups.data());
+        if (term) {
+            ga.pos = P->pos.get();
+            ga.Rb = y;
+            ga.TS = net->term_states;
+        }
+        return ESL_OK;
+    };
+    uint32_t largest = 0;  // states of the largest SCC
+    for (const uint4& c : P->h_scc) largest = std::max(largest, c.y + c.w);
     bool first_launch = true;
     for (const SwGroup& g : P->groups) {
         // debug timing: wall time of the group with the stream drained on both sides
@@ -3557,6 +3594,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - g_t0).count();
         };
         a.beg = g.beg;
+        a.ob = g.beg + g.ne;
         a.Qo = a.IQe = nullptr;
         a.ne = g.ne;
         a.no = g.no;
@@ -3578,44 +3616,11 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         const bool resident = g.resident && (!g.split || K >= kSccClusterMin);
         if (resident || K <= 32) {
             SccArgs ga{};
-            ga.a = a;
-            ga.og_ptr = P->og_ptr.get();
-            ga.og_ent = P->og_ent.get();
-            ga.x0 = x0;
-            ga.x0_ld = x0_ld;
-            ga.warm = term ? nullptr : o.d_warm;
-            ga.warm_ld = (size_t)net->N;
-            ga.rev = P->rev.get();
-            ga.Z = Z;
-            const int slots[12] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
-            const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
-            for (int j = 0; j < (resident ? (big ? 5 : 0) : 12); j++) {
-                const bool even = slots[j] == W_W64 || slots[j] == W_IQE;
-                ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(even ? P->max_even : P->max_odd, 1) * Kp * 8,
-                                            &st_);
-            }
-            if (!resident) {
-                ga.bar = reinterpret_cast<unsigned*>(d_cnt) + 8;
-                ga.part = (double*)ws.get(W_PART, (size_t)2 * ctx->sm_count * 3 * 32 * 8, &st_);
-            }
-            if (st_ != ESL_OK) return st_;
-            ga.tol2 = tol * tol;
-            ga.accept2 = kSwAcceptRel * kSwAcceptRel;
-            ga.max_iters = max_iters;
-            ga.max_outer = g.kind == 2 ? max_refine : max_refine + 3;
-            ga.stall = g.kind == 2 ? kSwStall64 : kSwStall;
-            ga.ratio = loc_ratio;
-            ga.fail = loc_fail;
-            ga.iters = loc_iters + (&g - P->groups.data());
-            if (term) {
-                ga.pos = P->pos.get();
-                ga.Rb = y;
-                ga.TS = net->term_states;
-            }
+            ESL_TRY(scc_args(g, resident, ga));
             st.local_groups++;
             const bool overlap = !first_launch;
             first_launch = false;
-            if (resident) ESL_TRY(launch_scc(ctx, P, g, term, overlap, ga));
+            if (resident) ESL_TRY(launch_scc(ctx, P, g, 0, term, overlap, ga));
             else ESL_TRY(launch_scc_grid(ctx, g, term, ga));
             if (debug_on()) {
                 ESL_CUDA(cudaStreamSynchronize(s));
@@ -3624,6 +3629,43 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             }
             continue;
         }
+        // ---- grid-wide Krylov ----
+        // The SCCs of a group share no edge: those beyond a cluster are solved one by one,
+        // each with its own coefficients and end, the others and the singletons by k_sw_scc.
+        // As one block the group's iterations served the union of the SCCs' spectra on all of
+        // its rows (316,541 rows in SCCs of 126,976, 63,488, 63,488, 30,688, 30,688 and fewer
+        // states, 512 systems: 420 -> 312 ms).
+        std::vector<SwGroup> pieces;
+        for (uint32_t j = g.s0; j < g.s0 + g.ns && scc_rows(P->h_scc[j]) > kSccClusterRows; j++) {
+            const uint4& c = P->h_scc[j];
+            SwGroup q = g;
+            q.beg = c.x;
+            q.ne = c.y;
+            q.ob = c.z;
+            q.no = c.w;
+            // (the share of the rows, for the measurement hook)
+            q.nin = (uint64_t)((double)g.nin * (c.y + c.w) / std::max<uint32_t>(g.ne + g.no, 1));
+            pieces.push_back(q);
+        }
+        if (pieces.size() < g.ns || (!term && g.singles > 0)) {
+            SccArgs ga{};
+            const bool overlap = !first_launch;
+            first_launch = false;
+            ESL_TRY(scc_args(g, true, ga));
+            st.local_groups++;
+            ESL_TRY(launch_scc(ctx, P, g, (uint32_t)pieces.size(), term, overlap, ga));
+        }
+        for (const SwGroup& g : pieces) {
+        const uint32_t rows = g.ne + g.no;
+        a.beg = g.beg;
+        a.ob = g.ob;
+        a.ne = g.ne;
+        a.no = g.no;
+        a.flags = nullptr;
+        a.KT = KT64;
+        a.Qo = a.IQe = nullptr;
+        a.gam = nullptr;
+        a.inv_s = 1.0 / (double)std::max<uint32_t>(rows, 1);
         double* Bv = (double*)ws.get(W_BV, (size_t)P->max_rows * Kp * 8, &st_);
         if (st_ != ESL_OK) return st_;
         ESL_COUNT_LAUNCH();
@@ -3633,7 +3675,6 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             k_sw_rhs<false><<<row_grid(rows, Kp, KT64, ctx->sm_count), kSwT, sm64, s>>>(
                 a, P->og_ptr.get(), P->og_ent.get(), x0, x0_ld, Z, Bv);
         ESL_CUDA(cudaGetLastError());
-        // ---- grid-wide Krylov group ----
         st.krylov_groups++;
         const size_t vo = (size_t)std::max<uint32_t>(P->max_odd, 1) * Kp, ve = (size_t)std::max<uint32_t>(P->max_even, 1) * Kp;
         double* bS = (double*)ws.get(W_BS, vo * 8, &st_);
@@ -3652,7 +3693,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         void* vTT = ws.get(W_TT, vo * es, &st_);
         void* vD = ws.get(W_D, vo * es, &st_);
         if (st_ != ESL_OK) return st_;
-        double* X64 = Z + (size_t)(g.beg + g.ne) * Kp;  // the odd rows of the group, in place
+        double* X64 = Z + (size_t)g.ob * Kp;  // the odd rows, in place
         // tiles narrow enough that one tile's slice of a gathered vector stays in L2
         // the network's autotuned slice budget, or the default
         const int tmb = net->tune_tile_mb > 0 ? net->tune_tile_mb : ctx->tune_tile_mb;
@@ -3701,7 +3742,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ~NvtxRange() {
                 if (on) nvtxRangePop();
             }
-        } nvtx_range(!term && g.ne + g.no == P->max_rows);
+        } nvtx_range(!term && rows == largest);
         auto true_residual = [&]() -> int {
             a.flags = nullptr;
             a.KT = gKT64;
@@ -4096,6 +4137,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
                 fprintf(stderr, "[esl-sweep]   iterations per system: min %d p50 %d p90 %d p99 %d max %d\n",
                         its.front(), its[K / 2], its[(K * 9) / 10], its[(K * 99) / 100], its.back());
             }
+        }
         }
     }
     // masses into the terminal SCCs

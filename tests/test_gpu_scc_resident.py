@@ -6,7 +6,8 @@ or both set).  The split of the mass between them needs the transient solve, the
 the deflated one (dense up to 128 states).  2^(d-1) rows of each
 parity: d = 2 (a warp), 8 and 9 (several systems per CTA, one), 11 (one row per thread,
 1,024 threads), 12 and 13 (several rows per thread, the largest resident SCC), 14 (above
-it: the cooperative grid for few systems, clusters of two CTAs for more) and 15 (of four).
+it: the cooperative grid for few systems, clusters of two CTAs for more), 15 (of four) and 16
+(the row kernels).
 Batches: one system, a ragged tile, one more than a warp's lanes.
 
 Tolerance: the solver stops at a relative residual of 1e-10 and the tests of the other
@@ -43,7 +44,7 @@ def cube_with_exits(d):
 
 @pytest.mark.parametrize("d,B,R", [(2, 1, 1), (2, 33, 1), (8, 5, 1), (9, 3, 2), (11, 1, 1), (11, 33, 1), (12, 2, 1),
                                    (13, 1, 1), (13, 3, 1), (14, 1, 1),
-                                   (14, 9, 2), (14, 33, 1), (15, 8, 1)])
+                                   (14, 9, 2), (14, 33, 1), (15, 8, 1), (16, 33, 1)])
 @pytest.mark.parametrize("method", ["direct", "mixed"])
 def test_cube_with_exits(esl, d, B, R, method):
     n = d + 2
