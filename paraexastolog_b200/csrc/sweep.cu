@@ -1967,8 +1967,9 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             });
             sum(red1, v);
             rr = v[0];
-            if (dense && outer == 0 && !done && !(rr < b2)) {
-                // a zero start is better (a singular block, overflow)
+            if (dense && outer == 0 && act && !(rr < b2)) {
+                // a zero start is better (a singular block, overflow), and the answer where
+                // the SCC gets no mass (b2 == 0: done already, whatever the pivots were)
                 each(so, [&](int r, int idx) {
                     g.Z[(size_t)(od0 + r) * Kp + k] = 0.0;
                     R.set(idx, BS.get(idx));
