@@ -36,7 +36,8 @@ def _newer(target: str, deps) -> bool:
 def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(OUT_DIR, exist_ok=True)
     objs = []
-    headers = [os.path.join(CSRC, "esl_internal.h"), os.path.join(REPO, "include", "esl_b200.h")]
+    headers = [os.path.join(CSRC, "esl_internal.h"), os.path.join(CSRC, "scc_plan.h"),
+               os.path.join(REPO, "include", "esl_b200.h")]
     flags = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-extended-lambda",
                     "-I" + os.path.join(REPO, "include"), "-I" + CSRC]
     for src in SOURCES:

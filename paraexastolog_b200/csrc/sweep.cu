@@ -43,6 +43,7 @@
 #include <nvtx3/nvToolsExt.h>
 
 #include "esl_internal.h"
+#include "scc_plan.h"
 
 namespace esl {
 namespace {
@@ -1317,7 +1318,7 @@ struct SccArgs {
     size_t warm_ld;
     const uint32_t* rev; // per slot, flips whose reverse of the row's entries exists (null: the out-mask)
     double* Z;           // [slot][Kp]
-    double* own[12];     // group-sized scratch: 5 odd-row vectors (kSccBig), all 12 (kSccGrid)
+    double* own[kOwnCount];  // group-sized scratch, see SccOwn (kSccBig: the first five)
     unsigned* bar;       // kSccGrid: barrier arrivals (0 before the launch), and a failure flag
     double* part;        // kSccGrid: 2 x CTAs x 3 x KS partial sums
     double tol2, accept2;
@@ -1608,16 +1609,23 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     const size_t Kp = a.Kp;
     const bool act = k < a.K;
     // both with a zero row past the last, for the entries that a row of a slice lacks
-    double* A = GRID ? g.own[5] : rate + ((size_t)(2 * a.n) << lks);  // odd rows: the vector whose product is formed
-    double* W = GRID ? g.own[6] : A + ((size_t)(sm + 1) << lks);      // even rows: its elimination
+    double* A = GRID ? g.own[kOwnA] : rate + ((size_t)(2 * a.n) << lks);  // odd rows: the vector whose product is formed
+    double* W = GRID ? g.own[kOwnW] : A + ((size_t)(sm + 1) << lks);      // even rows: its elimination
     double* red0 = GRID ? rate + ((size_t)(2 * a.n) << lks) : W + ((size_t)(le_rows + 1) << lks);
     double* red1 = red0 + ((size_t)(2 * (nact >> 5)) << lks);
     double* red2 = red1 + ((size_t)(3 * (nact >> 5)) << lks);
     SccVec<MEM> R, V, P, T, IQ, R0, D, dS, q, BS;
     if constexpr (GRID) {
-        SccVec<MEM>* const all[10] = {&R0, &D, &dS, &q, &BS, &R, &V, &P, &T, &IQ};
-#pragma unroll
-        for (int j = 0; j < 10; j++) all[j]->mem = g.own[j < 5 ? j : j + 2];
+        R0.mem = g.own[kOwnR0];
+        D.mem = g.own[kOwnD];
+        dS.mem = g.own[kOwnDS];
+        q.mem = g.own[kOwnQ];
+        BS.mem = g.own[kOwnBS];
+        R.mem = g.own[kOwnR];
+        V.mem = g.own[kOwnV];
+        P.mem = g.own[kOwnP];
+        T.mem = g.own[kOwnT];
+        IQ.mem = g.own[kOwnIQ];
     }
     if constexpr (BIG) {
         R.mem = red2 + ((size_t)(nact >> 5) << lks);
@@ -1627,11 +1635,11 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         IQ.mem = T.mem + ((size_t)lo_rows << lks);
         // the SCC's block of odd rows x Kp of a group vector, tile by tile (row by row there)
         const size_t o = (size_t)(sc.z - a.beg - a.ne) * Kp + (size_t)tile * KS * sc.w + (CLUSTER ? rank * kSccMaxRows : 0);
-        R0.mem = g.own[0] + o;
-        D.mem = g.own[1] + o;
-        dS.mem = g.own[2] + o;
-        q.mem = g.own[3] + o;
-        BS.mem = g.own[4] + o;
+        R0.mem = g.own[kOwnR0] + o;
+        D.mem = g.own[kOwnD] + o;
+        dS.mem = g.own[kOwnDS] + o;
+        q.mem = g.own[kOwnQ] + o;
+        BS.mem = g.own[kOwnBS] + o;
     }
     // one row per thread: its first two lines stay in registers
     uint4 ee[2], eo[2];
@@ -3554,13 +3562,10 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         ga.warm_ld = (size_t)net->N;
         ga.rev = P->rev.get();
         ga.Z = Z;
-        const int slots[12] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
+        const int slots[kOwnCount] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
         const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
-        for (int j = 0; j < (resident ? (big ? 5 : 0) : 12); j++) {
-            const bool even = slots[j] == W_W64 || slots[j] == W_IQE;
-            ga.own[j] = (double*)ws.get(slots[j], (size_t)std::max<uint32_t>(even ? P->max_even : P->max_odd, 1) * Kp * 8,
-                                        &st_);
-        }
+        for (int j = 0; j < (resident ? (big ? kOwnBS + 1 : 0) : kOwnCount); j++)
+            ga.own[j] = (double*)ws.get(slots[j], (size_t)scc_own_rows(j, P->max_even, P->max_odd) * Kp * 8, &st_);
         if (!resident) {
             ga.bar = reinterpret_cast<unsigned*>(d_cnt) + 8;
             ga.part = (double*)ws.get(W_PART, (size_t)2 * ctx->sm_count * 3 * 32 * 8, &st_);
