@@ -285,6 +285,11 @@ int masks_from_csc(int n, const int32_t* indptr, const int32_t* rows, uint32_t* 
 
 // graph.cu
 int build_graph(esl_ctx* ctx, esl_net* net);
+// Bound of a wait at the barrier of a cooperative launch (seconds), and the one for its
+// test: with ESL_BARRIER_TIMEOUT_TEST=1 (read per call) the barriers expect one arrival more
+// than there are CTAs, so that the wait runs out and the call returns ESL_ERR_TIMEOUT.
+constexpr unsigned kBarrierPolls = 1u << 24, kBarrierTestPolls = 1u << 10;
+bool barrier_timeout_test();
 
 // solve.cu
 void free_workspace(void* w);

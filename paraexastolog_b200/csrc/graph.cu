@@ -53,7 +53,6 @@ inline unsigned blocks_for(uint64_t N) { return (unsigned)((N + kThreads - 1) / 
 // 28 rounds whose live sets shrink 2.5 times slower.
 constexpr int kSccT = 1024;
 constexpr uint32_t kReached = 0x80000000u;
-constexpr unsigned kBarrierPolls = 1u << 24;  // bound of a barrier wait (seconds)
 
 struct GraphState {        // device, zeroed before the launch
     unsigned arrived;      // grid barrier: arrivals so far
@@ -76,6 +75,8 @@ struct GraphArgs {
     uint64_t* keys;
     int32_t* vals;
     int64_t budget;    // passes per fixpoint
+    unsigned polls;    // bound of a barrier wait
+    unsigned missing;  // arrivals that never come (0, or 1 when the bounded wait is tested)
     GraphState* st;
 };
 
@@ -90,20 +91,26 @@ __device__ __forceinline__ uint32_t priority_of(uint32_t v, int n) {
     return (v * 0xC2B2AE35u) & m;
 }
 
-// Grid barrier with a bounded wait; false once the launch has failed anywhere.
-__device__ bool grid_barrier(GraphState* st, unsigned& target) {
+// Grid barrier with a bounded wait; false once the launch has failed anywhere.  One thread
+// reads the status for its CTA: threads that read it themselves could see it change between
+// their reads, and part of a CTA would leave while the rest waits for it.
+__device__ bool grid_barrier(const GraphArgs& g, unsigned& target) {
+    __shared__ bool s_ok;
+    GraphState* st = g.st;
     __syncthreads();
     target += gridDim.x;
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(&st->arrived, 1u);
         unsigned polls = 0;
-        while (*(volatile unsigned*)&st->arrived < target && *(volatile int*)&st->status != 2)
-            if (++polls > kBarrierPolls) atomicExch(&st->status, 2);
+        // (the difference, not the order: the arrivals may wrap around)
+        while ((int)(*(volatile unsigned*)&st->arrived - target) < 0 && *(volatile int*)&st->status != 2)
+            if (++polls > g.polls) atomicExch(&st->status, 2);
         __threadfence();
+        s_ok = *(volatile int*)&st->status == 0;
     }
     __syncthreads();
-    return *(volatile int*)&st->status == 0;
+    return s_ok;
 }
 
 // Calls fn on the values of arr at the neighbours of v in mask, eight at a time (0 past the
@@ -128,7 +135,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
     GraphState* st = g.st;
     uint32_t* list = g.list + (size_t)cta * g.cap;
     __shared__ unsigned s_warp[kSccT / 32 + 1];
-    unsigned target = 0, phase = 0;
+    unsigned target = g.missing, phase = 0;
     // state i of this CTA
     auto state_at = [&](uint32_t i) { return ((i >> 5) * ctas + cta) * 32u + (i & 31u); };
     const uint32_t chunks = (g.N + 31) / 32;
@@ -176,7 +183,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
             used += p;
             if (cta == 0 && tid == 0) st->changed[(phase + 1) % 3] = 0;
             if (__syncthreads_or(ch) && tid == 0) st->changed[phase % 3] = 1;
-            if (!grid_barrier(st, target)) return false;
+            if (!grid_barrier(g, target)) return false;
             const unsigned any = *(volatile unsigned*)&st->changed[phase % 3];
             phase++;
             if (!any) return true;
@@ -194,7 +201,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
         g.canon[v] = 0x7FFFFFFF;
         g.level[v] = 1;
     }
-    if (!grid_barrier(st, target)) return;
+    if (!grid_barrier(g, target)) return;
     uint32_t live = g.N;
     unsigned round = 0;
     bool seeded = false;
@@ -223,7 +230,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
         if (cta == 0 && tid == 0) st->live[(round + 1) % 3] = 0;
         if (tid == 0 && count) atomicAdd(&st->live[round % 3], count);
         for (uint32_t i = tid; i < count; i += kSccT) __stcg(g.color + list[i], priority_of(list[i], g.n) + 1u);
-        if (!grid_barrier(st, target)) return;
+        if (!grid_barrier(g, target)) return;
         live = *(volatile unsigned*)&st->live[round % 3];
         if (live == 0) break;
         // largest priority among the live ancestors
@@ -280,12 +287,12 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
         const uint32_t v = state_at(i);
         if (v < g.N) atomicMin(&g.canon[g.lab[v]], (int32_t)v);
     }
-    if (!grid_barrier(st, target)) return;
+    if (!grid_barrier(g, target)) return;
     for (uint32_t i = tid; i < own; i += kSccT) {
         const uint32_t v = state_at(i);
         if (v < g.N) g.lab[v] = __ldcg(g.canon + g.lab[v]);
     }
-    if (!grid_barrier(st, target)) return;
+    if (!grid_barrier(g, target)) return;
     // levels, stored at the SCC's label: 1 + the largest level among successor SCCs.  The
     // list takes each state's flips that leave its SCC, the colours a copy of its SCC's
     // level, which neighbours read without going through the label.
@@ -302,7 +309,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
         }
         list[i] = x;
     }
-    if (!grid_barrier(st, target)) return;
+    if (!grid_barrier(g, target)) return;
     if (!fixpoint(own, g.N > 2u * kSccT * ctas ? 1u : 4u, false, [&](uint32_t i) {
             const uint32_t v = state_at(i);
             if (v >= g.N) return false;
@@ -392,6 +399,11 @@ __global__ void k_domain_masks(int n, uint64_t N, const uint32_t* __restrict__ F
 
 }  // namespace
 
+bool barrier_timeout_test() {
+    const char* e = getenv("ESL_BARRIER_TIMEOUT_TEST");
+    return e && e[0] == '1';
+}
+
 int build_graph(esl_ctx* ctx, esl_net* net) {
     const uint64_t N = (uint64_t)net->N;
     const int n = net->n;
@@ -438,6 +450,9 @@ int build_graph(esl_ctx* ctx, esl_net* net) {
         // a pass can only fail to progress once per state (or the context's budget)
         ga.budget = ctx->graph_sweeps > 0 ? ctx->graph_sweeps : (int64_t)N + 64;
         ga.st = state.get();
+        const bool no_end = barrier_timeout_test();
+        ga.polls = no_end ? kBarrierTestPolls : kBarrierPolls;
+        ga.missing = no_end ? 1 : 0;
         ESL_CUDA(cudaMemsetAsync(state.get(), 0, sizeof(GraphState), s));
         GraphState h{};
         {
