@@ -1320,6 +1320,7 @@ struct SccArgs {
     double* Z;           // [slot][Kp]
     double* own[kOwnCount];  // group-sized scratch, see SccOwn (kSccBig: the first five)
     unsigned* bar;       // kSccGrid: barrier arrivals (0 before the launch), and a failure flag
+    unsigned polls, missing;  // kSccGrid: bound of a barrier wait; arrivals that never come (a test's)
     double* part;        // kSccGrid: 2 x CTAs x 3 x KS partial sums
     double tol2, accept2;
     int max_iters, max_outer, stall;
@@ -1333,30 +1334,32 @@ struct SccArgs {
 };
 
 // Barrier of a cooperative launch.  A wait is bounded: past the bound it sets the failure
-// flag and neither this CTA nor, once they see the flag, the others wait any more (their
-// iteration budgets end the launch; the host reports the flag).
-constexpr unsigned kGridPolls = 1u << 24;
+// flag, which ends the other CTAs' waits too.  A CTA whose wait ended that way is `dead`, all
+// of its threads alike: it takes no part in later barriers and sums and leaves its loops, so
+// that the CTAs that still run read nothing that it wrote afterwards into their decisions.
 struct GridBarrier {
     unsigned* bar;
-    unsigned target;
+    unsigned target, polls;
     bool dead;
     __device__ __forceinline__ void wait() {
+        __shared__ bool s_dead;
         __syncthreads();
+        if (dead) return;
         target += gridDim.x;
-        if (threadIdx.x == 0 && !dead) {
+        if (threadIdx.x == 0) {
+            bool gone = false;
             __threadfence();
             atomicAdd(bar, 1u);
-            unsigned polls = 0;
-            while ((int)(*(volatile unsigned*)bar - target) < 0) {
-                if (*(volatile unsigned*)(bar + 1)) {
-                    dead = true;
-                    break;
-                }
-                if (++polls > kGridPolls) atomicExch(bar + 1, 1u);
+            unsigned n = 0;
+            while (!gone && (int)(*(volatile unsigned*)bar - target) < 0) {
+                if (*(volatile unsigned*)(bar + 1)) gone = true;
+                else if (++n > polls) atomicExch(bar + 1, 1u);
             }
             __threadfence();
+            s_dead = gone;
         }
         __syncthreads();
+        dead = s_dead;
     }
 };
 
@@ -1741,7 +1744,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     constexpr auto odd_rows = std::false_type{};
     // barrier of all threads of the item, and sums over them (see scc_sum); a grid's CTAs
     // add up their sums in one order, so that they take the same decisions
-    GridBarrier gb = {g.bar, 0u, false};
+    GridBarrier gb = {g.bar, g.missing, g.polls, false};
     auto sync = [&]() {
         if constexpr (GRID) gb.wait();
         else if constexpr (CLUSTER) cluster_sync();
@@ -1767,6 +1770,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             }
         }
         if constexpr (GRID) {
+            if (gb.dead) return;
             double* part = g.part + (size_t)(sums++ & 1u) * ((size_t)gridDim.x * 3 << lks);
             if (team.tid < KS)
 #pragma unroll
@@ -1962,7 +1966,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     }
     double prev = 0.0, rr = b2;
     int noimp = 0, its = 0;
-    for (int outer = 0;; outer++) {
+    for (int outer = 0; !gb.dead; outer++) {
         if (outer > 0 || warm || dense) {
             // true residual r = b - S x
             load_x();
@@ -2020,7 +2024,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         sync();
         double rho = 1.0, best = 1.0;
         int it = 0, stall = 0;
-        while (__any_sync(0xffffffffu, run)) {
+        while (!gb.dead && __any_sync(0xffffffffu, run)) {
             elim();
             double v1[1] = {0.0};
             apply([&](int idx, double y) {
@@ -2071,6 +2075,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         its += it;
         if (started) each(so, [&](int r, int idx) { g.Z[(size_t)(od0 + r) * Kp + k] += nrm * D.get(idx); });
     }
+    if (gb.dead) return;  // the call fails
     // even rows from the odd solution
     load_x();
     double total[1] = {0.0};
@@ -3192,7 +3197,7 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
 // SM, take more systems while shared memory holds them and the SMs stay filled.
 constexpr int kSccPairs = 256;
 constexpr int kSccClusterMin = 8;  // fewer systems: kSccGrid uses more of the chip
-constexpr size_t kSccClusterSmem = kSccMaxSmem - 256;  // (static exchange buffers)
+constexpr size_t kSccDynSmem = kSccMaxSmem - 256;  // beside the static arrays of kSccCluster and kSccGrid
 constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
 // overlap: the launch may start, up to its first read of the sweep's vectors, before the
 // previous one ends (not for the sweep's first: the rates are being written).
@@ -3229,7 +3234,7 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t skip
         cfg.attrs = attr;
         cfg.numAttrs = overlap ? 2 : 1;
         auto kern = defl ? k_sw_scc<kSccCluster, true> : k_sw_scc<kSccCluster, false>;
-        ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccClusterSmem));
+        ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccDynSmem));
         ESL_COUNT_LAUNCH();
         ESL_CUDA(cudaLaunchKernelEx(&cfg, kern, ga));
         overlap = true;
@@ -3337,7 +3342,7 @@ int launch_scc_grid(esl_ctx* ctx, const SwGroup& g, bool defl, SccArgs ga) {
     const size_t smem = ((size_t)(2 * ga.a.n + 6 * (kSccThreadsBig / 32)) << lks) * 8;
     const void* kern = defl ? (const void*)k_sw_scc<kSccGrid, true> : (const void*)k_sw_scc<kSccGrid, false>;
     if (smem > 48 * 1024)
-        ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
+        ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccDynSmem));
     ESL_CUDA(cudaMemsetAsync(ga.bar, 0, sizeof(unsigned), ctx->stream));
     void* args[] = {&ga};
     ESL_COUNT_LAUNCH();
@@ -3568,6 +3573,9 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             ga.own[j] = (double*)ws.get(slots[j], (size_t)scc_own_rows(j, P->max_even, P->max_odd) * Kp * 8, &st_);
         if (!resident) {
             ga.bar = reinterpret_cast<unsigned*>(d_cnt) + 8;
+            const bool no_end = barrier_timeout_test();
+            ga.polls = no_end ? kBarrierTestPolls : kBarrierPolls;
+            ga.missing = no_end ? 1 : 0;
             ga.part = (double*)ws.get(W_PART, (size_t)2 * ctx->sm_count * 3 * 32 * 8, &st_);
         }
         if (st_ != ESL_OK) return st_;
