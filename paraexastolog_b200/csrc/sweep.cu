@@ -1284,25 +1284,11 @@ __global__ void __launch_bounds__(kSwT) k_sw_warm_scale(SwArgs a, const double* 
 // The SCCs of a launch are listed largest first and cut into buckets of equal KS and team
 // size.  CTAs past the last item serve the group's singleton SCCs (rows without in-group
 // predecessors): z = b / q.
-constexpr int kSccMaxRows = 4096;  // most odd (or even) rows of an SCC solved by one CTA
-// Most CTAs that share a larger one.  512 systems: SCCs of 16K states (two) 11.2 -> 6 ms and
+// Most CTAs that share an SCC beyond kSccMaxRows rows of a parity.  512 systems: SCCs of 16K states (two) 11.2 -> 6 ms and
 // of 26K to 31K (four) 31 -> 28 and 22 -> 14 ms against the row kernels; of 53K to 58K states
 // (eight) 31 -> 38 and 64 -> 78 ms.
 constexpr int kSccMaxCluster = 4;
 constexpr uint32_t kSccClusterRows = kSccMaxRows * kSccMaxCluster;
-// threads of a CTA with one row per thread (128 registers each), and with several
-constexpr int kSccThreads = 512, kSccThreadsBig = 1024;
-constexpr int kSccBuckets = 16;    // most (KS, team size) pairs of a launch
-constexpr size_t kSccMaxSmem = 227 * 1024;
-
-struct SccBucket {
-    uint32_t cta0, items;  // first CTA, work items
-    uint32_t scc0;         // first SCC (relative to SccArgs::scc)
-    uint32_t stride;       // doubles of shared memory per team
-    uint8_t lks, lteam;    // log2 KS, log2 threads of a team
-    uint8_t teams;         // teams per CTA
-};
-
 struct SccArgs {
     SwArgs a;
     const uint4* scc;  // the launch's SCCs: (first even slot, even rows, first odd slot, odd rows)
@@ -1511,29 +1497,12 @@ struct SccVec {
     }
 };
 
-// SCCs of at most kSccDense odd rows are solved by elimination: a Krylov iteration is a
-// chain of FP64 reductions, about 4 us however small the SCC, an elimination step one
-// barrier and a division (n=12 x 64 rate sets 1.93 -> 1.5 ms; at 32 rows the steps cost as
-// much as the iterations, n=22 67 -> 61 ms).  A budget of fewer iterations than rows is too
-// small for it.
-constexpr int kSccDense = 16;
-__host__ __device__ inline bool scc_dense(int so, int max_iters) { return so <= kSccDense && so <= max_iters; }
-__host__ __device__ inline int scc_dense_ld(int so) { return (so + 1) | 1; }
-
 // 1 / x to about an ulp: two Newton steps from a single-precision reciprocal (not finite
 // where x is outside its range; the elimination's residual check then rejects the result)
 __device__ __forceinline__ double scc_recip(double x) {
     double r = (double)(1.0f / (float)x);
     r = fma(r, fma(-x, r, 1.0), r);
     return fma(r, fma(-x, r, 1.0), r);
-}
-
-// shared-memory doubles of a work item (see the carving in k_sw_scc)
-__host__ __device__ inline size_t scc_smem_doubles(bool big, bool dense, int n, int se, int so, int lks, int nact) {
-    const size_t m = (size_t)(se > so ? se : so), KS = (size_t)1 << lks;
-    return (m + 1 + se + 1 + 2 * n + 6 * (size_t)(nact >> 5) + (big ? 4 * (size_t)so + se : 0) +
-            (dense ? (size_t)so * scc_dense_ld(so) + 2 : 0)) *
-           KS;
 }
 
 // kSccSmall: SCCs of at most kSccThreads rows of either parity, a thread per row and
@@ -3192,19 +3161,13 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
 }
 
 // Launches k_sw_scc over group g without its first `skip` SCCs: its SCCs of more than kSccThreads rows, then the others
-// with its singleton rows.  KS, the systems of one CTA, is the largest power of two that
-// keeps (row, system) pairs of small SCCs within kSccPairs threads; large SCCs, one CTA per
-// SM, take more systems while shared memory holds them and the SMs stay filled.
-constexpr int kSccPairs = 256;
+// with its singleton rows (see plan_scc_launch).
 constexpr int kSccClusterMin = 8;  // fewer systems: kSccGrid uses more of the chip
 constexpr size_t kSccDynSmem = kSccMaxSmem - 256;  // beside the static arrays of kSccCluster and kSccGrid
-constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
 // overlap: the launch may start, up to its first read of the sweep's vectors, before the
 // previous one ends (not for the sweep's first: the rates are being written).
 int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t skip, bool defl, bool overlap, SccArgs ga) {
     const int K = ga.a.K, n = ga.a.n;
-    int lmax = 0;
-    while (lmax < 5 && (1 << lmax) < K) lmax++;
     ga.scc = P->scc.get() + g.s0;
     ga.scc_sl = P->scc_sl.get() + g.s0;
     ga.sl = P->sl.get();
@@ -3245,77 +3208,39 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t skip
     for (int part = 0; part < 2; part++) {
         const bool big = part == 0;
         const uint32_t j0 = big ? nsplit : nbig, j1 = big ? nbig : g.ns;
-        // buckets, and the items that a CTA per item would make
-        uint64_t all = 0;
-        ga.nb = 0;
-        for (uint32_t j = j0; j < j1; j++) {
-            const int se = (int)list[j].y, so = (int)list[j].w, m = std::max(se, so);
-            const bool dense = !big && !defl && scc_dense(so, ga.max_iters);
-            auto lteam = [&](int l) {
-                int t = big ? 10 : 5;
-                while (!big && (1 << t) < (m << l)) t++;
-                return t;
-            };
-            auto doubles = [&](int l) { return scc_smem_doubles(big, dense, n, se, so, l, 1 << lteam(l)); };
-            int lks = 0;
-            if (big)
-                while (lks < lmax && doubles(lks + 1) * 8 <= kSccMaxSmem &&
-                       (uint64_t)(nbig - nsplit) * (uint64_t)((K + (2 << lks) - 1) >> (lks + 1)) >= (uint64_t)ctx->sm_count)
-                    lks++;
+        std::vector<SccShape> shapes;
+        for (uint32_t j = j0; j < j1; j++)
+            if (!shapes.empty() && shapes.back().even == list[j].y && shapes.back().odd == list[j].w)
+                shapes.back().count++;
             else
-                while (lks < lmax && (m << (lks + 1)) <= kSccPairs &&
-                       (!dense || doubles(lks + 1) * 8 <= kSccDenseSmem))
-                    lks++;
-            // an SCC's KS is at least that of the larger ones before it
-            if (ga.nb > 0) lks = std::max<int>(lks, ga.b[ga.nb - 1].lks);
-            const int lt = lteam(lks);
-            if (ga.nb == 0 || ga.b[ga.nb - 1].lks != lks || ga.b[ga.nb - 1].lteam != lt) {
-                if (ga.nb == kSccBuckets) return fail(ESL_ERR_INVALID, "too many buckets");
-                ga.b[ga.nb++] = SccBucket{0, 0, j, 0, (uint8_t)lks, (uint8_t)lt, 1};
-            }
-            SccBucket& b = ga.b[ga.nb - 1];
-            const uint64_t its = (uint64_t)((K + (1 << lks) - 1) >> lks);
-            if (all + its > 0x3FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
-            b.items += (uint32_t)its;
-            all += its;
-            b.stride = std::max<uint32_t>(b.stride, (uint32_t)doubles(lks));
-        }
-        // Items share CTAs once there are more of them than SMs; a CTA then has the threads
-        // of the largest team at least
-        int threads = 32;
-        size_t smem = 0;
-        uint32_t items = 0, ctas = 0;
-        for (int j = 0; j < ga.nb; j++) threads = std::max(threads, 1 << ga.b[j].lteam);
-        if (!big && all > (uint64_t)ctx->sm_count) threads = std::max(threads, kSccPairs);
-        for (int j = 0; j < ga.nb; j++) {
-            SccBucket& b = ga.b[j];
-            if (!big && all > (uint64_t)ctx->sm_count)
-                b.teams = (uint8_t)std::max<size_t>(
-                    1, std::min<size_t>({(size_t)(threads >> b.lteam), (size_t)16, kSccTeamSmem / (b.stride * 8)}));
-            b.cta0 = items;
-            items += (b.items + b.teams - 1) / b.teams;
-            smem = std::max(smem, (size_t)b.teams * b.stride * 8);
-        }
-        ga.ctas = items;
+                shapes.push_back({list[j].y, list[j].w, 1});
+        SccLaunch L;
+        if (!plan_scc_launch(shapes.data(), shapes.size(), j0, big, defl, K, n, ga.max_iters, ctx->sm_count, L))
+            return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
+        std::copy(L.b, L.b + L.nb, ga.b);
+        ga.nb = L.nb;
+        ga.ctas = L.ctas;
+        int threads = L.threads;
+        uint32_t singles = 0;  // CTAs for the singleton rows
         if (!big && !defl && g.singles > 0) {
             threads = std::max(threads, 128);
             const uint64_t pairs = (uint64_t)(g.ne + g.no) * (uint64_t)K;
-            ctas = (uint32_t)std::max<uint64_t>(
+            singles = (uint32_t)std::max<uint64_t>(
                 1, std::min<uint64_t>((pairs + threads - 1) / threads, (uint64_t)ctx->sm_count * 8));
         }
-        if (items + ctas == 0) continue;
+        if (L.ctas + singles == 0) continue;
         auto go = [&](auto kern) -> int {
             // the same limit from every thread: contexts set it concurrently
-            if (smem > 48 * 1024)
+            if (L.smem > 48 * 1024)
                 ESL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSccMaxSmem));
             ESL_COUNT_LAUNCH();
             cudaLaunchAttribute attr{};
             attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr.val.programmaticStreamSerializationAllowed = 1;
             cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3(items + ctas);
+            cfg.gridDim = dim3(L.ctas + singles);
             cfg.blockDim = dim3(threads);
-            cfg.dynamicSmemBytes = smem;
+            cfg.dynamicSmemBytes = L.smem;
             cfg.stream = ctx->stream;
             cfg.attrs = &attr;
             cfg.numAttrs = overlap ? 1 : 0;

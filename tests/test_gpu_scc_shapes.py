@@ -1,0 +1,53 @@
+"""`k_sw_scc` on SCCs of unequal parities and odd sizes, on graphs made for it.
+
+The graphs come in as tables (`Net.from_csc`); a solve is checked by its own equations
+(`tests/hypercube.py`): relative residual and L1 error of the masses <= 1e-9.
+"""
+import numpy as np
+import pytest
+
+import hypercube as H
+from paraexastolog_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def esl():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import paraexastolog_b200 as E
+    E.lib()
+    return E
+
+
+def solve_and_check(esl, F, sizes, B, seed, method=None, systems=3):
+    """One batch on the graph F, whose largest SCCs have `sizes` states; the first and last
+    systems and one between them are checked."""
+    n = int(np.log2(F.size))
+    rng = np.random.default_rng(seed)
+    rates = synth.log_uniform_rates(rng, n, B)
+    x0 = rng.dirichlet(np.ones(F.size))
+    ctx = esl.Context(0, torch.cuda.Stream())
+    indptr, rows = (torch.as_tensor(a, device="cuda") for a in H.csc(F))
+    net = esl.Net.from_csc(ctx, n, indptr, rows)
+    offsets = net.export()[1].cpu().numpy()
+    assert np.array_equal(np.sort(np.diff(offsets))[::-1][:len(sizes)], np.sort(sizes)[::-1])
+    occ = torch.empty((B, F.size), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    res = esl.solve_batch(ctx, net, rates, x0[None], method=esl.METHOD_DIRECT if method is None else method,
+                          occupation=occ)
+    assert res.report.converged == 1 and res.report.fallback_systems == 0
+    for b in np.unique(np.linspace(0, B - 1, systems).astype(int)):
+        H.check(F, rates[b], x0, occ[b].cpu().numpy(), res.x_inf[b, 0].cpu().numpy())
+    return res
+
+
+def test_two_sccs_whose_footprints_grow(esl):
+    """The second SCC has fewer rows of its larger parity and the larger footprint: two systems
+    of the first fit a CTA, of the second one does."""
+    rng = np.random.default_rng(1)
+    parts = [H.random_part(rng, 13, 2400, 1760), H.random_part(rng, 13, 2100, 2100) | (1 << 13)]
+    solve_and_check(esl, H.masks(rng, 14, parts), [4160, 4200], 148, 2)
