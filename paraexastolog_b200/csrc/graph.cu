@@ -74,7 +74,7 @@ struct GraphArgs {
     uint32_t cap;      // states per CTA
     uint64_t* keys;
     int32_t* vals;
-    int64_t budget;    // passes per fixpoint
+    int64_t budget;    // phases per fixpoint
     unsigned polls;    // bound of a barrier wait
     unsigned missing;  // arrivals that never come (0, or 1 when the bounded wait is tested)
     GraphState* st;
@@ -173,21 +173,21 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
     // Runs pass(place) over the CTA's first `count` list places until a whole phase changes
     // nothing: `passes` sweeps per phase while the states are few (a sweep is then shorter
     // than a barrier).  `seeded`: this thread changed states that the passes read since the
-    // last barrier, which the first phase may not see everywhere.  False: failed.
-    auto fixpoint = [&](uint32_t count, unsigned passes, bool seeded, auto pass) -> bool {
+    // last barrier, which the first phase may not see everywhere, so that it does not count.
+    // A phase gets at least as far as one sweep that reads only what the phase before it left;
+    // the budget is in such sweeps.  False: failed.
+    auto fixpoint = [&](uint32_t count, unsigned passes, bool after_seeds, bool seeded, int64_t budget, auto pass) -> bool {
         bool ch = seeded;
-        for (int64_t used = 0;; ch = false) {
-            const unsigned p = (unsigned)min((int64_t)passes, max(g.budget - used, (int64_t)1));
-            for (unsigned k = 0; k < p; k++)
+        for (int64_t used = after_seeds ? 0 : 1;; ch = false, used++) {
+            for (unsigned k = 0; k < passes; k++)
                 for (uint32_t i = tid; i < count; i += kSccT) ch |= pass(i);
-            used += p;
             if (cta == 0 && tid == 0) st->changed[(phase + 1) % 3] = 0;
             if (__syncthreads_or(ch) && tid == 0) st->changed[phase % 3] = 1;
             if (!grid_barrier(g, target)) return false;
             const unsigned any = *(volatile unsigned*)&st->changed[phase % 3];
             phase++;
             if (!any) return true;
-            if (used >= g.budget) {
+            if (used >= budget) {
                 if (tid == 0) atomicCAS(&st->status, 0, 1);
                 // every CTA sees the same flag and budget: all leave here
                 return false;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
     };
     for (;; round++) {
         const unsigned passes = live > 2u * kSccT * ctas ? 1u : 4u;
-        if (!fixpoint(count, passes, seeded, trim)) return;
+        if (!fixpoint(count, passes, round > 0, seeded, g.budget, trim)) return;
         count = compact(count, false);
         if (cta == 0 && tid == 0) st->live[(round + 1) % 3] = 0;
         if (tid == 0 && count) atomicAdd(&st->live[round % 3], count);
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
         live = *(volatile unsigned*)&st->live[round % 3];
         if (live == 0) break;
         // largest priority among the live ancestors
-        if (!fixpoint(count, passes, false, [&](uint32_t i) {
+        if (!fixpoint(count, passes, false, false, g.budget, [&](uint32_t i) {
                 const uint32_t v = list[i], c = __ldcg(g.color + v);
                 uint32_t m = c;
                 for_neighbours(v, g.G[v], g.color, [&](const uint32_t (&x)[8]) {
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
                 seeded = true;
             }
         }
-        if (!fixpoint(count, passes, seeded, [&](uint32_t i) {
+        if (!fixpoint(count, passes, true, seeded, g.budget, [&](uint32_t i) {
                 const uint32_t v = list[i], c = __ldcg(g.color + v);
                 if (c & kReached) return false;
                 bool hit = false;
@@ -295,7 +295,9 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
     if (!grid_barrier(g, target)) return;
     // levels, stored at the SCC's label: 1 + the largest level among successor SCCs.  The
     // list takes each state's flips that leave its SCC, the colours a copy of its SCC's
-    // level, which neighbours read without going through the label.
+    // level, which neighbours read without going through the label.  The state that raises its
+    // SCC's level raises its own copy with it, the SCC's other states theirs a pass later: a
+    // level costs one pass behind singletons and two behind larger SCCs, hence twice the budget.
     for (uint32_t i = tid; i < own; i += kSccT) {
         const uint32_t v = state_at(i);
         uint32_t x = 0;
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
         list[i] = x;
     }
     if (!grid_barrier(g, target)) return;
-    if (!fixpoint(own, g.N > 2u * kSccT * ctas ? 1u : 4u, false, [&](uint32_t i) {
+    if (!fixpoint(own, g.N > 2u * kSccT * ctas ? 1u : 4u, false, false, 2 * g.budget, [&](uint32_t i) {
             const uint32_t v = state_at(i);
             if (v >= g.N) return false;
             const int32_t c = g.lab[v];
@@ -328,6 +330,7 @@ __global__ void __launch_bounds__(kSccT, 1) k_scc(const GraphArgs g) {
             });
             if (best >= l && best > 0) {
                 atomicMax(&g.level[c], (int32_t)best + 1);
+                __stcg(g.color + v, best + 1);
                 ch = true;
             }
             return ch;
@@ -447,7 +450,7 @@ int build_graph(esl_ctx* ctx, esl_net* net) {
         ga.list = list.get();
         ga.keys = keys.get();
         ga.vals = vals.get();
-        // a pass can only fail to progress once per state (or the context's budget)
+        // a sweep can only fail to progress once per state (or the context's budget)
         ga.budget = ctx->graph_sweeps > 0 ? ctx->graph_sweeps : (int64_t)N + 64;
         ga.st = state.get();
         const bool no_end = barrier_timeout_test();
