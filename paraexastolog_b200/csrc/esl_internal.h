@@ -284,6 +284,9 @@ int masks_from_csc(int n, const int32_t* indptr, const int32_t* rows, uint32_t* 
                    unsigned long long* d_bad, cudaStream_t s);
 
 // graph.cu
+// stable sort of (key, value) pairs by key; tmp: scratch, grown as needed
+int sort_pairs(const uint64_t* keys, uint64_t* keys_out, const int32_t* vals, int32_t* vals_out, size_t count,
+               DevBuf<uint8_t>& tmp, cudaStream_t s);
 int build_graph(esl_ctx* ctx, esl_net* net);
 // Bound of a wait at the barrier of a cooperative launch (seconds), and the one for its
 // test: with ESL_BARRIER_TIMEOUT_TEST=1 (read per call) the barriers expect one arrival more

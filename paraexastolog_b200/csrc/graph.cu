@@ -402,6 +402,15 @@ __global__ void k_domain_masks(int n, uint64_t N, const uint32_t* __restrict__ F
 
 }  // namespace
 
+int sort_pairs(const uint64_t* keys, uint64_t* keys_out, const int32_t* vals, int32_t* vals_out, size_t count,
+               DevBuf<uint8_t>& tmp, cudaStream_t s) {
+    size_t bytes = 0;
+    ESL_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys, keys_out, vals, vals_out, (int64_t)count, 0, 64, s));
+    if (tmp.n < bytes) ESL_TRY(tmp.alloc(bytes));
+    ESL_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), bytes, keys, keys_out, vals, vals_out, (int64_t)count, 0, 64, s));
+    return ESL_OK;
+}
+
 bool barrier_timeout_test() {
     const char* e = getenv("ESL_BARRIER_TIMEOUT_TEST");
     return e && e[0] == '1';
@@ -481,13 +490,8 @@ int build_graph(esl_ctx* ctx, esl_net* net) {
         DevBuf<uint8_t> head;
         ESL_TRY(keys_out.alloc(N));
         ESL_TRY(net->order.alloc(N));
-        size_t tmp_bytes = 0;
-        ESL_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.get(), keys_out.get(), vals.get(),
-                                                 net->order.get(), (int64_t)N, 0, 64, s));
         DevBuf<uint8_t> tmp;
-        ESL_TRY(tmp.alloc(tmp_bytes));
-        ESL_CUDA(cub::DeviceRadixSort::SortPairs(tmp.get(), tmp_bytes, keys.get(), keys_out.get(), vals.get(),
-                                                 net->order.get(), (int64_t)N, 0, 64, s));
+        ESL_TRY(sort_pairs(keys.get(), keys_out.get(), vals.get(), net->order.get(), N, tmp, s));
         // SCC heads
         ESL_TRY(pos.alloc(N));
         ESL_TRY(head.alloc(N));

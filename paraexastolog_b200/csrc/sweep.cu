@@ -89,6 +89,9 @@ struct SwGroup {
     int max_odd;           // local groups: most odd rows of one SCC
     uint64_t nin;          // in-group predecessor entries of the group's rows
     uint32_t s0, ns;       // the group's SCCs of >= 2 states: range in SweepPlan::scc
+    uint32_t sh0, nsh;     // their shapes: range in SweepPlan::shapes
+    uint32_t l0, nlarge;   // those beyond a cluster (the first ones): range in SweepPlan::large
+    uint32_t most;         // most rows of one parity of an SCC (0: singletons only)
     bool resident;         // every one of them fits a CTA or a cluster of k_sw_scc
     bool split;            // one of them needs a cluster
     uint32_t singles;      // rows that are SCCs of their own
@@ -106,13 +109,18 @@ struct SweepPlan {
     DevBuf<uint32_t> og_ptr, og_ent;     // predecessors in earlier groups
     DevBuf<uint32_t> tp_ptr, tp_ent;     // transient predecessors of terminal position p
     DevBuf<uint32_t> lsc_off;            // local SCCs: offsets into lsc_slots
-    // SCCs of >= 2 states, group by group, largest first: (first even slot, even rows,
-    // first odd slot, odd rows); an SCC's even and odd slots are one run each
+    // SCCs of >= 2 states in the order of scc_sort_key: (first even slot, even rows, first odd
+    // slot, odd rows); an SCC's even and odd slots are one run each.  The host keeps their
+    // shapes, and the places of those beyond a cluster: a network may have millions of SCCs.
     DevBuf<uint4> scc;
-    std::vector<uint4> h_scc;
+    DevBuf<uint64_t> scc_key;  // (while the plan is built)
+    std::vector<SccShape> shapes;
+    std::vector<uint4> large;
     // Predecessors of the rows of SCCs solved by one CTA (k_sw_scc), by slices of 32 rows of
     // one parity: scc_sl = an SCC's first even and first odd slice, sl = a slice's (lines,
-    // first line of ell).  Line j holds entries 4j .. 4j + 3 of each row, 16 bytes a row:
+    // first line of ell).  Line j holds entries 4j .. 4j + 3 of 32 rows, 16 bytes a row; a narrow
+    // SCC's (scc_narrow) are as wide as the parity has rows and sl holds their place in ell,
+    // behind those of the others.  An entry is the
     // local row of the other parity << 9 | rate index << 3, so that masked and shifted they
     // are byte offsets (row * 8 after >> 6); past a row's last entry the local row is the
     // other parity's row count.  In an SCC split over a cluster the local row is the owner's
@@ -1613,6 +1621,11 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         q.mem = g.own[kOwnQ] + o;
         BS.mem = g.own[kOwnBS] + o;
     }
+    // line j of a slice of even or odd rows
+    const bool narrow = !MEM && scc_narrow(sc.y, sc.w);
+    auto line_at = [&](const uint2& sl, uint32_t j, uint32_t rows) {
+        return g.ell + (narrow ? (size_t)(sl.y + j * rows) : (size_t)(sl.y + j) * 32);
+    };
     // one row per thread: its first two lines stay in registers
     uint4 ee[2], eo[2];
     uint2 le = make_uint2(0u, 0u), lo = make_uint2(0u, 0u);
@@ -1630,8 +1643,8 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             if (!DEFL) og_o = make_uint2(g.og_ptr[od0 + rs], g.og_ptr[od0 + rs + 1]);
         }
         for (int j = 0; j < 2; j++) {
-            if (j < (int)le.x) ee[j] = __ldg(g.ell + (size_t)(le.y + j) * 32 + (rs & 31));
-            if (j < (int)lo.x) eo[j] = __ldg(g.ell + (size_t)(lo.y + j) * 32 + (rs & 31));
+            if (j < (int)le.x) ee[j] = __ldg(line_at(le, j, sc.y) + (rs & 31));
+            if (j < (int)lo.x) eo[j] = __ldg(line_at(lo, j, sc.w) + (rs & 31));
         }
     }
     const uint32_t rate_at = shared_addr(rate + s);
@@ -1704,7 +1717,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             double acc = 0.0;
             if (l.x > 0) ell_add(acc, EVEN ? ee[0] : eo[0], xs, rate_at, lks);
             if (l.x > 1) ell_add(acc, EVEN ? ee[1] : eo[1], xs, rate_at, lks);
-            for (uint32_t j = 2; j < l.x; j++)
+            for (uint32_t j = 2; j < l.x; j++)  // (not narrow)
                 ell_add(acc, __ldg(g.ell + (size_t)(l.y + j) * 32 + (rs & 31)), xs, rate_at, lks);
             fn(rs, (rs << lks) | s, acc);
         }
@@ -1825,7 +1838,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             const uint2 sl = __ldg(g.sl + first.y + (r >> 5));
             for (uint32_t j = 0; j < 4 * sl.x; j++) {
                 const uint32_t e =
-                    __ldg(reinterpret_cast<const uint32_t*>(g.ell + (size_t)(sl.y + j / 4) * 32 + (r & 31)) + j % 4);
+                    __ldg(reinterpret_cast<const uint32_t*>(line_at(sl, j / 4, sc.w) + (r & 31)) + j % 4);
                 diag(e >> 3 & 63u, CLUSTER ? lds_cluster(shared_addr(A) + (e >> 6 & 0xFFF8u), e >> 22) : A[((e >> 9) << lks) | s]);
             }
         }
@@ -1848,7 +1861,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         at(rs, rs) = q.get(0);
         at(rs, so) = R.get(0);
         for (uint32_t j = 0; j < lo.x; j++) {
-            const uint4 e4 = __ldg(g.ell + (size_t)(lo.y + j) * 32 + (rs & 31));
+            const uint4 e4 = __ldg(line_at(lo, j, sc.w) + (rs & 31));
             const uint32_t es[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -1857,7 +1870,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
                 const double w = rate[((es[u] >> 3 & 63u) << lks) | s] * A[(er << lks) | s];
                 const uint2 sl = __ldg(g.sl + first.x + (er >> 5));
                 for (uint32_t i = 0; i < sl.x; i++) {
-                    const uint4 f4 = __ldg(g.ell + (size_t)(sl.y + i) * 32 + (er & 31));
+                    const uint4 f4 = __ldg(line_at(sl, i, sc.y) + (er & 31));
                     const uint32_t fs[4] = {f4.x, f4.y, f4.z, f4.w};
 #pragma unroll
                     for (int x = 0; x < 4; x++)
@@ -2162,9 +2175,8 @@ int build_terminal_plan(const std::vector<int32_t>& order, const std::vector<int
             }
             (par ? g.no : g.ne) = (uint32_t)rows.size() - g.beg - (par ? g.ne : 0);
         }
-        g.s0 = (uint32_t)TP->h_scc.size();
+        g.s0 = (uint32_t)TP->groups.size();
         g.ns = 1;
-        TP->h_scc.push_back(make_uint4(g.beg, g.ne, g.beg + g.ne, g.no));
         TP->max_rows = std::max(TP->max_rows, g.ne + g.no);
         TP->max_even = std::max(TP->max_even, g.ne);
         TP->max_odd = std::max(TP->max_odd, g.no);
@@ -2490,13 +2502,15 @@ __global__ void k_pl_scc2(int NT, const uint32_t* __restrict__ ssize, uint32_t* 
 __global__ void k_pl_scc_list(int NT, int T, int TS, const int32_t* __restrict__ offsets,
                               const uint32_t* __restrict__ gid_incl, const uint32_t* __restrict__ ssize,
                               const uint32_t* __restrict__ E, const uint32_t* __restrict__ info,
-                              const uint32_t* __restrict__ idx, uint4* __restrict__ out) {
+                              const uint32_t* __restrict__ idx, uint4* __restrict__ out,
+                              uint64_t* __restrict__ key) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= NT || ssize[c] < 2) return;
     const uint32_t* in = info + (size_t)(gid_incl[c] - 1) * 8;
     const uint32_t p0 = in[0], ne = in[1], cs = (uint32_t)(offsets[T + c] - TS), ce = cs + ssize[c];
     const uint32_t er = E[cs] - E[p0], se = E[ce] - E[cs];
     out[idx[c]] = make_uint4(p0 + er, se, p0 + ne + (cs - p0) - er, ssize[c] - se);
+    key[idx[c]] = scc_sort_key(gid_incl[c] - 1, se, ssize[c] - se);
 }
 
 // slot of every transient position: rows, slot_of (by state), group of each slot
@@ -2738,6 +2752,7 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         for (uint32_t g = 0; g < G; g++) n2 += h_info[(size_t)g * 8 + 6];
         if (n2 > 0) {
             ESL_TRY(P->scc.alloc(n2));
+            ESL_TRY(P->scc_key.alloc(n2));
             ESL_COUNT_LAUNCH();
             k_pl_scc2<<<nblk((uint64_t)NT + 1), 256, 0, s>>>(NT, ssize.get(), qsize.get());
             DevBuf<uint32_t> sidx;
@@ -2745,11 +2760,8 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
             ESL_TRY(scan_excl(tmp, qsize.get(), sidx.get(), (uint32_t)NT + 1, s));
             ESL_COUNT_LAUNCH();
             k_pl_scc_list<<<nblk(NT), 256, 0, s>>>(NT, T, TS, offsets, gid.get(), ssize.get(), E.get(), info.get(),
-                                                   sidx.get(), P->scc.get());
+                                                   sidx.get(), P->scc.get(), P->scc_key.get());
             ESL_CUDA(cudaGetLastError());
-            P->h_scc.resize(n2);
-            ESL_CUDA(cudaMemcpyAsync(P->h_scc.data(), P->scc.get(), (size_t)n2 * sizeof(uint4), cudaMemcpyDeviceToHost,
-                                     s));
         }
         ESL_TRY(P->ig_ent.alloc(std::max<uint32_t>(tot[0], 1)));
         ESL_TRY(P->og_ent.alloc(std::max<uint32_t>(tot[1], 1)));
@@ -2854,10 +2866,11 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
 }
 
 // Most rows of one parity of an SCC
-inline uint32_t scc_rows(const uint4& c) { return std::max(c.y, c.w); }
+__host__ __device__ inline uint32_t scc_rows(const uint4& c) { return c.y > c.w ? c.y : c.w; }
 
 // Slices of SCC j (see SweepPlan::sl): source[slice] = (first slot, rows | 64 and the cluster
-// rank << 7 for an SCC split over a cluster, first slot of the other parity, its rows)
+// rank << 7 for an SCC split over a cluster | 512 for a narrow one, first slot of the other
+// parity, its rows)
 __global__ void k_pl_slices(uint32_t count, const uint4* __restrict__ scc, const uint2* __restrict__ scc_sl,
                             uint4* __restrict__ source) {
     const uint32_t j = blockIdx.x;
@@ -2866,33 +2879,45 @@ __global__ void k_pl_slices(uint32_t count, const uint4* __restrict__ scc, const
     const uint2 f = scc_sl[j];
     if (f.x == kNoSlot) return;  // not solved by a CTA or a cluster
     const bool split = max(c.y, c.w) > (uint32_t)kSccMaxRows;
+    const uint32_t narrow = scc_narrow(c.y, c.w) ? 512u : 0u;
     for (uint32_t r = threadIdx.x * 32; r < c.y; r += blockDim.x * 32)
-        source[f.x + r / 32] = make_uint4(c.x + r, min(32u, c.y - r) | (split ? 64u | r / kSccMaxRows << 7 : 0u), c.z, c.w);
+        source[f.x + r / 32] =
+            make_uint4(c.x + r, min(32u, c.y - r) | (split ? 64u | r / kSccMaxRows << 7 : 0u) | narrow, c.z, c.w);
     for (uint32_t r = threadIdx.x * 32; r < c.w; r += blockDim.x * 32)
-        source[f.y + r / 32] = make_uint4(c.z + r, min(32u, c.w - r) | (split ? 64u | r / kSccMaxRows << 7 : 0u), c.x, c.y);
+        source[f.y + r / 32] =
+            make_uint4(c.z + r, min(32u, c.w - r) | (split ? 64u | r / kSccMaxRows << 7 : 0u) | narrow, c.x, c.y);
 }
 
-// One warp per slice.  FILL false: its line count (four entries a line, the most of a row);
-// true: the lines.
+// One warp per slice.  FILL false: its lines (four entries a line, the most of a row) in
+// size[w], or for a narrow SCC its places in ell in size[slices + w] (the other one 0); true:
+// the lines, from the exclusive sums of these.
 template <bool FILL>
 __global__ void k_pl_ell(uint32_t slices, const uint4* __restrict__ source, const uint32_t* __restrict__ ig_ptr,
-                         const uint32_t* __restrict__ ig_ent, uint32_t* __restrict__ width,
+                         const uint32_t* __restrict__ ig_ent, uint32_t* __restrict__ size,
                          const uint32_t* __restrict__ off, uint2* __restrict__ sl, uint4* __restrict__ ell) {
     const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= slices) return;
     const uint4 src = source[w];
-    const bool row = lane < (src.y & 63u);
+    const bool narrow = src.y & 512u;
+    const uint32_t rows = src.y & 63u, width = narrow ? rows : 32u;
+    const bool row = lane < rows;
     const uint32_t p = row ? ig_ptr[src.x + lane] : 0u;
     const uint32_t cnt = row ? ig_ptr[src.x + lane + 1] - p : 0u;
+    const uint32_t lines = (__reduce_max_sync(0xFFFFFFFFu, cnt) + 3) / 4;
     if (!FILL) {
-        const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, cnt);
-        if (lane == 0) width[w] = (most + 3) / 4;
+        if (lane == 0) {
+            size[w] = narrow ? 0u : lines;
+            size[slices + w] = narrow ? lines * width : 0u;
+        }
         return;
     }
-    const uint32_t lines = width[w];
+    // (the narrow slices' sums go on from the lines of the others: off[slices])
+    const uint32_t first = narrow ? off[slices] * 31 + off[slices + w] : off[w];
+    uint4* out = ell + (narrow ? (size_t)first : (size_t)first * 32);
+    if (lane == 0) sl[w] = make_uint2(lines, first);
+    if (lane >= width) return;
     const bool split = src.y & 64u;  // (see kSccCluster)
-    const uint32_t none = split ? (src.y >> 7) << 13 | (uint32_t)kSccMaxRows : src.w;
-    if (lane == 0) sl[w] = make_uint2(lines, off[w]);
+    const uint32_t none = split ? (src.y >> 7 & 3u) << 13 | (uint32_t)kSccMaxRows : src.w;
     for (uint32_t j = 0; j < lines; j++) {
         uint32_t e[4];
 #pragma unroll
@@ -2903,70 +2928,178 @@ __global__ void k_pl_ell(uint32_t slices, const uint4* __restrict__ source, cons
                 e[u] = (split ? (r / kSccMaxRows) << 13 | r % kSccMaxRows : r) << 9 | (uint32_t)ent_rate(x) << 3;
             }
         }
-        ell[((size_t)off[w] + j) * 32 + lane] = make_uint4(e[0], e[1], e[2], e[3]);
+        out[(size_t)j * width + lane] = make_uint4(e[0], e[1], e[2], e[3]);
     }
 }
 
-// Sorts each group's SCC list by decreasing size (the launch order of k_sw_scc: a group
-// lasts as long as the CTA of its largest SCC, which must not start behind the small ones)
-// and lays out the predecessor lines of the SCCs that a CTA or a cluster solves.  Any SCC of
-// at most kSccMaxRows rows of either parity fits a CTA's shared memory at one system.
+// slices of `rows` rows of one parity of an SCC (0: neither a CTA nor a cluster solves it)
+__host__ __device__ inline uint32_t scc_slices(const uint4& c, uint32_t rows) {
+    return scc_rows(c) > kSccClusterRows ? 0u : (rows + 31) / 32;
+}
+
+// The sorted list: SCC i = in[place[i]].  head[i]: it begins a shape of its group; slices[i]:
+// its slices (both with one more, zero, entry for the scans)
+__global__ void k_pl_scc_sorted(uint32_t count, const uint4* __restrict__ in, const uint64_t* __restrict__ key,
+                                const int32_t* __restrict__ place, uint4* __restrict__ out, uint32_t* __restrict__ head,
+                                uint32_t* __restrict__ slices) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > count) return;
+    if (i == count) {
+        head[i] = slices[i] = 0;
+        return;
+    }
+    const uint4 c = in[place[i]], b = in[place[i ? i - 1 : 0]];
+    out[i] = c;
+    head[i] = (i == 0 || key[i] >> 38 != key[i - 1] >> 38 || c.y != b.y || c.w != b.w) ? 1u : 0u;
+    slices[i] = scc_slices(c, c.y) + scc_slices(c, c.w);
+}
+// scc_sl, and of every shape's first SCC (its place, even rows, odd rows, group)
+__global__ void k_pl_scc_shapes(uint32_t count, const uint4* __restrict__ scc, const uint64_t* __restrict__ key,
+                                const uint32_t* __restrict__ head, const uint32_t* __restrict__ shape,
+                                const uint32_t* __restrict__ slice, uint2* __restrict__ scc_sl,
+                                uint4* __restrict__ shapes) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const uint4 c = scc[i];
+    const bool kept = scc_rows(c) <= kSccClusterRows;
+    scc_sl[i] = kept ? make_uint2(slice[i], slice[i] + scc_slices(c, c.y)) : make_uint2(kNoSlot, kNoSlot);
+    if (head[i]) shapes[shape[i]] = make_uint4(i, c.y, c.w, (uint32_t)(key[i] >> 38));
+}
+
+// Sorts the SCC list (scc_sort_key), lists its shapes and lays out the predecessor lines of the
+// SCCs that a CTA or a cluster solves.  Any SCC of at most kSccMaxRows rows of either parity
+// fits a CTA's shared memory at one system.  A short list is sorted on the host (`list`, or
+// read back where that is null), a long one on the device.
 static_assert((2 * (kSccMaxRows + 1) + 2 * 26 + 6 * (kSccThreadsBig / 32) + 5 * kSccMaxRows) * 8 <= (int)kSccMaxSmem - 256,
               "k_sw_scc's arrays");
-int finish_scc_list(esl_ctx* ctx, SweepPlan* P) {
-    for (SwGroup& g : P->groups) {
-        const auto b = P->h_scc.begin() + g.s0, e = b + g.ns;
-        std::stable_sort(b, e, [](const uint4& x, const uint4& y) { return scc_rows(x) > scc_rows(y); });
-        g.singles = g.ne + g.no;
-        for (auto c = b; c != e; ++c) g.singles -= c->y + c->w;
-        g.resident = g.ns == 0 || scc_rows(*b) <= kSccClusterRows;
-        g.split = g.ns > 0 && scc_rows(*b) > (uint32_t)kSccMaxRows;
-    }
-    if (P->h_scc.empty()) return ESL_OK;
+constexpr uint32_t kSccHostSort = 1024;
+int finish_scc_list(esl_ctx* ctx, SweepPlan* P, const std::vector<uint4>* list) {
     cudaStream_t s = ctx->stream;
-    const uint32_t count = (uint32_t)P->h_scc.size();
-    std::vector<uint2> first(count, make_uint2(kNoSlot, kNoSlot));
-    uint32_t slices = 0;
-    for (const SwGroup& g : P->groups)
-        for (uint32_t j = g.s0; j < g.s0 + g.ns; j++) {
-            if (scc_rows(P->h_scc[j]) > kSccClusterRows) continue;
-            first[j].x = slices;
-            slices += (P->h_scc[j].y + 31) / 32;
-            first[j].y = slices;
-            slices += (P->h_scc[j].w + 31) / 32;
-        }
-    if (!P->scc.get()) ESL_TRY(P->scc.alloc(count));
-    ESL_TRY(P->scc_sl.alloc(count));
-    ESL_CUDA(cudaMemcpyAsync(P->scc.get(), P->h_scc.data(), (size_t)count * sizeof(uint4), cudaMemcpyHostToDevice, s));
-    ESL_CUDA(cudaMemcpyAsync(P->scc_sl.get(), first.data(), (size_t)count * sizeof(uint2), cudaMemcpyHostToDevice, s));
-    DevBuf<uint4> source;
-    DevBuf<uint32_t> width, off;
+    uint32_t count = 0, slices = 0;
+    for (const SwGroup& g : P->groups) count += g.ns;
     DevBuf<uint8_t> tmp;
-    ESL_TRY(source.alloc(std::max(slices, 1u)));
-    ESL_TRY(width.alloc((size_t)slices + 1));
-    ESL_TRY(off.alloc((size_t)slices + 1));
-    ESL_TRY(P->sl.alloc(std::max(slices, 1u)));
-    uint32_t lines = 0;
-    if (slices > 0) {
+    std::vector<uint4> shapes;  // (first SCC, even rows, odd rows, group)
+    if (count > 0) ESL_TRY(P->scc_sl.alloc(count));
+    if (count > 0 && (list || count <= kSccHostSort)) {
+        std::vector<uint4> h(count);
+        if (list) {
+            h = *list;
+            ESL_TRY(P->scc.alloc(count));
+        } else {
+            ESL_CUDA(cudaMemcpyAsync(h.data(), P->scc.get(), (size_t)count * sizeof(uint4), cudaMemcpyDeviceToHost, s));
+            ESL_CUDA(cudaStreamSynchronize(s));
+        }
+        std::vector<uint2> first(count, make_uint2(kNoSlot, kNoSlot));
+        for (uint32_t gi = 0; gi < P->groups.size(); gi++) {
+            const SwGroup& g = P->groups[gi];
+            std::stable_sort(h.begin() + g.s0, h.begin() + g.s0 + g.ns, [](const uint4& x, const uint4& y) {
+                return scc_sort_key(0, x.y, x.w) < scc_sort_key(0, y.y, y.w);
+            });
+            for (uint32_t j = g.s0; j < g.s0 + g.ns; j++) {
+                const uint4& c = h[j];
+                if (j == g.s0 || c.y != h[j - 1].y || c.w != h[j - 1].w) shapes.push_back(make_uint4(j, c.y, c.w, gi));
+                if (scc_rows(c) > kSccClusterRows) continue;
+                first[j].x = slices;
+                first[j].y = slices + scc_slices(c, c.y);
+                slices = first[j].y + scc_slices(c, c.w);
+            }
+        }
+        ESL_CUDA(cudaMemcpyAsync(P->scc.get(), h.data(), (size_t)count * sizeof(uint4), cudaMemcpyHostToDevice, s));
+        ESL_CUDA(cudaMemcpyAsync(P->scc_sl.get(), first.data(), (size_t)count * sizeof(uint2), cudaMemcpyHostToDevice, s));
+    } else if (count > 0) {
+        DevBuf<uint4> sorted, d_shapes;
+        DevBuf<uint64_t> key;
+        DevBuf<int32_t> place0, place;
+        DevBuf<uint32_t> head, shape, nsl, slice;
+        ESL_TRY(sorted.alloc(count));
+        ESL_TRY(key.alloc(count));
+        ESL_TRY(place0.alloc(count));
+        ESL_TRY(place.alloc(count));
         ESL_COUNT_LAUNCH();
-        k_pl_slices<<<count, 32, 0, s>>>(count, P->scc.get(), P->scc_sl.get(), source.get());
-        ESL_CUDA(cudaMemsetAsync(width.get() + slices, 0, 4, s));
+        k_sw_iota<<<nblk(count), 256, 0, s>>>((int)count, place0.get());
+        ESL_TRY(sort_pairs(P->scc_key.get(), key.get(), place0.get(), place.get(), count, tmp, s));
+        for (DevBuf<uint32_t>* b : {&head, &shape, &nsl, &slice}) ESL_TRY(b->alloc((size_t)count + 1));
         ESL_COUNT_LAUNCH();
-        k_pl_ell<false><<<nblk((uint64_t)slices * 32), 256, 0, s>>>(slices, source.get(), P->ig_ptr.get(),
-                                                                    P->ig_ent.get(), width.get(), nullptr, nullptr,
-                                                                    nullptr);
-        ESL_TRY(scan_excl(tmp, width.get(), off.get(), slices + 1, s));
-        ESL_CUDA(cudaMemcpyAsync(&lines, off.get() + slices, 4, cudaMemcpyDeviceToHost, s));
+        k_pl_scc_sorted<<<nblk((uint64_t)count + 1), 256, 0, s>>>(count, P->scc.get(), key.get(), place.get(), sorted.get(),
+                                                                  head.get(), nsl.get());
+        ESL_TRY(scan_excl(tmp, head.get(), shape.get(), count + 1, s));
+        ESL_TRY(scan_excl(tmp, nsl.get(), slice.get(), count + 1, s));
+        uint32_t n_shapes = 0;
+        ESL_CUDA(cudaMemcpyAsync(&n_shapes, shape.get() + count, 4, cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaMemcpyAsync(&slices, slice.get() + count, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
-        ESL_TRY(P->ell.alloc((size_t)lines * 32));
+        ESL_TRY(d_shapes.alloc(n_shapes));
         ESL_COUNT_LAUNCH();
-        k_pl_ell<true><<<nblk((uint64_t)slices * 32), 256, 0, s>>>(slices, source.get(), P->ig_ptr.get(),
-                                                                   P->ig_ent.get(), width.get(), off.get(),
-                                                                   P->sl.get(), P->ell.get());
+        k_pl_scc_shapes<<<nblk(count), 256, 0, s>>>(count, sorted.get(), key.get(), head.get(), shape.get(), slice.get(),
+                                                    P->scc_sl.get(), d_shapes.get());
         ESL_CUDA(cudaGetLastError());
+        shapes.resize(n_shapes);
+        ESL_CUDA(cudaMemcpyAsync(shapes.data(), d_shapes.get(), (size_t)n_shapes * sizeof(uint4), cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaStreamSynchronize(s));
+        std::swap(P->scc.p, sorted.p);
+        std::swap(P->scc.n, sorted.n);
     }
+    P->scc_key.release();
+    for (SwGroup& g : P->groups) g.singles = g.ne + g.no;
+    for (size_t j = 0; j < shapes.size(); j++) {
+        const uint4& x = shapes[j];
+        SwGroup& g = P->groups[x.w];
+        const uint32_t next = j + 1 < shapes.size() ? shapes[j + 1].x : count, many = next - x.x, rows = std::max(x.y, x.z);
+        if (g.nsh++ == 0) {
+            g.sh0 = (uint32_t)P->shapes.size();
+            g.l0 = (uint32_t)P->large.size();
+            g.most = rows;
+        }
+        P->shapes.push_back({x.y, x.z, many});
+        g.singles -= (x.y + x.z) * many;
+        if (rows > kSccClusterRows) {
+            g.nlarge += many;
+            P->large.resize(P->large.size() + many);
+            ESL_CUDA(cudaMemcpyAsync(P->large.data() + P->large.size() - many, P->scc.get() + x.x,
+                                     (size_t)many * sizeof(uint4), cudaMemcpyDeviceToHost, s));
+            ESL_CUDA(cudaStreamSynchronize(s));
+        }
+    }
+    for (SwGroup& g : P->groups) {
+        g.resident = g.nlarge == 0;
+        g.split = g.most > (uint32_t)kSccMaxRows;
+    }
+    // (the uploads above read vectors of this function)
+    if (slices == 0) {
+        ESL_CUDA(cudaStreamSynchronize(s));
+        return ESL_OK;
+    }
+    DevBuf<uint4> source;
+    DevBuf<uint32_t> size, off;
+    ESL_TRY(source.alloc(slices));
+    ESL_TRY(size.alloc(2 * (size_t)slices + 1));
+    ESL_TRY(off.alloc(2 * (size_t)slices + 1));
+    ESL_TRY(P->sl.alloc(slices));
+    uint32_t total[2] = {0, 0};  // lines of 32 rows, and these and the places of narrow ones
+    ESL_COUNT_LAUNCH();
+    k_pl_slices<<<count, 32, 0, s>>>(count, P->scc.get(), P->scc_sl.get(), source.get());
+    ESL_CUDA(cudaMemsetAsync(size.get() + 2 * (size_t)slices, 0, 4, s));
+    ESL_COUNT_LAUNCH();
+    k_pl_ell<false><<<nblk((uint64_t)slices * 32), 256, 0, s>>>(slices, source.get(), P->ig_ptr.get(), P->ig_ent.get(),
+                                                                size.get(), nullptr, nullptr, nullptr);
+    ESL_TRY(scan_excl(tmp, size.get(), off.get(), 2 * slices + 1, s));
+    ESL_CUDA(cudaMemcpyAsync(&total[0], off.get() + slices, 4, cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaMemcpyAsync(&total[1], off.get() + 2 * (size_t)slices, 4, cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaStreamSynchronize(s));
+    ESL_TRY(P->ell.alloc((size_t)total[0] * 31 + total[1]));
+    ESL_COUNT_LAUNCH();
+    k_pl_ell<true><<<nblk((uint64_t)slices * 32), 256, 0, s>>>(slices, source.get(), P->ig_ptr.get(), P->ig_ent.get(),
+                                                               size.get(), off.get(), P->sl.get(), P->ell.get());
+    ESL_CUDA(cudaGetLastError());
     ESL_CUDA(cudaStreamSynchronize(s));
     return ESL_OK;
+}
+
+// the SCC list of a plan whose groups are one SCC each
+std::vector<uint4> one_scc_per_group(const SweepPlan* P) {
+    std::vector<uint4> list;
+    for (const SwGroup& g : P->groups) list.push_back(make_uint4(g.beg, g.ne, g.beg + g.ne, g.no));
+    return list;
 }
 
 int build_plan(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
@@ -2979,8 +3112,11 @@ int build_plan(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     }
     SweepPlan* P = nullptr;
     ESL_TRY(build_plan_device(ctx, net, P));
-    int rc = finish_scc_list(ctx, P);
-    if (rc == ESL_OK && P->term) rc = finish_scc_list(ctx, P->term);
+    int rc = finish_scc_list(ctx, P, nullptr);
+    if (rc == ESL_OK && P->term) {
+        const std::vector<uint4> list = one_scc_per_group(P->term);
+        rc = finish_scc_list(ctx, P->term, &list);
+    }
     if (rc != ESL_OK) {
         delete P;
         return rc;
@@ -3032,7 +3168,6 @@ int build_whole_plan(esl_ctx* ctx, const esl_net* net, bool back, SweepPlan*& ou
                 (par ? g.no : g.ne)++;
             }
     g.ns = 1;
-    P->h_scc.push_back(make_uint4(0, g.ne, g.ne, g.no));
     P->max_rows = M;
     P->max_even = g.ne;
     P->max_odd = g.no;
@@ -3081,7 +3216,8 @@ int build_whole_plan(esl_ctx* ctx, const esl_net* net, bool back, SweepPlan*& ou
     up(P->tp_ent, tp);
     if (back) up(P->rev, rev);
     if (rc == ESL_OK && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(ESL_ERR_CUDA, "plan upload failed");
-    if (rc == ESL_OK) rc = finish_scc_list(ctx, P.get());
+    const std::vector<uint4> list = one_scc_per_group(P.get());
+    if (rc == ESL_OK) rc = finish_scc_list(ctx, P.get(), &list);
     if (rc != ESL_OK) return rc;
     mnet->sweep_free = free_plan_sweep;
     out = P.get();
@@ -3172,25 +3308,27 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t skip
     ga.scc_sl = P->scc_sl.get() + g.s0;
     ga.sl = P->sl.get();
     ga.ell = P->ell.get();
-    const uint4* list = P->h_scc.data() + g.s0;
-    uint32_t nsplit = skip;
-    while (nsplit < g.ns && scc_rows(list[nsplit]) > (uint32_t)kSccMaxRows) nsplit++;
+    const SccShape *sh = P->shapes.data() + g.sh0, *sh_end = sh + g.nsh;
+    auto rows = [](const SccShape& x) { return std::max(x.even, x.odd); };
+    uint32_t j = 0;  // SCCs before shape sh
+    for (; j < skip; sh++) j += sh->count;
     // SCCs split over clusters: one launch per cluster size
-    for (uint32_t j = skip; j < nsplit;) {
-        auto size = [&](uint32_t i) { return (scc_rows(list[i]) + kSccMaxRows - 1) / kSccMaxRows; };
-        uint32_t j1 = j + 1;
-        while (j1 < nsplit && size(j1) == size(j)) j1++;
-        if ((uint64_t)(j1 - j) * K * size(j) > 0x7FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
+    while (sh < sh_end && rows(*sh) > (uint32_t)kSccMaxRows) {
+        auto size_of = [&](const SccShape& x) { return (rows(x) + kSccMaxRows - 1) / kSccMaxRows; };
+        const uint32_t size = size_of(*sh);
+        uint32_t j1 = j;
+        for (; sh < sh_end && size_of(*sh) == size; sh++) j1 += sh->count;
+        if ((uint64_t)(j1 - j) * K * size > 0x7FFFFFFFull) return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
         ga.nb = 1;
         ga.b[0] = SccBucket{0, (j1 - j) * (uint32_t)K, j, 0, 0, 10, 1};
         cudaLaunchAttribute attr[2]{};
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = size(j);
+        attr[0].val.clusterDim.x = size;
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((j1 - j) * (uint32_t)K * size(j));
+        cfg.gridDim = dim3((j1 - j) * (uint32_t)K * size);
         cfg.blockDim = dim3(kSccThreadsBig);
         cfg.dynamicSmemBytes = scc_smem_doubles(true, false, n, kSccMaxRows, kSccMaxRows, 0, kSccThreadsBig) * 8;
         cfg.stream = ctx->stream;
@@ -3203,19 +3341,13 @@ int launch_scc(esl_ctx* ctx, const SweepPlan* P, const SwGroup& g, uint32_t skip
         overlap = true;
         j = j1;
     }
-    uint32_t nbig = nsplit;
-    while (nbig < g.ns && scc_rows(list[nbig]) > (uint32_t)kSccThreads) nbig++;
     for (int part = 0; part < 2; part++) {
         const bool big = part == 0;
-        const uint32_t j0 = big ? nsplit : nbig, j1 = big ? nbig : g.ns;
-        std::vector<SccShape> shapes;
-        for (uint32_t j = j0; j < j1; j++)
-            if (!shapes.empty() && shapes.back().even == list[j].y && shapes.back().odd == list[j].w)
-                shapes.back().count++;
-            else
-                shapes.push_back({list[j].y, list[j].w, 1});
+        const SccShape* sh0 = sh;
+        const uint32_t j0 = j;
+        for (; sh < sh_end && (!big || rows(*sh) > (uint32_t)kSccThreads); sh++) j += sh->count;
         SccLaunch L;
-        if (!plan_scc_launch(shapes.data(), shapes.size(), j0, big, defl, K, n, ga.max_iters, ctx->sm_count, L))
+        if (!plan_scc_launch(sh0, (size_t)(sh - sh0), j0, big, defl, K, n, ga.max_iters, ctx->sm_count, L))
             return fail(ESL_ERR_TOO_LARGE, "too many systems for one call");
         std::copy(L.b, L.b + L.nb, ga.b);
         ga.nb = L.nb;
@@ -3493,7 +3625,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         ga.rev = P->rev.get();
         ga.Z = Z;
         const int slots[kOwnCount] = {W_R0, W_D, W_DS64, W_QO, W_BS, W_PH, W_W64, W_R, W_V, W_SH, W_TT, W_IQE};
-        const bool big = g.ns > 0 && scc_rows(P->h_scc[g.s0]) > (uint32_t)kSccThreads;
+        const bool big = g.most > (uint32_t)kSccThreads;
         for (int j = 0; j < (resident ? (big ? kOwnBS + 1 : 0) : kOwnCount); j++)
             ga.own[j] = (double*)ws.get(slots[j], (size_t)scc_own_rows(j, P->max_even, P->max_odd) * Kp * 8, &st_);
         if (!resident) {
@@ -3520,7 +3652,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         return ESL_OK;
     };
     uint32_t largest = 0;  // states of the largest SCC
-    for (const uint4& c : P->h_scc) largest = std::max(largest, c.y + c.w);
+    for (const SccShape& x : P->shapes) largest = std::max(largest, x.even + x.odd);
     bool first_launch = true;
     for (const SwGroup& g : P->groups) {
         // debug timing: wall time of the group with the stream drained on both sides
@@ -3575,8 +3707,8 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         // its rows (316,541 rows in SCCs of 126,976, 63,488, 63,488, 30,688, 30,688 and fewer
         // states, 512 systems: 420 -> 312 ms).
         std::vector<SwGroup> pieces;
-        for (uint32_t j = g.s0; j < g.s0 + g.ns && scc_rows(P->h_scc[j]) > kSccClusterRows; j++) {
-            const uint4& c = P->h_scc[j];
+        for (uint32_t j = g.l0; j < g.l0 + g.nlarge; j++) {
+            const uint4& c = P->large[j];
             SwGroup q = g;
             q.beg = c.x;
             q.ne = c.y;

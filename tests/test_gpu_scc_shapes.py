@@ -51,3 +51,36 @@ def test_two_sccs_whose_footprints_grow(esl):
     rng = np.random.default_rng(1)
     parts = [H.random_part(rng, 13, 2400, 1760), H.random_part(rng, 13, 2100, 2100) | (1 << 13)]
     solve_and_check(esl, H.masks(rng, 14, parts), [4160, 4200], 148, 2)
+
+
+def tiny_sccs(n):
+    """One free node (bit 0) beside nodes that only decay: 2^(n-1) - 1 SCCs of two states, and
+    two terminal states without edges."""
+    v = np.arange(1 << n, dtype=np.int64)
+    return np.where(v > 1, v | 1, 0).astype(np.uint32)
+
+
+@pytest.mark.parametrize("n,B", [(4, 3), (11, 1), (12, 40), (17, 2)])
+def test_many_tiny_sccs(esl, n, B):
+    solve_and_check(esl, tiny_sccs(n), [2] * ((1 << (n - 1)) - 1), B, n)
+
+
+def test_many_tiny_sccs_take_little_memory(esl):
+    """Network, plan and workspace of a solve with 524,287 SCCs: under 700 bytes per state (the
+    padded vectors of one system are 256 of them)."""
+    n = 20
+    rng = np.random.default_rng(3)
+    rates = synth.log_uniform_rates(rng, n, 1)
+    x0 = torch.as_tensor(rng.dirichlet(np.ones(1 << n))[None], device="cuda")
+    indptr, rows = (torch.as_tensor(a, device="cuda") for a in H.csc(tiny_sccs(n)))
+    out = torch.empty((1, 1, 1 << n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    esl.lib().esl_trim_cache()
+    before = torch.cuda.mem_get_info()[0]
+    ctx = esl.Context(0)
+    net = esl.Net.from_csc(ctx, n, indptr, rows)
+    res = esl.solve_batch(ctx, net, rates, x0, method=esl.METHOD_DIRECT, out=out)
+    assert res.report.converged == 1
+    torch.cuda.synchronize()
+    esl.lib().esl_trim_cache()
+    assert before - torch.cuda.mem_get_info()[0] < 700 << n
