@@ -2024,9 +2024,13 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         ESL_CUDA(cudaMemsetAsync(d_x_inf, 0, (size_t)K * N * 8, s));
         if (d_marg) ESL_CUDA(cudaMemsetAsync(d_marg, 0, (size_t)K * n * 8, s));
         ESL_COUNT_LAUNCH();
-        // up to eight CTAs of several states per thread for a system
-        const int parts = std::max(1, std::min(8, (TS + 4 * kScatterT - 1) / (4 * kScatterT)));
-        k_scatter_xinf<<<dim3(parts, K), kScatterT, (size_t)n * kScatterT * 8, s>>>(
+        // CTAs per system: a state per thread; with marginals, whose atomics a CTA costs, as many
+        // as fill the GPU, at least eight of four states per thread (262,144 terminal states, one
+        // solve: 208 us without and 245 us with marginals, 495 and 693 us with eight CTAs; 64
+        // systems 414 and 568 us, 642 and 837 us with eight)
+        const int full = (TS + kScatterT - 1) / kScatterT, eight = std::min(8, (full + 3) / 4);
+        const int parts = std::max(1, d_marg ? std::max(eight, std::min(full, (16 * ctx->sm_count + K - 1) / K)) : full);
+        k_scatter_xinf<<<dim3(parts, K), kScatterT, d_marg ? (size_t)n * kScatterT * 8 : 0, s>>>(
             n, T, TS, R, N, net->order.get(), net->term_of.get(), Rb, y, d_x_inf, d_marg);
         ESL_CUDA(cudaGetLastError());
     }
