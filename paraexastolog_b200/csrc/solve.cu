@@ -1910,6 +1910,7 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         const int rc = sweep_whole(ctx, net, K, R, d_rates, d_x0, N, o, y, sw);
         if (rc == ESL_OK) {
             agg.iters += sw.iters;
+            agg.refinements = sw.refinements;
             agg.relres = std::max(agg.relres, sw.relres);
             swept = true;
         } else if (rc != ESL_ERR_NOT_CONVERGED) {

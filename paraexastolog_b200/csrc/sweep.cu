@@ -1320,7 +1320,7 @@ struct SccArgs {
     int max_iters, max_outer, stall;
     unsigned long long* ratio;  // per system: max over SCCs of final |r|^2 / |b|^2 (bits of a double >= 0)
     int* fail;                  // per system: 1 once an SCC stays above the acceptance residual
-    int* iters;                 // the group's most inner iterations
+    int *iters, *refines;       // the group's most inner iterations and refinement steps
     // deflated (terminal) groups: kernels into Rb[k][pos[slot]], normalised to sum 1
     const uint32_t* pos;
     double* Rb;
@@ -1948,7 +1948,8 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     }
     double prev = 0.0, rr = b2;
     int noimp = 0, its = 0;
-    for (int outer = 0; !gb.dead; outer++) {
+    int outer = 0;  // refinement steps taken
+    for (; !gb.dead; outer++) {
         if (outer > 0 || warm || dense) {
             // true residual r = b - S x
             load_x();
@@ -2084,6 +2085,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         atomicMax(g.ratio + k, (unsigned long long)__double_as_longlong(b2 > 0.0 ? rr / b2 : 0.0));
         if (failed) g.fail[k] = 1;
         atomicMax(g.iters, its);
+        atomicMax(g.refines, outer);
     }
 }
 
@@ -3577,8 +3579,8 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     int* iscal = (int*)ws.get(W_ISCAL, (size_t)I_NISCAL * Kp * 4, &st_);
     int* d_cnt = (int*)ws.get(W_CNT, 64, &st_);
     // results of the SCC-resident groups: per system max |r|^2/|b|^2 and failure flag, per
-    // group the most iterations
-    const size_t loc_bytes = (size_t)Kp * 12 + P->groups.size() * 4;
+    // group the most iterations and refinement steps
+    const size_t loc_bytes = (size_t)Kp * 12 + P->groups.size() * 8;
     unsigned long long* loc_ratio = (unsigned long long*)ws.get(W_LOC, loc_bytes, &st_);
     if (st_ != ESL_OK) return st_;
     int* loc_fail = reinterpret_cast<int*>(loc_ratio + Kp);
@@ -3644,6 +3646,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         ga.ratio = loc_ratio;
         ga.fail = loc_fail;
         ga.iters = loc_iters + (&g - P->groups.data());
+        ga.refines = ga.iters + P->groups.size();
         if (term) {
             ga.pos = P->pos.get();
             ga.Rb = y;
@@ -4238,6 +4241,11 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         if (h_bar[1]) return fail(ESL_ERR_TIMEOUT, "a grid barrier of the level sweep did not complete in time");
         std::vector<int> h_its(P->groups.size());
         std::memcpy(h_its.data(), h_loc.data() + (size_t)Kp * 12, h_its.size() * 4);
+        for (size_t j = 0; j < P->groups.size(); j++) {
+            int steps;
+            std::memcpy(&steps, h_loc.data() + (size_t)Kp * 12 + (P->groups.size() + j) * 4, 4);
+            st.refinements = std::max(st.refinements, steps);
+        }
         for (int k = 0; k < K; k++) {
             double ratio;
             int bad;
