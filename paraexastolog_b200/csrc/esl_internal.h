@@ -308,6 +308,7 @@ constexpr int kDenseTerminalMax = 128;
 struct SweepStats {
     int iters = 0, refinements = 0, local_groups = 0, krylov_groups = 0, compactions = 0;
     double relres = 0.0;
+    double relres_kept = 0.0;  // of the systems not in `failed` (SCC-resident groups)
     std::vector<int32_t> failed;
 };
 bool sweep_supported(const esl_net* net);
@@ -322,7 +323,8 @@ int sweep_terminal(esl_ctx* ctx, const esl_net* net, int B, const double* rates,
 void free_sweep_workspace(void* w);
 // The transient part of a small network as one block (whole_supported): forward masses as
 // sweep_forward, and the absorption matrix L (T x N, terminal states included) of the first
-// rate set.  ESL_ERR_NOT_CONVERGED: nothing usable was written, another path must solve it.
+// rate set.  ESL_ERR_NOT_CONVERGED: another path must solve the systems in `failed` (all of
+// them, and L, where it is empty).
 bool whole_supported(const esl_net* net);
 int sweep_whole(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const double* rates, const double* x0, size_t x0_ld,
                 const esl_solve_opts& o, double* y, SweepStats& st);

@@ -536,9 +536,10 @@ __global__ void k_zero_r(int K, KState* st) {
 
 // ---- right-hand sides ---------------------------------------------------------------
 // forward: b = x0 on transient states; backward (system = (rate set, terminal t)):
-// b_v = sum of rates of edges v -> terminal t.  Written in both halves.
+// b_v = sum of rates of edges v -> terminal t.  Written in both halves.  x0_sys (forward): an x0
+// row per system, not per right-hand side.
 template <bool FWD>
-__global__ void k_rhs(Layout L, int n, const double* __restrict__ rates, const double* __restrict__ x0,
+__global__ void k_rhs(Layout L, int n, int x0_sys, const double* __restrict__ rates, const double* __restrict__ x0,
                       size_t x0_ld, const uint32_t* __restrict__ F, const int32_t* __restrict__ term_of,
                       double* __restrict__ bE, double* __restrict__ bO) {
     __shared__ double s_rate[64];
@@ -548,7 +549,7 @@ __global__ void k_rhs(Layout L, int n, const double* __restrict__ rates, const d
     uint32_t h = blockIdx.x * kT + threadIdx.x;
     if (h >= L.H) return;
     const size_t o = (size_t)k * L.ld;
-    const int r = k % L.nrhs;
+    const int r = x0_sys ? k : k % L.nrhs;
 #pragma unroll
     for (int par = 0; par < 2; par++) {
         uint32_t v = state_of(h, par);
@@ -1018,7 +1019,8 @@ namespace {
 enum Slot {
     S_BE, S_BS, S_DS, S_X64, S_R64, S_W64, S_ZE, S_ST, S_ACT,
     S_R, S_R0, S_PH, S_V, S_SH, S_T, S_D, S_W,
-    S_M0, S_M1, S_F0, S_F1, S_RB, S_Y, S_SUM, S_BIG, S_PIN, S_BO, S_LIST, S_XT, S_RT, S_ACTLIST, S_ZEF, S_ZOF, S_ZEB, S_ZOB, S_RSUB, S_XSUB, S_LUOFF, S_LUSYS, S_LU, S_COUNT
+    S_M0, S_M1, S_F0, S_F1, S_RB, S_Y, S_SUM, S_BIG, S_PIN, S_BO, S_LIST, S_XT, S_RT, S_ACTLIST, S_ZEF, S_ZOF, S_ZEB, S_ZOB, S_RSUB, S_XSUB, S_LUOFF, S_LUSYS, S_LU,
+    S_MISS, S_MISSR, S_MISSX, S_MISSY, S_COUNT
 };
 
 struct SolveOut {
@@ -1905,16 +1907,46 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         }
         swept = true;
     }
+    // the systems of the whole-system form: all, or those that one resident block missed
+    struct {
+        int K, R, x0_sys;
+        const double *rates, *x0, *warm;
+        double* y;
+        const int32_t* missed;  // their places among the K systems, or null
+    } w = {K, R, 0, d_rates, d_x0, o.d_warm, y, nullptr};
     if (!swept && has_transient && o.method == ESL_METHOD_FP64 && whole_supported(net)) {
         SweepStats sw;
         const int rc = sweep_whole(ctx, net, K, R, d_rates, d_x0, N, o, y, sw);
+        agg.iters += sw.iters;
         if (rc == ESL_OK) {
-            agg.iters += sw.iters;
             agg.refinements = sw.refinements;
             agg.relres = std::max(agg.relres, sw.relres);
             swept = true;
         } else if (rc != ESL_ERR_NOT_CONVERGED) {
             return rc;
+        } else if (!sw.failed.empty() && (int)sw.failed.size() < K) {
+            agg.relres = std::max(agg.relres, sw.relres_kept);
+            w.K = (int)sw.failed.size();
+            w.R = 1;
+            w.x0_sys = 1;
+            w.warm = nullptr;
+            int32_t* missed = (int32_t*)ws.get(S_MISS, (size_t)w.K * 4, &st_);
+            double* r_sub = (double*)ws.get(S_MISSR, (size_t)w.K * 2 * n * 8, &st_);
+            double* x_sub = (double*)ws.get(S_MISSX, (size_t)w.K * N * 8, &st_);
+            w.y = (double*)ws.get(S_MISSY, (size_t)w.K * T * 8, &st_);
+            if (st_ != ESL_OK) return st_;
+            ESL_CUDA(cudaMemcpyAsync(missed, sw.failed.data(), (size_t)w.K * 4, cudaMemcpyHostToDevice, s));
+            for (int j = 0; j < w.K; j++) {
+                const int k = sw.failed[j];
+                ESL_CUDA(cudaMemcpyAsync(r_sub + (size_t)j * 2 * n, d_rates + (size_t)(k / R) * 2 * n, 2 * n * 8,
+                                         cudaMemcpyDeviceToDevice, s));
+                ESL_CUDA(cudaMemcpyAsync(x_sub + (size_t)j * N, d_x0 + (size_t)(k % R) * N, N * 8,
+                                         cudaMemcpyDeviceToDevice, s));
+            }
+            ESL_CUDA(cudaMemsetAsync(w.y, 0, (size_t)w.K * T * 8, s));
+            w.missed = missed;
+            w.rates = r_sub;
+            w.x0 = x_sub;
         } else {
             ESL_CUDA(cudaMemsetAsync(y, 0, (size_t)K * T * 8, s));
         }
@@ -1923,8 +1955,8 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         // terminal masses are in y
     } else if (has_transient) {
         Layout L;
-        ESL_TRY(make_layout(ctx, ws, net, 0, nullptr, true, L, R));
-        const size_t vec = (size_t)K * L.ld;
+        ESL_TRY(make_layout(ctx, ws, net, 0, nullptr, true, L, w.R));
+        const size_t vec = (size_t)w.K * L.ld;
         double* ZE = nullptr;
         double* ZO = nullptr;
         int rc = ESL_OK;
@@ -1944,15 +1976,16 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
             double* bE = (double*)ws.get(S_BE, vec * 8, &st_);
             double* bO = (double*)ws.get(S_BO, vec * 8, &st_);
             if (st_ != ESL_OK) return st_;
-            dim3 g = grid2(L.H, K);
+            dim3 g = grid2(L.H, w.K);
             ESL_COUNT_LAUNCH();
-            k_rhs<true><<<g, kT, 0, s>>>(L, n, d_rates, d_x0, N, net->F.get(), net->term_of.get(), bE, bO);
+            k_rhs<true><<<g, kT, 0, s>>>(L, n, w.x0_sys, w.rates, w.x0, N, net->F.get(), net->term_of.get(), bE, bO);
             ESL_CUDA(cudaGetLastError());
             double *x64 = nullptr, *zE = nullptr;
-            rc = krylov_solve<true>(ctx, ws, L, d_rates, K, bE, bO, o.d_warm, N, o, x64, zE, so);
+            const double kept = agg.relres;  // of the systems that the block solved
+            rc = krylov_solve<true>(ctx, ws, L, w.rates, w.K, bE, bO, w.warm, N, o, x64, zE, so);
             agg.iters += so.iters;
             agg.refinements = so.refinements;
-            agg.relres = so.relres;
+            agg.relres = std::max(w.missed ? kept : 0.0, so.relres);
             agg.converged = so.converged;
             // keep the whole-system result out of the Krylov scratch slots
             ws.swap(S_X64, S_ZOF);
@@ -1962,10 +1995,10 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
             if (rc == ESL_ERR_NOT_CONVERGED) {
                 // fallback: systems that missed the budget go through the block solve
                 std::vector<int32_t> failed;
-                for (int k = 0; k < K; k++)
+                for (int k = 0; k < w.K; k++)
                     if (so.sys_relres[k] > kAcceptRel) failed.push_back(k);
                 const int Kf = (int)failed.size();
-                if (debug_enabled()) fprintf(stderr, "[esl] block-solve fallback for %d of %d systems\n", Kf, K);
+                if (debug_enabled()) fprintf(stderr, "[esl] block-solve fallback for %d of %d systems\n", Kf, w.K);
                 double* r_sub = (double*)ws.get(S_RSUB, (size_t)Kf * 2 * n * 8, &st_);
                 double* x_sub = (double*)ws.get(S_XSUB, (size_t)Kf * N * 8, &st_);
                 int32_t* d_failed = (int32_t*)ws.get(S_LIST, (size_t)Kf * 4, &st_);
@@ -1974,9 +2007,9 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
                 if (st_ != ESL_OK) return st_;
                 for (int j = 0; j < Kf; j++) {
                     const int k = failed[j];
-                    ESL_CUDA(cudaMemcpyAsync(r_sub + (size_t)j * 2 * n, d_rates + (size_t)(k / R) * 2 * n, 2 * n * 8,
+                    ESL_CUDA(cudaMemcpyAsync(r_sub + (size_t)j * 2 * n, w.rates + (size_t)(k / w.R) * 2 * n, 2 * n * 8,
                                              cudaMemcpyDeviceToDevice, s));
-                    ESL_CUDA(cudaMemcpyAsync(x_sub + (size_t)j * N, d_x0 + (size_t)(k % R) * N, N * 8,
+                    ESL_CUDA(cudaMemcpyAsync(x_sub + (size_t)j * N, w.x0 + (size_t)(w.x0_sys ? k : k % w.R) * N, N * 8,
                                              cudaMemcpyDeviceToDevice, s));
                 }
                 ESL_CUDA(cudaMemcpyAsync(d_failed, failed.data(), (size_t)Kf * 4, cudaMemcpyHostToDevice, s));
@@ -1989,8 +2022,8 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
                 agg.fallback_systems += Kf;
                 agg.dense_systems += sb.dense_systems;
                 agg.converged = sb.converged;
-                double worst = 0.0;
-                for (int k = 0; k < K; k++)
+                double worst = w.missed ? kept : 0.0;
+                for (int k = 0; k < w.K; k++)
                     if (so.sys_relres[k] <= kAcceptRel) worst = std::max(worst, so.sys_relres[k]);
                 agg.relres = std::max(worst, sb.relres);
                 dim3 gs((unsigned)((L.ld + 255) / 256), (unsigned)Kf);
@@ -2003,9 +2036,13 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
         }
         if (rc != ESL_OK && rc != ESL_ERR_NOT_CONVERGED) return rc;
         ESL_COUNT_LAUNCH();
-        k_terminal_mass<<<dim3((TS + 127) / 128, K), 128, 0, s>>>(n, T, TS, R, 0, L.ld, d_rates, d_x0, N,
+        k_terminal_mass<<<dim3((TS + 127) / 128, w.K), 128, 0, s>>>(n, T, TS, w.R, w.x0_sys, L.ld, w.rates, w.x0, N,
                                                                     net->order.get(), net->term_of.get(),
-                                                                    net->G.get(), ZE, ZO, y);
+                                                                    net->G.get(), ZE, ZO, w.y);
+        if (w.missed) {
+            ESL_COUNT_LAUNCH();
+            k_set_rows<<<dim3((T + 127) / 128, w.K), 128, 0, s>>>(T, w.missed, w.y, y);
+        }
         ESL_CUDA(cudaGetLastError());
         if (rc == ESL_ERR_NOT_CONVERGED) {
             if (rep) {
@@ -2060,7 +2097,7 @@ int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, 
             if (st_ != ESL_OK) return st_;
             dim3 g = grid2(L.H, T);
             ESL_COUNT_LAUNCH();
-            k_rhs<false><<<g, kT, 0, s>>>(L, n, d_rates, d_x0, N, net->F.get(), net->term_of.get(), bE, bO);
+            k_rhs<false><<<g, kT, 0, s>>>(L, n, 0, d_rates, d_x0, N, net->F.get(), net->term_of.get(), bE, bO);
             ESL_CUDA(cudaGetLastError());
             double *x64 = nullptr, *zE = nullptr;
             SolveOut so;

@@ -4253,6 +4253,7 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
             std::memcpy(&bad, h_loc.data() + (size_t)Kp * 8 + (size_t)k * 4, 4);
             st.relres = std::max(st.relres, std::sqrt(ratio));
             if (bad) failed[k] = 1;
+            else st.relres_kept = std::max(st.relres_kept, std::sqrt(ratio));
         }
         // groups of larger SCCs add their iterations, groups of small ones run beside them
         int small = 0;
