@@ -331,7 +331,7 @@ int sweep_whole(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const double*
 int sweep_absorption(esl_ctx* ctx, const esl_net* net, const double* rates, const esl_solve_opts& o, double* d_L,
                      SweepStats& st);
 // checksums (FNV-1a 64) of the 12 parts of a freshly built level-sweep plan: rows, desc,
-// ig_ptr, ig_ent, og_ptr, og_ent, tp_ptr, tp_ent, lsc_off, lsc_ne, lsc_slots, group table;
+// ig_ptr, ig_ent, og_ptr, og_ent, tp_ptr, tp_ent, SCC list, slices, lines, group table;
 // host != 0 builds it with the host reference builder instead of the device one
 int plan_checksums_for(esl_ctx* ctx, const esl_net* net, int host, uint64_t* out, int cap);
 // states whose warm start the sweep's grid-wide Krylov groups read (their odd-parity rows)

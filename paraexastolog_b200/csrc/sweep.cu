@@ -85,8 +85,6 @@ struct SwGroup {
     uint32_t ob;           // first odd slot (beg + ne, except in a piece of a group)
     int kind;              // 0 singletons, 1 SCCs of at most kSwLocalMax states, 2 larger ones
     int max_scc;
-    uint32_t scc0, nscc;   // local groups: range in the local SCC list (SCCs of >= 2 states)
-    int max_odd;           // local groups: most odd rows of one SCC
     uint64_t nin;          // in-group predecessor entries of the group's rows
     uint32_t s0, ns;       // the group's SCCs of >= 2 states: range in SweepPlan::scc
     uint32_t sh0, nsh;     // their shapes: range in SweepPlan::shapes
@@ -100,7 +98,7 @@ struct SwGroup {
 };
 
 struct SweepPlan {
-    uint32_t M = 0, max_rows = 0, max_even = 0, max_odd = 0, max_even_local = 0, max_odd_local = 0;
+    uint32_t M = 0, max_rows = 0, max_even = 0, max_odd = 0;
     int TS = 0;
     std::vector<SwGroup> groups;
     DevBuf<uint2> rows;                  // per slot: (state, out-mask)
@@ -108,7 +106,6 @@ struct SweepPlan {
     DevBuf<uint32_t> ig_ptr, ig_ent;     // predecessors inside the group: slot << 6 | rate index
     DevBuf<uint32_t> og_ptr, og_ent;     // predecessors in earlier groups
     DevBuf<uint32_t> tp_ptr, tp_ent;     // transient predecessors of terminal position p
-    DevBuf<uint32_t> lsc_off;            // local SCCs: offsets into lsc_slots
     // SCCs of >= 2 states in the order of scc_sort_key: (first even slot, even rows, first odd
     // slot, odd rows); an SCC's even and odd slots are one run each.  The host keeps their
     // shapes, and the places of those beyond a cluster: a network may have millions of SCCs.
@@ -127,8 +124,6 @@ struct SweepPlan {
     // rank << 13 | its row there, and past the last entry the own rank's row kSccMaxRows.
     DevBuf<uint2> scc_sl, sl;
     DevBuf<uint4> ell;
-    DevBuf<uint32_t> lsc_ne;             // local SCCs: number of even-parity slots (listed first)
-    DevBuf<uint32_t> lsc_slots;          // local SCCs: slots, SCC by SCC
     // terminal plan: per slot, the state's position in the reordering
     DevBuf<uint32_t> pos;
     // backward plan of the whole transient part: per slot, the in-mask among transient states
@@ -2225,6 +2220,63 @@ int build_terminal_plan(const std::vector<int32_t>& order, const std::vector<int
     return ESL_OK;
 }
 
+int finish_scc_list(esl_ctx* ctx, SweepPlan* P, const std::vector<uint4>* list);
+
+// The lines of SweepPlan::sl and ell made on the host from the predecessor lists, in place of
+// those that finish_scc_list made.
+int host_lines(esl_ctx* ctx, SweepPlan* P, const std::vector<uint32_t>& ig_ptr, const std::vector<uint32_t>& ig) {
+    uint32_t count = 0;
+    for (const SwGroup& g : P->groups) count += g.ns;
+    if (count == 0 || !P->sl.get()) return ESL_OK;
+    cudaStream_t s = ctx->stream;
+    std::vector<uint4> scc(count), wide, narrow;
+    ESL_CUDA(cudaMemcpyAsync(scc.data(), P->scc.get(), (size_t)count * sizeof(uint4), cudaMemcpyDeviceToHost, s));
+    ESL_CUDA(cudaStreamSynchronize(s));
+    std::vector<uint2> sl;
+    std::vector<uint8_t> is_narrow;
+    for (const uint4& c : scc) {
+        if (std::max(c.y, c.w) > kSccClusterRows) continue;
+        const bool nar = scc_narrow(c.y, c.w), split = std::max(c.y, c.w) > (uint32_t)kSccMaxRows;
+        for (int par = 0; par < 2; par++) {
+            const uint32_t slot0 = par ? c.z : c.x, rows = par ? c.w : c.y, other = par ? c.x : c.z,
+                           others = par ? c.y : c.w;
+            for (uint32_t r0 = 0; r0 < rows; r0 += 32) {
+                const uint32_t here = std::min(32u, rows - r0), width = nar ? here : 32u;
+                uint32_t most = 0;
+                for (uint32_t r = r0; r < r0 + here; r++) most = std::max(most, ig_ptr[slot0 + r + 1] - ig_ptr[slot0 + r]);
+                const uint32_t lines = (most + 3) / 4;
+                std::vector<uint4>& out = nar ? narrow : wide;
+                sl.push_back(make_uint2(lines, (uint32_t)(nar ? out.size() : out.size() / 32)));
+                is_narrow.push_back(nar);
+                const uint32_t none = split ? r0 / kSccMaxRows << 13 | (uint32_t)kSccMaxRows : others;
+                for (uint32_t j = 0; j < lines; j++)
+                    for (uint32_t l = 0; l < width; l++) {
+                        uint32_t e[4];
+                        for (uint32_t u = 0; u < 4; u++) {
+                            const uint32_t p = l < here ? ig_ptr[slot0 + r0 + l] + 4 * j + u : 0;
+                            if (l < here && p < ig_ptr[slot0 + r0 + l + 1]) {
+                                const uint32_t x = ig[p], r = (x >> 6) - other;
+                                e[u] = (split ? (r / kSccMaxRows) << 13 | r % kSccMaxRows : r) << 9 | (x & 63u) << 3;
+                            } else {
+                                e[u] = none << 9;
+                            }
+                        }
+                        out.push_back(make_uint4(e[0], e[1], e[2], e[3]));
+                    }
+            }
+        }
+    }
+    for (size_t i = 0; i < sl.size(); i++)
+        if (is_narrow[i]) sl[i].y += (uint32_t)wide.size();
+    wide.insert(wide.end(), narrow.begin(), narrow.end());
+    ESL_TRY(P->sl.alloc(sl.size()));
+    ESL_TRY(P->ell.alloc(wide.size()));
+    ESL_CUDA(cudaMemcpyAsync(P->sl.get(), sl.data(), sl.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
+    ESL_CUDA(cudaMemcpyAsync(P->ell.get(), wide.data(), wide.size() * sizeof(uint4), cudaMemcpyHostToDevice, s));
+    ESL_CUDA(cudaStreamSynchronize(s));
+    return ESL_OK;
+}
+
 // The plan built on the host from copies of the net's arrays: the reference the device
 // builder (build_plan_device) is checked against, bit for bit.
 int build_plan_host(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
@@ -2251,7 +2303,7 @@ int build_plan_host(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     std::vector<uint32_t> slot_of(N, 0xFFFFFFFFu);
     std::vector<uint2> rows;
     rows.reserve(M);
-    std::vector<uint32_t> lsc_off{0}, lsc_ne, lsc_slots;
+    std::vector<uint4> list;  // SCCs of >= 2 states
     for (int c = T; c < n_sccs;) {
         int c1 = c, mx = 0;
         while (c1 < n_sccs && levels[c1] == levels[c]) {
@@ -2272,33 +2324,20 @@ int build_plan_host(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
             }
             (par ? g.no : g.ne) = (uint32_t)rows.size() - g.beg - (par ? g.ne : 0);
         }
-        if (g.kind == 1) {
-            // SCCs of >= 2 states, each with its even-parity slots first
-            g.scc0 = (uint32_t)lsc_ne.size();
-            for (int cc = c; cc < c1; cc++) {
-                const int sz = offsets[cc + 1] - offsets[cc];
-                if (sz < 2) continue;
-                uint32_t ne = 0;
-                for (int par = 0; par < 2; par++)
-                    for (int p = offsets[cc]; p < offsets[cc + 1]; p++) {
-                        const uint32_t v = (uint32_t)order[p];
-                        if ((uint32_t)(__builtin_popcount(v) & 1) != (uint32_t)par) continue;
-                        lsc_slots.push_back(slot_of[v]);
-                        ne += par == 0;
-                    }
-                lsc_off.push_back((uint32_t)lsc_slots.size());
-                lsc_ne.push_back(ne);
-                g.max_odd = std::max(g.max_odd, sz - (int)ne);
-            }
-            g.nscc = (uint32_t)lsc_ne.size() - g.scc0;
+        g.s0 = (uint32_t)list.size();
+        uint32_t er = 0, orr = 0;  // rows of the SCCs before, of either parity
+        for (int cc = c; cc < c1; cc++) {
+            uint32_t ne = 0, no = 0;
+            for (int p = offsets[cc]; p < offsets[cc + 1]; p++)
+                (__builtin_popcount((uint32_t)order[p]) & 1 ? no : ne)++;
+            if (ne + no >= 2) list.push_back(make_uint4(g.beg + er, ne, g.beg + g.ne + orr, no));
+            er += ne;
+            orr += no;
         }
+        g.ns = (uint32_t)list.size() - g.s0;
         P->max_rows = std::max(P->max_rows, g.ne + g.no);
         P->max_even = std::max(P->max_even, g.ne);
         P->max_odd = std::max(P->max_odd, g.no);
-        if (g.kind == 1) {
-            P->max_even_local = std::max(P->max_even_local, g.ne);
-            P->max_odd_local = std::max(P->max_odd_local, g.no);
-        }
         P->groups.push_back(g);
         c = c1;
     }
@@ -2402,10 +2441,9 @@ int build_plan_host(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     up32(P->og_ent, og);
     up32(P->tp_ptr, tp_ptr);
     up32(P->tp_ent, tp);
-    up32(P->lsc_off, lsc_off);
-    up32(P->lsc_ne, lsc_ne);
-    up32(P->lsc_slots, lsc_slots);
     if (rc == ESL_OK && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(ESL_ERR_CUDA, "sweep plan upload failed");
+    if (rc == ESL_OK) rc = finish_scc_list(ctx, P, &list);
+    if (rc == ESL_OK) rc = host_lines(ctx, P, ig_ptr, ig);
     if (rc == ESL_OK) rc = build_terminal_plan(order, offsets, T, F, G, s, P->term);
     if (rc != ESL_OK) {
         delete P;
@@ -2453,34 +2491,27 @@ __global__ void k_pl_even(uint32_t M, int TS, const int32_t* __restrict__ order,
 }
 
 // Group g (one warp): info[g] = (first position, even rows, odd rows, kind, largest SCC,
-// first SCC, SCCs of >= 2 states, most odd rows of one of them); local groups flag their
-// SCCs of >= 2 states for the CTA-local lists.
+// first SCC, SCCs of >= 2 states).
 __global__ void k_pl_groups(int T, int TS, const int32_t* __restrict__ offsets, const uint32_t* __restrict__ gid_incl,
                             int NT, const uint32_t* __restrict__ gfirst, const uint32_t* __restrict__ ssize,
-                            const uint32_t* __restrict__ E, uint32_t* __restrict__ info, uint32_t* __restrict__ qual) {
+                            const uint32_t* __restrict__ E, uint32_t* __restrict__ info) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int G = (int)gid_incl[NT - 1];
     if (warp >= G) return;
     const uint32_t c0 = gfirst[warp], c1 = gfirst[warp + 1];
     const uint32_t p0 = (uint32_t)(offsets[T + c0] - TS), p1 = (uint32_t)(offsets[T + c1] - TS);
-    uint32_t mx = 0, n2 = 0, mo = 0;
+    uint32_t mx = 0, n2 = 0;
     for (uint32_t c = c0 + lane; c < c1; c += 32) {
         const uint32_t sz = ssize[c];
         mx = max(mx, sz);
-        if (sz >= 2) {
-            n2++;
-            const uint32_t cs = (uint32_t)(offsets[T + c] - TS), ce = cs + sz;
-            mo = max(mo, sz - (E[ce] - E[cs]));
-        }
+        if (sz >= 2) n2++;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         mx = max(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-        mo = max(mo, __shfl_xor_sync(0xFFFFFFFFu, mo, o));
         n2 += __shfl_xor_sync(0xFFFFFFFFu, n2, o);
     }
     const uint32_t kind = mx == 1 ? 0u : (mx <= (uint32_t)kSwLocalMax ? 1u : 2u);
-    for (uint32_t c = c0 + lane; c < c1; c += 32) qual[c] = (kind == 1 && ssize[c] >= 2) ? 1u : 0u;
     if (lane == 0) {
         const uint32_t ne = E[p1] - E[p0];
         uint32_t* o = info + (size_t)warp * 8;
@@ -2491,7 +2522,6 @@ __global__ void k_pl_groups(int T, int TS, const int32_t* __restrict__ offsets, 
         o[4] = mx;
         o[5] = c0;
         o[6] = n2;
-        o[7] = mo;
     }
 }
 
@@ -2596,49 +2626,14 @@ __global__ void k_pl_tpreds(int TS, const int32_t* __restrict__ order, const uin
     if (COUNT) cnt[p] = c;
 }
 
-// per group: first local-SCC list entry and in-group predecessor entries
-__global__ void k_pl_gtail(int G, const uint32_t* __restrict__ info, const uint32_t* __restrict__ qidx,
-                           const uint32_t* __restrict__ ig_ptr, uint32_t* __restrict__ gtail) {
+// per group: in-group predecessor entries
+__global__ void k_pl_gtail(int G, const uint32_t* __restrict__ info, const uint32_t* __restrict__ ig_ptr,
+                           uint32_t* __restrict__ gtail) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= G) return;
     const uint32_t* in = info + (size_t)g * 8;
     const uint32_t b = in[0], e = in[0] + in[1] + in[2];
-    gtail[2 * g] = qidx[in[5]];
-    gtail[2 * g + 1] = ig_ptr[e] - ig_ptr[b];
-}
-
-// CTA-local SCC lists: slots of each flagged SCC, even-parity ones first
-__global__ void k_pl_lsc(uint32_t M, int T, int TS, const int32_t* __restrict__ offsets, const int32_t* __restrict__ order,
-                         const uint32_t* __restrict__ E, const uint32_t* __restrict__ sccpos,
-                         const uint32_t* __restrict__ qual, const uint32_t* __restrict__ qidx,
-                         const uint32_t* __restrict__ qoff, const uint32_t* __restrict__ ssize,
-                         const uint32_t* __restrict__ slot_of, uint32_t* __restrict__ lsc_off,
-                         uint32_t* __restrict__ lsc_ne, uint32_t* __restrict__ lsc_slots, uint32_t Q) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= M) return;
-    const uint32_t c = sccpos[p] - 1;
-    if (!qual[c]) return;
-    const uint32_t cs = (uint32_t)(offsets[T + c] - TS), sz = ssize[c];
-    const uint32_t ne = E[cs + sz] - E[cs];
-    const uint32_t v = (uint32_t)order[TS + p];
-    const bool even = (__popc(v) & 1) == 0;
-    const uint32_t er = E[p] - E[cs];
-    const uint32_t local = even ? er : ne + (p - cs) - er;
-    lsc_slots[qoff[c] + local] = slot_of[v];
-    if (p == cs) {
-        const uint32_t j = qidx[c];
-        lsc_off[j] = qoff[c];
-        lsc_ne[j] = ne;
-        if (j + 1 == Q) lsc_off[Q] = qoff[c] + sz;
-    }
-}
-
-// qsize = size of a flagged SCC, else 0 (one more, zero, entry for the scan)
-__global__ void k_pl_qsize(int NT, const uint32_t* __restrict__ qual, const uint32_t* __restrict__ ssize,
-                           uint32_t* __restrict__ qsize) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c > NT) return;
-    qsize[c] = (c < NT && qual[c]) ? ssize[c] : 0u;
+    gtail[g] = ig_ptr[e] - ig_ptr[b];
 }
 
 // exclusive scan of n + 1 counts (the last one 0) into out[0 .. n], on the stream
@@ -2677,19 +2672,15 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
     const int32_t* order = net->order.get();
     const int32_t* offsets = net->offsets.get();
     std::vector<uint32_t> h_info, h_tail;
-    uint32_t G = 0, tot[5] = {0, 0, 0, 0, 0};
+    uint32_t G = 0, tot[3] = {0, 0, 0};
     if (M > 0) {
-        DevBuf<uint32_t> gflag, gid, ssize, gfirst, info, qual, qidx, qsize, qoff, pos_head, sccpos, ev, E, slot_grp,
-            cnt_in, cnt_out, gtail;
+        DevBuf<uint32_t> gflag, gid, ssize, gfirst, info, pos_head, sccpos, ev, E, slot_grp, cnt_in, cnt_out,
+            gtail;
         ESL_TRY(gflag.alloc(NT));
         ESL_TRY(gid.alloc(NT));
         ESL_TRY(ssize.alloc(NT));
         ESL_TRY(gfirst.alloc(NT + 1));
         ESL_TRY(info.alloc((size_t)NT * 8));
-        ESL_TRY(qual.alloc(NT + 1));
-        ESL_TRY(qidx.alloc(NT + 1));
-        ESL_TRY(qsize.alloc(NT + 1));
-        ESL_TRY(qoff.alloc(NT + 1));
         ESL_TRY(pos_head.alloc(M));
         ESL_TRY(sccpos.alloc(M));
         ESL_TRY(ev.alloc((size_t)M + 1));
@@ -2698,7 +2689,6 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         ESL_TRY(cnt_in.alloc((size_t)M + 1));
         ESL_TRY(cnt_out.alloc((size_t)M + 1));
         ESL_CUDA(cudaMemsetAsync(pos_head.get(), 0, (size_t)M * 4, s));
-        ESL_CUDA(cudaMemsetAsync(qual.get(), 0, (size_t)(NT + 1) * 4, s));
         ESL_COUNT_LAUNCH();
         k_pl_sccs<<<nblk(NT), 256, 0, s>>>(T, NT, TS, offsets, net->levels.get(), gflag.get(), ssize.get(),
                                            pos_head.get());
@@ -2711,13 +2701,8 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         ESL_TRY(scan_incl(tmp, pos_head.get(), sccpos.get(), M, s));
         ESL_COUNT_LAUNCH();
         k_pl_groups<<<nblk((uint64_t)NT * 32), 256, 0, s>>>(T, TS, offsets, gid.get(), NT, gfirst.get(), ssize.get(),
-                                                            E.get(), info.get(), qual.get());
+                                                            E.get(), info.get());
         ESL_CUDA(cudaGetLastError());
-        // CTA-local lists: index and slot offset of every flagged SCC
-        ESL_TRY(scan_excl(tmp, qual.get(), qidx.get(), (uint32_t)NT + 1, s));
-        ESL_COUNT_LAUNCH();
-        k_pl_qsize<<<nblk((uint64_t)NT + 1), 256, 0, s>>>(NT, qual.get(), ssize.get(), qsize.get());
-        ESL_TRY(scan_excl(tmp, qsize.get(), qoff.get(), (uint32_t)NT + 1, s));
         ESL_TRY(P->rows.alloc(M));
         ESL_COUNT_LAUNCH();
         k_pl_slots<<<nblk(M), 256, 0, s>>>(M, TS, order, net->F.get(), E.get(), sccpos.get(), gid.get(), info.get(),
@@ -2736,30 +2721,29 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         // the group count and the group table
         ESL_CUDA(cudaMemcpyAsync(&G, gid.get() + NT - 1, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
-        ESL_TRY(gtail.alloc((size_t)G * 2));
+        ESL_TRY(gtail.alloc(G));
         ESL_COUNT_LAUNCH();
-        k_pl_gtail<<<nblk(G), 256, 0, s>>>((int)G, info.get(), qidx.get(), P->ig_ptr.get(), gtail.get());
+        k_pl_gtail<<<nblk(G), 256, 0, s>>>((int)G, info.get(), P->ig_ptr.get(), gtail.get());
         ESL_CUDA(cudaGetLastError());
         h_info.resize((size_t)G * 8);
-        h_tail.resize((size_t)G * 2);
+        h_tail.resize(G);
         ESL_CUDA(cudaMemcpyAsync(h_info.data(), info.get(), (size_t)G * 32, cudaMemcpyDeviceToHost, s));
-        ESL_CUDA(cudaMemcpyAsync(h_tail.data(), gtail.get(), (size_t)G * 8, cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaMemcpyAsync(h_tail.data(), gtail.get(), (size_t)G * 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaMemcpyAsync(&tot[0], P->ig_ptr.get() + M, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaMemcpyAsync(&tot[1], P->og_ptr.get() + M, 4, cudaMemcpyDeviceToHost, s));
-        ESL_CUDA(cudaMemcpyAsync(&tot[2], qidx.get() + NT, 4, cudaMemcpyDeviceToHost, s));
-        ESL_CUDA(cudaMemcpyAsync(&tot[3], qoff.get() + NT, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
-        // the list of SCCs of >= 2 states (qsize and qoff are free again)
+        // the list of SCCs of >= 2 states
         uint32_t n2 = 0;
         for (uint32_t g = 0; g < G; g++) n2 += h_info[(size_t)g * 8 + 6];
         if (n2 > 0) {
             ESL_TRY(P->scc.alloc(n2));
             ESL_TRY(P->scc_key.alloc(n2));
-            ESL_COUNT_LAUNCH();
-            k_pl_scc2<<<nblk((uint64_t)NT + 1), 256, 0, s>>>(NT, ssize.get(), qsize.get());
-            DevBuf<uint32_t> sidx;
+            DevBuf<uint32_t> flag, sidx;
+            ESL_TRY(flag.alloc((size_t)NT + 1));
             ESL_TRY(sidx.alloc((size_t)NT + 1));
-            ESL_TRY(scan_excl(tmp, qsize.get(), sidx.get(), (uint32_t)NT + 1, s));
+            ESL_COUNT_LAUNCH();
+            k_pl_scc2<<<nblk((uint64_t)NT + 1), 256, 0, s>>>(NT, ssize.get(), flag.get());
+            ESL_TRY(scan_excl(tmp, flag.get(), sidx.get(), (uint32_t)NT + 1, s));
             ESL_COUNT_LAUNCH();
             k_pl_scc_list<<<nblk(NT), 256, 0, s>>>(NT, T, TS, offsets, gid.get(), ssize.get(), E.get(), info.get(),
                                                    sidx.get(), P->scc.get(), P->scc_key.get());
@@ -2772,16 +2756,6 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         k_pl_preds<false><<<nblk(M), 256, 0, s>>>(M, P->rows.get(), net->G.get(), slot_of.get(), slot_grp.get(),
                                                   info.get(), nullptr, nullptr, P->ig_ptr.get(), P->og_ptr.get(),
                                                   P->ig_ent.get(), P->og_ent.get(), P->desc.get());
-        ESL_TRY(P->lsc_off.alloc((size_t)tot[2] + 1));
-        ESL_TRY(P->lsc_ne.alloc(std::max<uint32_t>(tot[2], 1)));
-        ESL_TRY(P->lsc_slots.alloc(std::max<uint32_t>(tot[3], 1)));
-        ESL_CUDA(cudaMemsetAsync(P->lsc_off.get(), 0, 4, s));
-        if (tot[2] > 0) {
-            ESL_COUNT_LAUNCH();
-            k_pl_lsc<<<nblk(M), 256, 0, s>>>(M, T, TS, offsets, order, E.get(), sccpos.get(), qual.get(), qidx.get(),
-                                             qoff.get(), ssize.get(), slot_of.get(), P->lsc_off.get(), P->lsc_ne.get(),
-                                             P->lsc_slots.get(), tot[2]);
-        }
         ESL_CUDA(cudaGetLastError());
     } else {
         ESL_TRY(P->rows.alloc(1));
@@ -2790,12 +2764,8 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         ESL_TRY(P->og_ptr.alloc(1));
         ESL_TRY(P->ig_ent.alloc(1));
         ESL_TRY(P->og_ent.alloc(1));
-        ESL_TRY(P->lsc_off.alloc(1));
-        ESL_TRY(P->lsc_ne.alloc(1));
-        ESL_TRY(P->lsc_slots.alloc(1));
         ESL_CUDA(cudaMemsetAsync(P->ig_ptr.get(), 0, 4, s));
         ESL_CUDA(cudaMemsetAsync(P->og_ptr.get(), 0, 4, s));
-        ESL_CUDA(cudaMemsetAsync(P->lsc_off.get(), 0, 4, s));
     }
     // transient predecessors of the terminal positions
     {
@@ -2809,9 +2779,9 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
                                                        nullptr);
         }
         ESL_TRY(scan_excl(tmp, cnt.get(), P->tp_ptr.get(), (uint32_t)TS + 1, s));
-        ESL_CUDA(cudaMemcpyAsync(&tot[4], P->tp_ptr.get() + TS, 4, cudaMemcpyDeviceToHost, s));
+        ESL_CUDA(cudaMemcpyAsync(&tot[2], P->tp_ptr.get() + TS, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaStreamSynchronize(s));
-        ESL_TRY(P->tp_ent.alloc(std::max<uint32_t>(tot[4], 1)));
+        ESL_TRY(P->tp_ent.alloc(std::max<uint32_t>(tot[2], 1)));
         if (TS > 0) {
             ESL_COUNT_LAUNCH();
             k_pl_tpreds<false><<<nblk(TS), 256, 0, s>>>(TS, order, net->G.get(), slot_of.get(), nullptr,
@@ -2830,22 +2800,13 @@ int build_plan_device(esl_ctx* ctx, const esl_net* net, SweepPlan*& out) {
         gr.kind = (int)in[3];
         gr.max_scc = (int)in[4];
         gr.term = -1;
-        if (gr.kind == 1) {
-            gr.scc0 = h_tail[2 * g];
-            gr.nscc = in[6];
-            gr.max_odd = (int)in[7];
-        }
-        gr.nin = h_tail[2 * g + 1];
+        gr.nin = h_tail[g];
         gr.s0 = s0;
         gr.ns = in[6];
         s0 += gr.ns;
         P->max_rows = std::max(P->max_rows, gr.ne + gr.no);
         P->max_even = std::max(P->max_even, gr.ne);
         P->max_odd = std::max(P->max_odd, gr.no);
-        if (gr.kind == 1) {
-            P->max_even_local = std::max(P->max_even_local, gr.ne);
-            P->max_odd_local = std::max(P->max_odd_local, gr.no);
-        }
         P->groups.push_back(gr);
     }
     ESL_CUDA(cudaStreamSynchronize(s));
@@ -3176,16 +3137,13 @@ int build_whole_plan(esl_ctx* ctx, const esl_net* net, bool back, SweepPlan*& ou
     std::vector<uint32_t> ig_ptr(M + 1, 0), og_ptr(M + 1, 0), ig, tp_ptr{0}, tp;
     std::vector<uint4> desc(M);
     auto entries = [&](uint32_t v, std::vector<uint32_t>& e) {
-        uint32_t kept_flips = 0;
         for (uint32_t m = back ? F[v] : G[v]; m; m &= m - 1) {
             const uint32_t i = (uint32_t)__builtin_ctz(m), su = slot_of[v ^ (1u << i)];
             if (su == kNoSlot) continue;
             // the rate of the edge's source: the neighbour's, or (back) the row's own
             const uint32_t b = ((v >> i) & 1u) ^ (back ? 0u : 1u);
             e.push_back((su << kEntShift) | (2u * i + b));
-            kept_flips |= 1u << i;
         }
-        return kept_flips;
     };
     for (uint32_t sl = 0; sl < M; sl++) {
         const uint32_t v = rows[sl].x;
@@ -3470,15 +3428,13 @@ int dev_checksum(const void* d, size_t words, cudaStream_t s, uint64_t& h) {
 
 int plan_checksums(esl_ctx* ctx, const SweepPlan& P, uint64_t (&h)[12]) {
     cudaStream_t s = ctx->stream;
-    uint32_t ig = 0, og = 0, tp = 0, Q = 0, L = 0;
-    for (const SwGroup& g : P.groups)
-        if (g.kind == 1) Q += g.nscc;
+    uint32_t ig = 0, og = 0, tp = 0, count = 0;
+    for (const SwGroup& g : P.groups) count += g.ns;
     if (P.M) {
         ESL_CUDA(cudaMemcpyAsync(&ig, P.ig_ptr.get() + P.M, 4, cudaMemcpyDeviceToHost, s));
         ESL_CUDA(cudaMemcpyAsync(&og, P.og_ptr.get() + P.M, 4, cudaMemcpyDeviceToHost, s));
     }
     ESL_CUDA(cudaMemcpyAsync(&tp, P.tp_ptr.get() + P.TS, 4, cudaMemcpyDeviceToHost, s));
-    ESL_CUDA(cudaMemcpyAsync(&L, P.lsc_off.get() + Q, 4, cudaMemcpyDeviceToHost, s));
     ESL_CUDA(cudaStreamSynchronize(s));
     ESL_TRY(dev_checksum(P.rows.get(), (size_t)P.M * 2, s, h[0]));
     ESL_TRY(dev_checksum(P.desc.get(), (size_t)P.M * 4, s, h[1]));
@@ -3488,9 +3444,11 @@ int plan_checksums(esl_ctx* ctx, const SweepPlan& P, uint64_t (&h)[12]) {
     ESL_TRY(dev_checksum(P.og_ent.get(), og, s, h[5]));
     ESL_TRY(dev_checksum(P.tp_ptr.get(), (size_t)P.TS + 1, s, h[6]));
     ESL_TRY(dev_checksum(P.tp_ent.get(), tp, s, h[7]));
-    ESL_TRY(dev_checksum(P.lsc_off.get(), (size_t)Q + 1, s, h[8]));
-    ESL_TRY(dev_checksum(P.lsc_ne.get(), Q, s, h[9]));
-    ESL_TRY(dev_checksum(P.lsc_slots.get(), L, s, h[10]));
+    ESL_TRY(dev_checksum(P.scc.get(), (size_t)count * 4, s, h[8]));
+    uint64_t first_slices = 0;
+    ESL_TRY(dev_checksum(P.scc_sl.get(), (size_t)count * 2, s, first_slices));
+    ESL_TRY(dev_checksum(P.sl.get(), P.sl.n * 2, s, h[9]));
+    ESL_TRY(dev_checksum(P.ell.get(), P.ell.n * 4, s, h[10]));
     uint64_t g = 1469598103934665603ull;
     auto mix = [&](uint64_t x) {
         g ^= x;
@@ -3502,16 +3460,19 @@ int plan_checksums(esl_ctx* ctx, const SweepPlan& P, uint64_t (&h)[12]) {
         mix(gr.no);
         mix((uint64_t)gr.kind);
         mix((uint64_t)gr.max_scc);
-        mix(gr.kind == 1 ? gr.scc0 : 0);
-        mix(gr.kind == 1 ? gr.nscc : 0);
-        mix(gr.kind == 1 ? (uint64_t)gr.max_odd : 0);
         mix(gr.nin);
+        for (uint32_t x : {gr.s0, gr.ns, gr.sh0, gr.nsh, gr.l0, gr.nlarge, gr.most, gr.singles}) mix(x);
+        mix(gr.resident);
+        mix(gr.split);
     }
+    for (const SccShape& x : P.shapes)
+        for (uint32_t y : {x.even, x.odd, x.count}) mix(y);
+    for (const uint4& c : P.large)
+        for (uint32_t y : {c.x, c.y, c.z, c.w}) mix(y);
+    mix(first_slices);
     mix(P.max_rows);
     mix(P.max_even);
     mix(P.max_odd);
-    mix(P.max_even_local);
-    mix(P.max_odd_local);
     h[11] = g;
     return ESL_OK;
 }
@@ -3523,6 +3484,7 @@ int plan_checksums_for(esl_ctx* ctx, const esl_net* net, int host, uint64_t* out
     SweepPlan* P = nullptr;
     ESL_TRY(host ? build_plan_host(ctx, net, P) : build_plan_device(ctx, net, P));
     std::unique_ptr<SweepPlan> keep(P);
+    if (!host) ESL_TRY(finish_scc_list(ctx, P, nullptr));
     uint64_t h[12];
     ESL_TRY(plan_checksums(ctx, *P, h));
     for (int i = 0; i < cap && i < 12; i++) out[i] = h[i];

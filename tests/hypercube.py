@@ -24,9 +24,12 @@ def random_part(rng, d, even, odd):
     inside = np.zeros(N, bool)
     for _ in range(500):
         for p in (0, 1):
-            have = int((inside & (par == p)).sum())
-            free = np.flatnonzero(~inside & (par == p))
-            inside[rng.choice(free, want[p] - have, replace=False)] = True
+            need = want[p] - int((inside & (par == p)).sum())
+            free = ~inside & (par == p)
+            near = free & np.any([inside[np.arange(N) ^ (1 << i)] for i in range(d)], axis=0)
+            if need <= near.sum():  # next to what there is, once there is enough of it
+                free = near
+            inside[rng.choice(np.flatnonzero(free), need, replace=False)] = True
         v = np.flatnonzero(inside)
         src, dst = [], []
         for i in range(d):

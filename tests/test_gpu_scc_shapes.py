@@ -84,3 +84,25 @@ def test_many_tiny_sccs_take_little_memory(esl):
     torch.cuda.synchronize()
     esl.lib().esl_trim_cache()
     assert before - torch.cuda.mem_get_info()[0] < 700 << n
+
+
+def mixed_sizes(rng):
+    """n = 17: SCCs beyond a cluster, of three CTAs, of one, of one row per thread, and of the
+    sizes around the narrow ones, all in one level group."""
+    parts = [H.random_part(rng, 16, 16500, 16390)]
+    for k, (even, odd) in enumerate([(5000, 4990), (4097, 900), (4096, 4000), (600, 513)]):
+        parts.append(H.random_part(rng, 13 if even <= 4096 else 14, even, odd) | (4 + k) << 14)
+    small = [(512, 500), (33, 32), (32, 20), (9, 7), (8, 8), (8, 3), (1, 1), (1, 2), (17, 16)]
+    for k, (even, odd) in enumerate(small):
+        # in the other half of the last region
+        at = 7 << 14 | 1 << 13 | (0 if k == 0 else (7 + k) << 7)
+        parts.append(H.random_part(rng, 10 if k == 0 else 7, even, odd) | at)
+    return parts
+
+
+@pytest.mark.parametrize("which", ["tiny", "mixed"])
+def test_device_plan_equals_host_plan(esl, which):
+    F = tiny_sccs(12) if which == "tiny" else H.masks(np.random.default_rng(7), 17, mixed_sizes(np.random.default_rng(6)))
+    ctx = esl.Context(0)
+    net = esl.Net.from_csc(ctx, int(np.log2(F.size)), *(torch.as_tensor(a, device="cuda") for a in H.csc(F)))
+    assert np.array_equal(net.plan_checksums(host_builder=False), net.plan_checksums(host_builder=True))
