@@ -46,27 +46,31 @@ def random_part(rng, d, even, odd):
     raise ValueError("no connected part found")
 
 
-def masks(rng, n, parts, exits=0.2):
+def masks(rng, n, parts, exits=0.2, singles=False):
     """Flip masks of a graph in which each part (an array of states) is an SCC of its own, with
-    edges to states outside all parts from about `exits` of its states."""
+    edges to states outside all parts from about `exits` of its states.  singles: odd states
+    outside the parts flow into even ones, which keep no edges, and so do the parts, from their
+    odd states: all of them are one level group."""
     N = 1 << n
     part_of = np.full(N, -1, np.int64)
     for j, p in enumerate(parts):
         part_of[p] = j
     F = np.zeros(N, np.uint32)
     for j, p in enumerate(parts):
+        may = parity(p) == 1 if singles else np.ones(len(p), bool)
         out = np.zeros(len(p), bool)
         for i in range(n):
             t = part_of[p ^ (1 << i)]
-            leave = (t < 0) & (rng.random(len(p)) < exits / n * 4)
+            leave = may & (t < 0) & (rng.random(len(p)) < exits / n * 4)
             out |= leave
             F[p[(t == j) | leave]] |= np.uint32(1 << i)
         if not out.any():  # one exit at least
-            for s in p:
-                i = next((i for i in range(n) if part_of[s ^ (1 << i)] < 0), None)
-                if i is not None:
-                    F[s] |= np.uint32(1 << i)
-                    break
+            s, i = next((s, i) for s in p[may] for i in range(n) if part_of[s ^ (1 << i)] < 0)
+            F[s] |= np.uint32(1 << i)
+    if singles:
+        v = np.flatnonzero((part_of < 0) & (parity(np.arange(N)) == 1))
+        for i in range(n):
+            F[v[(part_of[v ^ (1 << i)] < 0) & (rng.random(len(v)) < 0.3)]] |= np.uint32(1 << i)
     return F
 
 
