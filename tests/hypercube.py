@@ -111,3 +111,12 @@ def check(F, rates, x0, z, x_inf, tol=1e-9):
     want = np.where(transient, 0.0, x0 + inflow)
     assert np.abs(x_inf - want).sum() <= tol, np.abs(x_inf - want).sum()
     assert abs(x_inf.sum() - x0.sum()) <= tol
+
+
+def check_stationary(F, rates, part, x_inf, tol=1e-9):
+    """x_inf of one system is the stationary distribution of a part without exits: the relative
+    L1 residual of the balance equations is within tol, and nothing is left outside."""
+    q, inflow = flows(F, rates, x_inf)
+    assert np.abs(q * x_inf - inflow).sum() <= tol * (q * x_inf).sum()
+    assert abs(x_inf[part].sum() - 1.0) <= tol and abs(x_inf.sum() - 1.0) <= tol
+    assert x_inf.min() >= -tol

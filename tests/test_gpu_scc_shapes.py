@@ -53,6 +53,48 @@ def test_two_sccs_whose_footprints_grow(esl):
     solve_and_check(esl, H.masks(rng, 14, parts), [4160, 4200], 148, 2)
 
 
+# (even, odd) rows and systems: both sides of one row per thread (512), unequal parities, a CTA;
+# clusters of two to four CTAs (from 8 systems) whose last CTA has few rows, a partial slice of
+# 32, or none of one parity, and their cooperative grid (fewer systems); beyond a cluster
+SHAPES = [(512, 512, 3), (511, 512, 33), (513, 200, 5), (513, 513, 1), (4096, 900, 2), (900, 4096, 150), (4096, 4095, 1),
+          (4097, 900, 8), (4097, 4096, 3), (5000, 8192, 9), (8300, 8200, 8), (9000, 4000, 9), (4000, 9000, 34),
+          (12289, 12300, 8), (16384, 13000, 10), (16385, 16000, 17)]
+
+
+def cube_of(even, odd):
+    """A cube with room for the part: one more dimension where one parity has few rows."""
+    return int(np.ceil(np.log2(2 * max(even, odd)))) + (3 * min(even, odd) < 2 * max(even, odd))
+
+
+@pytest.mark.parametrize("even,odd,B", SHAPES)
+def test_transient_shapes(esl, even, odd, B):
+    rng = np.random.default_rng(even + odd)
+    d = cube_of(even, odd)
+    solve_and_check(esl, H.masks(rng, d + 1, [H.random_part(rng, d, even, odd)]), [even + odd], B, odd)
+
+
+@pytest.mark.parametrize("even,odd,B", SHAPES)
+def test_terminal_shapes(esl, even, odd, B):
+    """The same parts without exits: the deflated solves."""
+    rng = np.random.default_rng(even + odd)
+    d = cube_of(even, odd)
+    part = H.random_part(rng, d, even, odd)
+    v = np.arange(1 << d)
+    inside = np.isin(v, part)
+    F = np.zeros(1 << d, np.uint32)
+    for i in range(d):
+        F[inside & inside[v ^ (1 << i)]] |= np.uint32(1 << i)
+    rates = synth.log_uniform_rates(rng, d, B)
+    x0 = np.where(inside, 1.0 / len(part), 0.0)
+    ctx = esl.Context(0, torch.cuda.Stream())
+    net = esl.Net.from_csc(ctx, d, *(torch.as_tensor(a, device="cuda") for a in H.csc(F)))
+    assert np.diff(net.export()[1].cpu().numpy()).max() == even + odd
+    torch.cuda.synchronize()
+    res = esl.solve_batch(ctx, net, rates, x0[None], method=esl.METHOD_DIRECT)
+    for b in np.unique([0, B // 2, B - 1]):
+        H.check_stationary(F, rates[b], part, res.x_inf[b, 0].cpu().numpy())
+
+
 def tiny_sccs(n):
     """One free node (bit 0) beside nodes that only decay: 2^(n-1) - 1 SCCs of two states, and
     two terminal states without edges."""
