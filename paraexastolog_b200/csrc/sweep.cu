@@ -3618,80 +3618,13 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
     };
     uint32_t largest = 0;  // states of the largest SCC
     for (const SccShape& x : P->shapes) largest = std::max(largest, x.even + x.odd);
-    bool first_launch = true;
-    for (const SwGroup& g : P->groups) {
-        // debug timing: wall time of the group with the stream drained on both sides
-        std::chrono::steady_clock::time_point g_t0;
-        if (debug_on()) {
-            ESL_CUDA(cudaStreamSynchronize(s));
-            g_t0 = std::chrono::steady_clock::now();
-        }
-        auto g_ms = [&]() {
-            return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - g_t0).count();
-        };
-        a.beg = g.beg;
-        a.ob = g.beg + g.ne;
-        a.Qo = a.IQe = nullptr;
-        a.ne = g.ne;
-        a.no = g.no;
-        a.flags = nullptr;
-        a.KT = KT64;
-        const uint32_t rows = g.ne + g.no;
-        a.gam = nullptr;
-        a.inv_s = 1.0 / (double)std::max<uint32_t>(rows, 1);
-        // singleton SCCs only: a row kernel, or the singleton CTAs of k_sw_scc, whose lanes
-        // hold rows when there are fewer than 32 systems
-        if (g.kind == 0 && K >= 32) {
-            ESL_COUNT_LAUNCH();
-            k_sw_rhs<true><<<row_grid(rows, Kp, KT64, ctx->sm_count), kSwT, sm64, s>>>(
-                a, P->og_ptr.get(), P->og_ent.get(), x0, x0_ld, Z, nullptr);
-            ESL_CUDA(cudaGetLastError());
-            continue;
-        }
-        // (kSccGrid: where the rule lies, see there)
-        const bool resident = g.resident && (!g.split || K >= kSccClusterMin);
-        if (resident || K <= 32) {
-            SccArgs ga{};
-            ESL_TRY(scc_args(g, resident, ga));
-            st.local_groups++;
-            const bool overlap = !first_launch;
-            first_launch = false;
-            if (resident) ESL_TRY(launch_scc(ctx, P, g, 0, term, overlap, ga));
-            else ESL_TRY(launch_scc_grid(ctx, g, term, ga));
-            if (debug_on()) {
-                ESL_CUDA(cudaStreamSynchronize(s));
-                fprintf(stderr, "[esl-sweep] local group beg %u even %u odd %u max_scc %d sccs %u singles %u, %.3f ms\n",
-                        g.beg, g.ne, g.no, g.max_scc, g.ns, g.singles, g_ms());
-            }
-            continue;
-        }
-        // ---- grid-wide Krylov ----
-        // The SCCs of a group share no edge: those beyond a cluster are solved one by one,
-        // each with its own coefficients and end, the others and the singletons by k_sw_scc.
-        // As one block the group's iterations served the union of the SCCs' spectra on all of
-        // its rows (316,541 rows in SCCs of 126,976, 63,488, 63,488, 30,688, 30,688 and fewer
-        // states, 512 systems: 420 -> 312 ms).
-        std::vector<SwGroup> pieces;
-        for (uint32_t j = g.l0; j < g.l0 + g.nlarge; j++) {
-            const uint4& c = P->large[j];
-            SwGroup q = g;
-            q.beg = c.x;
-            q.ne = c.y;
-            q.ob = c.z;
-            q.no = c.w;
-            // (the share of the rows, for the measurement hook)
-            q.nin = (uint64_t)((double)g.nin * (c.y + c.w) / std::max<uint32_t>(g.ne + g.no, 1));
-            pieces.push_back(q);
-        }
-        if (pieces.size() < g.ns || (!term && g.singles > 0)) {
-            SccArgs ga{};
-            const bool overlap = !first_launch;
-            first_launch = false;
-            ESL_TRY(scc_args(g, true, ga));
-            st.local_groups++;
-            ESL_TRY(launch_scc(ctx, P, g, (uint32_t)pieces.size(), term, overlap, ga));
-        }
-        for (const SwGroup& g : pieces) {
+    // debug timing: wall time of a group with the stream drained on both sides
+    std::chrono::steady_clock::time_point g_t0;
+    auto g_ms = [&]() {
+        return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - g_t0).count();
+    };
+    // Grid-wide Krylov solve of one SCC of a group by the row kernels.
+    auto solve_rows = [&](const SwGroup& g) -> int {
         const uint32_t rows = g.ne + g.no;
         a.beg = g.beg;
         a.ob = g.ob;
@@ -4174,7 +4107,77 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
                         its.front(), its[K / 2], its[(K * 9) / 10], its[(K * 99) / 100], its.back());
             }
         }
+        return ESL_OK;
+    };
+    bool first_launch = true;
+    for (const SwGroup& g : P->groups) {
+        if (debug_on()) {
+            ESL_CUDA(cudaStreamSynchronize(s));
+            g_t0 = std::chrono::steady_clock::now();
         }
+        a.beg = g.beg;
+        a.ob = g.beg + g.ne;
+        a.Qo = a.IQe = nullptr;
+        a.ne = g.ne;
+        a.no = g.no;
+        a.flags = nullptr;
+        a.KT = KT64;
+        const uint32_t rows = g.ne + g.no;
+        a.gam = nullptr;
+        a.inv_s = 1.0 / (double)std::max<uint32_t>(rows, 1);
+        // singleton SCCs only: a row kernel, or the singleton CTAs of k_sw_scc, whose lanes
+        // hold rows when there are fewer than 32 systems
+        if (g.kind == 0 && K >= 32) {
+            ESL_COUNT_LAUNCH();
+            k_sw_rhs<true><<<row_grid(rows, Kp, KT64, ctx->sm_count), kSwT, sm64, s>>>(
+                a, P->og_ptr.get(), P->og_ent.get(), x0, x0_ld, Z, nullptr);
+            ESL_CUDA(cudaGetLastError());
+            continue;
+        }
+        // (kSccGrid: where the rule lies, see there)
+        const bool resident = g.resident && (!g.split || K >= kSccClusterMin);
+        if (resident || K <= 32) {
+            SccArgs ga{};
+            ESL_TRY(scc_args(g, resident, ga));
+            st.local_groups++;
+            const bool overlap = !first_launch;
+            first_launch = false;
+            if (resident) ESL_TRY(launch_scc(ctx, P, g, 0, term, overlap, ga));
+            else ESL_TRY(launch_scc_grid(ctx, g, term, ga));
+            if (debug_on()) {
+                ESL_CUDA(cudaStreamSynchronize(s));
+                fprintf(stderr, "[esl-sweep] local group beg %u even %u odd %u max_scc %d sccs %u singles %u, %.3f ms\n",
+                        g.beg, g.ne, g.no, g.max_scc, g.ns, g.singles, g_ms());
+            }
+            continue;
+        }
+        // ---- grid-wide Krylov ----
+        // The SCCs of a group share no edge: those beyond a cluster are solved one by one,
+        // each with its own coefficients and end, the others and the singletons by k_sw_scc.
+        // As one block the group's iterations served the union of the SCCs' spectra on all of
+        // its rows (316,541 rows in SCCs of 126,976, 63,488, 63,488, 30,688, 30,688 and fewer
+        // states, 512 systems: 420 -> 312 ms).
+        std::vector<SwGroup> pieces;
+        for (uint32_t j = g.l0; j < g.l0 + g.nlarge; j++) {
+            const uint4& c = P->large[j];
+            SwGroup q = g;
+            q.beg = c.x;
+            q.ne = c.y;
+            q.ob = c.z;
+            q.no = c.w;
+            // (the share of the rows, for the measurement hook)
+            q.nin = (uint64_t)((double)g.nin * (c.y + c.w) / std::max<uint32_t>(g.ne + g.no, 1));
+            pieces.push_back(q);
+        }
+        if (pieces.size() < g.ns || (!term && g.singles > 0)) {
+            SccArgs ga{};
+            const bool overlap = !first_launch;
+            first_launch = false;
+            ESL_TRY(scc_args(g, true, ga));
+            st.local_groups++;
+            ESL_TRY(launch_scc(ctx, P, g, (uint32_t)pieces.size(), term, overlap, ga));
+        }
+        for (const SwGroup& q : pieces) ESL_TRY(solve_rows(q));
     }
     // masses into the terminal SCCs
     a.flags = nullptr;
