@@ -236,7 +236,7 @@ int esl_solve_host(esl_ctx* ctx, const esl_model* m, int B, const double* rates,
  *      accumulation) predicts the log occupation of a transient state under a rate set
  *      from: 20 node bits, the log outgoing rate sum, 16 terminal-reachability bits
  *      and 40 log rates.  Its prediction is the warm start (esl_solve_opts.d_warm) of
- *      the level sweep's grid-wide Krylov groups; the solve itself is unchanged and
+ *      the level groups with an SCC above 512 states; the solve itself is unchanged and
  *      still decides convergence.  Networks of at most 20 nodes; the handle refers to
  *      `net`, which must outlive it.  Training labels come from esl_solve_batch with
  *      esl_solve_opts.d_occupation.  Parameters: W1[128][77], b1[128], W2[128][128],
@@ -246,7 +246,7 @@ int esl_mlp_create(esl_ctx* ctx, const esl_net* net, uint64_t seed, esl_mlp** ou
 /* waits for the device, then frees; touches neither the context nor the net, so it may
  * come after either has been freed */
 int esl_mlp_free(esl_mlp* mlp);
-/* number of states it predicts (odd-parity rows of the grid-wide level groups) and the
+/* number of states it predicts (odd-parity rows of the level groups with an SCC above 512 states) and the
  * label standardisation log z = mu + sigma * y */
 int esl_mlp_info(const esl_mlp* mlp, int* n_targets, float* mu, float* sigma);
 int esl_mlp_targets(const esl_mlp* mlp, uint32_t* d_states);  /* n_targets states */

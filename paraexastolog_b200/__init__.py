@@ -407,8 +407,8 @@ MLP_PARAMS = 26625
 
 class Mlp:
     """Learned warm start of one network's transient solve (``esl_mlp_*``): a 3-layer
-    MLP (77 -> 128 -> 128 -> 1) predicting the log occupation of the states whose warm
-    start the level sweep's grid-wide Krylov groups read.  Keeps ``net`` alive."""
+    MLP (77 -> 128 -> 128 -> 1) predicting the log occupation of the odd-parity states of
+    the level groups with an SCC above 512 states.  Keeps ``net`` alive."""
 
     def __init__(self, ctx: Context, net: Net, seed: int = 0):
         self.ctx, self.net = ctx, net

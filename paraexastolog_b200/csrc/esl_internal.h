@@ -334,7 +334,8 @@ int sweep_absorption(esl_ctx* ctx, const esl_net* net, const double* rates, cons
 // ig_ptr, ig_ent, og_ptr, og_ent, tp_ptr, tp_ent, SCC list, slices, lines, group table;
 // host != 0 builds it with the host reference builder instead of the device one
 int plan_checksums_for(esl_ctx* ctx, const esl_net* net, int host, uint64_t* out, int cap);
-// states whose warm start the sweep's grid-wide Krylov groups read (their odd-parity rows)
+// the states that the learned warm start predicts: odd-parity rows of the level groups with an
+// SCC above 512 states (the sweep reads a warm start for every SCC that it solves by Krylov)
 int sweep_targets(esl_ctx* ctx, const esl_net* net, std::vector<uint32_t>& states);
 int solve_batch(esl_ctx* ctx, const esl_net* net, int B, const double* d_rates, int R, const double* d_x0,
                 double* d_x_inf, double* d_marg, double* d_R, double* d_L, const esl_solve_opts* opts,

@@ -42,10 +42,11 @@ inline unsigned blocks_for(uint64_t N) { return (unsigned)((N + kThreads - 1) / 
 // over their states between two grid barriers, and the barriers only decide termination
 // (a phase in which no state changed).  With a launch per pass and a host read of the flag
 // per few passes, launches and reads took most of the time: the n=20 network 27.4 ms (1,587
-// launches, 474 reads) against 8.4 ms here, the n=13 one 4.1 against 1.0 ms.  A pass over
+// launches, 474 reads) against 7.8 ms here, the n=13 one 4.1 against 1.0 ms.  A pass over
 // 2^20 states (17 us) is bound by the L2 traffic of the neighbour reads (whole-warp walks of
 // the union of flips and four states in flight measured the same), a pass over few states
-// by round trips to L2, a level per pass at worst (114 passes, 2.1 ms, at n=20).
+// by round trips to L2, a level per pass at worst (the n=20 network has 143 levels; the state
+// that raises a level raises its own copy in the same pass: 8.9 -> 7.8 ms).
 //
 // A CTA owns the 32-state chunks c with c % grid == its index, which spreads live states
 // evenly, and keeps the list of its live states.  Colours are pseudo-random priorities

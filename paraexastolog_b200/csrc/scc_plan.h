@@ -19,8 +19,13 @@ constexpr int kSccMaxRows = 4096;  // most odd (or even) rows of an SCC solved b
 constexpr int kSccThreads = 512, kSccThreadsBig = 1024;
 constexpr int kSccBuckets = 16;    // most (KS, team size) pairs of a launch
 constexpr size_t kSccMaxSmem = 227 * 1024;
-constexpr int kSccPairs = 256;     // (row, system) pairs of a small SCC's team at most
-constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;  // two CTAs per SM
+// (row, system) pairs of a small SCC's team at most: n=12 x 64 rate sets, one n=22 solve and
+// n=17 x 185 systems 1.22, 36.6 and 12.9 ms; 128: 1.22, 36.2, 12.8; 512: 1.26, 37.5, 12.9
+constexpr int kSccPairs = 256;
+// Shared memory of an elimination (it takes fewer systems above that: 24 KB 1.217 ms at n=12 x 64,
+// 12 KB 1.232, 48 KB 1.218), and of the teams of a CTA (two CTAs per SM; 55 and 220 KB are within
+// 1% of it in the cases above)
+constexpr size_t kSccDenseSmem = 24 * 1024, kSccTeamSmem = 110 * 1024;
 
 // SCCs of at most kSccDense odd rows are solved by elimination: a Krylov iteration is a
 // chain of FP64 reductions, about 4 us however small the SCC, an elimination step one

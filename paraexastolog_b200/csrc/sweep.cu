@@ -14,11 +14,16 @@
 //   - singleton SCCs only: z_v = b_v / q_v;
 //   - otherwise BiCGStab on the odd-parity Schur complement.  Every edge flips one bit, so
 //     the graph is bipartite by popcount parity and the even rows are eliminated exactly.
-//     The right preconditioner is the Schur diagonal.  Groups whose SCCs have at most
-//     kSccMaxRows rows of either parity run in one launch, a CTA per (SCC, few systems)
-//     with its vectors on chip and in FP64 throughout (k_sw_scc); larger groups run one
-//     grid-wide kernel per step, their inner iterations in FP64 (ESL_METHOD_DIRECT) or
-//     FP32 (ESL_METHOD_MIXED) inside FP64 iterative refinement on the true residual.
+//     The right preconditioner is the Schur diagonal.  Where an SCC is solved depends on its
+//     larger parity and the number of systems K:
+//       up to kSccMaxRows rows: one CTA per (SCC, few systems), vectors on chip (k_sw_scc);
+//       up to kSccMaxCluster times as many: a cluster per (SCC, system) for K >=
+//       kSccClusterMin, else the group is one block of a cooperative grid (kSccGrid);
+//       beyond: the cooperative grid for K <= 32; for more systems the row kernels, one
+//       launch per step, SCC by SCC, and the group's other SCCs and singletons as above.
+//     k_sw_scc is FP64 throughout; the row kernels' inner iterations are FP64
+//     (ESL_METHOD_DIRECT) or FP32 (ESL_METHOD_MIXED) inside FP64 iterative refinement on
+//     the true residual.
 //
 // Layout: every vector is [row][system], the Kp (K rounded up to 32) systems of a row
 // contiguous.  A warp handles 32 systems of one state, so every neighbour gather reads a
@@ -83,7 +88,8 @@ enum IScal { I_FLAGS, I_ITERS, I_NOIMP, I_TOTAL, I_STALL, I_NISCAL };
 struct SwGroup {
     uint32_t beg, ne, no;  // first slot, even rows, odd rows
     uint32_t ob;           // first odd slot (beg + ne, except in a piece of a group)
-    int kind;              // 0 singletons, 1 SCCs of at most kSwLocalMax states, 2 larger ones
+    int kind;              // 0 singletons, 1 SCCs of at most kSwLocalMax states, 2 larger ones (their
+                           // odd rows are the learned warm start's targets)
     int max_scc;
     uint64_t nin;          // in-group predecessor entries of the group's rows
     uint32_t s0, ns;       // the group's SCCs of >= 2 states: range in SweepPlan::scc
@@ -1272,8 +1278,8 @@ __global__ void __launch_bounds__(kSwT) k_sw_warm_scale(SwArgs a, const double* 
 }
 
 // ---- SCC-resident refinement --------------------------------------------------------------
-// One CTA solves one SCC for KS systems (a power of two chosen per SCC) from right-hand
-// side to result: the two vectors the operator gathers (the search direction and its
+// One CTA (a team of its warps, a cluster or a cooperative grid: see the modes below) solves
+// one SCC for KS systems (a power of two chosen per SCC) from right-hand side to result: the two vectors the operator gathers (the search direction and its
 // even-row elimination) stay in shared memory, a thread's own rows in registers, and the
 // CTA stops with its own systems.  A Krylov iteration is bounded by its chain of FP64
 // reductions, barriers and shared-memory gathers (3.9 us at 256 rows, 27 us at 4,096)
@@ -3258,7 +3264,11 @@ dim3 row_grid(uint32_t rows, int Kp, int KT, int sm_count, int S = 1) {
 
 // Launches k_sw_scc over group g without its first `skip` SCCs: its SCCs of more than kSccThreads rows, then the others
 // with its singleton rows (see plan_scc_launch).
-constexpr int kSccClusterMin = 8;  // fewer systems: kSccGrid uses more of the chip
+// Fewer systems: kSccGrid, which uses more of the chip for one SCC but solves the group's SCCs as
+// one block.  A lone SCC of 16,384 (two CTAs) and 32,768 states (four), in ms, grid and clusters:
+// 4 systems 1.26 / 1.65 and 1.36 / 1.77, 8: 1.30 / 1.65 and 1.43 / 1.78, 10: 1.50 / 1.68 and
+// 2.15 / 1.82, 32: 2.42 / 1.86 and 3.25 / 1.90.
+constexpr int kSccClusterMin = 8;
 constexpr size_t kSccDynSmem = kSccMaxSmem - 256;  // beside the static arrays of kSccCluster and kSccGrid
 // overlap: the launch may start, up to its first read of the sweep's vectors, before the
 // previous one ends (not for the sweep's first: the rates are being written).
@@ -3700,8 +3710,9 @@ int sweep_run(esl_ctx* ctx, const esl_net* net, SweepPlan* P, bool term, int K, 
         const double* warm = term ? nullptr : o.d_warm;
         k_sw_init<<<go, kSwT, 0, s>>>(a, warm, (size_t)net->N, bS, dS64, X64);
         ESL_CUDA(cudaGetLastError());
-        // An NVTX range names the grid solve of the largest level group, so that a
-        // profiler can select that group's launches (`ncu --nvtx --nvtx-include
+        // An NVTX range names the row-kernel solve of the network's largest transient SCC (of
+        // each, where several are that large; of none, where k_sw_scc solves it), so that a
+        // profiler can select its launches (`ncu --nvtx --nvtx-include
         // "esl_largest_level_group/"`); without a profiler attached it costs nothing.
         struct NvtxRange {
             bool on;
@@ -4254,8 +4265,8 @@ int sweep_forward(esl_ctx* ctx, const esl_net* net, int K, int nrhs, const doubl
 }
 
 // The whole-system form is solved as one resident block while CTA-sized (8,192 transient
-// states of a network of at most 13 nodes): its Krylov launches, seven per iteration over
-// vectors of one state each, took 1.2 ms where the block takes 0.3 (n=11, one system).
+// states of a network of at most 13 nodes): its Krylov solve, seven launches per iteration
+// however few the states, took 1.2 ms where the block takes 0.3 (n=11, one system).
 bool whole_supported(const esl_net* net) {
     return net->n <= 13 && net->N - net->term_states >= 4 && (int64_t)net->term_states < net->N;
 }
