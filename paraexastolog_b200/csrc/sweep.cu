@@ -1328,35 +1328,34 @@ struct SccArgs {
     int TS;
 };
 
-// Barrier of a cooperative launch.  A wait is bounded: past the bound it sets the failure
-// flag, which ends the other CTAs' waits too.  A CTA whose wait ended that way is `dead`, all
-// of its threads alike: it takes no part in later barriers and sums and leaves its loops, so
-// that the CTAs that still run read nothing that it wrote afterwards into their decisions.
-struct GridBarrier {
-    unsigned* bar;
-    unsigned target, polls;
-    bool dead;
-    __device__ __forceinline__ void wait() {
-        __shared__ bool s_dead;
-        __syncthreads();
-        if (dead) return;
-        target += gridDim.x;
-        if (threadIdx.x == 0) {
-            bool gone = false;
-            __threadfence();
-            atomicAdd(bar, 1u);
-            unsigned n = 0;
-            while (!gone && (int)(*(volatile unsigned*)bar - target) < 0) {
-                if (*(volatile unsigned*)(bar + 1)) gone = true;
-                else if (++n > polls) atomicExch(bar + 1, 1u);
+// Barrier of a cooperative launch (target: the arrivals it waits for).  A wait is bounded: past
+// the bound it sets the failure flag, which ends the other CTAs' waits too.  A CTA whose wait
+// ended that way is gone: it takes no part in later barriers and sums and leaves its loops, so
+// that the CTAs that still run read nothing that it wrote afterwards into their decisions.  Its
+// threads learn of it through a flag that changes only between the two __syncthreads of a
+// wait: read outside of them it is the same for all.
+__device__ __forceinline__ volatile int& grid_gone() {
+    __shared__ int s_gone;
+    return *const_cast<volatile int*>(&s_gone);
+}
+__device__ __forceinline__ void grid_wait(const SccArgs& g, unsigned& target) {
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0 && !grid_gone()) {
+        __threadfence();
+        atomicAdd(g.bar, 1u);
+        unsigned n = 0;
+        while ((int)(*(volatile unsigned*)g.bar - target) < 0) {
+            if (*(volatile unsigned*)(g.bar + 1)) {
+                grid_gone() = 1;
+                break;
             }
-            __threadfence();
-            s_dead = gone;
+            if (++n > g.polls) atomicExch(g.bar + 1, 1u);
         }
-        __syncthreads();
-        dead = s_dead;
+        __threadfence();
     }
-};
+    __syncthreads();
+}
 
 // a team's barrier: `threads` of the CTA, named by the team
 struct SccTeam {
@@ -1727,9 +1726,15 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     constexpr auto odd_rows = std::false_type{};
     // barrier of all threads of the item, and sums over them (see scc_sum); a grid's CTAs
     // add up their sums in one order, so that they take the same decisions
-    GridBarrier gb = {g.bar, g.missing, g.polls, false};
+    unsigned target = g.missing;
+    auto gone = [&]() {
+        if constexpr (GRID) return grid_gone() != 0;
+        else return false;
+    };
+    if constexpr (GRID)
+        if (threadIdx.x == 0) grid_gone() = 0;
     auto sync = [&]() {
-        if constexpr (GRID) gb.wait();
+        if constexpr (GRID) grid_wait(g, target);
         else if constexpr (CLUSTER) cluster_sync();
         else scc_sync(team);
     };
@@ -1753,12 +1758,11 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
             }
         }
         if constexpr (GRID) {
-            if (gb.dead) return;
             double* part = g.part + (size_t)(sums++ & 1u) * ((size_t)gridDim.x * 3 << lks);
-            if (team.tid < KS)
+            if (team.tid < KS && !gone())  // (a return here instead spills 50 bytes a thread)
 #pragma unroll
                 for (int j = 0; j < NV; j++) __stcg(part + ((size_t)(blockIdx.x * 3 + j) << lks) + s, v[j]);
-            gb.wait();
+            grid_wait(g, target);
 #pragma unroll
             for (int j = 0; j < NV; j++) v[j] = 0.0;
             for (int c = team.tid >> lks; c < (int)gridDim.x; c += nact >> lks)
@@ -1950,7 +1954,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
     double prev = 0.0, rr = b2;
     int noimp = 0, its = 0;
     int outer = 0;  // refinement steps taken
-    for (; !gb.dead; outer++) {
+    for (;; outer++) {
         if (outer > 0 || warm || dense) {
             // true residual r = b - S x
             load_x();
@@ -2008,7 +2012,7 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
         sync();
         double rho = 1.0, best = 1.0;
         int it = 0, stall = 0;
-        while (!gb.dead && __any_sync(0xffffffffu, run)) {
+        while (!gone() && __any_sync(0xffffffffu, run)) {
             elim();
             double v1[1] = {0.0};
             apply([&](int idx, double y) {
@@ -2056,10 +2060,11 @@ __global__ void __launch_bounds__(MODE == kSccSmall ? kSccThreads : kSccThreadsB
                 rho = v2[1];
             }
         }
+        if (gone()) break;
         its += it;
         if (started) each(so, [&](int r, int idx) { g.Z[(size_t)(od0 + r) * Kp + k] += nrm * D.get(idx); });
     }
-    if (gb.dead) return;  // the call fails
+    if (gone()) return;  // the call fails
     // even rows from the odd solution
     load_x();
     double total[1] = {0.0};
