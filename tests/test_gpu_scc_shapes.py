@@ -144,7 +144,8 @@ def mixed_sizes(rng):
 
 @pytest.mark.parametrize("which", ["tiny", "mixed"])
 def test_device_plan_equals_host_plan(esl, which):
-    F = tiny_sccs(12) if which == "tiny" else H.masks(np.random.default_rng(7), 17, mixed_sizes(np.random.default_rng(6)))
+    """8,191 SCCs of two states, whose list is sorted on the device, and every other kind."""
+    F = tiny_sccs(14) if which == "tiny" else H.masks(np.random.default_rng(7), 17, mixed_sizes(np.random.default_rng(6)))
     ctx = esl.Context(0)
     net = esl.Net.from_csc(ctx, int(np.log2(F.size)), *(torch.as_tensor(a, device="cuda") for a in H.csc(F)))
     assert np.array_equal(net.plan_checksums(host_builder=False), net.plan_checksums(host_builder=True))
